@@ -344,19 +344,21 @@ namespace lla {
 // Factor the column-major n x n W in place.  On a FAST failure or a
 // near-singular FAST factorisation, W is re-imported from (R, drs, dcs) and
 // factored in EXACT order, whose verdict stands.  *fail receives the failing
-// row or -1.
+// row or -1; *timed_out says that a bounded device wait gave up.
 template <typename T>
 cudaError_t factor_on_device(Ctx &c, T *W, int64_t n, int64_t ld, bool exact, const T *R,
-                             int64_t drs, int64_t dcs, int64_t *fail) {
+                             int64_t drs, int64_t dcs, int64_t *fail, int *timed_out) {
+    *timed_out = 0;
     cudaError_t e;
     Words w;
     if ((e = reset_words(c)) != cudaSuccess) return e;
     if (!exact) {
         if ((e = c.aux_d.ensure(sizeof(T) * n)) != cudaSuccess) return e;
         e = launch_status(potrf_fast_launch<T>(W, n, ld, &dev_words(c)->info, (T *)c.aux_d.p,
-                                               &dev_words(c)->min_ratio, c.stream));
+                                               &dev_words(c)->min_ratio, &dev_words(c)->err_word, nullptr, c.stream));
         if (e != cudaSuccess) return e;
         if ((e = read_words(c, w)) != cudaSuccess) return e;
+        if ((*timed_out = (w.err_word == LLA_ERR_TIMEOUT))) return cudaSuccess;
         if (w.info < 0 && !(w.min_ratio < kPivotGuard)) {
             *fail = -1;
             return cudaSuccess;
@@ -392,9 +394,9 @@ cudaError_t trsm_on_device(Ctx &c, const T *M, int64_t ld, int64_t n, int lower,
 }
 
 template cudaError_t factor_on_device<double>(Ctx &, double *, int64_t, int64_t, bool,
-                                              const double *, int64_t, int64_t, int64_t *);
+                                              const double *, int64_t, int64_t, int64_t *, int *);
 template cudaError_t factor_on_device<float>(Ctx &, float *, int64_t, int64_t, bool, const float *,
-                                             int64_t, int64_t, int64_t *);
+                                             int64_t, int64_t, int64_t *, int *);
 template cudaError_t trsm_on_device<double>(Ctx &, const double *, int64_t, int64_t, int, int,
                                             const double *, double *, int64_t, int64_t, bool, int *);
 template cudaError_t trsm_on_device<float>(Ctx &, const float *, int64_t, int64_t, int, int,
@@ -435,7 +437,9 @@ int cholesky_impl(T *a, int64_t rows, int64_t cols, int64_t rs, int64_t cs, int 
     const T *R = (const T *)c->raw_a.p;
     LLA_TRY_CUDA(launch_status(import_launch<T>(R, drs, dcs, n, n, W, n, c->stream)));
     int64_t fail = -1;
-    LLA_TRY_CUDA(factor_on_device<T>(*c, W, n, n, use_exact(n), R, drs, dcs, &fail));
+    int to = 0;
+    LLA_TRY_CUDA(factor_on_device<T>(*c, W, n, n, use_exact(n), R, drs, dcs, &fail, &to));
+    if (to) return lla__set_status(err, LLA_ERR_TIMEOUT);
     const int mode = fail >= 0 ? EXPORT_FAIL : (dirty ? EXPORT_LOWER : EXPORT_LOWER_ZERO_UPPER);
     LLA_TRY_CUDA(launch_status(export_launch<T>(W, n, (T *)c->raw_a.p, drs, dcs, n, n, mode, fail,
                                                 c->stream)));
@@ -456,7 +460,9 @@ int factor_then(Ctx *c, T *a, int64_t n, int64_t rs, int64_t cs, bool &failed, l
     const T *R = (const T *)c->raw_a.p;
     LLA_TRY_CUDA(launch_status(import_launch<T>(R, drs, dcs, n, n, W, n, c->stream)));
     int64_t fail = -1;
-    LLA_TRY_CUDA(factor_on_device<T>(*c, W, n, n, use_exact(n), R, drs, dcs, &fail));
+    int to = 0;
+    LLA_TRY_CUDA(factor_on_device<T>(*c, W, n, n, use_exact(n), R, drs, dcs, &fail, &to));
+    if (to) return lla__set_status(err, LLA_ERR_TIMEOUT);
     const int mode = fail >= 0 ? EXPORT_FAIL : EXPORT_LOWER;  // self keeps the dirty factor (:140)
     LLA_TRY_CUDA(launch_status(export_launch<T>(W, n, (T *)c->raw_a.p, drs, dcs, n, n, mode, fail,
                                                 c->stream)));
@@ -696,7 +702,9 @@ int orthonormalize_impl(const T *v, int64_t rows, int64_t cols, int64_t rs, int6
     LLA_TRY_CUDA(launch_status(atb_launch<T>(WV, n, WV, n, n, k, k, G, k, (T *)c->lob_p.p, 1, c->stream)));
     LLA_TRY_CUDA(cudaMemcpyAsync(Gc, G, sizeof(T) * k * k, cudaMemcpyDeviceToDevice, c->stream));
     int64_t fail = -1;
-    LLA_TRY_CUDA(factor_on_device<T>(*c, G, k, k, use_exact(k), Gc, 1, k, &fail));
+    int to = 0;
+    LLA_TRY_CUDA(factor_on_device<T>(*c, G, k, k, use_exact(k), Gc, 1, k, &fail, &to));
+    if (to) return lla__set_status(err, LLA_ERR_TIMEOUT);
     if (fail >= 0) return not_pd(err, fail);
     // L: lower factor, upper part zeroed (cholesky_into)
     View vl{(char *)l, k, k, lrs, lcs, sizeof(T)};
@@ -707,7 +715,6 @@ int orthonormalize_impl(const T *v, int64_t rows, int64_t cols, int64_t rs, int6
     if (n > 0) {
         // V^T (k x n), L Z = V^T, U = Z^T
         LLA_TRY_CUDA(launch_status(import_launch<T>(WV, n, 1, k, n, VT, k, c->stream)));
-        int to = 0;
         LLA_TRY_CUDA(trsm_on_device<T>(*c, G, k, k, /*lower=*/1, /*trans=*/0, nullptr, VT, k, n, use_exact(k), &to));
         if (to) return lla__set_status(err, LLA_ERR_TIMEOUT);
         LLA_TRY_CUDA(launch_status(import_launch<T>(VT, k, 1, n, k, WV, n, c->stream)));
@@ -815,6 +822,19 @@ int lla_dposv_refined(const double *a, int64_t rows, int64_t cols, int64_t rs, i
 
 // ---- device-resident entry points -----------------------------------------
 
+// The calling thread's device-call status word (allocated and zeroed once;
+// the asynchronous device entry points record a timed-out wait there).
+static cudaError_t device_status_word(Ctx &c, cudaStream_t st, int **out) {
+    cudaError_t e = c.status_dev.ensure(sizeof(int));
+    if (e != cudaSuccess) return e;
+    if (!c.status_clear) {
+        if ((e = cudaMemsetAsync(c.status_dev.p, 0, sizeof(int), st)) != cudaSuccess) return e;
+        c.status_clear = true;
+    }
+    *out = (int *)c.status_dev.p;
+    return cudaSuccess;
+}
+
 template <typename T>
 static int potrf_device_impl(T *dA, int64_t n, int64_t ld, int algo, int64_t *d_info, void *stream,
                              lla_error *err) {
@@ -834,23 +854,12 @@ static int potrf_device_impl(T *dA, int64_t n, int64_t ld, int algo, int64_t *d_
             potrf_exact_launch<T>(dA, (T *)c->dev_s.p, (T *)c->dev_d.p, n, ld, d_info, st)));
     } else {
         LLA_TRY_CUDA(c->dev_d.ensure(sizeof(T) * n));
+        int *sticky = nullptr;
+        LLA_TRY_CUDA(device_status_word(*c, st, &sticky));
         LLA_TRY_CUDA(launch_status(
-            potrf_fast_launch<T>(dA, n, ld, d_info, (T *)c->dev_d.p, nullptr, st)));
+            potrf_fast_launch<T>(dA, n, ld, d_info, (T *)c->dev_d.p, nullptr, nullptr, sticky, st)));
     }
     return LLA_OK;
-}
-
-// The calling thread's device-call status word (allocated and zeroed once;
-// the asynchronous device entry points record a timed-out wait there).
-static cudaError_t device_status_word(Ctx &c, cudaStream_t st, int **out) {
-    cudaError_t e = c.status_dev.ensure(sizeof(int));
-    if (e != cudaSuccess) return e;
-    if (!c.status_clear) {
-        if ((e = cudaMemsetAsync(c.status_dev.p, 0, sizeof(int), st)) != cudaSuccess) return e;
-        c.status_clear = true;
-    }
-    *out = (int *)c.status_dev.p;
-    return cudaSuccess;
 }
 
 template <typename T>

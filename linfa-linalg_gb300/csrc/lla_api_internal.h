@@ -70,7 +70,7 @@ Ctx *get_ctx(lla_error *err);
 
 template <typename T>
 cudaError_t factor_on_device(Ctx &c, T *W, int64_t n, int64_t ld, bool exact, const T *R,
-                             int64_t drs, int64_t dcs, int64_t *fail);
+                             int64_t drs, int64_t dcs, int64_t *fail, int *timed_out);
 template <typename T>
 cudaError_t trsm_on_device(Ctx &c, const T *M, int64_t ld, int64_t n, int lower, int trans,
                            const T *diag, T *B, int64_t ldb, int64_t m, bool exact, int *timed_out);

@@ -16,10 +16,15 @@ namespace lla {
 template <typename T>
 int potrf_exact_launch(T *W, T *S, T *D, int64_t n, int64_t ld, int64_t *d_info, cudaStream_t st);
 // FAST needs diag0 (n) scratch and min_ratio (device double, preset to a
-// large value) for the near-singular guard.
+// large value) for the near-singular guard.  err_word (optional, device int, 0
+// on entry) and sticky (optional, never cleared by the launch) receive
+// LLA_ERR_TIMEOUT when a bounded wait gave up.
 template <typename T>
 int potrf_fast_launch(T *W, int64_t n, int64_t ld, int64_t *d_info, T *diag0, double *min_ratio,
-                      cudaStream_t st);
+                      int *err_word, int *sticky, cudaStream_t st);
+// Its FP64 form (lla_fp64_chol.cu).
+int potrf_fast64_launch(double *W, int64_t n, int64_t ld, int64_t *d_info, double *diag0, double *min_ratio,
+                        int *err_word, int *sticky, cudaStream_t st);
 
 // Triangular solve op(T) X = B in place (see lla_trsm.cu).  ws: trsm_ws_ints
 // ints of scratch; err_word: device int, 0 on entry; sticky (optional): a

@@ -517,7 +517,7 @@ __global__ void __launch_bounds__(256, 2) lowp_panel_kernel(float *L, int64_t ld
 int lowp_factor_launch(float *L, int64_t n, int64_t ld, const lla_refine_opts &opts, int64_t *info,
                        float *diag0, double *min_ratio, Ctx *c, cudaStream_t st) {
     const int upd = opts.update;
-    if (upd == LLA_UPDATE_FP32) return potrf_fast_launch<float>(L, n, ld, info, diag0, min_ratio, st);
+    if (upd == LLA_UPDATE_FP32) return potrf_fast_launch<float>(L, n, ld, info, diag0, min_ratio, nullptr, nullptr, st);
     const bool fp16 = (upd == LLA_UPDATE_FP16 || upd == LLA_UPDATE_FP16X3);
     const int terms = (upd == LLA_UPDATE_BF16 || upd == LLA_UPDATE_FP16) ? 1
                       : (upd == LLA_UPDATE_BF16X6)                        ? 3

@@ -830,8 +830,13 @@ extern "C" int lla_dposv_refined_device(const double *dA, int64_t n, int64_t lda
         int64_t minus1 = -1;
         MX_TRY(cudaMemcpyAsync(info, &minus1, sizeof(int64_t), cudaMemcpyHostToDevice, st));
         MX_TRY(cudaMemcpyAsync(min_ratio, &big, sizeof(double), cudaMemcpyHostToDevice, st));
-        MX_TRY(last_err(potrf_fast_launch<double>(F, n, n, info, (double *)w.fdiag.p, min_ratio, st)));
+        MX_TRY(last_err(potrf_fast_launch<double>(F, n, n, info, (double *)w.fdiag.p, min_ratio, err_word, nullptr, st)));
         MX_TRY(read_words(4));
+        if (((int *)(hw + 3))[1] != 0) {  // a bounded wait of the factorisation gave up
+            r.ms_fallback = ms_since(t0);
+            if (rep) *rep = r;
+            return lla__set_status(err, LLA_ERR_TIMEOUT);
+        }
         int64_t finfo;
         std::memcpy(&finfo, hw + 2, sizeof(int64_t));
         if (finfo >= 0 || !(hw[1] >= kFallbackPivotGuard)) {

@@ -103,4 +103,83 @@ __host__ __device__ __forceinline__ void oz_digits_packed4(const int64_t (&b)[4]
     }
 }
 
+// ---- balanced 8-bit digits (the FP64 trailing update, lla_fp64_chol.cu) ----
+//
+// An integer of up to 9 bits magnitude 2^7 is exact in BF16, so signed digits
+// in [-128, 128] carry 8 bits each: seven of them hold a value rounded to the
+// nearest multiple of 2^(e-55), where the truncated 7-bit digits above need
+// eight for 56 bits.
+constexpr int kOzBal = 7;
+
+// a rounded to the nearest multiple of 2^(e-55) (|a| < 2^e), as that integer
+// (|V| <= 2^55); zero for inf and NaN.  Integer operations only.
+__host__ __device__ __forceinline__ int64_t oz_fixed55(int64_t bits, int e) {
+    const int eb = (int)((bits >> 52) & 0x7ff);
+    uint64_t mant = (uint64_t)bits & ((1ull << 52) - 1);
+    if (eb != 0) mant |= 1ull << 52;
+    const int shift = (eb != 0 ? eb : 1) - 1075 + 55 - e;  // <= 2 since |a| < 2^e
+    uint64_t V = 0;
+    if (eb != 0x7ff) {
+        if (shift >= 0)
+            V = mant << shift;
+        else if (shift >= -54)
+            V = (mant + (1ull << (-shift - 1))) >> (-shift);
+    }
+    return bits < 0 ? -(int64_t)V : (int64_t)V;
+}
+
+// Balanced digits p = 0..6 (most significant first, V = sum_p d_p 256^(6-p)) of
+// two values as BF16 pairs, a in the low half of each word.  Adding 128 to every
+// digit makes the digits plain bytes (the top one 0..256); a byte in the
+// mantissa of 2^23, minus 2^23 + 128, is the signed digit, exact in FP32, and
+// its upper 16 bits are its BF16.
+__host__ __device__ __forceinline__ void oz_balanced_pair(int64_t va, int64_t vb, uint32_t (&out)[kOzBal]) {
+    const uint64_t bias = 0x0080808080808080ull;
+    const uint64_t wa = (uint64_t)va + bias, wb = (uint64_t)vb + bias;
+#pragma unroll
+    for (int p = 0; p < kOzBal; ++p) {
+        const int s = 8 * (kOzBal - 1 - p);
+        const uint32_t mask = p == 0 ? 0x1ffu : 0xffu;
+        const uint32_t ma = 0x4b000000u | ((uint32_t)(wa >> s) & mask), mb = 0x4b000000u | ((uint32_t)(wb >> s) & mask);
+        float fa, fb;
+        memcpy(&fa, &ma, 4);
+        memcpy(&fb, &mb, 4);
+        fa -= 8388736.f;
+        fb -= 8388736.f;
+        uint32_t ba, bb;
+        memcpy(&ba, &fa, 4);
+        memcpy(&bb, &fb, 4);
+        out[p] = oz_pack_bf16(ba, bb);
+    }
+}
+
+// The double nearest to T 2^s, |T| < 2^63 (ties to even): integer operations
+// only for results in the normal range, the plain product otherwise.
+__host__ __device__ __forceinline__ double oz_scaled_double(int64_t T, int s) {
+    if (T == 0) return 0.0;
+    const uint64_t u = T < 0 ? 0ull - (uint64_t)T : (uint64_t)T;
+#ifdef __CUDA_ARCH__
+    const int lz = __clzll((long long)u);
+#else
+    const int lz = __builtin_clzll(u);
+#endif
+    const uint64_t v = u << lz;
+    uint64_t m = v >> 11;  // 53 bits, the leading one at bit 52
+    const uint32_t rem = (uint32_t)v & 0x7ffu;
+    m += (rem > 0x400u || (rem == 0x400u && (m & 1))) ? 1 : 0;
+    const int ex = 63 - lz + s + 1022;  // biased exponent minus one: the leading one of m adds it
+    if (ex < 0 || ex >= 0x7fd) return ldexp((double)T, s);
+    const uint64_t b = ((uint64_t)T & 0x8000000000000000ull) | (((uint64_t)ex << 52) + m);
+    double d;
+    memcpy(&d, &b, 8);
+    return d;
+}
+
+// Smallest e with |v| < 2^e for the bit pattern of a finite |v| (0 and
+// subnormals: -1022, which holds for all of them).
+__host__ __device__ __forceinline__ int oz_bits_exponent(uint64_t abs_bits) {
+    const int eb = (int)(abs_bits >> 52);
+    return eb == 0 ? -1022 : eb - 1022;
+}
+
 }  // namespace lla

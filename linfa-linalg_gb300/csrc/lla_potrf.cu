@@ -14,10 +14,7 @@
 // rounded separately, so the factor is bit-identical to the reference's.
 //
 // FAST mode is LAPACK-style right-looking (A22 -= L21 L21^T in place) with
-// fused multiply-add; the FP64 trailing update runs on the FP64 tensor pipe
-// (mma.sync m16n8k16 .f64), measured on GB300 at 1.05-1.10 TFLOP/s with
-// GEMM-like operand use, about the DFMA rate (1.02 TFLOP/s): FP64 is the
-// scarce resource on this GPU either way.
+// fused multiply-add; this file holds the FP32 form, lla_fp64_chol.cu the FP64 one.
 #include "lla_common.cuh"
 #include "lla_kernels.h"
 #include "lla_prof.h"
@@ -276,84 +273,6 @@ __global__ void __launch_bounds__(128) potrf_fast_panel(T *W, int64_t ld, int64_
         if (k < b) cm(W, ld, j, p + k) = av[k];
 }
 
-// FAST FP64 trailing update on the FP64 tensor pipe: A22 -= L21 L21^T on
-// 64 x 64 lower tiles, panel width b <= 64 (zero-padded to a multiple of 16).
-// 4 warps in 2 x 2, each a 32 x 32 sub-tile of 2 x 4 m16n8k16 MMAs.
-// Fragment layout of mma.m16n8k16.row.col.f64 (g = lane/4, t = lane%4):
-//   A (16x16): a[i] = A[g + 8*(i&1)][t + 4*(i>>1)],  i = 0..7
-//   B (16x8) : b[i] = B[t + 4*i][g],                 i = 0..3
-//   C (16x8) : c[i] = C[g + 8*(i>>1)][2*t + (i&1)],  i = 0..3
-constexpr int kDmmaStride = 68;  // 68 = 4 (mod 16): conflict-free fragment reads
-
-__global__ void __launch_bounds__(128) potrf_fast_update_dmma(double *W, int64_t ld, int64_t n,
-                                                              int64_t p, int b,
-                                                              const int64_t *info) {
-    __shared__ double lj[32][kDmmaStride];  // [k][row], one 32-wide slice of the panel
-    __shared__ double lk[32][kDmmaStride];
-    if (*(volatile const int64_t *)info >= 0) return;
-    const int64_t q = p + b;
-    int64_t I, J;
-    tri_tile(blockIdx.x, I, J);
-    const int64_t j0 = q + I * 64, k0 = q + J * 64;
-    const int tid = threadIdx.x;
-    const int bp = (b + 15) & ~15;
-    const int warp = tid / 32, lane = tid % 32;
-    const int g = lane >> 2, t = lane & 3;
-    const int wr = (warp & 1) * 32, wc = (warp >> 1) * 32;
-    double acc[2][4][4];
-#pragma unroll
-    for (int mi = 0; mi < 2; ++mi)
-#pragma unroll
-        for (int ni = 0; ni < 4; ++ni)
-#pragma unroll
-            for (int i = 0; i < 4; ++i) acc[mi][ni][i] = 0.0;
-    for (int kh = 0; kh < bp; kh += 32) {
-      const int kw = min(32, bp - kh);
-      __syncthreads();
-      for (int e = tid; e < 64 * kw; e += 128) {
-          const int r = e % 64, k = e / 64;
-          const bool kin = kh + k < b;
-          lj[k][r] = (kin && j0 + r < n) ? cm(W, ld, j0 + r, p + kh + k) : 0.0;
-          lk[k][r] = (kin && k0 + r < n) ? cm(W, ld, k0 + r, p + kh + k) : 0.0;
-      }
-      __syncthreads();
-      for (int kk = 0; kk < kw; kk += 16) {
-        double af[2][8], bf[4][4];
-#pragma unroll
-        for (int mi = 0; mi < 2; ++mi)
-#pragma unroll
-            for (int i = 0; i < 8; ++i)
-                af[mi][i] = lj[kk + t + 4 * (i >> 1)][wr + mi * 16 + g + 8 * (i & 1)];
-#pragma unroll
-        for (int ni = 0; ni < 4; ++ni)
-#pragma unroll
-            for (int i = 0; i < 4; ++i) bf[ni][i] = lk[kk + t + 4 * i][wc + ni * 8 + g];
-#pragma unroll
-        for (int mi = 0; mi < 2; ++mi)
-#pragma unroll
-            for (int ni = 0; ni < 4; ++ni)
-                asm volatile(
-                    "mma.sync.aligned.m16n8k16.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, "
-                    "{%4,%5,%6,%7,%8,%9,%10,%11}, {%12,%13,%14,%15}, {%0,%1,%2,%3};\n"
-                    : "+d"(acc[mi][ni][0]), "+d"(acc[mi][ni][1]), "+d"(acc[mi][ni][2]),
-                      "+d"(acc[mi][ni][3])
-                    : "d"(af[mi][0]), "d"(af[mi][1]), "d"(af[mi][2]), "d"(af[mi][3]),
-                      "d"(af[mi][4]), "d"(af[mi][5]), "d"(af[mi][6]), "d"(af[mi][7]),
-                      "d"(bf[ni][0]), "d"(bf[ni][1]), "d"(bf[ni][2]), "d"(bf[ni][3]));
-      }
-    }
-#pragma unroll
-    for (int mi = 0; mi < 2; ++mi)
-#pragma unroll
-        for (int ni = 0; ni < 4; ++ni)
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const int64_t j = j0 + wr + mi * 16 + g + 8 * (i >> 1);
-                const int64_t k2 = k0 + wc + ni * 8 + 2 * t + (i & 1);
-                if (j < n && k2 <= j) cm(W, ld, j, k2) -= acc[mi][ni][i];
-            }
-}
-
 // Saves the input diagonal (for the fast path's pivot-ratio guard).
 template <typename T>
 __global__ void copy_diag(const T *W, int64_t ld, int64_t n, T *out) {
@@ -396,9 +315,10 @@ int potrf_exact_launch(T *W, T *S, T *D, int64_t n, int64_t ld, int64_t *d_info,
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
-template <typename T>
-int potrf_fast_launch(T *W, int64_t n, int64_t ld, int64_t *d_info, T *diag0, double *min_ratio,
-                      cudaStream_t st) {
+template <>
+int potrf_fast_launch<float>(float *W, int64_t n, int64_t ld, int64_t *d_info, float *diag0, double *min_ratio,
+                             int *, int *, cudaStream_t st) {
+    using T = float;
     {
         LaunchScope ls(K_MISC, st);
         copy_diag<T><<<(unsigned)ceil_div(n, 256), 256, 0, st>>>(W, ld, n, diag0);
@@ -418,24 +338,21 @@ int potrf_fast_launch(T *W, int64_t n, int64_t ld, int64_t *d_info, T *diag0, do
             }
             // algorithmic work: rest*(rest+1)/2 lower entries x b multiply-adds x 2
             LaunchScope ls(K_POTRF_FAST_UPDATE, st, (double)rest * (rest + 1) * b);
-            if constexpr (sizeof(T) == 8)
-                potrf_fast_update_dmma<<<(unsigned)tri_tiles(rest, 64), 128, 0, st>>>(
-                    (double *)W, ld, n, p, b, d_info);
-            else
-                potrf_update_simt<T, false><<<(unsigned)tri_tiles(rest, kUpdTile), 256, 0, st>>>(
-                    W, nullptr, ld, n, p, b, d_info);
+            potrf_update_simt<T, false><<<(unsigned)tri_tiles(rest, kUpdTile), 256, 0, st>>>(
+                W, nullptr, ld, n, p, b, d_info);
         }
     }
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
+}
+
+template <>
+int potrf_fast_launch<double>(double *W, int64_t n, int64_t ld, int64_t *d_info, double *diag0, double *min_ratio,
+                              int *err_word, int *sticky, cudaStream_t st) {
+    return potrf_fast64_launch(W, n, ld, d_info, diag0, min_ratio, err_word, sticky, st);
 }
 
 template int potrf_exact_launch<double>(double *, double *, double *, int64_t, int64_t, int64_t *,
                                         cudaStream_t);
 template int potrf_exact_launch<float>(float *, float *, float *, int64_t, int64_t, int64_t *,
                                        cudaStream_t);
-template int potrf_fast_launch<double>(double *, int64_t, int64_t, int64_t *, double *, double *,
-                                       cudaStream_t);
-template int potrf_fast_launch<float>(float *, int64_t, int64_t, int64_t *, float *, double *,
-                                      cudaStream_t);
-
 }  // namespace lla

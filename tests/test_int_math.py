@@ -1,0 +1,104 @@
+"""Integer building blocks of the FP64 factorisations, compiled on the host from
+the kernels' own headers: reciprocal roots in fixed point (csrc/lla_int_math.h),
+and the balanced digits, fixed-point values and 64-bit-to-double conversion of
+the FP64 trailing update (csrc/lla_oz_digits.h).  The references are the
+compiler's long double and integer arithmetic."""
+import os
+import shutil
+import subprocess
+import tempfile
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+CSRC = os.path.join(ROOT, "linfa-linalg_gb300", "csrc")
+
+HARNESS = r"""
+#include <cmath>
+#include <cstdio>
+#include <cstring>
+#include <random>
+#include "lla_int_math.h"
+#include "lla_oz_digits.h"
+using namespace lla;
+static long long bad = 0;
+#define CHECK(c, ...) do { if (!(c) && bad++ < 5) std::printf(__VA_ARGS__); } while (0)
+int main() {
+    std::mt19937_64 g(7);
+    // reciprocal roots: within one unit in the last place, any positive normal argument
+    for (long t = 0; t < 2000000; ++t) {
+        uint64_t b = g() & 0x7fffffffffffffffull;
+        if (t % 5 == 0) b = (b & 0x000fffffffffffffull) | ((1021ull + g() % 5) << 52);
+        if (t % 7 == 0) b &= ~0xffffffffffull;             // few mantissa bits
+        if (t % 11 == 0) b |= 0x000ffffffffffff0ull;        // mantissa near the top
+        if (!im_positive_normal(b)) continue;
+        const double d = im_double(b), y = im_rsqrt(d);
+        const long double want = 1.0L / sqrtl((long double)d);
+        const double w = (double)want;
+        const long double ulp = (long double)w - (long double)std::nextafter(w, 0.0);
+        CHECK(fabsl((long double)y - want) <= ulp, "rsqrt(%a) = %a\n", d, y);
+    }
+    for (double d : {0.0, -0.0, -1.0, 5e-324, 2.2250738585072009e-308, HUGE_VAL, -HUGE_VAL, std::nan("")})
+        CHECK(!im_positive_normal(im_bits(d)), "normal(%a)\n", d);
+    CHECK(im_positive_normal(im_bits(2.2250738585072014e-308)) && im_positive_normal(im_bits(1.7976931348623157e308)), "ends\n");
+    // digits: V = nearest multiple of 2^(e-55), its seven balanced digits exact in BF16
+    std::uniform_real_distribution<double> U(0.5, 1.0);
+    for (long t = 0; t < 400000; ++t) {
+        const int e = (int)(g() % 1601) - 800;
+        int64_t v[2];
+        double a[2];
+        for (int u = 0; u < 2; ++u) {
+            a[u] = std::ldexp(U(g), e - (int)(g() % 62));
+            if (g() & 1) a[u] = -a[u];
+            if (t % 101 == u) a[u] = t & 1 ? 0.0 : -0.0;
+            if (t % 103 == u) a[u] = std::ldexp(std::nextafter(1.0, 0.0), e);
+            v[u] = oz_fixed55((int64_t)im_bits(a[u]), e);
+            const long double x = std::ldexp((long double)a[u], 55 - e);
+            CHECK(fabsl(x - (long double)v[u]) <= 0.5L, "fixed(%a, %d)\n", a[u], e);
+        }
+        CHECK(oz_bits_exponent(im_bits(std::fabs(a[0]))) <= e || a[0] == 0, "exponent(%a)\n", a[0]);
+        uint32_t q[kOzBal];
+        oz_balanced_pair(v[0], v[1], q);
+        for (int u = 0; u < 2; ++u) {
+            int64_t s = 0;
+            for (int p = 0; p < kOzBal; ++p) {
+                const uint32_t w = (u ? q[p] & 0xffff0000u : q[p] << 16);
+                float f;
+                std::memcpy(&f, &w, 4);
+                CHECK(std::fabs(f) <= 128.f && f == std::rint(f), "digit %g\n", f);
+                s = s * 256 + (int64_t)f;
+            }
+            CHECK(s == v[u], "digits of %lld\n", (long long)v[u]);
+        }
+    }
+    // 64-bit integer times a power of two, rounded to nearest even
+    for (long t = 0; t < 1000000; ++t) {
+        int64_t T = (int64_t)g() >> (g() % 64);
+        if (T == INT64_MIN) T = 0;
+        if (t % 3 == 0) T = (T >> 12 << 12) | 0x400;  // ties
+        const int s = (int)(g() % 1900) - 1000;
+        const double got = oz_scaled_double(T, s), want = (double)std::ldexp((long double)T, s);
+        const bool sub = std::fabs(want) < 2.3e-308;   // subnormal results round twice
+        CHECK(im_bits(got) == im_bits(want) || (T == 0 && got == 0) || (sub && std::fabs(got - want) <= 5e-324),
+              "scaled(%lld, %d) = %a, %a\n", (long long)T, s, got, want);
+    }
+    std::printf("bad %lld\n", bad);
+    return bad != 0;
+}
+"""
+
+
+@pytest.mark.parametrize("seed_error", ["0.0f", "-2.4e-7f", "2.4e-7f"])
+def test_integer_math_on_host(seed_error):
+    """`seed_error`: relative error put on the FP32 seed (the hardware's is below 2^-22)."""
+    cxx = shutil.which("g++") or shutil.which("c++")
+    if cxx is None:
+        pytest.skip("no host C++ compiler")
+    with tempfile.TemporaryDirectory() as d:
+        src, exe = os.path.join(d, "t.cpp"), os.path.join(d, "t")
+        with open(src, "w") as f:
+            f.write(HARNESS)
+        subprocess.run([cxx, "-O2", "-std=c++17", "-ffp-contract=off", f"-DIM_SEED_ERROR={seed_error}", "-I", CSRC,
+                        src, "-o", exe], check=True)
+        r = subprocess.run([exe], capture_output=True, text=True)
+        assert r.returncode == 0, r.stdout

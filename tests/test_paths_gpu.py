@@ -37,3 +37,99 @@ def test_refined_slices_of_well_conditioned_systems_converge(gpu_lla, n, m, shif
     R = B - A @ X
     be = (R.abs().amax(0) / (A.abs().sum(1).amax() * X.abs().amax(0) + B.abs().amax(0))).max()
     assert float(be) <= 1.1e-13  # the default tolerance, plus the check's own rounding
+
+
+def _potrf(gpu_lla, torch, A, ld=None):
+    """FAST device factor of A in a buffer of leading dimension ld (column-major)."""
+    n = A.shape[0]
+    ld = ld or n
+    buf = torch.full((n, ld), -7.0, dtype=A.dtype, device="cuda")
+    buf[:, :n] = A.T
+    L = buf.T[:n]
+    info = gpu_lla.potrf_device(L, algo=gpu_lla.ALGO_FAST)
+    torch.cuda.synchronize()
+    assert ld == n or bool((buf[:, n:] == -7.0).all()), "rows below the matrix were written"
+    return L, int(info.item())
+
+
+@pytest.mark.parametrize("n", [1, 2, 63, 64, 65, 127, 128, 129, 192, 193, 257, 320, 1000])
+@pytest.mark.parametrize("pad", [0, 3])
+def test_fast_fp64_factor(gpu_lla, n, pad):
+    """Digit-sliced trailing updates: edges of the 64-column panels, the 128-row
+    tiles and the pairs of panels, against ||L L^T - A|| <= 10 n eps ||A||; the
+    upper triangle stays untouched."""
+    torch = _torch()
+    A, g = _spd(torch, n, 0.5, n)
+    d = torch.exp2(20 * torch.rand(n, dtype=torch.float64, device="cuda", generator=g) - 10)
+    A = A * d[:, None] * d[None, :]
+    A = torch.tril(A) + torch.tril(A, -1).T
+    L, info = _potrf(gpu_lla, torch, A, n + pad)
+    assert info == -1
+    low = torch.tril(L)
+    S = A / d[:, None] / d[None, :]
+    R = (low @ low.T) / d[:, None] / d[None, :] - S
+    assert float(R.norm() / S.norm()) <= 10 * n * 2.2e-16
+    assert bool((torch.triu(L, 1) == torch.triu(A, 1)).all())
+
+
+@pytest.mark.parametrize("row", [0, 1, 30, 31, 32, 33, 63, 64, 65, 100, 127, 128, 200, 255, 299])
+def test_fast_fp64_factor_reports_the_failing_row(gpu_lla, row):
+    torch = _torch()
+    A, _ = _spd(torch, 300, 1.0, 3)
+    A[row, row] = -1.0
+    L, info = _potrf(gpu_lla, torch, A)
+    assert info == row
+    if row:
+        R = torch.linalg.cholesky(A[:row, :row])
+        assert float((torch.tril(L[:row, :row]) - R).norm() / R.norm()) <= 10 * 300 * 2.2e-16
+
+
+def test_fast_fp64_factor_non_finite_and_subnormal_rows(gpu_lla):
+    """A row without digits (NaN) spoils what a FMA factorisation would spoil and nothing else;
+    a subnormal pivot is a pivot."""
+    torch = _torch()
+    n, bad = 300, 170
+    A, _ = _spd(torch, n, 1.0, 5)
+    R = torch.linalg.cholesky(A)
+    A[bad, 3] = A[3, bad] = float("nan")
+    L, info = _potrf(gpu_lla, torch, A)
+    assert info == -1
+    ok = torch.ones(n, n, dtype=torch.bool, device="cuda").tril()
+    ok[bad, 3:] = False
+    ok[bad + 1:, bad:] = False
+    assert float((L - R)[ok].abs().max()) <= 1e-13
+    assert bool(torch.isnan(L[bad, 3:bad + 1]).all()) and bool(torch.isnan(torch.diagonal(L)[bad:]).all())
+    D = torch.eye(130, dtype=torch.float64, device="cuda")
+    D[70, 70] = 4.0e-310
+    L, info = _potrf(gpu_lla, torch, D)
+    assert info == -1 and abs(float(L[70, 70]) - 2.0e-155) <= 1e-168 and float(L[129, 129]) == 1.0
+
+
+def test_fast_fp64_factor_on_two_streams_and_in_a_graph(gpu_lla):
+    """Concurrent factorisations of one thread, and replays of a captured one, share no scratch."""
+    torch = _torch()
+    n = 700
+    mats = [_spd(torch, n, 1.0, 20 + i)[0] for i in range(4)]
+    want = [_potrf(gpu_lla, torch, A)[0].clone() for A in mats]
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    out = [A.clone().T for A in mats]
+    infos = [torch.empty(1, dtype=torch.int64, device="cuda") for _ in mats]
+    torch.cuda.synchronize()
+    for i, (L, f) in enumerate(zip(out, infos)):
+        gpu_lla.potrf_device(L, algo=gpu_lla.ALGO_FAST, info=f, stream=streams[i % 2])
+    torch.cuda.synchronize()
+    for L, w, f in zip(out, want, infos):
+        assert int(f.item()) == -1 and bool((L == w).all())
+    L = mats[0].clone().T
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=streams[0]):
+        gpu_lla.potrf_device(L, algo=gpu_lla.ALGO_FAST, info=infos[0], stream=torch.cuda.current_stream())
+    other = mats[1].clone().T
+    for i in (1, 2):
+        L.copy_(mats[i].T)
+        torch.cuda.synchronize()
+        graph.replay()
+        gpu_lla.potrf_device(other, algo=gpu_lla.ALGO_FAST, info=infos[1], stream=streams[1])
+        torch.cuda.synchronize()
+        assert bool((L == want[i]).all())
+        assert i != 1 or bool((other == want[1]).all())
