@@ -97,4 +97,61 @@ __host__ __device__ __forceinline__ double im_rsqrt(double d) {
     return im_double(((uint64_t)(1021 - h) << 52) + ((y + 128) >> 8));
 }
 
+// ---- correctly rounded quotients by one divisor ------------------------------
+//
+// a / d with the reciprocal of d's mantissa in fixed point: one high product
+// gives the quotient's mantissa with nine or ten bits to spare, below the true
+// value by less than two units of the last one.  That decides the rounding (to
+// nearest; a quotient of two doubles is never a midpoint) unless the spare bits
+// are one short of a half.
+struct ImDivisor {
+    uint64_t D;   // mantissa of d, 2^52 <= D < 2^53
+    uint64_t V;   // floor(2^115 / D)
+    int32_t e;    // exponent field of d, sign in bit 11
+    int32_t ok;   // d is a normal number
+};
+
+__host__ __device__ __forceinline__ ImDivisor im_divisor(double d) {
+    const uint64_t b = im_bits(d);
+    ImDivisor v;
+    v.e = (int32_t)(b >> 52);
+    v.ok = im_positive_normal(b & 0x7fffffffffffffffull);
+    v.D = (b & 0x000fffffffffffffull) | 0x0010000000000000ull;
+    // D 2^-52 in [1, 2) and its reciprocal to 53 bits, then one exact correction:
+    // E = 2^115 - V D is below 2^64 in magnitude, so its low 64 bits are E
+    const double y = 1.0 / im_double((b & 0x000fffffffffffffull) | 0x3ff0000000000000ull);  // (1/2, 1]
+    uint64_t V = (uint64_t)(y * 9223372036854775808.0);  // y 2^63, exact
+    if (V > 0x7fffffffffffffffull) V = 0x7fffffffffffffffull;
+    int64_t E = (int64_t)(0ull - V * v.D);
+    const int64_t k = (int64_t)((double)E * (y * 2.220446049250313e-16));  // E / D, within one of it
+    V += (uint64_t)k;
+    E -= k * (int64_t)v.D;
+    while (E < 0) {
+        --V;
+        E += (int64_t)v.D;
+    }
+    while (E >= (int64_t)v.D) {
+        ++V;
+        E -= (int64_t)v.D;
+    }
+    v.V = V;
+    return v;
+}
+
+// a / d; ok says whether it is IEEE division's result (a zero or normal a over a
+// normal d with exponents well inside the range, and no undecided rounding).
+__host__ __device__ __forceinline__ double im_div(double a, const ImDivisor &d, bool &ok) {
+    const uint64_t b = im_bits(a);
+    const uint64_t A = (b & 0x000fffffffffffffull) | 0x0010000000000000ull;
+    const bool lt = A < d.D, zero = (b << 1) == 0;              // lt: quotient of the mantissas below 1
+    const uint64_t hi = im_mulhi(A << 11, d.V);                 // A / D 2^62, less than two above hi
+    const uint64_t m = lt ? (hi + 256) >> 9 : (hi + 512) >> 10; // 53 bits, or 2^53
+    const int ea = (int)(b >> 52) & 0x7ff, q = ea - (d.e & 0x7ff);
+    const uint64_t sign = (b ^ ((uint64_t)(uint32_t)d.e << 52)) & 0x8000000000000000ull;
+    const uint64_t e = (uint64_t)(q + 1022 - (lt ? 1 : 0)) << 52;  // biased, minus the leading one of m
+    const bool undecided = ((uint32_t)hi & (lt ? 511u : 1023u)) == (lt ? 255u : 511u);
+    ok = d.ok && (zero || (ea != 0 && ea != 0x7ff && q > -1020 && q < 1020 && !undecided));
+    return im_double(zero ? sign : sign | (e + m));
+}
+
 }  // namespace lla

@@ -21,11 +21,26 @@
 // kSpinLimit polls the CTA records LLA_ERR_TIMEOUT in `err_word`, publishes
 // its flag and returns, so a fault elsewhere cannot hang the device.
 //
+// What bounds it is the chain from row block to row block: hand-off, the last
+// coupling tile, the solve of the diagonal block.  One warp owns one right-hand
+// side of the block (lane = row) and goes from poll to publication alone; the
+// CTA's warps share only the coupling tiles, copied one tile ahead into two
+// buffers, and the diagonal block, which is loaded and prepared before the
+// first wait.  An FP64 instruction takes 64 cycles of its sub-partition, so the
+// solve of a block keeps few of them in its chain: in EXACT mode the division by
+// the diagonal is done in integers (lla_int_math.h), in FAST mode the rows are divided by their diagonal beforehand and
+// a step is one FMA.  Four right-hand sides a CTA: one warp per sub-partition.
+// Per row block, before -> now: EXACT f64 25 -> 11 us (n = 512), EXACT f32 7.1 ->
+// 3.7 us (n = 1000, 8 right-hand sides), FAST f64 30 -> 7.3 us (n = 8192, 16
+// right-hand sides; 1.03 ms of the 1.9 ms solve is the FP64 pipe's share), FAST
+// f32 9.4 -> 2.0 us (n = 6001, 3 right-hand sides).
+//
 // T[r, c] (logical) = trans ? M[c, r] : M[r, c]; `diag` (optional) overrides
 // the diagonal as the reference's diag_fn does (src/triangular.rs:133-144).
 #include <atomic>
 
 #include "lla_common.cuh"
+#include "lla_int_math.h"
 #include "lla_kernels.h"
 #include "lla_prof.h"
 
@@ -33,6 +48,7 @@ namespace lla {
 
 constexpr int kTrsmNb = 32;
 constexpr int kTrsmMaxMc = 8;
+constexpr int kTrsmMc = 4;  // right-hand sides a CTA (8 where the flags would not fit otherwise)
 
 __device__ __forceinline__ int ld_acquire(const int *p) {
     int v;
@@ -40,29 +56,56 @@ __device__ __forceinline__ int ld_acquire(const int *p) {
     return v;
 }
 
-__device__ __forceinline__ void st_release(int *p, int v) {
-    asm volatile("st.release.gpu.b32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+__device__ __forceinline__ void or_release(int *p, int v) {
+    asm volatile("red.release.gpu.global.or.b32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
+template <typename T>
+__device__ __forceinline__ void cp_async_elem(T *dst, const T *src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src),
+                 "n"(sizeof(T))
+                 : "memory");
+}
+
+// Warps of a CTA: one per right-hand side; at least four copy the tiles.
+static int trsm_warps(int mc) { return std::max(mc, kTrsmMc); }
+
+// The division of the reference's substitution by a divisor that is known early;
+// ok says, off the chain, whether the quotient is IEEE division's, and the solve
+// repeats a block with IEEE division if one was not.
+template <typename T>
+struct TrsmDivisor;
+template <>
+struct TrsmDivisor<float> {
+    float d;
+    __device__ __forceinline__ explicit TrsmDivisor(float v) { d = v; }
+    __device__ __forceinline__ float divide(float b, bool &ok) const {
+        ok = true;
+        return __fdiv_rn(b, d);
+    }
+};
+template <>
+struct TrsmDivisor<double> {
+    ImDivisor q;
+    __device__ __forceinline__ explicit TrsmDivisor(double v) { q = im_divisor(v); }
+    __device__ __forceinline__ double divide(double b, bool &ok) const { return im_div(b, q, ok); }
+};
+
 template <typename T, bool kExact>
-__global__ void __launch_bounds__(256) trsm_lookback(const T *__restrict__ M, int64_t ld, int64_t n,
-                                                     int lower, int trans,
-                                                     const T *__restrict__ diag, T *B, int64_t ldb,
-                                                     int64_t m, int mc, int n_chunks, int *ws,
-                                                     int *err_word, int *sticky, long long spin_limit,
-                                                     int lose_first) {
+__global__ void __launch_bounds__(kTrsmNb *kTrsmMaxMc) trsm_lookback(const T *__restrict__ M, int64_t ld, int64_t n,
+                                                                   int lower, int trans, const T *__restrict__ diag,
+                                                                   T *B, int64_t ldb, int64_t m, int mc, int n_chunks,
+                                                                   int *ws, int *err_word, int *sticky,
+                                                                   long long spin_limit, int lose_first) {
     using Ar = Arith<T>;
-    __shared__ T ts[kTrsmNb][kTrsmNb + 1];
-    __shared__ T xs[kTrsmMaxMc][kTrsmNb];
-    __shared__ T dg[kTrsmNb];
-    __shared__ int s_ticket, s_abort;
+    __shared__ T ts[2][kTrsmNb][kTrsmNb + 1];  // coupling tiles, [term][row]
+    __shared__ T td[kTrsmNb][kTrsmNb + 1];     // diagonal block, [term][row]
+    __shared__ __align__(16) T xs[kTrsmMaxMc][kTrsmNb];  // a solved block, by right-hand side
+    __shared__ int s_ticket;
     const int tx = threadIdx.x, ty = threadIdx.y;
     const int tid = ty * kTrsmNb + tx, nthr = kTrsmNb * blockDim.y;
     int *counter = ws, *flags = ws + 1;
-    if (tid == 0) {
-        s_ticket = atomicAdd(counter, 1);
-        s_abort = 0;
-    }
+    if (tid == 0) s_ticket = atomicAdd(counter, 1);
     __syncthreads();
     // failure injection (tests only): the first item is lost -- never solved,
     // never published -- so every wait on it runs out
@@ -70,92 +113,138 @@ __global__ void __launch_bounds__(256) trsm_lookback(const T *__restrict__ M, in
     const int64_t rb = s_ticket / n_chunks;
     const int cc = s_ticket % n_chunks;
     const int64_t col = (int64_t)cc * mc + ty;
-    const bool col_ok = ty < mc && col < m;
+    const bool col_ok = ty < mc && col < m;  // uniform for the warp
     auto row_of = [&](int64_t t) -> int64_t { return lower ? t : n - 1 - t; };
-    auto tval = [&](int64_t r, int64_t c) -> T { return trans ? M[c + r * ld] : M[r + c * ld]; };
-    const int64_t t_own = rb * kTrsmNb + tx;
-    const bool row_ok = t_own < n;
-    const int64_t r_own = row_ok ? row_of(t_own) : 0;
-    T bv = (row_ok && col_ok) ? B[r_own + col * ldb] : T(0);
+    const int64_t t0 = rb * kTrsmNb;
+    const int bs = (int)(n - t0 < kTrsmNb ? n - t0 : kTrsmNb);
+    // element e of a tile: consecutive e -> consecutive memory (rows, or terms when transposed)
+    auto copy_tile = [&](T(*dst)[kTrsmNb + 1], int64_t u0, int terms) {
+        for (int e = tid; e < kTrsmNb * kTrsmNb; e += nthr) {
+            const int x = trans ? e / kTrsmNb : e % kTrsmNb, y = trans ? e % kTrsmNb : e / kTrsmNb;
+            if (x < bs && y < terms) {
+                const int64_t r = row_of(t0 + x), c = row_of(u0 + y);
+                cp_async_elem(&dst[y][x], trans ? &M[c + r * ld] : &M[r + c * ld]);
+            } else {
+                dst[y][x] = T(0);
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    copy_tile(td, t0, bs);
+    if (rb > 0) copy_tile(ts[0], 0, kTrsmNb);
+    const int64_t r_own = row_of(t0 + (tx < bs ? tx : 0));
+    T bv = (tx < bs && col_ok) ? B[r_own + col * ldb] : T(0);
+    const T dv = tx < bs ? (diag ? diag[r_own] : M[r_own + r_own * ld]) : T(1);
+    const TrsmDivisor<T> dq(dv);
+    // FAST: 1 / dv in two parts, so that b times it is rounded once, like the quotient
+    const T rinv = kExact ? T(0) : Ar::div(T(1), dv);
+    const T rlo = kExact ? T(0) : Ar::mul(Ar::fma_(-dv, rinv, T(1)), rinv);
+    if (rb > 0)
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+    else
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    // FAST: the rows are divided by their diagonal, so that a step of the solve is
+    // one FMA -- unless that would leave the comfortable range of the type (a zero,
+    // tiny, huge or non-finite diagonal or entry): then a step divides.
+    bool scaled = false;
+    if (!kExact) {
+        const T big = sizeof(T) == 8 ? T(1.3e154) : T(1.8e19f), small = T(1) / big;
+        bool in_range = abs(rinv) <= big && abs(rinv) >= small;
+        for (int y = ty; y < kTrsmNb; y += blockDim.y) {  // this lane's row
+            const T t = abs(td[y][tx]), u = t * abs(rinv);
+            in_range = in_range && (t == T(0) || y >= tx || (u <= big && u >= small));
+        }
+        scaled = __syncthreads_and(in_range) != 0;
+        if (scaled)
+            for (int y = ty; y < kTrsmNb; y += blockDim.y) td[y][tx] *= rinv;
+    }
 
+    bool abort = false;
     for (int64_t q = 0; q < rb; ++q) {
-        if (tid == 0) {
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        // tile q has landed for everyone, and tile q - 1's buffer is free; the barrier carries the
+        // verdict of the last wait, so that all warps leave together
+        if (__syncthreads_or(abort)) {
+            abort = true;
+            break;
+        }
+        if (q + 1 < rb) copy_tile(ts[(q + 1) & 1], (q + 1) * kTrsmNb, kTrsmNb);
+        if (col_ok) {
             const int *f = flags + q * n_chunks + cc;
             long long spins = 0;
-            while (ld_acquire(f) == 0) {
+            while (!((ld_acquire(f) >> ty) & 1)) {
                 if (*(volatile int *)err_word != 0) {
-                    s_abort = 1;
+                    abort = true;
                     break;
                 }
                 if (++spins > spin_limit) {
-                    atomicCAS(err_word, 0, (int)LLA_ERR_TIMEOUT);
-                    if (sticky) atomicCAS(sticky, 0, (int)LLA_ERR_TIMEOUT);
-                    s_abort = 1;
+                    if (tx == 0) {
+                        atomicCAS(err_word, 0, (int)LLA_ERR_TIMEOUT);
+                        if (sticky) atomicCAS(sticky, 0, (int)LLA_ERR_TIMEOUT);
+                    }
+                    abort = true;
                     break;
                 }
-                __nanosleep(64);
+                if (spins > 64) __nanosleep(64);
+            }
+            abort = __any_sync(0xffffffffu, abort);
+            // solved block q (always a full block: q < rb), one row a lane
+            __syncwarp();  // (the previous block's values have been read)
+            xs[ty][tx] = abort ? T(0) : __ldcg(&B[row_of(q * kTrsmNb + tx) + col * ldb]);
+            __syncwarp();
+            const T(*tq)[kTrsmNb + 1] = ts[q & 1];
+#pragma unroll
+            for (int y0 = 0; y0 < kTrsmNb; y0 += 8) {
+                T xv[8], tv[8];
+#pragma unroll
+                for (int y = 0; y < 8; ++y) {
+                    xv[y] = xs[ty][y0 + y];
+                    tv[y] = tq[y0 + y][tx];
+                }
+#pragma unroll
+                for (int y = 0; y < 8; ++y)
+                    bv = kExact ? Ar::sub(bv, Ar::mul(xv[y], tv[y])) : Ar::fma_(-xv[y], tv[y], bv);
             }
         }
-        __syncthreads();
-        if (s_abort) break;
-        // solved block q (always a full block: q < rb) and the tile T[block rb, block q]
-        for (int e = tid; e < kTrsmNb * mc; e += nthr) {
-            const int x = e % kTrsmNb, y = e / kTrsmNb;
-            const int64_t c = (int64_t)cc * mc + y;
-            xs[y][x] = (c < m) ? __ldcg(&B[row_of(q * kTrsmNb + x) + c * ldb]) : T(0);
-        }
-        for (int e = tid; e < kTrsmNb * kTrsmNb; e += nthr) {
-            const int x = trans ? e / kTrsmNb : e % kTrsmNb;  // consecutive e -> consecutive memory
-            const int y = trans ? e % kTrsmNb : e / kTrsmNb;
-            const int64_t tr = rb * kTrsmNb + x;
-            ts[x][y] = (tr < n) ? tval(row_of(tr), row_of(q * kTrsmNb + y)) : T(0);
-        }
-        __syncthreads();
-        if (row_ok && col_ok) {
-#pragma unroll 8
-            for (int y = 0; y < kTrsmNb; ++y) {
-                if (kExact)
-                    bv = Ar::sub(bv, Ar::mul(xs[ty][y], ts[tx][y]));
-                else
-                    bv = Ar::fma_(-xs[ty][y], ts[tx][y], bv);
-            }
-        }
-        __syncthreads();
     }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    if (!kExact) __syncthreads();  // (the first block met no barrier after the scaling of td)
 
-    if (!s_abort) {
-        const int64_t left = n - rb * kTrsmNb;
-        const int bs = left < kTrsmNb ? (int)left : kTrsmNb;
-        for (int e = tid; e < kTrsmNb * kTrsmNb; e += nthr) {
-            const int x = trans ? e / kTrsmNb : e % kTrsmNb;
-            const int y = trans ? e % kTrsmNb : e / kTrsmNb;
-            ts[x][y] = (x < bs && y < bs) ? tval(row_of(rb * kTrsmNb + x), row_of(rb * kTrsmNb + y))
-                                          : T(0);
-        }
-        if (tid < bs) {
-            const int64_t r = row_of(rb * kTrsmNb + tid);
-            dg[tid] = diag ? diag[r] : M[r + r * ld];
-        }
-        __syncthreads();
-        for (int y = 0; y < bs; ++y) {
-            if (tx == y) {
-                const T xv = Ar::div(bv, dg[y]);  // coeff = b[i,k] / diag  (:117-119)
-                bv = xv;
-                xs[ty][y] = xv;
+    if (!abort && col_ok) {
+        if (scaled) {
+            bv = Ar::fma_(bv, rinv, Ar::mul(bv, rlo));
+#pragma unroll 4
+            for (int y = 0; y < bs; ++y) {
+                const T xy = __shfl_sync(0xffffffffu, bv, y);
+                const T nb = Ar::fma_(-xy, td[y][tx], bv);
+                if (tx > y) bv = nb;
             }
-            __syncthreads();
-            if (tx > y && tx < bs) {
-                if (kExact)
-                    bv = Ar::sub(bv, Ar::mul(xs[ty][y], ts[tx][y]));
-                else
-                    bv = Ar::fma_(-xs[ty][y], ts[tx][y], bv);
+        } else {
+            const T b0 = bv;
+            bool ok = true;
+#pragma unroll 4
+            for (int y = 0; y < bs; ++y) {
+                bool quot_ok;
+                const T xy = __shfl_sync(0xffffffffu, dq.divide(bv, quot_ok), y);  // coeff = b[i,k] / diag  (:117-119)
+                ok = ok && (tx != y || quot_ok);
+                const T nb = kExact ? Ar::sub(bv, Ar::mul(xy, td[y][tx])) : Ar::fma_(-xy, td[y][tx], bv);
+                bv = tx == y ? xy : (tx > y ? nb : bv);
+            }
+            if (!__all_sync(0xffffffffu, ok)) {
+                bv = b0;
+#pragma unroll 1
+                for (int y = 0; y < bs; ++y) {
+                    const T xy = __shfl_sync(0xffffffffu, Ar::div(bv, dv), y);
+                    const T nb = kExact ? Ar::sub(bv, Ar::mul(xy, td[y][tx])) : Ar::fma_(-xy, td[y][tx], bv);
+                    bv = tx == y ? xy : (tx > y ? nb : bv);
+                }
             }
         }
     }
-    if (row_ok && col_ok) B[r_own + col * ldb] = bv;
-    __threadfence();
-    __syncthreads();
-    if (tid == 0) st_release(flags + rb * n_chunks + cc, 1);
+    if (tx < bs && col_ok) B[r_own + col * ldb] = bv;
+    __syncwarp();  // the warp's stores, then its bit of the block's flag
+    if (tx == 0) or_release(flags + rb * n_chunks + cc, 1 << ty);
 }
 
 // One-shot failure injection for the tests of timeout reporting
@@ -179,11 +268,11 @@ int trsm_launch(const T *M, int64_t ld, int64_t n, int lower, int trans, const T
                 int64_t ldb, int64_t m, bool exact, int *ws, int *err_word, cudaStream_t st,
                 int *sticky) {
     if (n == 0 || m == 0) return 0;
-    const int mc = (int)std::min<int64_t>(kTrsmMaxMc, m);
+    const int mc = (int)std::min<int64_t>(kTrsmMc, m);
     const int64_t chunks = ceil_div(m, mc);
     const int64_t R = ceil_div(n, kTrsmNb);
     if (cudaMemsetAsync(ws, 0, sizeof(int) * (1 + R * chunks), st) != cudaSuccess) return -1;
-    const dim3 block(kTrsmNb, mc);
+    const dim3 block(kTrsmNb, trsm_warps(mc));
     const unsigned grid = (unsigned)(R * chunks);
     const TrsmWaitCfg wc = take_wait_cfg();
     // algorithmic work: n^2 * m flops (n(n-1)/2 multiply-adds and n divisions per column)
@@ -201,7 +290,7 @@ int trsm_launch(const T *M, int64_t ld, int64_t n, int lower, int trans, const T
 
 size_t trsm_ws_ints(int64_t n, int64_t m) {
     if (n == 0 || m == 0) return 1;
-    const int mc = (int)std::min<int64_t>(kTrsmMaxMc, m);
+    const int mc = (int)std::min<int64_t>(kTrsmMc, m);
     return (size_t)(1 + ceil_div(n, kTrsmNb) * ceil_div(m, mc));
 }
 
@@ -280,9 +369,10 @@ extern "C" int lla_dtrsm_device_noalloc(const double *dL, int64_t n, int64_t ld,
         return lla__set_status(err, LLA_ERR_INVALID_ARG);
     lla__set_status(err, LLA_OK);
     if (n == 0 || m == 0) return LLA_OK;
-    const int mc = (int)std::min<int64_t>(kTrsmMaxMc, m);
-    const int64_t chunks = ceil_div(m, mc);
+    // the limit is that of eight right-hand sides a CTA; fewer where their flags fit too
     const int64_t R = ceil_div(n, kTrsmNb);
+    const int mc = (int)std::min<int64_t>(R * ceil_div(m, kTrsmMc) <= kNoAllocMaxFlags ? kTrsmMc : kTrsmMaxMc, m);
+    const int64_t chunks = ceil_div(m, mc);
     if (R * chunks > kNoAllocMaxFlags) return lla__set_status(err, LLA_ERR_TOO_LARGE);
     int *scratch = nullptr;
     cudaError_t e = noalloc_scratch(&scratch);
@@ -292,7 +382,7 @@ extern "C" int lla_dtrsm_device_noalloc(const double *dL, int64_t n, int64_t ld,
     e = cudaMemsetAsync(scratch, 0, sizeof(int) * (size_t)(1 + R * chunks), st);
     if (e == cudaSuccess) e = cudaMemsetAsync(err_word, 0, sizeof(int), st);
     if (e != cudaSuccess) return lla__set_cuda_error(err, e);
-    const dim3 block(kTrsmNb, mc);
+    const dim3 block(kTrsmNb, trsm_warps(mc));
     const unsigned grid = (unsigned)(R * chunks);
     // trans = 0: L X = B (lower, ascending); trans = 1: L^T X = B (descending)
     const int lower = trans ? 0 : 1;

@@ -1,5 +1,5 @@
 """Integer building blocks of the FP64 factorisations, compiled on the host from
-the kernels' own headers: reciprocal roots in fixed point (csrc/lla_int_math.h),
+the kernels' own headers: reciprocal roots and quotients in fixed point (csrc/lla_int_math.h),
 and the balanced digits, fixed-point values and 64-bit-to-double conversion of
 the FP64 trailing update (csrc/lla_oz_digits.h).  The references are the
 compiler's long double and integer arithmetic."""
@@ -41,6 +41,28 @@ int main() {
     for (double d : {0.0, -0.0, -1.0, 5e-324, 2.2250738585072009e-308, HUGE_VAL, -HUGE_VAL, std::nan("")})
         CHECK(!im_positive_normal(im_bits(d)), "normal(%a)\n", d);
     CHECK(im_positive_normal(im_bits(2.2250738585072014e-308)) && im_positive_normal(im_bits(1.7976931348623157e308)), "ends\n");
+    // quotients: IEEE division's where they say so, refused about once in 700
+    long taken = 0, refused = 0;
+    for (long t = 0; t < 300000; ++t) {
+        uint64_t db = g();
+        if (t % 3) db = (db & 0x800fffffffffffffull) | ((1000ull + g() % 40) << 52);
+        if (t % 5 == 0) db &= ~0xfffffffffffull;
+        if (t % 7 == 0) db |= 0xfffffffffffffull;
+        const double d = im_double(db);
+        const ImDivisor v = im_divisor(d);
+        for (int k = 0; k < 6; ++k) {
+            uint64_t ab = g();
+            if (k & 1) ab = (ab & 0x800fffffffffffffull) | ((1000ull + g() % 40) << 52);
+            if (k == 2) ab = im_bits(im_double((g() & 0x000ffffffff00000ull) | (1023ull << 52)) * d);
+            if (k == 4) ab &= 0x8000000000000000ull;
+            const double a = im_double(ab);
+            bool ok;
+            const double q = im_div(a, v, ok);
+            CHECK(!ok || im_bits(q) == im_bits(a / d), "%a / %a = %a\n", a, d, q);
+            if (k == 3 && t % 3 && im_positive_normal(ab & ~(1ull << 63))) (ok ? taken : refused)++;
+        }
+    }
+    CHECK(refused < taken / 300 && refused > taken / 2000, "refused %ld of %ld\n", refused, taken);
     // digits: V = nearest multiple of 2^(e-55), its seven balanced digits exact in BF16
     std::uniform_real_distribution<double> U(0.5, 1.0);
     for (long t = 0; t < 400000; ++t) {

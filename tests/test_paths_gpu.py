@@ -133,3 +133,69 @@ def test_fast_fp64_factor_on_two_streams_and_in_a_graph(gpu_lla):
         torch.cuda.synchronize()
         assert bool((L == want[i]).all())
         assert i != 1 or bool((other == want[1]).all())
+
+
+def _tri(n, dtype, seed, scale):
+    """Well-conditioned lower triangle, rows scaled by 2^U(-scale, scale)."""
+    rng = np.random.default_rng(seed)
+    t = np.tril(rng.standard_normal((n, n)) / np.sqrt(n), -1) + np.diag(rng.uniform(1, 2, n) * rng.choice((-1, 1), n))
+    d = np.exp2(np.round(rng.uniform(-scale, scale, n)))
+    return (t * d[:, None]).astype(dtype), d
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("n,m", [(1, 1), (31, 3), (32, 4), (33, 5), (65, 9), (257, 2)])
+@pytest.mark.parametrize("scale", [0, 60, 600])
+def test_fast_substitution_forms(gpu_lla, dtype, n, m, scale):
+    """FAST triangular solves in both directions, with row scales inside and outside the
+    range in which rows are divided by their diagonal beforehand: scaling the rows of T and
+    of B by powers of two changes nothing."""
+    torch = _torch()
+    if scale > 60 and dtype == np.float32:
+        pytest.skip("outside the type's exponent range")
+    t, d = _tri(n, dtype, n + m, scale)
+    b0 = np.random.default_rng(m).standard_normal((n, m))
+    eps = np.finfo(dtype).eps
+    for trans in (0, 1):
+        # trans = 1 solves T^T x = b, where the scales are those of the unknowns
+        b = (b0 * d[:, None] if not trans else b0).astype(dtype)
+        L = torch.from_numpy(np.ascontiguousarray(t.T)).cuda().T
+        X = torch.from_numpy(np.ascontiguousarray(b.T)).cuda().T
+        gpu_lla.trsm_device(L, X, trans, algo=gpu_lla.ALGO_FAST)
+        gpu_lla.device_status()
+        x = X.cpu().numpy().astype(np.float64)
+        base = (t.astype(np.float64) / d[:, None])
+        y = x * d[:, None] if trans else x
+        r = (base.T if trans else base) @ y - b0
+        den = np.abs(base).sum(1).max() * np.abs(y).max() + np.abs(b0).max()
+        assert np.abs(r).max() <= 10 * max(n, 4) * eps * den
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+def test_exact_division_fallbacks_match_the_oracle(gpu_lla, dtype):
+    """Quotients that the integer division does not take (subnormal, overflowing, infinite and
+    NaN values, zero diagonals) repeat the block with IEEE division: bit-identical to the oracle."""
+    from oracle import oracle as ora
+    n, tiny = 70, np.finfo(dtype).tiny
+    t, _ = _tri(n, dtype, 9, 0)
+    b = np.random.default_rng(1).standard_normal((n, 6)).astype(dtype)
+    b[:, 1] *= tiny
+    b[:, 2] = 0
+    b[5, 2] = -0.0
+    b[:, 3] *= np.finfo(dtype).max / 8
+    b[40, 4] = np.inf
+    b[41, 5] = np.nan
+    with np.errstate(all="ignore"):
+        for k, v in ((None, 0), (33, 0.0), (50, tiny / 4), (66, np.inf)):
+            tt = t.copy()
+            if k is not None:
+                tt[k, k] = v
+            want, got = b.copy(), b.copy()
+            ora.solve_triangular_inplace(tt, want, "lower")
+            prev = gpu_lla.set_algorithm(gpu_lla.ALGO_EXACT)
+            try:
+                gpu_lla.solve_triangular_inplace(tt, got, "lower")
+            finally:
+                gpu_lla.set_algorithm(prev)
+            same = (got == want) | (np.isnan(got) & np.isnan(want))
+            assert same.all() and (np.signbit(got) == np.signbit(want))[~np.isnan(want)].all(), (k, v)
