@@ -97,44 +97,44 @@ __host__ __device__ __forceinline__ double im_rsqrt(double d) {
     return im_double(((uint64_t)(1021 - h) << 52) + ((y + 128) >> 8));
 }
 
+__host__ __device__ __forceinline__ int64_t im_mulhi_s(int64_t a, int64_t b) {
+#ifdef __CUDA_ARCH__
+    return __mul64hi(a, b);
+#else
+    return (int64_t)(((__int128)a * b) >> 64);
+#endif
+}
+
 // ---- correctly rounded quotients by one divisor ------------------------------
 //
-// a / d with the reciprocal of d's mantissa in fixed point: one high product
-// gives the quotient's mantissa with nine or ten bits to spare, below the true
-// value by less than two units of the last one.  That decides the rounding (to
-// nearest; a quotient of two doubles is never a midpoint) unless the spare bits
-// are one short of a half.
+// 2^115 / D for the divisor's mantissa D as V + F 2^-32: V to 53 bits, F from
+// the exact remainder E = 2^115 - V D (below 2^63 in magnitude, so its low 64
+// bits are E).  A product with it gives the quotient's mantissa with some 40 bits
+// to spare, which decide the rounding (to nearest; a quotient of two doubles is
+// never a midpoint) unless they lie within a few units of a half.
 struct ImDivisor {
     uint64_t D;   // mantissa of d, 2^52 <= D < 2^53
-    uint64_t V;   // floor(2^115 / D)
+    uint64_t V;
+    int64_t F;    // |F| < 2^43
     int32_t e;    // exponent field of d, sign in bit 11
     int32_t ok;   // d is a normal number
 };
+
+// V: 2^115 / D to a relative 2^-53.
+__host__ __device__ __forceinline__ void im_reciprocal(ImDivisor &v, uint64_t D, uint64_t V) {
+    v.D = D;
+    v.V = V;
+    v.F = im_mulhi_s((int64_t)(0ull - V * D), (int64_t)V) >> 19;
+}
 
 __host__ __device__ __forceinline__ ImDivisor im_divisor(double d) {
     const uint64_t b = im_bits(d);
     ImDivisor v;
     v.e = (int32_t)(b >> 52);
     v.ok = im_positive_normal(b & 0x7fffffffffffffffull);
-    v.D = (b & 0x000fffffffffffffull) | 0x0010000000000000ull;
-    // D 2^-52 in [1, 2) and its reciprocal to 53 bits, then one exact correction:
-    // E = 2^115 - V D is below 2^64 in magnitude, so its low 64 bits are E
     const double y = 1.0 / im_double((b & 0x000fffffffffffffull) | 0x3ff0000000000000ull);  // (1/2, 1]
-    uint64_t V = (uint64_t)(y * 9223372036854775808.0);  // y 2^63, exact
-    if (V > 0x7fffffffffffffffull) V = 0x7fffffffffffffffull;
-    int64_t E = (int64_t)(0ull - V * v.D);
-    const int64_t k = (int64_t)((double)E * (y * 2.220446049250313e-16));  // E / D, within one of it
-    V += (uint64_t)k;
-    E -= k * (int64_t)v.D;
-    while (E < 0) {
-        --V;
-        E += (int64_t)v.D;
-    }
-    while (E >= (int64_t)v.D) {
-        ++V;
-        E -= (int64_t)v.D;
-    }
-    v.V = V;
+    const uint64_t V = (uint64_t)(y * 9223372036854775808.0);  // y 2^63, exact
+    im_reciprocal(v, (b & 0x000fffffffffffffull) | 0x0010000000000000ull, V - (V >> 63));  // below 2^63
     return v;
 }
 
@@ -142,16 +142,48 @@ __host__ __device__ __forceinline__ ImDivisor im_divisor(double d) {
 // normal d with exponents well inside the range, and no undecided rounding).
 __host__ __device__ __forceinline__ double im_div(double a, const ImDivisor &d, bool &ok) {
     const uint64_t b = im_bits(a);
-    const uint64_t A = (b & 0x000fffffffffffffull) | 0x0010000000000000ull;
-    const bool lt = A < d.D, zero = (b << 1) == 0;              // lt: quotient of the mantissas below 1
-    const uint64_t hi = im_mulhi(A << 11, d.V);                 // A / D 2^62, less than two above hi
-    const uint64_t m = lt ? (hi + 256) >> 9 : (hi + 512) >> 10; // 53 bits, or 2^53
+    const uint64_t An = ((b << 11) & 0x7ffffffffffff800ull) | 0x8000000000000000ull;  // a's mantissa, leading one on top
+    const bool lt = An < (d.D << 11), zero = (b << 1) == 0;  // lt: quotient of the mantissas below 1
+    // A / D 2^62 = hi . lo, to about 2^-30
+    const uint64_t lo0 = An * d.V, hi0 = im_mulhi(An, d.V);
+    int64_t G = im_mulhi_s((int64_t)(An >> 1), d.F);         // An F 2^-65
+    const uint64_t lo = lo0 + ((uint64_t)G << 33);
+    const uint64_t hi = hi0 + (uint64_t)(G >> 31) + (lo < lo0 ? 1 : 0);
+    const uint64_t m = lt ? (hi + 256) >> 9 : (hi + 512) >> 10;  // 53 bits, or 2^53
     const int ea = (int)(b >> 52) & 0x7ff, q = ea - (d.e & 0x7ff);
     const uint64_t sign = (b ^ ((uint64_t)(uint32_t)d.e << 52)) & 0x8000000000000000ull;
     const uint64_t e = (uint64_t)(q + 1022 - (lt ? 1 : 0)) << 52;  // biased, minus the leading one of m
-    const bool undecided = ((uint32_t)hi & (lt ? 511u : 1023u)) == (lt ? 255u : 511u);
+    // spare bits and the top of lo, seen from a half
+    const int32_t spare = (int32_t)((uint32_t)hi & (lt ? 511u : 1023u)) - (lt ? 256 : 512), top = (int32_t)(lo >> 32) >> 8;
+    const bool undecided = (spare == -1 && top == -1) || (spare == 0 && top == 0);
     ok = d.ok && (zero || (ea != 0 && ea != 0x7ff && q > -1020 && q < 1020 && !undecided));
     return im_double(zero ? sign : sign | (e + m));
+}
+
+// sqrt(d), correctly rounded, and the divisor it becomes; d positive and normal.
+// The reciprocal root y (2^-60) gives the root to 54 bits or one unit less; the
+// exact remainder corrects it, and a root is never a midpoint of two doubles.
+// y is also the divisor's reciprocal to 2^-53.
+__host__ __device__ __forceinline__ double im_sqrt(double d, ImDivisor &v) {
+    const uint64_t b = im_bits(d);
+    const int eb = (int)(b >> 52);
+    const int odd = (eb & 1) ^ 1;  // d = m 2^(2h), m in [1, 4)
+    const int h = (eb - 1023 - odd) >> 1;
+    const uint64_t X = (b & 0x000fffffffffffffull) | 0x0010000000000000ull;
+    const uint64_t M = X << (10 + odd);
+    const uint32_t fb = ((uint32_t)(127 + odd) << 23) | ((uint32_t)(b >> 29) & 0x7fffffu);
+    float mf;
+    memcpy(&mf, &fb, 4);
+    const uint64_t y = im_rsqrt_q61(M, mf);
+    // S = floor(sqrt(m) 2^53), or one less
+    uint64_t S = (im_mulhi(M, y) - 16) >> 6;
+    const int64_t rem = (int64_t)((X << (54 + odd)) - S * S);  // m 2^106 - S^2, modulo 2^64
+    S += rem > (int64_t)(2 * S) ? 1 : 0;
+    const uint64_t D = (S + 1) >> 1;
+    im_reciprocal(v, D, (y << 2) - (y >> 61));  // (below 2^63 for y = 1 too)
+    v.e = h + 1023;
+    v.ok = 1;
+    return im_double(((uint64_t)(h + 1022) << 52) + D);
 }
 
 }  // namespace lla

@@ -16,100 +16,263 @@
 // FAST mode is LAPACK-style right-looking (A22 -= L21 L21^T in place) with
 // fused multiply-add; this file holds the FP32 form, lla_fp64_chol.cu the FP64 one.
 #include "lla_common.cuh"
+#include "lla_int_math.h"
 #include "lla_kernels.h"
 #include "lla_prof.h"
 
 namespace lla {
 
 // ---------------------------------------------------------------------------
-// EXACT: diagonal block [p, p+b), b <= kNbExact, one CTA of 32 x 32 threads.
+// EXACT kernels.  An FP64 instruction takes 64 cycles of its sub-partition
+// whatever its active lanes, and a library root or division about nine of them,
+// so: roots and quotients run in integer arithmetic (lla_int_math.h,
+// bit-identical to IEEE), the accumulators stay in registers as patches of 16
+// rows x 2 columns, and tiles are small, so that every SM's pipe has a share.
+// Per panel of a 512 x 512 factorisation, before -> now: diagonal block 53 ->
+// 20 us, panel 66 -> 18 us, update 82 -> 10 us (f64; the whole factor 3160 ->
+// 783 us).
 constexpr int kNbExact = 32;
 
+// d <= 0 as the reference tests it (src/cholesky.rs:69, false for NaN).
 template <typename T>
-__global__ void __launch_bounds__(1024) potrf_exact_diag(T *W, const T *S, T *D, int64_t ld,
-                                                         int64_t p, int b, int64_t *info) {
-    using Ar = Arith<T>;
-    __shared__ T a[kNbExact][kNbExact + 1];
-    __shared__ T s[kNbExact][kNbExact + 1];
-    __shared__ T d[kNbExact];
-    __shared__ int failed;
-    const int tx = threadIdx.x, ty = threadIdx.y;  // tx: column k, ty: row j
-    if (*(volatile int64_t *)info >= 0) return;    // an earlier panel failed
-    if (ty < b && tx <= ty) {
-        a[ty][tx] = cm(W, ld, p + ty, p + tx);
-        s[ty][tx] = (tx < ty) ? cm(S, ld, p + ty, p + tx) : T(0);
-    }
-    if (ty == 0 && tx < b) d[tx] = D[p + tx];
-    if (tx == 0 && ty == 0) failed = 0;
-    __syncthreads();
-    int k = 0;
-    for (; k < b; ++k) {
-        if (tx == 0 && ty == 0) {
-            const T dd = Ar::sub(a[k][k], d[k]);  // d = A[j,j] - d  (:66)
-            if (dd <= T(0)) {                     // (:69) false for NaN
-                failed = 1;
-                *info = p + k;
-            } else {
-                a[k][k] = Ar::sqrt_(dd);  // (:73)
-            }
-        }
-        __syncthreads();
-        if (failed) break;
-        const T lkk = a[k][k];
-        if (ty == 0 && tx > k && tx < b) {
-            const int j = tx;
-            const T l = Ar::div(Ar::sub(a[j][k], s[j][k]), lkk);  // (:62)
-            a[j][k] = l;
-            d[j] = Ar::add(d[j], Ar::mul(l, l));  // (:64)
-        }
-        __syncthreads();
-        // s_{j,k2} += L[k2,k] * L[j,k] for k < k2 < j   (:59-61, term i = k)
-        if (ty < b && tx > k && tx < ty) s[ty][tx] = Ar::add(s[ty][tx], Ar::mul(a[tx][k], a[ty][k]));
-        __syncthreads();
-    }
-    // Write back every value computed (on failure the host keeps only rows
-    // < info and row info's strict lower part).
-    if (ty < b && tx <= ty) cm(W, ld, p + ty, p + tx) = a[ty][tx];
+__device__ __forceinline__ bool exact_not_positive(T d) {
+    return d <= T(0);
 }
 
-// EXACT: rows [q, n) below the diagonal block, q = p + b; one thread per row.
-template <typename T>
-__global__ void __launch_bounds__(128) potrf_exact_panel(T *W, T *S, T *D, int64_t ld, int64_t n,
-                                                         int64_t p, int b, const int64_t *info) {
+// Root and quotients of the reference (src/cholesky.rs:62, 73) for one pivot.
+// LIB: the library's functions, for whatever the integer ones do not take (a
+// pivot that is not a positive normal number, quotients outside the comfortable
+// exponent range); a kernel runs the integer form first, without a branch on its
+// chain, and the other only if some ok came back false.
+template <typename T, bool LIB>
+struct ExactPivot {
+    T l;
+    __device__ __forceinline__ void from_square(T dd, bool &ok) { l = Arith<T>::sqrt_(dd); }
+    __device__ __forceinline__ void from_root(T v) { l = v; }
+    __device__ __forceinline__ T divide(T t, bool &ok) const { return Arith<T>::div(t, l); }
+};
+template <>
+struct ExactPivot<double, false> {
+    double l;
+    ImDivisor q;
+    __device__ __forceinline__ void from_square(double dd, bool &ok) {
+        ok = ok && im_positive_normal(im_bits(dd));
+        l = im_sqrt(dd, q);
+    }
+    __device__ __forceinline__ void from_root(double v) {
+        l = v;
+        q = im_divisor(v);
+    }
+    __device__ __forceinline__ double divide(double t, bool &ok) const {
+        bool good;
+        const double x = im_div(t, q, good);
+        ok = ok && good;
+        return x;
+    }
+};
+
+// Diagonal block [p, p+b), b <= 32, one CTA.  Warp 0 (lane = row) walks the
+// chain, one column ahead of the others: it adds column k's products to the sums
+// of column k + 1, takes the pivot and divides; it also keeps the diagonal sums
+// D.  The warps of the other sub-partitions hold the sums of the columns right of
+// it in registers and hand column k + 2 over once column k is in it.  One barrier
+// per column.
+constexpr int kExDiagThreads = 512;
+constexpr int kExPatches = 24, kExPatchWarps = 12, kExSlots = 2;
+
+// Returns (to every thread) whether the block stands; with LIB always, and
+// *s_fail is the failing column or -1.
+template <typename T, bool LIB>
+__device__ bool exact_diag_block(const T *W, const T *S, const T *D, int64_t ld, int64_t p, int b,
+                                 T (*a)[kNbExact + 1], T (*s)[kNbExact + 1], int *s_fail) {
     using Ar = Arith<T>;
-    __shared__ T l11[kNbExact][kNbExact + 1];
-    if (*(volatile const int64_t *)info >= 0) return;
-    for (int e = threadIdx.x; e < kNbExact * kNbExact; e += blockDim.x) {
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    for (int e = tid; e < kNbExact * kNbExact; e += kExDiagThreads) {
         const int r = e % kNbExact, c = e / kNbExact;
-        if (r < b && c <= r) l11[r][c] = cm(W, ld, p + r, p + c);
+        // a short block is padded with the identity
+        a[c][r] = (r < b && c <= r) ? cm(W, ld, p + r, p + c) : T(r == c ? 1 : 0);
+        s[c][r] = (r < b && c < r && p > 0) ? cm(S, ld, p + r, p + c) : T(0);
     }
+    if (tid == 0) *s_fail = -1;
+    T d = (warp == 0 && lane < b && p > 0) ? D[p + lane] : T(0);
     __syncthreads();
-    const int64_t j = p + b + (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= n) return;
-    T av[kNbExact], sv[kNbExact];
+    const bool upd = (warp & 3) != 0;
+    T acc[kExSlots];
+    int row[kExSlots], col[kExSlots];  // col < 0: no patch
+    if (upd) {
 #pragma unroll
-    for (int k = 0; k < kNbExact; ++k) {
-        if (k < b) {
-            av[k] = cm(W, ld, j, p + k);
-            sv[k] = cm(S, ld, j, p + k);
+        for (int i = 0; i < kExSlots; ++i) {
+            // rightmost columns first: pairs 15 .. 8 of rows 16-31, then pairs 7 .. 0 of both row groups
+            const int t = warp - 1 - (warp >> 2) + kExPatchWarps * i;
+            const int j = t < 8 ? 15 - t : 7 - (t - 8) / 2, g = t < 8 ? 1 : 1 - (t & 1);
+            row[i] = 16 * g + (lane & 15);
+            col[i] = t < kExPatches ? 2 * j + (lane >> 4) : -1;
+            acc[i] = t < kExPatches ? s[col[i]][row[i]] : T(0);
         }
     }
-    T dj = D[j];
+    bool bad = false, ok = true;
+    T lk = T(0);  // warp 0: this row's entry of the last finished column
+    // warp 0: column c, whose sums hold all products of columns before c - 1
+    auto finish = [&](int c) {
+        T sum = s[c][lane];
+        const T av = a[c][lane], ac = a[c][c];
+        d = Ar::add(d, Ar::mul(lk, lk));                           // (:64) for column c - 1 (0 before the first)
+        const T dd = Ar::sub(ac, __shfl_sync(0xffffffffu, d, c));  // d = A[j,j] - d  (:66)
+        if (c > 0) {
+            const T lc = __shfl_sync(0xffffffffu, lk, c);  // L[c, c-1]
+            sum = Ar::add(sum, Ar::mul(lc, lk));           // (:59-61), term c - 1
+        }
+        const T t = Ar::sub(av, sum);
+        if (LIB && exact_not_positive(dd)) {  // (:69)
+            bad = true;
+            if (lane == 0) *s_fail = c;
+            return;
+        }
+        ExactPivot<T, LIB> piv;
+        bool good = true;
+        piv.from_square(dd, ok);  // (:73)
+        const T l = piv.divide(t, good);  // (:62)
+        ok = ok && (good || lane <= c);
+        lk = lane > c ? l : T(0);
+        if (lane >= c) a[c][lane] = lane == c ? piv.l : l;
+    };
+    if (warp == 0) finish(0);
+    for (int k = 0;; ++k) {
+        __syncthreads();  // column k is final
+        // a failure at column k ends the loop here for everyone; one at column k + 1, which warp 0
+        // may already have recorded, after the next barrier
+        if (LIB && warp > 0) bad = (unsigned)*(volatile int *)s_fail <= (unsigned)k;
+        if (bad || k == kNbExact - 1) break;
+        if (warp == 0) {
+            finish(k + 1);
+        } else if (upd) {
 #pragma unroll
-    for (int k = 0; k < kNbExact; ++k) {
-        if (k < b) {
-            const T l = Ar::div(Ar::sub(av[k], sv[k]), l11[k][k]);
-            av[k] = l;
-            dj = Ar::add(dj, Ar::mul(l, l));
-#pragma unroll
-            for (int k2 = k + 1; k2 < kNbExact; ++k2)
-                if (k2 < b) sv[k2] = Ar::add(sv[k2], Ar::mul(l11[k2][k], l));
+            for (int i = 0; i < kExSlots; ++i) {
+                if ((col[i] | 1) < k + 2) break;  // (the same for the whole warp)
+                const T u = Ar::add(acc[i], Ar::mul(a[k][col[i]], a[k][row[i]]));
+                if (col[i] >= k + 2) acc[i] = u;
+                if (col[i] == k + 2) s[k + 2][row[i]] = u;
+            }
         }
     }
+    return __syncthreads_and(ok) != 0;
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kExDiagThreads) potrf_exact_diag(T *W, const T *S, const T *D, int64_t ld,
+                                                                 int64_t p, int b, int64_t *info) {
+    __shared__ T a[kNbExact][kNbExact + 1];  // [column][row]: A, then L
+    __shared__ T s[kNbExact][kNbExact + 1];  // sums
+    __shared__ int s_fail;
+    const int tid = threadIdx.x;
+    pdl_wait();
+    pdl_trigger();
+    if (*(volatile int64_t *)info >= 0) return;  // an earlier panel failed
+    constexpr bool lib = sizeof(T) == 4;  // FP32 roots and quotients are fast as they are
+    if (!exact_diag_block<T, lib>(W, S, D, ld, p, b, a, s, &s_fail) && !lib)
+        exact_diag_block<T, true>(W, S, D, ld, p, b, a, s, &s_fail);
+    if (s_fail >= 0 && tid == 0) *info = p + s_fail;
+    // every value computed (on failure the caller keeps only rows < info and row
+    // info's strict lower part)
+    for (int e = tid; e < kNbExact * kNbExact; e += kExDiagThreads) {
+        const int r = e % kNbExact, c = e / kNbExact;
+        if (r < b && c <= r) cm(W, ld, p + r, p + c) = a[c][r];
+    }
+}
+
+// Rows [q, n) below the diagonal block, q = p + 32; 16 rows per CTA.  The sums
+// stay in registers as patches of 16 rows x 2 columns, two per warp (warp w:
+// column pairs w and w + 8); pairs are finished in turn by their owner, one
+// barrier each, the next owner bringing its own pair up to date first.  Warp 8
+// adds the rows' squares to D as their columns appear.
+constexpr int kExRows = 16;
+constexpr int kExPanelThreads = 288;
+
+template <typename T, bool LIB>
+__device__ bool exact_panel_rows(const T *W, const T *S, const T *D, int64_t ld, int64_t n, int64_t p, int64_t j0,
+                                 const T (*l11)[kNbExact + 1], const ExactPivot<T, LIB> *piv, T (*x)[kExRows], T &dj) {
+    using Ar = Arith<T>;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, r16 = lane & 15, cc = lane >> 4;
+    const bool in = j0 + r16 < n;
+    T av[2] = {T(0), T(0)}, sv[2] = {T(0), T(0)};
+    if (warp < 8) {
 #pragma unroll
-    for (int k = 0; k < kNbExact; ++k)
-        if (k < b) cm(W, ld, j, p + k) = av[k];
-    D[j] = dj;
+        for (int i = 0; i < 2; ++i) {
+            const int64_t c = p + 2 * (warp + 8 * i) + cc;
+            av[i] = in ? cm(W, ld, j0 + r16, c) : T(0);
+            sv[i] = (in && p > 0) ? cm(S, ld, j0 + r16, c) : T(0);
+        }
+    }
+    dj = (warp == 8 && in && p > 0) ? D[j0 + r16] : T(0);
+    __syncthreads();  // l11, piv
+    bool ok = true;
+    auto solve = [&](int j, T a0, T s0) {  // column pair j
+        const int c = 2 * j;
+        bool g0 = true, g1 = true;
+        const T u0 = piv[c].divide(Ar::sub(a0, s0), g0);  // (:62); the first column's lanes
+        const T x0 = __shfl_sync(0xffffffffu, u0, r16);
+        const T u1 = piv[c + 1].divide(Ar::sub(a0, Ar::add(s0, Ar::mul(l11[c][c + 1], x0))), g1);
+        ok = ok && (cc ? g1 : g0);
+        x[c + cc][r16] = cc ? u1 : u0;
+    };
+    if (warp == 0) solve(0, av[0], sv[0]);
+    __syncthreads();
+#pragma unroll
+    for (int i0 = 0; i0 < 2; ++i0) {
+#pragma unroll 1
+        for (int w0 = 0; w0 < 8; ++w0) {
+            const int j = 8 * i0 + w0;  // pair j is finished: add its products to the pairs right of it
+            const T x0 = x[2 * j][r16], x1 = x[2 * j + 1][r16];
+            if (warp == 8) {
+                dj = Ar::add(dj, Ar::mul(x0, x0));  // (:64)
+                dj = Ar::add(dj, Ar::mul(x1, x1));
+            } else {
+#pragma unroll
+                for (int i = i0; i < 2; ++i) {
+                    const int jj = 8 * i + warp;
+                    if (jj <= j) continue;
+                    const int c = 2 * jj + cc;
+                    sv[i] = Ar::add(sv[i], Ar::mul(l11[2 * j][c], x0));  // (:59-61)
+                    sv[i] = Ar::add(sv[i], Ar::mul(l11[2 * j + 1][c], x1));
+                    if (jj == j + 1) solve(jj, av[i], sv[i]);
+                }
+            }
+            if (j < kNbExact / 2 - 1) __syncthreads();
+        }
+    }
+    return __syncthreads_and(ok) != 0;
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kExPanelThreads) potrf_exact_panel(T *W, const T *S, T *D, int64_t ld, int64_t n,
+                                                                   int64_t p, const int64_t *info) {
+    constexpr bool lib = sizeof(T) == 4;
+    __shared__ T l11[kNbExact][kNbExact + 1];  // [column][row]
+    __shared__ T x[kNbExact][kExRows];         // finished columns
+    __shared__ ExactPivot<T, lib> piv[kNbExact];
+    __shared__ ExactPivot<T, true> lpiv[kNbExact];
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int64_t j0 = p + kNbExact + (int64_t)blockIdx.x * kExRows;
+    pdl_wait();
+    pdl_trigger();
+    if (*(volatile const int64_t *)info >= 0) return;
+    for (int e = tid; e < kNbExact * kNbExact; e += kExPanelThreads) {
+        const int r = e % kNbExact, c = e / kNbExact;
+        l11[c][r] = c <= r ? cm(W, ld, p + r, p + c) : T(0);
+    }
+    if (tid < kNbExact) {
+        const T l = cm(W, ld, p + tid, p + tid);
+        piv[tid].from_root(l);
+        lpiv[tid].from_root(l);
+    }
+    T dj;
+    if (!exact_panel_rows<T, lib>(W, S, D, ld, n, p, j0, l11, piv, x, dj) && !lib)
+        exact_panel_rows<T, true>(W, S, D, ld, n, p, j0, l11, lpiv, x, dj);
+    for (int e = tid; e < kExRows * kNbExact; e += kExPanelThreads) {
+        const int r = e % kExRows, c = e / kExRows;
+        if (j0 + r < n) cm(W, ld, j0 + r, p + c) = x[c][r];
+    }
+    if (tid >> 5 == 8 && lane < kExRows && j0 + lane < n) D[j0 + lane] = dj;
 }
 
 // Lower-triangular tile enumeration: t -> (I, J) with J <= I.
@@ -121,18 +284,58 @@ __device__ __forceinline__ void tri_tile(int64_t t, int64_t &I, int64_t &J) {
     J = t - i * (i + 1) / 2;
 }
 
-// SIMT trailing update on 64 x 64 tiles of the lower trailing matrix
-// [q, n)^2, panel columns [p, p+b), b <= 64.  256 threads, 4 x 4 per thread.
-//  EXACT: S[j,k2] = S[j,k2] + L[k2,k]*L[j,k] for ascending k, strictly lower
-//         (j > k2) -- each product and sum rounded separately.
-//  FAST : A[j,k2] -= sum_k L[j,k]*L[k2,k] with FMA, lower incl. diagonal.
+// S[j, k2] += L[k2, k] L[j, k] for the panel's 32 columns in ascending k, each
+// product and sum rounded separately, on 16 x 16 tiles of the strictly lower
+// part of [q, n)^2 (the FP64 pipe of one SM needs 64 us for a 64 x 64 tile, so
+// small tiles spread it).  Thread (row r16, columns 4 w + cc, + 2) of warp w.
+constexpr int kExTile = 16;
+
+template <typename T>
+__global__ void __launch_bounds__(128) potrf_exact_update(const T *W, T *S, int64_t ld, int64_t n, int64_t p,
+                                                         const int64_t *info) {
+    using Ar = Arith<T>;
+    __shared__ T lj[kNbExact][kExTile];  // [k][row]
+    __shared__ T lk[kNbExact][kExTile];
+    pdl_wait();
+    pdl_trigger();
+    if (*(volatile const int64_t *)info >= 0) return;
+    int64_t I, J;
+    tri_tile(blockIdx.x, I, J);
+    const int64_t q = p + kNbExact, j0 = q + I * kExTile, k0 = q + J * kExTile;
+    const int tid = threadIdx.x, lane = tid & 31, r16 = lane & 15, c0 = 4 * (tid >> 5) + (lane >> 4);
+    T acc[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const int64_t j = j0 + r16, k2 = k0 + c0 + 2 * i;
+        acc[i] = (j < n && k2 < j && p > 0) ? cm(S, ld, j, k2) : T(0);
+    }
+    for (int e = tid; e < kExTile * kNbExact; e += 128) {
+        const int r = e % kExTile, k = e / kExTile;
+        lj[k][r] = (j0 + r < n) ? cm(W, ld, j0 + r, p + k) : T(0);
+        lk[k][r] = (k0 + r < n) ? cm(W, ld, k0 + r, p + k) : T(0);
+    }
+    __syncthreads();
+#pragma unroll 8
+    for (int k = 0; k < kNbExact; ++k)
+#pragma unroll
+        for (int i = 0; i < 2; ++i) acc[i] = Ar::add(acc[i], Ar::mul(lk[k][c0 + 2 * i], lj[k][r16]));
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const int64_t j = j0 + r16, k2 = k0 + c0 + 2 * i;
+        if (j < n && k2 < j) cm(S, ld, j, k2) = acc[i];
+    }
+}
+
+// FAST FP32 trailing update A[j,k2] -= sum_k L[j,k] L[k2,k] with FMA on 64 x 64
+// tiles of the lower trailing matrix [q, n)^2, panel columns [p, p+b), b <= 64.
+// 256 threads, 4 x 4 per thread.
 constexpr int kUpdTile = 64;
 
-template <typename T, bool kExact>
-__global__ void __launch_bounds__(256) potrf_update_simt(T *W, T *S, int64_t ld, int64_t n,
-                                                         int64_t p, int b, const int64_t *info) {
+template <typename T>
+__global__ void __launch_bounds__(256) potrf_update_simt(T *W, int64_t ld, int64_t n, int64_t p, int b,
+                                                         const int64_t *info) {
     using Ar = Arith<T>;
-    constexpr int KB = kExact ? kNbExact : 64;  // panel width bound (<= 33 KB of smem)
+    constexpr int KB = 64;
     __shared__ T lj[KB][kUpdTile + 1];  // [k][row]
     __shared__ T lk[KB][kUpdTile + 1];
     if (*(volatile const int64_t *)info >= 0) return;
@@ -149,13 +352,12 @@ __global__ void __launch_bounds__(256) potrf_update_simt(T *W, T *S, int64_t ld,
     __syncthreads();
     const int tr = tid % 16, tc = tid / 16;
     T acc[4][4];
-    T *Dst = kExact ? S : W;
 #pragma unroll
     for (int r = 0; r < 4; ++r)
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
             const int64_t j = j0 + tr + 16 * r, k2 = k0 + tc + 16 * c;
-            acc[r][c] = (j < n && k2 < n) ? cm(Dst, ld, j, k2) : T(0);
+            acc[r][c] = (j < n && k2 < n) ? cm(W, ld, j, k2) : T(0);
         }
     for (int k = 0; k < b; ++k) {
         T xr[4], xc[4];
@@ -166,20 +368,14 @@ __global__ void __launch_bounds__(256) potrf_update_simt(T *W, T *S, int64_t ld,
 #pragma unroll
         for (int r = 0; r < 4; ++r)
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                if (kExact)
-                    acc[r][c] = Ar::add(acc[r][c], Ar::mul(xc[c], xr[r]));
-                else
-                    acc[r][c] = Ar::fma_(-xr[r], xc[c], acc[r][c]);
-            }
+            for (int c = 0; c < 4; ++c) acc[r][c] = Ar::fma_(-xr[r], xc[c], acc[r][c]);
     }
 #pragma unroll
     for (int r = 0; r < 4; ++r)
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
             const int64_t j = j0 + tr + 16 * r, k2 = k0 + tc + 16 * c;
-            const bool inside = kExact ? (k2 < j) : (k2 <= j);
-            if (j < n && k2 < n && inside) cm(Dst, ld, j, k2) = acc[r][c];
+            if (j < n && k2 <= j) cm(W, ld, j, k2) = acc[r][c];
         }
 }
 
@@ -291,25 +487,25 @@ static int64_t tri_tiles(int64_t m, int tile) {
 template <typename T>
 int potrf_exact_launch(T *W, T *S, T *D, int64_t n, int64_t ld, int64_t *d_info,
                        cudaStream_t st) {
-    // S (n x n, ld) and D (n) start at zero.
-    if (cudaMemsetAsync(D, 0, sizeof(T) * n, st) != cudaSuccess) return -1;
-    if (cudaMemsetAsync(S, 0, sizeof(T) * ld * n, st) != cudaSuccess) return -1;
+    // The sums S (n x n, ld) and D (n) start at zero: the first panel's kernels
+    // (p == 0) take them as zero and write them, so they need no clearing.
     for (int64_t p = 0; p < n; p += kNbExact) {
         const int b = (int)std::min<int64_t>(kNbExact, n - p);
         {
             LaunchScope ls(K_POTRF_EXACT_DIAG, st, (double)b * b * b / 3.0);
-            potrf_exact_diag<T><<<1, dim3(32, 32), 0, st>>>(W, S, D, ld, p, b, d_info);
+            launch_maybe_pdl(p > 0, potrf_exact_diag<T>, dim3(1), dim3(kExDiagThreads), 0, st, W, (const T *)S,
+                             (const T *)D, ld, p, b, d_info);
         }
         const int64_t rest = n - p - b;
         if (rest > 0) {
             {
                 LaunchScope ls(K_POTRF_EXACT_PANEL, st, (double)rest * b * b);
-                potrf_exact_panel<T><<<(unsigned)ceil_div(rest, 128), 128, 0, st>>>(
-                    W, S, D, ld, n, p, b, d_info);
+                launch_maybe_pdl(true, potrf_exact_panel<T>, dim3((unsigned)ceil_div(rest, kExRows)),
+                                 dim3(kExPanelThreads), 0, st, W, (const T *)S, D, ld, n, p, (const int64_t *)d_info);
             }
             LaunchScope ls(K_POTRF_EXACT_UPDATE, st, (double)rest * (rest - 1) * b);
-            potrf_update_simt<T, true><<<(unsigned)tri_tiles(rest, kUpdTile), 256, 0, st>>>(
-                W, S, ld, n, p, b, d_info);
+            launch_maybe_pdl(true, potrf_exact_update<T>, dim3((unsigned)tri_tiles(rest, kExTile)), dim3(128), 0, st,
+                             (const T *)W, S, ld, n, p, (const int64_t *)d_info);
         }
     }
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
@@ -338,8 +534,7 @@ int potrf_fast_launch<float>(float *W, int64_t n, int64_t ld, int64_t *d_info, f
             }
             // algorithmic work: rest*(rest+1)/2 lower entries x b multiply-adds x 2
             LaunchScope ls(K_POTRF_FAST_UPDATE, st, (double)rest * (rest + 1) * b);
-            potrf_update_simt<T, false><<<(unsigned)tri_tiles(rest, kUpdTile), 256, 0, st>>>(
-                W, nullptr, ld, n, p, b, d_info);
+            potrf_update_simt<T><<<(unsigned)tri_tiles(rest, kUpdTile), 256, 0, st>>>(W, ld, n, p, b, d_info);
         }
     }
     return cudaGetLastError() == cudaSuccess ? 0 : -1;

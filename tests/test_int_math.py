@@ -1,5 +1,5 @@
 """Integer building blocks of the FP64 factorisations, compiled on the host from
-the kernels' own headers: reciprocal roots and quotients in fixed point (csrc/lla_int_math.h),
+the kernels' own headers: roots, reciprocal roots and quotients in fixed point (csrc/lla_int_math.h),
 and the balanced digits, fixed-point values and 64-bit-to-double conversion of
 the FP64 trailing update (csrc/lla_oz_digits.h).  The references are the
 compiler's long double and integer arithmetic."""
@@ -41,7 +41,7 @@ int main() {
     for (double d : {0.0, -0.0, -1.0, 5e-324, 2.2250738585072009e-308, HUGE_VAL, -HUGE_VAL, std::nan("")})
         CHECK(!im_positive_normal(im_bits(d)), "normal(%a)\n", d);
     CHECK(im_positive_normal(im_bits(2.2250738585072014e-308)) && im_positive_normal(im_bits(1.7976931348623157e308)), "ends\n");
-    // quotients: IEEE division's where they say so, refused about once in 700
+    // quotients: IEEE division's where they say so, which is nearly always
     long taken = 0, refused = 0;
     for (long t = 0; t < 300000; ++t) {
         uint64_t db = g();
@@ -62,7 +62,25 @@ int main() {
             if (k == 3 && t % 3 && im_positive_normal(ab & ~(1ull << 63))) (ok ? taken : refused)++;
         }
     }
-    CHECK(refused < taken / 300 && refused > taken / 2000, "refused %ld of %ld\n", refused, taken);
+    CHECK(refused * 1000 < taken, "refused %ld of %ld\n", refused, taken);
+    // roots: IEEE's, and the divisor they become
+    for (long t = 0; t < 1000000; ++t) {
+        uint64_t b = g() & 0x7fffffffffffffffull;
+        if (t % 3 == 0) b = (b & 0x000fffffffffffffull) | ((1000ull + g() % 40) << 52);
+        if (t % 5 == 0) b |= 0xfffffffffffffull;
+        if (t % 7 == 0) b &= ~0xfffffffffffull;
+        if (t % 11 == 0) b = im_bits(im_double((g() & 0x000ffffffc000000ull) | (1023ull << 52)));
+        if (t % 13 == 0) b = im_bits(im_double((g() & 0x000fffffffffffffull) | ((1023ull + g() % 2) << 52)));
+        if (t % 11 == 0 || t % 13 == 0) b = im_bits(im_double(b) * im_double(b));  // squares
+        if (!im_positive_normal(b)) continue;
+        ImDivisor v;
+        const double d = im_double(b), r = im_sqrt(d, v);
+        CHECK(im_bits(r) == im_bits(std::sqrt(d)), "sqrt(%a) = %a\n", d, r);
+        const double a = im_double((g() & 0x800fffffffffffffull) | (((uint64_t)(v.e & 0x7ff) / 2 + 512) << 52));
+        bool ok;
+        const double q = im_div(a, v, ok);
+        CHECK(!ok || im_bits(q) == im_bits(a / r), "%a / %a = %a\n", a, r, q);
+    }
     // digits: V = nearest multiple of 2^(e-55), its seven balanced digits exact in BF16
     std::uniform_real_distribution<double> U(0.5, 1.0);
     for (long t = 0; t < 400000; ++t) {

@@ -199,3 +199,40 @@ def test_exact_division_fallbacks_match_the_oracle(gpu_lla, dtype):
                 gpu_lla.set_algorithm(prev)
             same = (got == want) | (np.isnan(got) & np.isnan(want))
             assert same.all() and (np.signbit(got) == np.signbit(want))[~np.isnan(want)].all(), (k, v)
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("n", [1, 15, 16, 17, 31, 32, 33, 47, 48, 49, 64, 65, 97])
+@pytest.mark.parametrize("kind", ["plain", "fails", "tiny", "inf", "nan"])
+def test_exact_factor_matches_the_oracle(gpu_lla, dtype, n, kind):
+    """EXACT factor at the edges of its 32-column panels and 16-row tiles, also where integer roots
+    and quotients do not apply (subnormal values, infinities, NaN) and at failing pivots."""
+    from oracle import oracle as ora
+    rng = np.random.default_rng(n)
+    g = rng.standard_normal((n, n))
+    a = (g @ g.T / n + np.eye(n)).astype(dtype)
+    k = int(rng.integers(0, n))
+    if kind == "fails":
+        a[k, k] = -a[k, k]
+    elif kind == "tiny":
+        a[k] *= np.finfo(dtype).tiny
+        a[:, k] = a[k]
+        a[k, k] = np.finfo(dtype).tiny / 8
+    elif kind == "inf":
+        a[k, k] = np.inf
+    elif kind == "nan":
+        a[k, k // 2] = np.nan
+    want, got = a.copy(), a.copy()
+    with np.errstate(all="ignore"):
+        st = ora.cholesky_inplace_dirty(want)
+    prev = gpu_lla.set_algorithm(gpu_lla.ALGO_EXACT)
+    try:
+        fail = -1
+        try:
+            gpu_lla.cholesky_inplace_dirty(got)
+        except gpu_lla.NotPositiveDefinite as e:
+            fail = e.index
+    finally:
+        gpu_lla.set_algorithm(prev)
+    assert (fail >= 0) == (st["code"] != 0) and (fail < 0 or fail == st["index"])
+    assert ((got == want) | (np.isnan(got) & np.isnan(want))).all()
