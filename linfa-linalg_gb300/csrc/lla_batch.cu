@@ -32,7 +32,9 @@
 #include "../../include/lla_gb300.h"
 #include "lla_autotune.h"
 #include "lla_common.cuh"
+#include "lla_int_math.h"
 #include "lla_kernels.h"
+#include "lla_oz_digits.h"
 #include "lla_prof.h"
 
 namespace lla {
@@ -46,111 +48,409 @@ __device__ __forceinline__ T shfl(T v, int src) {
     return __shfl_sync(0xffffffffu, v, src);
 }
 
-// One warp: Cholesky of the bs x bs block at sD (row-major [32][33] in shared
-// memory); returns the first failing local row or -1.  Lane i holds row i.
+// Shared memory of one CTA.
+//  dg   : diagonal block, dg[c * kBDs + r] = L[r][c] while factoring (and its
+//         transpose in the backward pass), identity-padded;
+//  rinv : reciprocals of L's diagonal, all n;
+//  rhs  : right-hand sides as extra rows, rhs[k * kBMaxN + i];
+//  panel: FP32: the finished panel rows, panel[c * kBPs + r]; FP64: their digits,
+//         panel[(d * kBRows + r) * 32 + k], and expo[r], the rows' exponents.
+constexpr int kBDs = 36;                     // 16-byte rows in both types
+constexpr int kBRows = kBMaxN - kBNb + 16;   // FP64 panel rows: trailing and right-hand sides, to whole 16-row tiles
+constexpr int kBPs = kBMaxN + 4;             // FP32: to whole 32-row tiles
+static_assert(kBMaxN - kBNb + kBMaxRhs <= kBRows && kBRows <= kBMaxN, "panel rows");
+constexpr int kBNonFinite = 1 << 20;
 template <typename T>
-__device__ int warp_potrf32(T *sD, int bs, int lane) {
-    T v[32];
+struct BatchSmem {
+    T dg[kBNb * kBDs];
+    T rinv[kBMaxN];
+    T rhs[kBMaxRhs * kBMaxN];
+    T piv[kBNb];
+    int expo[kBRows];
+    int fail;
+    alignas(16) unsigned char panel[sizeof(T) == 4 ? 4 * kBNb * kBPs : kOzBal * kBRows * kBNb];
+};
+
+// 1 / sqrt(d), d positive and normal: FP32 approximation and one Newton step;
+// FP64 in fixed point (lla_int_math.h).
+__device__ __forceinline__ float batch_rsqrt(float d) {
+    const float y = im_rsqrt_seed(d);
+    return fmaf(0.5f * y, fmaf(-d * y, y, 1.f), y);
+}
+__device__ __forceinline__ bool batch_normal(float d) { return d >= 1.1754944e-38f && d <= 3.4028235e38f; }
+
+// Factors the identity-padded 32 x 32 block in sm.dg; sm.rinv[kb ..] receives the
+// reciprocal pivots, the block L with its exact roots.  sm.fail: failing column.
+// FP32: one warp, a row a lane, shuffles.
+__device__ void batch_diag(BatchSmem<float> &sm, int kb, int bs) {
+    const int lane = threadIdx.x & 31;
+    if (threadIdx.x < 32) {
+        float v[32], dk = 1.f;
 #pragma unroll
-    for (int c = 0; c < 32; ++c) v[c] = (lane < bs && c <= lane) ? sD[lane * 33 + c] : T(0);
-    int fail = -1;
+        for (int c = 0; c < 32; ++c) v[c] = sm.dg[c * kBDs + lane];
+        int fail = -1;
 #pragma unroll
-    for (int c = 0; c < 32; ++c) {
-        if (c < bs && fail < 0) {
-            const T piv = shfl(v[c], c);
-            if (!(piv > T(0))) {
-                fail = c;  // non-positive pivot (NaN does not fail, as in the reference: `d <= 0`)
-                if (piv != piv) fail = -1;
+        for (int c = 0; c < 32; ++c) {
+            const float d = shfl(v[c], c);
+            float y = batch_rsqrt(d);
+            if (!batch_normal(d)) {  // (uniform) not positive (NaN does not fail, as in the reference: `d <= 0`), or special
+                if (d <= 0.f && fail < 0) fail = c;
+                y = 1.f / sqrtf(d);
             }
-            if (fail < 0) {
-                const T lcc = sqrt(piv);
-                if (lane == c) v[c] = lcc;
-                if (lane > c) v[c] = v[c] / lcc;
+            if (lane == c) {
+                dk = d;
+                sm.rinv[kb + c] = y;
+            }
+            v[c] *= y;
 #pragma unroll
-                for (int c2 = c + 1; c2 < 32; ++c2) {
-                    const T t = shfl(v[c], c2);
-                    if (c2 < bs && lane >= c2) v[c2] = fma(-v[c], t, v[c2]);
-                }
+            for (int c2 = c + 1; c2 < 32; ++c2) v[c2] = fmaf(-v[c], shfl(v[c], c2), v[c2]);
+        }
+#pragma unroll
+        for (int c = 0; c < 32; ++c)
+            if (c <= lane) sm.dg[c * kBDs + lane] = c == lane ? sqrtf(dk) : v[c];
+        if (lane == 0 && fail >= 0) sm.fail = kb + fail;
+    }
+    __syncthreads();
+}
+
+// FP64: an FP64 instruction takes 64 cycles of its sub-partition, so the block is
+// shared out: warp 0 walks the pivots, a pair of columns at a time and one pair
+// ahead, and the warps of the other sub-partitions apply the finished pairs to the
+// rest in patches of 16 rows x 2 columns.
+__device__ void batch_diag(BatchSmem<double> &sm, int kb, int bs) {
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    double *a = sm.dg;
+    auto pivots = [&](int c) {
+        double u = a[c * kBDs + lane], v = a[(c + 1) * kBDs + lane];
+        if (c > 0) {
+            const double *x0 = a + (c - 2) * kBDs, *x1 = a + (c - 1) * kBDs;
+            u = fma(-x1[lane], x1[c], fma(-x0[lane], x0[c], u));
+            v = fma(-x1[lane], x1[c + 1], fma(-x0[lane], x0[c + 1], v));
+        }
+        const double su = u, sv = v;
+        const double d0 = shfl(u, c);
+        double y0 = im_rsqrt(d0);
+        u *= y0;
+        v = fma(-u, shfl(u, c + 1), v);
+        double d1 = shfl(v, c + 1);
+        double y1 = im_rsqrt(d1);
+        v *= y1;
+        if (!im_positive_normal(im_bits(d0)) || !im_positive_normal(im_bits(d1))) {  // not positive, or special
+            int fail = d0 <= 0.0 ? c : -1;
+            y0 = 1.0 / sqrt(d0);
+            u = su * y0;
+            v = fma(-u, shfl(u, c + 1), sv);
+            d1 = shfl(v, c + 1);
+            if (d1 <= 0.0 && fail < 0) fail = c + 1;
+            y1 = 1.0 / sqrt(d1);
+            v *= y1;
+            if (lane == 0 && fail >= 0 && sm.fail < 0) sm.fail = kb + fail;
+        }
+        sm.piv[c] = d0;  // (every lane writes the same value)
+        sm.piv[c + 1] = d1;
+        sm.rinv[kb + c] = y0;
+        sm.rinv[kb + c + 1] = y1;
+        a[c * kBDs + lane] = u;
+        a[(c + 1) * kBDs + lane] = v;
+    };
+    if (warp == 0) pivots(0);
+    const int npw = (blockDim.x >> 7) * 3, pw = warp - 1 - (warp >> 2);
+    for (int k = 0; k < 15; ++k) {
+        __syncthreads();  // pair k is final
+        if (warp == 0) {
+            pivots(2 * k + 2);
+        } else if (warp & 3) {
+            const double *x0 = a + 2 * k * kBDs, *x1 = x0 + kBDs;
+            for (int t = pw; t < 24; t += npw) {  // rightmost pairs first
+                const int j = t < 8 ? 15 - t : 7 - (t - 8) / 2, g = t < 8 ? 1 : 1 - (t & 1);
+                if (j < k + 2) break;
+                const int r = 16 * g + (lane & 15), c = 2 * j + (lane >> 4);
+                a[c * kBDs + r] = fma(-x1[r], x1[c], fma(-x0[r], x0[c], a[c * kBDs + r]));
             }
         }
     }
-    if (lane < bs) {
+    __syncthreads();
+    if (tid < 32) a[tid * kBDs + tid] = sqrt(sm.piv[tid]);
+    __syncthreads();
+}
+
+// Trailing update of rows rr (0 .. rows - 1: trailing rows q + rr; rows .. rows +
+// m - 1: right-hand sides) and columns j < rows, j <= rr, from the panel.
+// FP32: warp tiles of 32 x 32, a thread 4 rows (stride 8) x 8 columns.
+__device__ void batch_update(BatchSmem<float> &sm, float *A, int n, int q, int kb, int rows, int m) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+    const float *P = reinterpret_cast<const float *>(sm.panel);
+    const int R = (rows + m + 31) / 32, C = (rows + 31) / 32;
+    const int lr = lane & 7, lc = (lane >> 3) * 8;
+    for (int t = warp; t < R * C; t += nw) {
+        const int I = t / C, J = t % C;
+        if (J > I) continue;
+        const int i0 = 32 * I + lr, j0 = 32 * J + lc;
+        float acc[4][8];
+        float *const Aq = A + q + (int64_t)(q + j0) * n;
 #pragma unroll
-        for (int c = 0; c < 32; ++c)
-            if (c <= lane) sD[lane * 33 + c] = v[c];
+        for (int u = 0; u < 4; ++u)
+#pragma unroll
+            for (int w = 0; w < 8; ++w) {
+                const int i = i0 + 8 * u, j = j0 + w;
+                acc[u][w] = 0.f;
+                if (j < rows && j <= i) {
+                    if (i < rows)
+                        acc[u][w] = Aq[i + w * n];
+                    else if (i < rows + m)
+                        acc[u][w] = sm.rhs[(i - rows) * kBMaxN + q + j];
+                }
+            }
+#pragma unroll 4
+        for (int k = 0; k < kBNb; ++k) {
+            float xr[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) xr[u] = P[k * kBPs + i0 + 8 * u];
+            const float4 c0 = *reinterpret_cast<const float4 *>(P + k * kBPs + j0);
+            const float4 c1 = *reinterpret_cast<const float4 *>(P + k * kBPs + j0 + 4);
+            const float xc[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+#pragma unroll
+                for (int w = 0; w < 8; ++w) acc[u][w] = fmaf(-xr[u], xc[w], acc[u][w]);
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+#pragma unroll
+            for (int w = 0; w < 8; ++w) {
+                const int i = i0 + 8 * u, j = j0 + w;
+                if (j < rows && j <= i) {
+                    if (i < rows)
+                        Aq[i + w * n] = acc[u][w];
+                    else if (i < rows + m)
+                        sm.rhs[(i - rows) * kBMaxN + q + j] = acc[u][w];
+                }
+            }
     }
+    __syncthreads();
+}
+
+// D (16 x 8, FP32) += A (16 x 16) B (16 x 8), FP16 operands.
+__device__ __forceinline__ void batch_mma(float (&d)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
+    asm volatile(
+        "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
+}
+// Four digits (bytes, biased by 128) as two pairs of FP16: 0x64xx is 1024 + xx.
+__device__ __forceinline__ void batch_digits(uint32_t w, uint32_t &lo, uint32_t &hi) {
+    const uint32_t a = __byte_perm(w, 0x64646464u, 0x4140), b = __byte_perm(w, 0x64646464u, 0x4342);
+    const uint32_t bias = 0x64806480u;  // 1152, 1152
+    asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(lo) : "r"(a), "r"(bias));
+    asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(hi) : "r"(b), "r"(bias));
+}
+
+// FP64: the product of the 32 panel columns on the tensor cores, from seven
+// balanced 8-bit digits per entry (exact in FP16, their products' sums exact in
+// the FP32 accumulators), one 64-bit integer per entry and one FP64 subtraction,
+// where FMAs would spend 32 FP64 instructions per entry (lla_fp64_chol.cu has the
+// scheme and its error).  Warp tiles of 16 x 8, K = 32 in two steps; the digits'
+// k order is permuted alike in both operands so that a thread's four are one word.
+__device__ void batch_update(BatchSmem<double> &sm, double *A, int n, int q, int kb, int rows, int m) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+    const int g = lane >> 2, t4 = lane & 3;
+    const int R = (rows + m + 15) / 16, C = (rows + 7) / 8;
+    for (int t = warp; t < R * C; t += nw) {
+        const int I = t / C, J = t % C;
+        if (8 * J > 16 * I + 15) continue;
+        const int i0 = 16 * I, j0 = 8 * J;
+        float acc[kOzBal][4];
+#pragma unroll
+        for (int l = 0; l < kOzBal; ++l)
+#pragma unroll
+            for (int u = 0; u < 4; ++u) acc[l][u] = 0.f;
+#pragma unroll
+        for (int ks = 0; ks < 2; ++ks) {
+            uint32_t fb[kOzBal][2];
+#pragma unroll
+            for (int d = 0; d < kOzBal; ++d)
+                batch_digits(*reinterpret_cast<const uint32_t *>(sm.panel + (d * kBRows + j0 + g) * kBNb + 8 * t4 + 4 * ks),
+                             fb[d][0], fb[d][1]);
+#pragma unroll
+            for (int d = 0; d < kOzBal; ++d) {
+                uint32_t fa[4];
+                const unsigned char *pa = sm.panel + (d * kBRows + i0 + g) * kBNb + 8 * t4 + 4 * ks;
+                batch_digits(*reinterpret_cast<const uint32_t *>(pa), fa[0], fa[2]);
+                batch_digits(*reinterpret_cast<const uint32_t *>(pa + 8 * kBNb), fa[1], fa[3]);
+#pragma unroll
+                for (int e = 0; e < kOzBal - d; ++e) batch_mma(acc[d + e], fa, fb[e]);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int i = i0 + g + 8 * (u >> 1), j = j0 + 2 * t4 + (u & 1);
+            if (j >= rows || j > i || i >= rows + m) continue;
+            double *w = i < rows ? &A[(q + i) + (int64_t)(q + j) * n] : &sm.rhs[(i - rows) * kBMaxN + q + j];
+            const int ei = sm.expo[i], ej = sm.expo[j];
+            if (ei == kBNonFinite || ej == kBNonFinite) {  // no digits: the FMA chain on the factor itself
+                double s = *w;
+                for (int k = 0; k < kBNb; ++k)
+                    s = fma(-(i < rows ? A[(q + i) + (int64_t)(kb + k) * n] : sm.rhs[(i - rows) * kBMaxN + kb + k]),
+                            A[(q + j) + (int64_t)(kb + k) * n], s);
+                *w = s;
+                continue;
+            }
+            long long lo = 128, hi = 0;
+#pragma unroll
+            for (int l = 4; l < kOzBal; ++l) lo += (long long)__float2int_rn(acc[l][u]) * (1 << (8 * (6 - l)));
+#pragma unroll
+            for (int l = 0; l < 4; ++l) hi += (long long)__float2int_rn(acc[l][u]) * (1 << (8 * (3 - l)));
+            *w -= oz_scaled_double(hi * 65536 + (lo >> 8), ei + ej - 54);
+        }
+    }
+    __syncthreads();
+}
+
+// Keeps a finished panel row (thread rr) for the update.
+__device__ __forceinline__ void batch_keep_row(BatchSmem<float> &sm, int rr, const float (&v)[kBNb]) {
+    float *P = reinterpret_cast<float *>(sm.panel);
+#pragma unroll
+    for (int c = 0; c < kBNb; ++c) P[c * kBPs + rr] = v[c];
+}
+__device__ __forceinline__ void batch_keep_row(BatchSmem<double> &sm, int rr, const double (&v)[kBNb]) {
+    uint64_t mx = 0;
+#pragma unroll
+    for (int c = 0; c < kBNb; ++c) {
+        const uint64_t b = im_bits(v[c]) & 0x7fffffffffffffffull;
+        mx = b > mx ? b : mx;
+    }
+    // one bit of headroom, so that the leading digit fits a byte as well
+    const bool fin = mx < 0x7ff0000000000000ull;
+    const int e = fin ? oz_bits_exponent(mx) + 1 : kBNonFinite;
+    sm.expo[rr] = e;
+    // words of four digits: k = 2 t, 2 t + 1, 2 t + 8, 2 t + 9 of step ks at byte 8 t + 4 ks
+#pragma unroll
+    for (int t = 0; t < 4; ++t) {
+        uint32_t w[2][kOzBal];
+#pragma unroll
+        for (int ks = 0; ks < 2; ++ks) {
+            uint64_t x[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int k = 16 * ks + 2 * t + (u & 1) + 8 * (u >> 1);
+                x[u] = (fin ? (uint64_t)oz_fixed55((int64_t)im_bits(v[k]), e) : 0ull) + 0x0080808080808080ull;
+            }
+#pragma unroll
+            for (int d = 0; d < kOzBal; ++d) {
+                const int s = 8 * (kOzBal - 1 - d);
+                w[ks][d] = (uint32_t)(x[0] >> s & 255) | (uint32_t)(x[1] >> s & 255) << 8 |
+                           (uint32_t)(x[2] >> s & 255) << 16 | (uint32_t)(x[3] >> s & 255) << 24;
+            }
+        }
+#pragma unroll
+        for (int d = 0; d < kOzBal; ++d)
+            *reinterpret_cast<uint2 *>(sm.panel + (d * kBRows + rr) * kBNb + 8 * t) = make_uint2(w[0][d], w[1][d]);
+    }
+}
+
+// Factor of one system by the whole CTA: A (n x n, column-major, ld = n) in
+// place (L in the lower triangle), right-looking with 32-column blocks; the m
+// right-hand sides in sm.rhs are carried along as rows below A, which makes them
+// L^-1 B.  Returns the first failing row (non-positive pivot) or -1; every thread
+// returns the same value.
+template <typename T>
+__device__ int batch_factor(T *A, int n, int m, BatchSmem<T> &sm) {
+    const int tid = threadIdx.x, nthr = blockDim.x;
+    if (tid == 0) sm.fail = -1;
+    __syncthreads();
+    for (int kb = 0; kb < n; kb += kBNb) {
+        const int bs = min(kBNb, n - kb), q = kb + bs, rows = n - q;
+        for (int e = tid; e < kBNb * kBNb; e += nthr) {
+            const int r = e % kBNb, c = e / kBNb;
+            sm.dg[c * kBDs + r] = (r < bs && c <= r) ? A[(kb + r) + (int64_t)(kb + c) * n] : T(r == c ? 1 : 0);
+        }
+        // the rows below the block, one a thread, fetched while the block is factored
+        const int total = rows + m;
+        T v[kBNb];
+        auto fetch = [&](int rr) {
+#pragma unroll
+            for (int c = 0; c < kBNb; ++c)
+                v[c] = c < bs ? (rr < rows ? A[(q + rr) + (int64_t)(kb + c) * n] : sm.rhs[(rr - rows) * kBMaxN + kb + c])
+                              : T(0);
+        };
+        if (tid < total) fetch(tid);
+        __syncthreads();
+        batch_diag(sm, kb, bs);
+        if (sm.fail >= 0) break;
+        for (int e = tid; e < kBNb * kBNb; e += nthr) {
+            const int r = e % kBNb, c = e / kBNb;
+            if (r < bs && c <= r) A[(kb + r) + (int64_t)(kb + c) * n] = sm.dg[c * kBDs + r];
+        }
+        for (int rr = tid; rr < total; rr += nthr) {
+            if (rr != tid) fetch(rr);
+#pragma unroll
+            for (int c = 0; c < kBNb; ++c) {
+                v[c] *= c < bs ? sm.rinv[kb + c] : T(1);
+#pragma unroll
+                for (int c2 = c + 1; c2 < kBNb; ++c2) v[c2] = fma(-v[c], sm.dg[c * kBDs + c2], v[c2]);
+            }
+#pragma unroll
+            for (int c = 0; c < kBNb; ++c)
+                if (c < bs) {
+                    if (rr < rows)
+                        A[(q + rr) + (int64_t)(kb + c) * n] = v[c];
+                    else
+                        sm.rhs[(rr - rows) * kBMaxN + kb + c] = v[c];
+                }
+            if (rows > 0) batch_keep_row(sm, rr, v);
+        }
+        __syncthreads();
+        if (rows > 0) batch_update(sm, A, n, q, kb, rows, m);
+    }
+    const int fail = sm.fail;
+    __syncthreads();
     return fail;
 }
 
-// Factor-and-solve of one system by the whole CTA: A (n x n, column-major,
-// ld = n) is factored in place (L in the lower triangle), B (n x m, leading
-// dimension ldb) is overwritten with X.  sD: [32][33], sP: [kBMaxN][33] shared
-// scratch.  Returns the first failing row (non-positive pivot) or -1; every
-// thread returns the same value.
+// L^T X = Y in place on sm.rhs for the factor in the lower triangle of A (ld = n)
+// and sm.rinv: blocks from the last, one warp per right-hand side in the block,
+// one thread per remaining column after it.
 template <typename T>
-__device__ int batch_factor(T *A, int n, T *sD, T *sP, int *s_fail) {
-    const int tid = threadIdx.x, nthr = blockDim.x, warp = tid >> 5, lane = tid & 31;
-    const int nwarps = nthr >> 5;
-    if (tid == 0) *s_fail = -1;
-    __syncthreads();
-    // ---- factor: right-looking, 32-column blocks ----
-    for (int kb = 0; kb < n; kb += kBNb) {
+__device__ void batch_backward(const T *A, int n, int m, BatchSmem<T> &sm) {
+    const int tid = threadIdx.x, nthr = blockDim.x, warp = tid >> 5, lane = tid & 31, nw = nthr >> 5;
+    for (int kb = (n - 1) / kBNb * kBNb; kb >= 0; kb -= kBNb) {
         const int bs = min(kBNb, n - kb);
-        for (int e = tid; e < 32 * 32; e += nthr) {
-            const int r = e % 32, c = e / 32;
-            if (r < bs && c <= r) sD[r * 33 + c] = A[(kb + r) + (int64_t)(kb + c) * n];
+        for (int e = tid; e < kBNb * kBNb; e += nthr) {
+            const int r = e % kBNb, c = e / kBNb;
+            sm.dg[r * kBDs + c] = (r < bs && c < r) ? A[(kb + r) + (int64_t)(kb + c) * n] : T(0);
         }
+        // the block's rows of column tid, fetched while the block is solved
+        T v[kBNb];
+        auto fetch = [&](int j) {
+#pragma unroll
+            for (int t = 0; t < kBNb; ++t) v[t] = t < bs ? A[(kb + t) + (int64_t)j * n] : T(0);
+        };
+        if (tid < kb) fetch(tid);
         __syncthreads();
-        if (warp == 0) {
-            const int f = warp_potrf32(sD, bs, lane);
-            if (lane == 0 && f >= 0) *s_fail = kb + f;
-        }
-        __syncthreads();
-        if (*s_fail >= 0) break;
-        for (int e = tid; e < 32 * 32; e += nthr) {
-            const int r = e % 32, c = e / 32;
-            if (r < bs && c <= r) A[(kb + r) + (int64_t)(kb + c) * n] = sD[r * 33 + c];
-        }
-        // panel: each row below the block solves against L_kk
-        const int q = kb + bs, rows = n - q;
-        for (int rr = tid; rr < rows; rr += nthr) {
-            const int r = q + rr;
-            T v[32];
+        for (int k = warp; k < m; k += nw) {
+            T z = lane < bs ? sm.rhs[k * kBMaxN + kb + lane] : T(0);
+            const T ri = lane < bs ? sm.rinv[kb + lane] : T(0);
 #pragma unroll
-            for (int c = 0; c < 32; ++c) v[c] = (c < bs) ? A[r + (int64_t)(kb + c) * n] : T(0);
-#pragma unroll
-            for (int c = 0; c < 32; ++c) {
-                if (c < bs) {
-                    v[c] = v[c] / sD[c * 33 + c];
-#pragma unroll
-                    for (int c2 = c + 1; c2 < 32; ++c2)
-                        if (c2 < bs) v[c2] = fma(-v[c], sD[c2 * 33 + c], v[c2]);
-                }
+            for (int c = kBNb - 1; c >= 0; --c) {
+                const T x = shfl(z * ri, c);
+                const T w = fma(-x, sm.dg[c * kBDs + lane], z);
+                z = lane == c ? x : (lane < c ? w : z);
             }
-#pragma unroll
-            for (int c = 0; c < 32; ++c) {
-                if (c < bs) {
-                    sP[rr * 33 + c] = v[c];
-                    A[r + (int64_t)(kb + c) * n] = v[c];
-                }
-            }
+            if (lane < bs) sm.rhs[k * kBMaxN + kb + lane] = z;
         }
         __syncthreads();
-        // trailing lower triangle, one column per warp, lanes over rows:
-        // A[i,j] -= sum_t P[i][t] P[j][t]
-        for (int j = warp; j < rows; j += nwarps) {
-            for (int i = j + lane; i < rows; i += 32) {
-                T acc = A[(q + i) + (int64_t)(q + j) * n];
-#pragma unroll 8
-                for (int t = 0; t < bs; ++t) acc = fma(-sP[i * 33 + t], sP[j * 33 + t], acc);
-                A[(q + i) + (int64_t)(q + j) * n] = acc;
+        for (int j = tid; j < kb; j += nthr) {
+            if (j != tid) fetch(j);
+            for (int k = 0; k < m; ++k) {
+                T s = sm.rhs[k * kBMaxN + j];
+#pragma unroll
+                for (int t = 0; t < kBNb; ++t)
+                    if (t < bs) s = fma(-v[t], sm.rhs[k * kBMaxN + kb + t], s);
+                sm.rhs[k * kBMaxN + j] = s;
             }
         }
         __syncthreads();
     }
-    const int fail = *s_fail;
-    __syncthreads();
-    return fail;
 }
 
 // L L^T X = B in place for the factor in the lower triangle of A (ld = n).
@@ -219,11 +519,22 @@ __device__ void batch_trsolve(const T *A, int n, T *B, int64_t ldb, int m, T *sD
     }
 }
 
+// Factor-and-solve of one system by the whole CTA: B (n x m, leading dimension
+// ldb) is overwritten with X (untouched when the factorisation fails).
 template <typename T>
-__device__ int batch_solve_one(T *A, int n, T *B, int64_t ldb, int m, T *sD, T *sP, int *s_fail) {
-    const int f = batch_factor<T>(A, n, sD, sP, s_fail);
+__device__ int batch_solve_one(T *A, int n, T *B, int64_t ldb, int m, BatchSmem<T> &sm) {
+    for (int e = threadIdx.x; e < n * m; e += blockDim.x) {
+        const int i = e % n, k = e / n;
+        sm.rhs[k * kBMaxN + i] = B[i + (int64_t)k * ldb];
+    }
+    const int f = batch_factor<T>(A, n, m, sm);
     if (f >= 0) return f;
-    batch_trsolve<T>(A, n, B, ldb, m, sD, sP);
+    batch_backward<T>(A, n, m, sm);
+    for (int e = threadIdx.x; e < n * m; e += blockDim.x) {
+        const int i = e % n, k = e / n;
+        B[i + (int64_t)k * ldb] = sm.rhs[k * kBMaxN + i];
+    }
+    __syncthreads();
     return -1;
 }
 
@@ -231,9 +542,8 @@ template <typename T>
 __global__ void __launch_bounds__(256, 2) batch_posv_kernel(const BatchItem *__restrict__ items, int64_t count, T *Apool,
                                   T *Bpool, int32_t *info, int *counter) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    T *sD = (T *)smem_raw;  // [32][33] diagonal block
-    T *sP = sD + 32 * 33;   // [kBMaxN][33] panel / block rows (row r at sP[r * 33])
-    __shared__ int s_item, s_fail;
+    BatchSmem<T> &sm = *reinterpret_cast<BatchSmem<T> *>(smem_raw);
+    __shared__ int s_item;
     const int tid = threadIdx.x;
     for (;;) {
         if (tid == 0) s_item = atomicAdd(counter, 1);
@@ -241,7 +551,7 @@ __global__ void __launch_bounds__(256, 2) batch_posv_kernel(const BatchItem *__r
         const int64_t it = s_item;
         if (it >= count) break;
         const BatchItem w = items[it];
-        const int f = batch_solve_one<T>(Apool + w.a_off, w.n, Bpool + w.b_off, w.n, w.m, sD, sP, &s_fail);
+        const int f = batch_solve_one<T>(Apool + w.a_off, w.n, Bpool + w.b_off, w.n, w.m, sm);
         if (tid == 0) info[w.idx] = f;
         __syncthreads();
     }
@@ -265,6 +575,10 @@ constexpr int kBRefIters = 5;
 // Stop at n eps / 16 (about what the plain FP64 batched solve reaches); a
 // system left above 10 n eps is re-solved in plain FP64.
 constexpr double kBRefTolPerN = 2.220446049250313e-16 / 16.0;
+// Shared memory of the factorisations (FP32, or FP64 in the fallback) and of the
+// FP32 solves ([32][33] and [kBMaxN][33] floats).
+constexpr size_t kBRefSpace = (sizeof(BatchSmem<double>) + 15) / 16 * 16;
+static_assert(kBRefSpace >= sizeof(BatchSmem<float>) && kBRefSpace >= 4 * (32 * 33 + kBMaxN * 33), "one space for all");
 constexpr size_t kBRefScratch = (size_t)kBMaxN * kBMaxN * 8 + (size_t)kBMaxN * kBMaxRhs * (4 + 8);
 
 // Column maxima of |X| and |R| (m <= kBMaxRhs columns each) over the CTA in one
@@ -356,10 +670,11 @@ __global__ void __launch_bounds__(256, 2) batch_posv_refined_kernel(const BatchI
                                                                    const double *Apool, double *Bpool,
                                                                    int32_t *info, int *counter, char *scratch) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    double *sDd = (double *)smem_raw;  // FP64 fallback: [32][33] + [kBMaxN][33]
-    float *sDf = (float *)smem_raw;    // FP32 factor and solves (same space)
-    double *sX = (double *)(smem_raw + sizeof(double) * (32 * 33 + kBMaxN * 33));  // [kBMaxN][kBMaxRhs]
-    __shared__ int s_item, s_fail;
+    BatchSmem<double> &smd = *reinterpret_cast<BatchSmem<double> *>(smem_raw);  // FP64 fallback
+    BatchSmem<float> &smf = *reinterpret_cast<BatchSmem<float> *>(smem_raw);    // FP32 factor (same space)
+    float *sDf = (float *)smem_raw;                                             // FP32 solves (same space)
+    double *sX = (double *)(smem_raw + kBRefSpace);                             // [kBMaxN][kBMaxRhs]
+    __shared__ int s_item;
     __shared__ double red[8 * 2 * kBMaxRhs];
     __shared__ double s_cb[kBMaxRhs];
     const int tid = threadIdx.x, nthr = blockDim.x;
@@ -402,7 +717,7 @@ __global__ void __launch_bounds__(256, 2) batch_posv_refined_kernel(const BatchI
         }
         __syncthreads();
         const double tol = kBRefTolPerN * n;
-        int f = batch_factor<float>(W, n, sDf, sDf + 32 * 33, &s_fail);
+        int f = batch_factor<float>(W, n, 0, smf);
         bool ok = f < 0;
         if (ok) {
             for (int e = tid; e < n * kBMaxRhs; e += nthr) sX[e] = 0.0;
@@ -460,7 +775,7 @@ __global__ void __launch_bounds__(256, 2) batch_posv_refined_kernel(const BatchI
                 if (i >= k) Wd[e] = A[e];
             }
             __syncthreads();
-            f = batch_solve_one<double>(Wd, n, B, n, m, sDd, sDd + 32 * 33, &s_fail);
+            f = batch_solve_one<double>(Wd, n, B, n, m, smd);
         } else {
             f = -1;
         }
@@ -469,7 +784,7 @@ __global__ void __launch_bounds__(256, 2) batch_posv_refined_kernel(const BatchI
     }
 }
 
-size_t batch_refined_smem() { return sizeof(double) * (32 * 33 + kBMaxN * 33 + kBMaxN * kBMaxRhs); }
+size_t batch_refined_smem() { return kBRefSpace + sizeof(double) * kBMaxN * kBMaxRhs; }
 size_t batch_refined_scratch_bytes(int ctas) { return (size_t)ctas * kBRefScratch; }
 
 // ---------------------------------------------------------------------------
@@ -500,7 +815,6 @@ __global__ void __launch_bounds__(256) serve_loop_kernel(ServeRing *ring, unsign
                                                         double *scratch, unsigned long long idle_ns) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ long long s_ticket;
-    __shared__ int s_fail;
     __shared__ ServeReq s_req;
     const int tid = threadIdx.x;
     double *myA = scratch + (size_t)blockIdx.x * kBMaxN * kBMaxN;
@@ -551,8 +865,8 @@ __global__ void __launch_bounds__(256) serve_loop_kernel(ServeRing *ring, unsign
                 if (i >= j) W[e] = A[i + (int64_t)j * q.lda];
             }
             __syncthreads();
-            double *sD = (double *)smem_raw;
-            f = batch_solve_one<double>(W, n, (double *)q.B, q.ldb, q.m, sD, sD + 32 * 33, &s_fail);
+            f = batch_solve_one<double>(W, n, (double *)q.B, q.ldb, q.m,
+                                        *reinterpret_cast<BatchSmem<double> *>(smem_raw));
         } else {
             float *W = (float *)myA;
             const float *A = (const float *)q.A;
@@ -561,8 +875,8 @@ __global__ void __launch_bounds__(256) serve_loop_kernel(ServeRing *ring, unsign
                 if (i >= j) W[e] = A[i + (int64_t)j * q.lda];
             }
             __syncthreads();
-            float *sD = (float *)smem_raw;
-            f = batch_solve_one<float>(W, n, (float *)q.B, q.ldb, q.m, sD, sD + 32 * 33, &s_fail);
+            f = batch_solve_one<float>(W, n, (float *)q.B, q.ldb, q.m,
+                                       *reinterpret_cast<BatchSmem<float> *>(smem_raw));
         }
         __syncthreads();  // every thread's writes of X precede the publication
         if (tid == 0) {
@@ -579,7 +893,8 @@ size_t serve_loop_scratch_bytes(int ctas) { return (size_t)ctas * kBMaxN * kBMax
 
 int serve_loop_launch(ServeRing *ring_dev, unsigned long long *d_next, double *scratch, int ctas,
                       double idle_us, cudaStream_t st) {
-    const size_t smem = sizeof(double) * (32 * 33 + kBMaxN * 33);
+    const size_t smem = sizeof(BatchSmem<double>);
+    static_assert(sizeof(BatchSmem<double>) >= sizeof(BatchSmem<float>), "one space for both types");
     static bool attr = false;
     if (!attr) {
         if (cudaFuncSetAttribute(serve_loop_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
@@ -620,7 +935,7 @@ struct lla_batch_plan {
     cudaStream_t g_stream = nullptr;
 };
 
-static size_t batch_smem(int dtype) { return (size_t)dtype * (32 * 33 + (size_t)kBMaxN * 33); }
+static size_t batch_smem(int dtype) { return dtype == 8 ? sizeof(BatchSmem<double>) : sizeof(BatchSmem<float>); }
 
 static bool cache_lookup(const std::string &key, int &cps, int &thr) { return lla::autotune_lookup(key, cps, thr); }
 static void cache_store(const std::string &key, int cps, int thr) { lla::autotune_store(key, cps, thr); }
