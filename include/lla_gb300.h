@@ -273,7 +273,7 @@ int lla_dtrsm_device_noalloc_status(void *stream, lla_error *err);
  * own operation order (src/cholesky.rs:51-76), whose verdict and failing row
  * are returned, as the host-view entry points do. */
 enum lla_update {
-    LLA_UPDATE_FP32 = 0,    /* FP32 SIMT trailing updates */
+    LLA_UPDATE_FP32 = 0,    /* FP32 factor (the FAST FP32 form: exact digits, one FP32 rounding per update) */
     LLA_UPDATE_BF16 = 1,    /* tcgen05: one BF16 term per operand, FP32 accumulation */
     LLA_UPDATE_BF16X3 = 3,  /* tcgen05: hi/lo BF16 split, three products */
     LLA_UPDATE_BF16X6 = 6,  /* tcgen05: three-level BF16 split, six products */

@@ -248,7 +248,7 @@ __device__ __forceinline__ void batch_digits(uint32_t w, uint32_t &lo, uint32_t 
 // FP64: the product of the 32 panel columns on the tensor cores, from seven
 // balanced 8-bit digits per entry (exact in FP16, their products' sums exact in
 // the FP32 accumulators), one 64-bit integer per entry and one FP64 subtraction,
-// where FMAs would spend 32 FP64 instructions per entry (lla_fp64_chol.cu has the
+// where FMAs would spend 32 FP64 instructions per entry (lla_fast_chol.cu has the
 // scheme and its error).  Warp tiles of 16 x 8, K = 32 in two steps; the digits'
 // k order is permuted alike in both operands so that a thread's four are one word.
 __device__ void batch_update(BatchSmem<double> &sm, double *A, int n, int q, int kb, int rows, int m) {

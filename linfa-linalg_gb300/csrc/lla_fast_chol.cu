@@ -1,33 +1,34 @@
-// lla_fp64_chol.cu -- FAST FP64 Cholesky: right-looking, lower triangle,
-// column-major, with the trailing update on the BF16 tensor cores by exact
-// integer digits.
+// lla_fast_chol.cu -- FAST Cholesky, FP64 and FP32: right-looking, lower
+// triangle, column-major, with the trailing update on the BF16 tensor cores by
+// exact integer digits.
 //
 // GB300 executes FP64 at about 1.7 operations per clock per SM (measured: one
 // FP64 warp instruction occupies its sub-partition for 64 cycles, whatever the
 // number of active lanes), 1/64 of the FP32 rate, so n^3/3 flops on the FP64
-// pipe take 176 ms at n = 8192 however they are tiled.  Here only the O(n^2)
-// parts stay there:
-//   diag   : 64 x 64 diagonal block, one CTA, FP64;
-//   panel  : L21 = A21 L11^-T, 64 columns, FP64 substitution; the finished rows
-//            are also cut into seven balanced 8-bit digits (lla_oz_digits.h)
-//            relative to each row's largest magnitude, exact in BF16;
+// pipe take 176 ms at n = 8192 however they are tiled; the FP32 pipe's n^3/3 is
+// 1 ms at n = 6001, but its rate needs large register tiles.  Here only the
+// O(n^2) parts stay on those pipes:
+//   diag   : 64 x 64 diagonal block, one CTA;
+//   panel  : L21 = A21 L11^-T, 64 columns, by substitution; the finished rows are
+//            also cut into balanced 8-bit digits (lla_oz_digits.h; seven for FP64,
+//            four for FP32) relative to each row's largest magnitude, exact in
+//            BF16;
 //   update : A22 -= L21 L21^T with tcgen05 MMAs on the digits.  Every product
 //            of digits is an integer of at most 14 bits, a level (sum of the
 //            products of equal weight) gathers at most 7 x 128 of them, so the
 //            FP32 accumulators hold exact integers (<= 2^24); they are combined
-//            in 64-bit integers and subtracted from A22 in FP64: one rounding
-//            per entry and 128 columns, where FMAs round once per column.
-// Digit products below 2^-56 of the row scales are dropped; the digits hold
-// each entry to 2^-56 of its row's largest one.  Measured against a 64-bit
-// reference the factor's error is no larger than the FP64 pipe's (see the
-// update kernel).  Panels go in pairs: the second one's 64 columns are brought
-// up to date by a narrow update with the first panel alone (K = 64), then one
-// update with both (K = 128) covers the rest, so the trailing matrix is read
-// and written once per 128 columns.
+//            in 64-bit integers and subtracted from A22 in its own type: one
+//            rounding per entry and 128 columns, where FMAs round once per column.
+// Digit products below 2^-56 (FP32: 2^-32) of the row scales are dropped; the
+// digits hold each entry to that fraction of its row's largest one.  Panels go in
+// pairs: the second one's 64 columns are brought up to date by a narrow update
+// with the first panel alone (K = 64), then one update with both (K = 128) covers
+// the rest, so the trailing matrix is read and written once per 128 columns.
 //
-// Measured, FP64 pipe before -> now: n = 8192 220 -> 15.1 ms, n = 2048 14.4 ->
-// 2.25 ms.  There is no size at which the FP64 pipe's update is faster: one
-// 64 x 64 tile of it took 70 us on its SM.
+// Measured, FMA updates before -> now (error against 64 bits the same or lower):
+// f64 n = 8192 220 -> 15.1 ms, n = 2048 14.4 -> 2.25 ms; f32 n = 6001 14.6 ->
+// 4.3 ms.  There is no size at which the FMA form is faster: one 64 x 64 tile of
+// the FP64 one took 70 us on its SM.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -49,6 +50,44 @@ constexpr int kFcNb = 64;             // panel width
 constexpr int kFcPair = 2 * kFcNb;    // columns per trailing update
 constexpr int kFcNonFinite = 1 << 20; // exponent word of a row that holds inf or NaN
 
+// What depends on the element type: digits, their fixed point and exponents, and
+// reciprocal roots (of positive normal numbers).
+template <typename T>
+struct Fc;
+template <>
+struct Fc<double> {
+    static constexpr int kDigits = kOzBal;
+    static constexpr int kShift = 62;  // digits of exponents e, f: products in units of 2^(e + f - kShift)
+    using Bits = unsigned long long;
+    static __device__ __forceinline__ Bits abs_bits(double v) {
+        return (Bits)__double_as_longlong(v) & 0x7fffffffffffffffull;
+    }
+    static __device__ __forceinline__ int exponent(Bits b) {
+        return b >= 0x7ff0000000000000ull ? kFcNonFinite : oz_bits_exponent(b);
+    }
+    static __device__ __forceinline__ int64_t fixed(double v, int e) { return oz_fixed55(__double_as_longlong(v), e); }
+    static __device__ __forceinline__ double rsqrt_(double d) { return im_rsqrt(d); }
+    static __device__ __forceinline__ bool normal(double d) { return im_positive_normal(im_bits(d)); }
+};
+template <>
+struct Fc<float> {
+    static constexpr int kDigits = kOzBal32;
+    static constexpr int kShift = 38;
+    using Bits = unsigned;
+    static __device__ __forceinline__ Bits abs_bits(float v) { return __float_as_uint(v) & 0x7fffffffu; }
+    // (-126 holds for zero and subnormals too)
+    static __device__ __forceinline__ int exponent(Bits b) {
+        return b >= 0x7f800000u ? kFcNonFinite : max((int)(b >> 23), 0) - 126;
+    }
+    static __device__ __forceinline__ int64_t fixed(float v, int e) { return oz_fixed31(__float_as_int(v), e); }
+    // FP32 approximation and one Newton step
+    static __device__ __forceinline__ float rsqrt_(float d) {
+        const float y = im_rsqrt_seed(d);
+        return fmaf(0.5f * y, fmaf(-d * y, y, 1.f), y);
+    }
+    static __device__ __forceinline__ bool normal(float d) { return __float_as_uint(d) - 0x800000u < 0x7f000000u; }
+};
+
 __device__ __forceinline__ void atomic_min_pos_f64(double *addr, double v) {
     // non-negative doubles order like their bit patterns
     if (v >= 0.0) atomicMin((unsigned long long *)addr, (unsigned long long)__double_as_longlong(v));
@@ -66,7 +105,7 @@ __device__ __forceinline__ void atomic_min_pos_f64(double *addr, double v) {
 // the other three sub-partitions keep the rest in registers, in patches of 16
 // rows x 2 columns (one FP64 instruction per column applied), and hand pair
 // k + 2 to warp 0 through shared memory once pair k is in it.  One barrier per
-// pair.  160 -> 35 us a block.
+// pair.  160 -> 33 us a block (FP32 67 -> 14 us).
 constexpr int kFcDiagThreads = 512;
 constexpr int kFcPatches = 80, kFcPatchWarps = 12, kFcSlots = 7;
 
@@ -92,58 +131,57 @@ __device__ __forceinline__ void fc_patch(int t, int &g, int &j) {
 // go to piv, their reciprocal roots to rv.  LOW: c < 32, both halves of the rows
 // (lane, lane + 32) take part.  Returns true when a pivot is not positive: its
 // column goes to *s_fail and the columns keep what is finished.
-template <bool LOW>
-__device__ __forceinline__ bool fc_pivot_pair(double (*a)[kFcNb], double *piv, double *rv, int *s_fail, int c,
-                                              int lane) {
-    double u0 = 0.0, v0 = 0.0, u1 = a[c][lane + 32], v1 = a[c + 1][lane + 32];
+template <typename T, bool LOW>
+__device__ __forceinline__ bool fc_pivot_pair(T (*a)[kFcNb], T *piv, T *rv, int *s_fail, int c, int lane) {
+    T u0 = T(0), v0 = T(0), u1 = a[c][lane + 32], v1 = a[c + 1][lane + 32];
     if (LOW) {
         u0 = a[c][lane];
         v0 = a[c + 1][lane];
     }
     if (c > 0) {
-        const double l00 = a[c - 2][c], l01 = a[c - 1][c], l10 = a[c - 2][c + 1], l11 = a[c - 1][c + 1];
-        const double x01 = a[c - 2][lane + 32], x11 = a[c - 1][lane + 32];
+        const T l00 = a[c - 2][c], l01 = a[c - 1][c], l10 = a[c - 2][c + 1], l11 = a[c - 1][c + 1];
+        const T x01 = a[c - 2][lane + 32], x11 = a[c - 1][lane + 32];
         if (LOW) {  // the half that holds the pivots first
-            const double x00 = a[c - 2][lane], x10 = a[c - 1][lane];
+            const T x00 = a[c - 2][lane], x10 = a[c - 1][lane];
             u0 = fma(-x10, l01, fma(-x00, l00, u0));
             v0 = fma(-x10, l11, fma(-x00, l10, v0));
         }
         u1 = fma(-x11, l01, fma(-x01, l00, u1));
         v1 = fma(-x11, l11, fma(-x01, l10, v1));
     }
-    const double su0 = u0, su1 = u1, sv0 = v0, sv1 = v1;
-    const double d0 = __shfl_sync(0xffffffffu, LOW ? u0 : u1, c & 31);
-    const double y0 = im_rsqrt(d0);
+    const T su0 = u0, su1 = u1, sv0 = v0, sv1 = v1;
+    const T d0 = __shfl_sync(0xffffffffu, LOW ? u0 : u1, c & 31);
+    const T y0 = Fc<T>::rsqrt_(d0);
     if (LOW) u0 *= y0;
     u1 *= y0;
-    const double l = __shfl_sync(0xffffffffu, LOW ? u0 : u1, (c + 1) & 31);
+    const T l = __shfl_sync(0xffffffffu, LOW ? u0 : u1, (c + 1) & 31);
     if (LOW) v0 = fma(-u0, l, v0);
     v1 = fma(-u1, l, v1);
-    const double d1 = __shfl_sync(0xffffffffu, LOW ? v0 : v1, (c + 1) & 31);
-    const double y1 = im_rsqrt(d1);
+    const T d1 = __shfl_sync(0xffffffffu, LOW ? v0 : v1, (c + 1) & 31);
+    const T y1 = Fc<T>::rsqrt_(d1);
     if (LOW) v0 *= y1;
     v1 *= y1;
-    double z0 = y0, z1 = y1;
+    T z0 = y0, z1 = y1;
     int fail = -1;
-    if (!im_positive_normal(im_bits(d0)) || !im_positive_normal(im_bits(d1))) {
+    if (!Fc<T>::normal(d0) || !Fc<T>::normal(d1)) {
         // not positive (false for NaN, as in the reference), subnormal, inf or NaN: again, with
         // the library's functions
         u0 = su0, u1 = su1, v0 = sv0, v1 = sv1;
-        if (d0 <= 0.0) {
+        if (d0 <= T(0)) {
             fail = c;
         } else {
-            z0 = 1.0 / sqrt(d0);
+            z0 = T(1) / sqrt(d0);
             u0 *= z0;
             u1 *= z0;
-            const double l2 = __shfl_sync(0xffffffffu, LOW ? u0 : u1, (c + 1) & 31);
+            const T l2 = __shfl_sync(0xffffffffu, LOW ? u0 : u1, (c + 1) & 31);
             v0 = fma(-u0, l2, v0);
             v1 = fma(-u1, l2, v1);
-            const double e1 = __shfl_sync(0xffffffffu, LOW ? v0 : v1, (c + 1) & 31);
+            const T e1 = __shfl_sync(0xffffffffu, LOW ? v0 : v1, (c + 1) & 31);
             piv[c + 1] = e1;
-            if (e1 <= 0.0) {
+            if (e1 <= T(0)) {
                 fail = c + 1;
             } else {
-                z1 = 1.0 / sqrt(e1);
+                z1 = T(1) / sqrt(e1);
                 v0 *= z1;
                 v1 *= z1;
             }
@@ -165,11 +203,12 @@ __device__ __forceinline__ bool fc_pivot_pair(double (*a)[kFcNb], double *piv, d
     return fail >= 0;
 }
 
-__global__ void __launch_bounds__(kFcDiagThreads) fc_diag_kernel(double *W, int64_t ld, int64_t p, int b,
-                                                                 const double *diag0, double *rinv, int64_t *info,
+template <typename T>
+__global__ void __launch_bounds__(kFcDiagThreads) fc_diag_kernel(T *W, int64_t ld, int64_t p, int b,
+                                                                 const T *diag0, T *rinv, int64_t *info,
                                                                  double *min_ratio) {
-    __shared__ double a[kFcNb][kFcNb];  // [column][row]
-    __shared__ double piv[kFcNb], rv[kFcNb];
+    __shared__ T a[kFcNb][kFcNb];  // [column][row]
+    __shared__ T piv[kFcNb], rv[kFcNb];
     __shared__ int s_fail;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     pdl_wait();
@@ -178,12 +217,12 @@ __global__ void __launch_bounds__(kFcDiagThreads) fc_diag_kernel(double *W, int6
     for (int e = tid; e < kFcNb * kFcNb; e += kFcDiagThreads) {
         const int r = e % kFcNb, c = e / kFcNb;
         // a short block is padded with the identity
-        a[c][r] = (r < b && c <= r) ? cm(W, ld, p + r, p + c) : (r == c ? 1.0 : 0.0);
+        a[c][r] = (r < b && c <= r) ? cm(W, ld, p + r, p + c) : T(r == c ? 1 : 0);
     }
     if (tid == 0) s_fail = -1;
     __syncthreads();
     const bool upd = (warp & 3) != 0;  // a patch warp (warps 4, 8 and 12 only load and store)
-    double acc[kFcSlots];
+    T acc[kFcSlots];
     int row[kFcSlots], col[kFcSlots];  // col < 0: no patch
     if (upd) {
 #pragma unroll
@@ -193,11 +232,11 @@ __global__ void __launch_bounds__(kFcDiagThreads) fc_diag_kernel(double *W, int6
             fc_patch(t, g, j);
             row[s] = 16 * g + (lane & 15);
             col[s] = t < kFcPatches ? 2 * j + (lane >> 4) : -1;
-            acc[s] = t < kFcPatches ? a[col[s]][row[s]] : 0.0;
+            acc[s] = t < kFcPatches ? a[col[s]][row[s]] : T(0);
         }
     }
     bool bad = false;
-    if (warp == 0) bad = fc_pivot_pair<true>(a, piv, rv, &s_fail, 0, lane);
+    if (warp == 0) bad = fc_pivot_pair<T, true>(a, piv, rv, &s_fail, 0, lane);
     for (int k = 0;; ++k) {
         __syncthreads();  // pair k is final
         // A pivot failure of pair k ends the loop for everyone here.  Warp 0 may already have
@@ -206,8 +245,8 @@ __global__ void __launch_bounds__(kFcDiagThreads) fc_diag_kernel(double *W, int6
         if (warp > 0) bad = (unsigned)*(volatile int *)&s_fail <= (unsigned)(2 * k + 1);
         if (bad || k == kFcNb / 2 - 1) break;
         if (warp == 0) {
-            bad = k < 15 ? fc_pivot_pair<true>(a, piv, rv, &s_fail, 2 * k + 2, lane)
-                         : fc_pivot_pair<false>(a, piv, rv, &s_fail, 2 * k + 2, lane);
+            bad = k < 15 ? fc_pivot_pair<T, true>(a, piv, rv, &s_fail, 2 * k + 2, lane)
+                         : fc_pivot_pair<T, false>(a, piv, rv, &s_fail, 2 * k + 2, lane);
         } else if (upd) {
 #pragma unroll
             for (int s = 0; s < kFcSlots; ++s) {
@@ -231,9 +270,9 @@ __global__ void __launch_bounds__(kFcDiagThreads) fc_diag_kernel(double *W, int6
     if (tid < kFcNb) {  // exact roots of the pivots, and the smallest relative pivot
         double ratio = 1.0e300;
         if (tid < done && tid < b) {
-            const double d = piv[tid];
+            const T d = piv[tid];
             a[tid][tid] = sqrt(d);
-            const double r0 = d / diag0[p + tid];
+            const double r0 = (double)d / (double)diag0[p + tid];
             if (r0 < ratio) ratio = r0;
         }
         if (min_ratio) {
@@ -267,14 +306,17 @@ __global__ void __launch_bounds__(kFcDiagThreads) fc_diag_kernel(double *W, int6
 constexpr int kFcRows = 16;
 constexpr int kFcPanelThreads = 256;
 
-__global__ void __launch_bounds__(kFcPanelThreads) fc_panel_kernel(double *W, int64_t ld, int64_t n, int64_t p,
-                                                                   int second, const double *rinv,
+template <typename T>
+__global__ void __launch_bounds__(kFcPanelThreads) fc_panel_kernel(T *W, int64_t ld, int64_t n, int64_t p,
+                                                                   int second, const T *rinv,
                                                                    __nv_bfloat16 *planes, int64_t plane_stride,
                                                                    int *expo, const int64_t *info) {
-    __shared__ double l11[kFcNb][kFcNb];        // [column][row]
-    __shared__ double x[kFcNb][kFcRows + 1];    // finished columns, [column][row]
-    __shared__ double rv[kFcNb];
-    __shared__ unsigned long long s_max[kFcPanelThreads / 16][kFcRows];
+    using Bits = typename Fc<T>::Bits;
+    constexpr int ND = Fc<T>::kDigits;
+    __shared__ T l11[kFcNb][kFcNb];           // [column][row]
+    __shared__ T x[kFcNb][kFcRows + 1];    // finished columns, [column][row]
+    __shared__ T rv[kFcNb];
+    __shared__ Bits s_max[kFcPanelThreads / 16][kFcRows];
     __shared__ int s_e[kFcRows];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int r16 = lane & 15, cc = lane >> 4;
@@ -283,20 +325,20 @@ __global__ void __launch_bounds__(kFcPanelThreads) fc_panel_kernel(double *W, in
     pdl_trigger();
     if (*(volatile const int64_t *)info >= 0) return;
     const bool in = j0 + r16 < n;
-    double acc[4];
+    T acc[4];
 #pragma unroll
-    for (int s = 0; s < 4; ++s) acc[s] = in ? cm(W, ld, j0 + r16, p + 2 * (warp + 8 * s) + cc) : 0.0;
+    for (int s = 0; s < 4; ++s) acc[s] = in ? cm(W, ld, j0 + r16, p + 2 * (warp + 8 * s) + cc) : T(0);
     for (int e = tid; e < kFcNb * kFcNb; e += kFcPanelThreads) {
         const int r = e % kFcNb, c = e / kFcNb;
-        l11[c][r] = c <= r ? cm(W, ld, p + r, p + c) : 0.0;
+        l11[c][r] = c <= r ? cm(W, ld, p + r, p + c) : T(0);
     }
     if (tid < kFcNb) rv[tid] = rinv[tid];
     __syncthreads();
     // solves column pair j (this warp's slot value v) and publishes it
-    auto solve = [&](int j, double v) {
+    auto solve = [&](int j, T v) {
         const int c = 2 * j;
-        double u = v * rv[c];
-        const double x0 = __shfl_sync(0xffffffffu, u, r16);
+        T u = v * rv[c];
+        const T x0 = __shfl_sync(0xffffffffu, u, r16);
         if (cc) u = fma(-x0, l11[c][c + 1], v) * rv[c + 1];
         x[c + cc][r16] = u;
     };
@@ -308,7 +350,7 @@ __global__ void __launch_bounds__(kFcPanelThreads) fc_panel_kernel(double *W, in
         for (int w0 = 0; w0 < 8; ++w0) {
             const int j = 8 * s0 + w0;  // pair j is finished: apply it to the pairs right of it
             if (j == kFcNb / 2 - 1) break;
-            const double x0 = x[2 * j][r16], x1 = x[2 * j + 1][r16];
+            const T x0 = x[2 * j][r16], x1 = x[2 * j + 1][r16];
 #pragma unroll
             for (int s = s0; s < 4; ++s) {
                 const int jj = 8 * s + warp;
@@ -325,22 +367,22 @@ __global__ void __launch_bounds__(kFcPanelThreads) fc_panel_kernel(double *W, in
         if (j0 + r < n) cm(W, ld, j0 + r, p + c) = x[c][r];
     }
     // the pair's first panel, in the space of L11
-    double(*x1)[kFcRows + 1] = reinterpret_cast<double(*)[kFcRows + 1]>(&l11[0][0]);
+    T(*x1)[kFcRows + 1] = reinterpret_cast<T(*)[kFcRows + 1]>(&l11[0][0]);
     if (second)
         for (int e = tid; e < kFcRows * kFcNb; e += kFcPanelThreads) {
             const int r = e % kFcRows, c = e / kFcRows;
-            x1[c][r] = j0 + r < n ? cm(W, ld, j0 + r, p - kFcNb + c) : 0.0;
+            x1[c][r] = j0 + r < n ? cm(W, ld, j0 + r, p - kFcNb + c) : T(0);
         }
     __syncthreads();
     // row maxima over the pair's columns so far, on the bit patterns
     {
         const int r = tid & 15, g = tid >> 4;  // 16 groups of columns
-        unsigned long long mx = 0ull;
+        Bits mx = 0;
         for (int c = g; c < kFcNb; c += kFcPanelThreads / 16) {
-            const unsigned long long v = (unsigned long long)__double_as_longlong(x[c][r]) & 0x7fffffffffffffffull;
+            const Bits v = Fc<T>::abs_bits(x[c][r]);
             mx = v > mx ? v : mx;
             if (second) {
-                const unsigned long long u = (unsigned long long)__double_as_longlong(x1[c][r]) & 0x7fffffffffffffffull;
+                const Bits u = Fc<T>::abs_bits(x1[c][r]);
                 mx = u > mx ? u : mx;
             }
         }
@@ -348,9 +390,9 @@ __global__ void __launch_bounds__(kFcPanelThreads) fc_panel_kernel(double *W, in
     }
     __syncthreads();
     if (tid < kFcRows) {
-        unsigned long long mx = 0ull;
+        Bits mx = 0;
         for (int g = 0; g < kFcPanelThreads / 16; ++g) mx = s_max[g][tid] > mx ? s_max[g][tid] : mx;
-        const int e = mx >= 0x7ff0000000000000ull ? kFcNonFinite : oz_bits_exponent(mx);
+        const int e = Fc<T>::exponent(mx);
         s_e[tid] = e;
         if (j0 + tid < n) expo[j0 + tid] = e;
     }
@@ -360,17 +402,17 @@ __global__ void __launch_bounds__(kFcPanelThreads) fc_panel_kernel(double *W, in
     for (int e = tid; e < kFcRows * cols / 4; e += kFcPanelThreads) {
         const int k4 = (e % (cols / 4)) * 4, r = e / (cols / 4);
         if (j0 + r >= n) continue;
-        const double(*xs)[kFcRows + 1] = second && k4 < kFcNb ? x1 : x;
+        const T(*xs)[kFcRows + 1] = second && k4 < kFcNb ? x1 : x;
         const int ks = k4 % kFcNb, ex = s_e[r];
         int64_t v[4];
 #pragma unroll
         for (int u = 0; u < 4; ++u)
-            v[u] = ex == kFcNonFinite ? 0 : oz_fixed55(__double_as_longlong(xs[ks + u][r]), ex);
-        uint32_t d0[kOzBal], d1[kOzBal];
+            v[u] = ex == kFcNonFinite ? 0 : Fc<T>::fixed(xs[ks + u][r], ex);
+        uint32_t d0[ND], d1[ND];
         oz_balanced_pair(v[0], v[1], d0);
         oz_balanced_pair(v[2], v[3], d1);
 #pragma unroll
-        for (int s = 0; s < kOzBal; ++s)
+        for (int s = 0; s < ND; ++s)
             *reinterpret_cast<uint2 *>(planes + s * plane_stride + (j0 + r) * kFcPair + k4) = make_uint2(d0[s], d1[s]);
     }
 }
@@ -394,16 +436,24 @@ constexpr int kFuM = 128, kFuN = 64, kFuK = 64;
 constexpr int kFuRing = 6;                         // stages of one row plane
 constexpr int kFuATile = kFuM * kFuK * 2;          // 16 KiB
 constexpr int kFuBTile = kFuN * kFuK * 2;          // 8 KiB
-constexpr int kFuBSet = kOzBal * kFuBTile;         // 56 KiB: all planes of a column tile's chunk
-constexpr int kFuSmem = 1024 + kFuRing * kFuATile + 2 * kFuBSet + 256;
+// All planes of a column tile's chunk (56 KiB for FP64).
+template <typename T>
+constexpr int kFuBSet = Fc<T>::kDigits *kFuBTile;
+template <typename T>
+constexpr int kFuSmem = 1024 + kFuRing * kFuATile + 2 * kFuBSet<T> + 256;
 constexpr int kFuEpi = 512;                        // 16 epilogue warps
 constexpr int kFuThreads = kFuEpi + 64;            // and the producer's and the MMA issuer's
-constexpr uint32_t kFuTmem = 512;                  // allocated columns (448 used)
+// Tensor memory: all 512 columns; FP64's seven levels fill 448 of them, FP32's
+// four levels leave room for a second set.
+constexpr uint32_t kFuTmem = 512;
+template <typename T>
+constexpr int kFuSets = Fc<T>::kDigits * kFuN * 2 <= (int)kFuTmem ? 2 : 1;
 
 // Entries of rows that hold inf or NaN, which have no digits: the FMA chain on
 // the factor itself.
-__device__ __noinline__ double fu_plain_entry(const double *W, int64_t ld, int64_t i, int64_t j, int64_t p0, int kext) {
-    double acc = W[i + j * ld];
+template <typename T>
+__device__ __noinline__ T fu_plain_entry(const T *W, int64_t ld, int64_t i, int64_t j, int64_t p0, int kext) {
+    T acc = W[i + j * ld];
     for (int k = 0; k < kext; ++k) acc = fma(-W[i + (p0 + k) * ld], W[j + (p0 + k) * ld], acc);
     return acc;
 }
@@ -422,21 +472,32 @@ __device__ __forceinline__ void fu_tile(int t, int narrow, int &I, int &J) {
     J = t - i * (i + 1);
 }
 
+// W - T 2^s, the product rounded to W's type first.
+__device__ __forceinline__ double fu_subtract(double w, long long T, int s) { return w - oz_scaled_double(T, s); }
+__device__ __forceinline__ float fu_subtract(float w, long long T, int s) {
+    const float t = __ll2float_rn(T);  // 2^t0 with 0 <= t0 <= 47
+    // 2^s as a float where it and the product stay normal, scalbnf elsewhere
+    const bool fits = s >= -120 && s <= 70;
+    return w - (fits ? t * __int_as_float((s + 127) << 23) : scalbnf(t, s));
+}
+
+template <typename T>
 __global__ void __launch_bounds__(kFuThreads, 1) fc_update_kernel(
-    const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, double *W, int64_t ld,
+    const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, T *W, int64_t ld,
     int64_t q, int64_t n, int64_t p0, int kchunks, int ntiles, int narrow, const int *__restrict__ expo,
     const int64_t *info, int *err_word, int *sticky) {
+    constexpr int ND = Fc<T>::kDigits, SETS = kFuSets<T>, BSET = kFuBSet<T>;
     extern __shared__ uint8_t smem_raw[];
     __shared__ int s_abort, s_skip;
     uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint8_t *sA = smem;
     uint8_t *sB = smem + kFuRing * kFuATile;
-    uint64_t *bars = (uint64_t *)(sB + 2 * kFuBSet);
-    uint32_t *tslot = (uint32_t *)(bars + 2 * kFuRing + 6);
+    uint64_t *bars = (uint64_t *)(sB + 2 * BSET);
+    uint32_t *tslot = (uint32_t *)(bars + 2 * kFuRing + 8);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t fullA0 = smem_u32(bars), emptyA0 = fullA0 + 8 * kFuRing;
     const uint32_t fullB0 = emptyA0 + 8 * kFuRing, emptyB0 = fullB0 + 16;
-    const uint32_t tfull = emptyB0 + 16, tempty = tfull + 8;
+    const uint32_t tfull = emptyB0 + 16, tempty = tfull + 16;  // + 8 per set
     if (tid == 0) {
         for (int s = 0; s < kFuRing; ++s) {
             mbar_init(fullA0 + 8 * s, 1);
@@ -446,8 +507,10 @@ __global__ void __launch_bounds__(kFuThreads, 1) fc_update_kernel(
             mbar_init(fullB0 + 8 * s, 1);
             mbar_init(emptyB0 + 8 * s, 1);
         }
-        mbar_init(tfull, 1);
-        mbar_init(tempty, kFuEpi);
+        for (int s = 0; s < SETS; ++s) {
+            mbar_init(tfull + 8 * s, 1);
+            mbar_init(tempty + 8 * s, kFuEpi);
+        }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         s_abort = 0;
     }
@@ -488,9 +551,9 @@ __global__ void __launch_bounds__(kFuThreads, 1) fc_update_kernel(
                         s_abort = 1;
                         break;
                     }
-                    mbar_expect_tx(fullB0 + 8 * xb, kFuBSet);
-                    tma_load_3d(smem_u32(sB + xb * kFuBSet), &tmB, kc * kFuK, rb, 0, fullB0 + 8 * xb);
-                    for (int s = 0; s < kOzBal; ++s, ++ga) {
+                    mbar_expect_tx(fullB0 + 8 * xb, BSET);
+                    tma_load_3d(smem_u32(sB + xb * BSET), &tmB, kc * kFuK, rb, 0, fullB0 + 8 * xb);
+                    for (int s = 0; s < ND; ++s, ++ga) {
                         const uint32_t st = ga % kFuRing, round = ga / kFuRing;
                         if (round > 0 && !mbar_wait(emptyA0 + 8 * st, (round - 1) & 1, err_word)) {
                             s_abort = 1;
@@ -506,7 +569,8 @@ __global__ void __launch_bounds__(kFuThreads, 1) fc_update_kernel(
         if (lane == 0) {  // MMA issuer
             uint32_t ga = 0, gb = 0, lt = 0;
             for (int t = blockIdx.x; t < ntiles && !*(volatile int *)&s_abort; t += gridDim.x, ++lt) {
-                if (lt > 0 && !mbar_wait(tempty, (lt - 1) & 1, err_word)) {
+                const uint32_t set = lt % SETS, use = lt / SETS;
+                if (use > 0 && !mbar_wait(tempty + 8 * set, (use - 1) & 1, err_word)) {
                     s_abort = 1;
                     break;
                 }
@@ -517,8 +581,8 @@ __global__ void __launch_bounds__(kFuThreads, 1) fc_update_kernel(
                         s_abort = 1;
                         break;
                     }
-                    const uint32_t b0 = smem_u32(sB + xb * kFuBSet);
-                    for (int s = 0; s < kOzBal; ++s, ++ga) {
+                    const uint32_t b0 = smem_u32(sB + xb * BSET);
+                    for (int s = 0; s < ND; ++s, ++ga) {
                         const uint32_t st = ga % kFuRing;
                         if (!mbar_wait(fullA0 + 8 * st, (ga / kFuRing) & 1, err_word)) {
                             s_abort = 1;
@@ -526,9 +590,9 @@ __global__ void __launch_bounds__(kFuThreads, 1) fc_update_kernel(
                         }
                         tc_fence_after();
                         const uint64_t ad = sw128_desc(smem_u32(sA + st * kFuATile));
-                        for (int t0 = 0; t0 < kOzBal - s; t0 += 4) {
-                            const int t1 = min(t0 + 4, kOzBal - s);
-                            const uint32_t dt = tmem + (uint32_t)((s + t0) * kFuN);
+                        for (int t0 = 0; t0 < ND - s; t0 += 4) {
+                            const int t1 = min(t0 + 4, ND - s);
+                            const uint32_t dt = tmem + set * (kFuTmem / SETS) + (uint32_t)((s + t0) * kFuN);
                             const uint32_t idesc = idesc0 | ((uint32_t)((kFuN * (t1 - t0)) >> 3) << 17);
                             const uint64_t bd = sw128_desc(b0 + (uint32_t)(t0 * kFuBTile));
 #pragma unroll
@@ -541,57 +605,59 @@ __global__ void __launch_bounds__(kFuThreads, 1) fc_update_kernel(
                     tc_commit(emptyB0 + 8 * xb);
                 }
                 if (*(volatile int *)&s_abort) break;
-                tc_commit(tfull);
+                tc_commit(tfull + 8 * set);
             }
         }
     } else {  // epilogue: warp w reads lane quarter w % 4, columns 16 (w / 4) .. + 15 of every level
         const int qw = warp & 3, cq = warp >> 2;
         const int r = qw * 32 + lane;
-        const uint32_t tcol = tmem + ((uint32_t)(qw * 32) << 16) + (uint32_t)(cq * 16);
+        const uint32_t tcol0 = tmem + ((uint32_t)(qw * 32) << 16) + (uint32_t)(cq * 16);
         uint32_t lt = 0;
         for (int t = blockIdx.x; t < ntiles; t += gridDim.x, ++lt) {
+            const uint32_t set = lt % SETS, use = lt / SETS, tcol = tcol0 + set * (kFuTmem / SETS);
             int I, J;
             fu_tile(t, narrow, I, J);
             const int64_t i = q + (int64_t)I * kFuM + r, jb = q + (int64_t)J * kFuN + cq * 16;
             const int nc = i < n ? (int)max((int64_t)0, min((int64_t)16, i - jb + 1)) : 0;  // columns j <= i
-            double *wp = W + i + jb * ld;
+            T *wp = W + i + jb * ld;
             // the entries and the columns' exponents (column lane & 15) are fetched before the
             // digits' products are ready
-            double w[16];
+            T w[16];
 #pragma unroll
-            for (int c = 0; c < 16; ++c) w[c] = c < nc ? wp[c * ld] : 0.0;
+            for (int c = 0; c < 16; ++c) w[c] = c < nc ? wp[c * ld] : T(0);
             const int64_t je = jb + (lane & 15);
             const int ejl = je < n ? expo[je] : 0;
             const int ei = i < n ? expo[i] : 0;
-            bool ok = mbar_wait(tfull, lt & 1, err_word);
+            bool ok = mbar_wait(tfull + 8 * set, use & 1, err_word);
             ok = __all_sync(0xffffffffu, ok) && !*(volatile int *)&s_abort;
             if (!ok) {
                 if (lane == 0) s_abort = 1;
                 break;
             }
             tc_fence_after();
-            // T = 2^-8 sum_d I_d 2^(8 (6 - d)): levels 4-6 first, rounded to eight bits less (below
-            // the dropped products, so that the sum fits 64 bits), then levels 0-3 at 2^16 and up
-            long long T[16];
+            // sum_d I_d 2^(8 (ND - 1 - d)).  FP64 needs it less eight bits to fit 64: levels 4-6
+            // first, rounded (below the dropped products), then levels 0-3 at 2^16 and up.
+            long long sum[16];
 #pragma unroll
             for (int g = 0; g < 2; ++g) {
                 long long s8[8];
                 uint32_t v[8];
+                if (ND > 4) {
 #pragma unroll
-                for (int c = 0; c < 8; ++c) s8[c] = 128;
+                    for (int c = 0; c < 8; ++c) s8[c] = 128;
 #pragma unroll
-                for (int d = 4; d < kOzBal; ++d) {
-                    tc_ld8_nowait(tcol + (uint32_t)(d * kFuN + g * 8), v);
-                    tc_wait_ld();
+                    for (int d = 4; d < ND; ++d) {
+                        tc_ld8_nowait(tcol + (uint32_t)(d * kFuN + g * 8), v);
+                        tc_wait_ld();
 #pragma unroll
-                    for (int c = 0; c < 8; ++c)
-                        s8[c] += (long long)__float2int_rn(__uint_as_float(v[c])) * (1 << (8 * (6 - d)));
+                        for (int c = 0; c < 8; ++c)
+                            s8[c] += (long long)__float2int_rn(__uint_as_float(v[c])) * (1 << (8 * (ND - 1 - d)));
+                    }
+#pragma unroll
+                    for (int c = 0; c < 8; ++c) sum[g * 8 + c] = s8[c] >> 8;
                 }
 #pragma unroll
-                for (int c = 0; c < 8; ++c) {
-                    T[g * 8 + c] = s8[c] >> 8;
-                    s8[c] = 0;
-                }
+                for (int c = 0; c < 8; ++c) s8[c] = 0;
 #pragma unroll
                 for (int d = 0; d < 4; ++d) {
                     tc_ld8_nowait(tcol + (uint32_t)(d * kFuN + g * 8), v);
@@ -601,10 +667,10 @@ __global__ void __launch_bounds__(kFuThreads, 1) fc_update_kernel(
                         s8[c] += (long long)__float2int_rn(__uint_as_float(v[c])) * (1 << (8 * (3 - d)));
                 }
 #pragma unroll
-                for (int c = 0; c < 8; ++c) T[g * 8 + c] += s8[c] << 16;
+                for (int c = 0; c < 8; ++c) sum[g * 8 + c] = ND > 4 ? sum[g * 8 + c] + (s8[c] << 16) : s8[c];
             }
             tc_fence_before();
-            asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(tempty) : "memory");
+            asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(tempty + 8 * set) : "memory");
             unsigned plain = 0;  // columns to do without digits
 #pragma unroll
             for (int c = 0; c < 16; ++c) {
@@ -614,7 +680,7 @@ __global__ void __launch_bounds__(kFuThreads, 1) fc_update_kernel(
                     if (nonfinite)
                         plain |= 1u << c;
                     else
-                        wp[c * ld] = w[c] - oz_scaled_double(T[c], ei + ej - 54);
+                        wp[c * ld] = fu_subtract(w[c], sum[c], ei + ej - Fc<T>::kShift + (ND > 4 ? 8 : 0));
                 }
             }
             while (plain) {
@@ -636,7 +702,8 @@ __global__ void __launch_bounds__(kFuThreads, 1) fc_update_kernel(
 }
 
 // Saves the input diagonal (for the pivot-ratio guard) and clears the status word.
-__global__ void fc_begin_kernel(const double *W, int64_t ld, int64_t n, double *out, int *err_word) {
+template <typename T>
+__global__ void fc_begin_kernel(const T *W, int64_t ld, int64_t n, T *out, int *err_word) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) out[i] = cm(W, ld, i, i);
     if (i == 0 && err_word) *err_word = 0;
@@ -655,10 +722,10 @@ static int fc_sms() {
     return sms;
 }
 
-static int fc_encode(PFN_cuTensorMapEncodeTiled_v12000 enc, CUtensorMap *m, void *planes, int64_t n, int rows,
-                     int nplanes) {
+static int fc_encode(PFN_cuTensorMapEncodeTiled_v12000 enc, CUtensorMap *m, void *planes, int64_t n, int digits,
+                     int rows, int nplanes) {
     const cuuint32_t estr[3] = {1, 1, 1};
-    const cuuint64_t dims[3] = {(cuuint64_t)kFcPair, (cuuint64_t)n, (cuuint64_t)kOzBal};
+    const cuuint64_t dims[3] = {(cuuint64_t)kFcPair, (cuuint64_t)n, (cuuint64_t)digits};
     const cuuint64_t strides[2] = {(cuuint64_t)kFcPair * 2, (cuuint64_t)n * kFcPair * 2};
     const cuuint32_t box[3] = {(cuuint32_t)kFuK, (cuuint32_t)rows, (cuuint32_t)nplanes};
     return enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, planes, dims, strides, box, estr,
@@ -668,46 +735,49 @@ static int fc_encode(PFN_cuTensorMapEncodeTiled_v12000 enc, CUtensorMap *m, void
                : -1;
 }
 
-int potrf_fast64_launch(double *W, int64_t n, int64_t ld, int64_t *d_info, double *diag0, double *min_ratio,
-                        int *err_word, int *sticky, cudaStream_t st) {
+template <typename T>
+int potrf_fast_launch(T *W, int64_t n, int64_t ld, int64_t *d_info, T *diag0, double *min_ratio, int *err_word,
+                      int *sticky, cudaStream_t st) {
+    constexpr int ND = Fc<T>::kDigits;
     static std::atomic<bool> attr{false};
     if (!attr.load()) {
-        if (cudaFuncSetAttribute(fc_update_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kFuSmem) != cudaSuccess)
+        if (cudaFuncSetAttribute(fc_update_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFuSmem<T>) !=
+            cudaSuccess)
             return -1;
         attr.store(true);
     }
     PFN_cuTensorMapEncodeTiled_v12000 enc = tma_encoder();
     if (!enc) return -1;
-    // digit planes [7][n][128], row exponents, reciprocal pivots, status word (own copy when
+    // digit planes [ND][n][128], row exponents, reciprocal pivots, status word (own copy when
     // the caller passes none)
-    const size_t planes_b = (size_t)kOzBal * n * kFcPair * 2, expo_b = ((size_t)n * 4 + 15) / 16 * 16;
+    const size_t planes_b = (size_t)ND * n * kFcPair * 2, expo_b = ((size_t)n * 4 + 15) / 16 * 16;
     StreamScratch ws(st);
     if (ws.alloc(planes_b + expo_b + kFcNb * 8 + 16) != cudaSuccess) return -1;
     char *base = (char *)ws.get();
     __nv_bfloat16 *planes = (__nv_bfloat16 *)base;
     int *expo = (int *)(base + planes_b);
-    double *rinv = (double *)(base + planes_b + expo_b);
+    T *rinv = (T *)(base + planes_b + expo_b);
     int *own_err = (int *)(base + planes_b + expo_b + kFcNb * 8);
     const int64_t pstride = n * kFcPair;
     int *ew = err_word ? err_word : own_err;
     CUtensorMap tmA, tmB;
-    if (fc_encode(enc, &tmA, planes, n, kFuM, 1) || fc_encode(enc, &tmB, planes, n, kFuN, kOzBal)) return -1;
+    if (fc_encode(enc, &tmA, planes, n, ND, kFuM, 1) || fc_encode(enc, &tmB, planes, n, ND, kFuN, ND)) return -1;
     {
         LaunchScope ls(K_MISC, st);
-        fc_begin_kernel<<<(unsigned)ceil_div(n, 256), 256, 0, st>>>(W, ld, n, diag0, err_word ? nullptr : own_err);
+        fc_begin_kernel<T><<<(unsigned)ceil_div(n, 256), 256, 0, st>>>(W, ld, n, diag0, err_word ? nullptr : own_err);
     }
     auto diag_panel = [&](int64_t p, int second) -> int64_t {  // rows left below the block
         const int b = (int)std::min<int64_t>(kFcNb, n - p);
         {
             LaunchScope ls(K_POTRF_FAST_DIAG, st, (double)b * b * b / 3.0);
-            launch_maybe_pdl(true, fc_diag_kernel, dim3(1), dim3(kFcDiagThreads), 0, st, W, ld, p, b,
-                             (const double *)diag0, rinv, d_info, min_ratio);
+            launch_maybe_pdl(true, fc_diag_kernel<T>, dim3(1), dim3(kFcDiagThreads), 0, st, W, ld, p, b,
+                             (const T *)diag0, rinv, d_info, min_ratio);
         }
         const int64_t rest = n - p - b;
         if (rest > 0) {
             LaunchScope ls(K_POTRF_FAST_PANEL, st, (double)rest * b * b);
-            launch_maybe_pdl(true, fc_panel_kernel, dim3((unsigned)ceil_div(rest, kFcRows)), dim3(kFcPanelThreads), 0,
-                             st, W, ld, n, p, second, (const double *)rinv, planes, pstride, expo,
+            launch_maybe_pdl(true, fc_panel_kernel<T>, dim3((unsigned)ceil_div(rest, kFcRows)), dim3(kFcPanelThreads), 0,
+                             st, W, ld, n, p, second, (const T *)rinv, planes, pstride, expo,
                              (const int64_t *)d_info);
         }
         return rest;
@@ -721,8 +791,8 @@ int potrf_fast64_launch(double *W, int64_t n, int64_t ld, int64_t *d_info, doubl
         // algorithmic work: entries of the lower part x columns x 2
         LaunchScope ls(K_POTRF_FAST_UPDATE, st,
                        ((double)m * cols - (double)cols * (cols - 1) / 2) * 2.0 * kchunks * kFuK);
-        launch_maybe_pdl(true, fc_update_kernel, dim3((unsigned)std::min<int64_t>(tiles, fc_sms())), dim3(kFuThreads),
-                         (size_t)kFuSmem, st, tmA, tmB, W, ld, q, n, p0, kchunks, (int)tiles, narrow,
+        launch_maybe_pdl(true, fc_update_kernel<T>, dim3((unsigned)std::min<int64_t>(tiles, fc_sms())), dim3(kFuThreads),
+                         (size_t)kFuSmem<T>, st, tmA, tmB, W, ld, q, n, p0, kchunks, (int)tiles, narrow,
                          (const int *)expo, (const int64_t *)d_info, ew, sticky);
     };
     for (int64_t p = 0; p < n; p += kFcPair) {
@@ -733,5 +803,10 @@ int potrf_fast64_launch(double *W, int64_t n, int64_t ld, int64_t *d_info, doubl
     }
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
+
+template int potrf_fast_launch<double>(double *, int64_t, int64_t, int64_t *, double *, double *, int *, int *,
+                                       cudaStream_t);
+template int potrf_fast_launch<float>(float *, int64_t, int64_t, int64_t *, float *, double *, int *, int *,
+                                      cudaStream_t);
 
 }  // namespace lla

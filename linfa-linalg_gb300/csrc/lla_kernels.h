@@ -22,9 +22,6 @@ int potrf_exact_launch(T *W, T *S, T *D, int64_t n, int64_t ld, int64_t *d_info,
 template <typename T>
 int potrf_fast_launch(T *W, int64_t n, int64_t ld, int64_t *d_info, T *diag0, double *min_ratio,
                       int *err_word, int *sticky, cudaStream_t st);
-// Its FP64 form (lla_fp64_chol.cu).
-int potrf_fast64_launch(double *W, int64_t n, int64_t ld, int64_t *d_info, double *diag0, double *min_ratio,
-                        int *err_word, int *sticky, cudaStream_t st);
 
 // Triangular solve op(T) X = B in place (see lla_trsm.cu).  ws: trsm_ws_ints
 // ints of scratch; err_word: device int, 0 on entry; sticky (optional): a

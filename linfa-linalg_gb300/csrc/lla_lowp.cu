@@ -517,7 +517,12 @@ __global__ void __launch_bounds__(256, 2) lowp_panel_kernel(float *L, int64_t ld
 int lowp_factor_launch(float *L, int64_t n, int64_t ld, const lla_refine_opts &opts, int64_t *info,
                        float *diag0, double *min_ratio, Ctx *c, cudaStream_t st) {
     const int upd = opts.update;
-    if (upd == LLA_UPDATE_FP32) return potrf_fast_launch<float>(L, n, ld, info, diag0, min_ratio, nullptr, nullptr, st);
+    if (upd == LLA_UPDATE_FP32) {
+        if (c->mixed.tcerr.ensure(4 * sizeof(int)) != cudaSuccess ||
+            cudaMemsetAsync(c->mixed.tcerr.p, 0, 4 * sizeof(int), st) != cudaSuccess)
+            return -1;
+        return potrf_fast_launch<float>(L, n, ld, info, diag0, min_ratio, (int *)c->mixed.tcerr.p, nullptr, st);
+    }
     const bool fp16 = (upd == LLA_UPDATE_FP16 || upd == LLA_UPDATE_FP16X3);
     const int terms = (upd == LLA_UPDATE_BF16 || upd == LLA_UPDATE_FP16) ? 1
                       : (upd == LLA_UPDATE_BF16X6)                        ? 3
@@ -647,13 +652,10 @@ extern "C" int lla_spotrf_mixed_device(float *dA, int64_t n, int64_t ld, int upd
         e = cudaGetLastError();
         return lla__set_cuda_error(err, e == cudaSuccess ? cudaErrorUnknown : e);
     }
-    if (update != LLA_UPDATE_FP32) {
-        int flag = 0;
-        if ((e = cudaMemcpyAsync(&flag, c->mixed.tcerr.p, sizeof(int), cudaMemcpyDeviceToHost, st)) !=
-                cudaSuccess ||
-            (e = cudaStreamSynchronize(st)) != cudaSuccess)
-            return lla__set_cuda_error(err, e);
-        if (flag) return lla__set_status(err, flag);
-    }
+    int flag = 0;
+    if ((e = cudaMemcpyAsync(&flag, c->mixed.tcerr.p, sizeof(int), cudaMemcpyDeviceToHost, st)) != cudaSuccess ||
+        (e = cudaStreamSynchronize(st)) != cudaSuccess)
+        return lla__set_cuda_error(err, e);
+    if (flag) return lla__set_status(err, flag);
     return LLA_OK;
 }

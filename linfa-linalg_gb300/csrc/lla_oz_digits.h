@@ -103,7 +103,7 @@ __host__ __device__ __forceinline__ void oz_digits_packed4(const int64_t (&b)[4]
     }
 }
 
-// ---- balanced 8-bit digits (the FP64 trailing update, lla_fp64_chol.cu) ----
+// ---- balanced 8-bit digits (the trailing updates, lla_fast_chol.cu) ----
 //
 // An integer of up to 9 bits magnitude 2^7 is exact in BF16, so signed digits
 // in [-128, 128] carry 8 bits each: seven of them hold a value rounded to the
@@ -139,6 +139,43 @@ __host__ __device__ __forceinline__ void oz_balanced_pair(int64_t va, int64_t vb
 #pragma unroll
     for (int p = 0; p < kOzBal; ++p) {
         const int s = 8 * (kOzBal - 1 - p);
+        const uint32_t mask = p == 0 ? 0x1ffu : 0xffu;
+        const uint32_t ma = 0x4b000000u | ((uint32_t)(wa >> s) & mask), mb = 0x4b000000u | ((uint32_t)(wb >> s) & mask);
+        float fa, fb;
+        memcpy(&fa, &ma, 4);
+        memcpy(&fb, &mb, 4);
+        fa -= 8388736.f;
+        fb -= 8388736.f;
+        uint32_t ba, bb;
+        memcpy(&ba, &fa, 4);
+        memcpy(&bb, &fb, 4);
+        out[p] = oz_pack_bf16(ba, bb);
+    }
+}
+
+// The same for FP32 values, to the nearest multiple of 2^(e-31) (|V| <= 2^31), in
+// four digits.
+constexpr int kOzBal32 = 4;
+__host__ __device__ __forceinline__ int64_t oz_fixed31(int32_t bits, int e) {
+    const int eb = (bits >> 23) & 0xff;
+    uint64_t mant = (uint32_t)bits & 0x7fffffu;
+    if (eb != 0) mant |= 0x800000u;
+    const int shift = (eb != 0 ? eb : 1) - 150 + 31 - e;  // <= 7 since |a| < 2^e
+    uint64_t V = 0;
+    if (eb != 0xff) {
+        if (shift >= 0)
+            V = mant << shift;
+        else if (shift >= -25)
+            V = (mant + (1ull << (-shift - 1))) >> (-shift);
+    }
+    return bits < 0 ? -(int64_t)V : (int64_t)V;
+}
+__host__ __device__ __forceinline__ void oz_balanced_pair(int64_t va, int64_t vb, uint32_t (&out)[kOzBal32]) {
+    const uint64_t bias = 0x80808080ull;
+    const uint64_t wa = (uint64_t)va + bias, wb = (uint64_t)vb + bias;
+#pragma unroll
+    for (int p = 0; p < kOzBal32; ++p) {
+        const int s = 8 * (kOzBal32 - 1 - p);
         const uint32_t mask = p == 0 ? 0x1ffu : 0xffu;
         const uint32_t ma = 0x4b000000u | ((uint32_t)(wa >> s) & mask), mb = 0x4b000000u | ((uint32_t)(wb >> s) & mask);
         float fa, fb;

@@ -111,6 +111,35 @@ int main() {
             CHECK(s == v[u], "digits of %lld\n", (long long)v[u]);
         }
     }
+    // the same for FP32 values: multiples of 2^(e-31), four digits
+    for (long t = 0; t < 400000; ++t) {
+        const int e = (int)(g() % 201) - 100;
+        int64_t v[2];
+        for (int u = 0; u < 2; ++u) {
+            float a = (float)std::ldexp(U(g), e - (int)(g() % 36));
+            if (std::fabs(a) >= std::ldexp(1.0, e)) a = std::nextafter((float)std::ldexp(1.0, e), 0.f);
+            if (g() & 1) a = -a;
+            if (t % 101 == u) a = t & 1 ? 0.f : -0.f;
+            if (t % 103 == u) a = std::nextafter((float)std::ldexp(1.0, e), 0.f);
+            int32_t b;
+            std::memcpy(&b, &a, 4);
+            v[u] = oz_fixed31(b, e);
+            CHECK(std::fabs(std::ldexp((double)a, 31 - e) - (double)v[u]) <= 0.5, "fixed31(%a, %d)\n", a, e);
+        }
+        uint32_t q[kOzBal32];
+        oz_balanced_pair(v[0], v[1], q);
+        for (int u = 0; u < 2; ++u) {
+            int64_t s = 0;
+            for (int p = 0; p < kOzBal32; ++p) {
+                const uint32_t w = (u ? q[p] & 0xffff0000u : q[p] << 16);
+                float f;
+                std::memcpy(&f, &w, 4);
+                CHECK(std::fabs(f) <= 128.f && f == std::rint(f), "digit %g\n", f);
+                s = s * 256 + (int64_t)f;
+            }
+            CHECK(s == v[u], "digits of %lld\n", (long long)v[u]);
+        }
+    }
     // 64-bit integer times a power of two, rounded to nearest even
     for (long t = 0; t < 1000000; ++t) {
         int64_t T = (int64_t)g() >> (g() % 64);

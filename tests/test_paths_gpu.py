@@ -54,34 +54,37 @@ def _potrf(gpu_lla, torch, A, ld=None):
 
 @pytest.mark.parametrize("n", [1, 2, 63, 64, 65, 127, 128, 129, 192, 193, 257, 320, 1000])
 @pytest.mark.parametrize("pad", [0, 3])
-def test_fast_fp64_factor(gpu_lla, n, pad):
+@pytest.mark.parametrize("dtype", ["float64", "float32"])
+def test_fast_factor(gpu_lla, n, pad, dtype):
     """Digit-sliced trailing updates: edges of the 64-column panels, the 128-row
     tiles and the pairs of panels, against ||L L^T - A|| <= 10 n eps ||A||; the
     upper triangle stays untouched."""
     torch = _torch()
     A, g = _spd(torch, n, 0.5, n)
     d = torch.exp2(20 * torch.rand(n, dtype=torch.float64, device="cuda", generator=g) - 10)
-    A = A * d[:, None] * d[None, :]
+    A = (A * d[:, None] * d[None, :]).to(getattr(torch, dtype))
     A = torch.tril(A) + torch.tril(A, -1).T
     L, info = _potrf(gpu_lla, torch, A, n + pad)
     assert info == -1
-    low = torch.tril(L)
-    S = A / d[:, None] / d[None, :]
+    low = torch.tril(L).double()
+    S = A.double() / d[:, None] / d[None, :]
     R = (low @ low.T) / d[:, None] / d[None, :] - S
-    assert float(R.norm() / S.norm()) <= 10 * n * 2.2e-16
+    assert float(R.norm() / S.norm()) <= 10 * n * torch.finfo(A.dtype).eps
     assert bool((torch.triu(L, 1) == torch.triu(A, 1)).all())
 
 
 @pytest.mark.parametrize("row", [0, 1, 30, 31, 32, 33, 63, 64, 65, 100, 127, 128, 200, 255, 299])
-def test_fast_fp64_factor_reports_the_failing_row(gpu_lla, row):
+@pytest.mark.parametrize("dtype", ["float64", "float32"])
+def test_fast_factor_reports_the_failing_row(gpu_lla, row, dtype):
     torch = _torch()
     A, _ = _spd(torch, 300, 1.0, 3)
+    A = A.to(getattr(torch, dtype))
     A[row, row] = -1.0
     L, info = _potrf(gpu_lla, torch, A)
     assert info == row
     if row:
-        R = torch.linalg.cholesky(A[:row, :row])
-        assert float((torch.tril(L[:row, :row]) - R).norm() / R.norm()) <= 10 * 300 * 2.2e-16
+        R = torch.linalg.cholesky(A[:row, :row].double())
+        assert float((torch.tril(L[:row, :row]) - R).norm() / R.norm()) <= 10 * 300 * torch.finfo(A.dtype).eps
 
 
 def test_fast_fp64_factor_non_finite_and_subnormal_rows(gpu_lla):
