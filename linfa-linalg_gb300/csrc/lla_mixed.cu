@@ -283,15 +283,25 @@ __global__ void update_x_kernel(double *X, int64_t ldx, const double *s, const f
 }
 
 // R = B - A_sym X on the FP64 tensor pipe (mma.sync m16n8k16 .f64).
-// CTA tile: 32 rows x 64 RHS columns, K chunks of 32; four warps, each 16 x 32
-// (four m16n8 MMAs per k16 step).  A_sym(i,k) reads the lower triangle:
-// A[i + k*lda] for k <= i, A[k + i*lda] otherwise.  Also colmax_r.
-constexpr int kResRows = 32, kResCols = 64, kResK = 32;
+// Four warps, each 16 rows x 8 NI right-hand sides: WC of them side by side along
+// the right-hand sides, the others along the rows; K chunks of 32.  The FP64 pipe
+// bounds it (16 x 8 x 16 multiply-adds take 1200 cycles of an SM), so the tile is
+// as wide as the right-hand sides need (8, 16, 32, or 64 columns at a time): with
+// 16 of them a 64-wide tile did four times the work (n = 3001: 1.30 -> 0.37 ms a
+// residual).  A_sym(i,k) reads the lower triangle: A[i + k*lda] for k <= i,
+// A[k + i*lda] otherwise.  Also colmax_r.
+constexpr int kResK = 32;
+template <int NI, int WC>
+struct ResTile {
+    static constexpr int kRows = 16 * (4 / WC), kCols = 8 * NI * WC;
+    static constexpr int kXStride = kCols == 8 ? 20 : kCols + 4;  // 4 (mod 16): conflict-free fragments
+};
 
 // K is split into `splits` contiguous ranges (blockIdx.z) so that the grid
 // covers the SMs in several full waves; with splits > 1 each range writes its
 // partial A_sym X into P[z] and residual_combine_kernel forms R = B - sum_z P[z]
 // in a fixed order (deterministic, no atomics).
+template <int NI, int WC>
 __global__ void __launch_bounds__(128) residual_dmma_kernel(const double *__restrict__ A, int64_t lda,
                                                             int64_t n, const double *__restrict__ X,
                                                             int64_t ldx, const double *__restrict__ B,
@@ -299,16 +309,17 @@ __global__ void __launch_bounds__(128) residual_dmma_kernel(const double *__rest
                                                             int64_t m, double *colmax_r, int splits,
                                                             double *P, const int *state) {
     if (refine_done(state)) return;
-    __shared__ double As[kResK][kResRows + 4];  // [k][row], stride 36 = 4 (mod 16)
-    __shared__ double Xs[kResK][kResCols + 4];  // [k][col], stride 68 = 4 (mod 16)
+    constexpr int kResRows = ResTile<NI, WC>::kRows, kResCols = ResTile<NI, WC>::kCols;
+    __shared__ double As[kResK][kResRows + 4];                 // [k][row], stride 4 (mod 16)
+    __shared__ double Xs[kResK][ResTile<NI, WC>::kXStride];    // [k][col]
     const int64_t i0 = (int64_t)blockIdx.x * kResRows;
     const int64_t c0 = (int64_t)blockIdx.y * kResCols;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int g = lane >> 2, t = lane & 3;
-    const int wr = (warp & 1) * 16, wc = (warp >> 1) * 32;
-    double acc[4][4];
+    const int wr = (warp / WC) * 16, wc = (warp % WC) * 8 * NI;
+    double acc[NI][4];
 #pragma unroll
-    for (int ni = 0; ni < 4; ++ni)
+    for (int ni = 0; ni < NI; ++ni)
 #pragma unroll
         for (int q = 0; q < 4; ++q) acc[ni][q] = 0.0;
     const int64_t kchunks = (n + kResK - 1) / kResK;
@@ -339,15 +350,15 @@ __global__ void __launch_bounds__(128) residual_dmma_kernel(const double *__rest
         __syncthreads();
 #pragma unroll
         for (int kk = 0; kk < kResK; kk += 16) {
-            double af[8], bf[4][4];
+            double af[8], bf[NI][4];
 #pragma unroll
             for (int q = 0; q < 8; ++q) af[q] = As[kk + t + 4 * (q >> 1)][wr + g + 8 * (q & 1)];
 #pragma unroll
-            for (int ni = 0; ni < 4; ++ni)
+            for (int ni = 0; ni < NI; ++ni)
 #pragma unroll
                 for (int q = 0; q < 4; ++q) bf[ni][q] = Xs[kk + t + 4 * q][wc + ni * 8 + g];
 #pragma unroll
-            for (int ni = 0; ni < 4; ++ni)
+            for (int ni = 0; ni < NI; ++ni)
                 asm volatile(
                     "mma.sync.aligned.m16n8k16.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, "
                     "{%4,%5,%6,%7,%8,%9,%10,%11}, {%12,%13,%14,%15}, {%0,%1,%2,%3};\n"
@@ -361,7 +372,7 @@ __global__ void __launch_bounds__(128) residual_dmma_kernel(const double *__rest
     if (splits > 1) {  // partial product of this K range
         double *Pz = P + (int64_t)blockIdx.z * n * m;
 #pragma unroll
-        for (int ni = 0; ni < 4; ++ni)
+        for (int ni = 0; ni < NI; ++ni)
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
                 const int64_t i = i0 + wr + g + 8 * (q >> 1);
@@ -372,7 +383,7 @@ __global__ void __launch_bounds__(128) residual_dmma_kernel(const double *__rest
     }
     // epilogue: R = B - acc, and column maxima of |R|
 #pragma unroll
-    for (int ni = 0; ni < 4; ++ni) {
+    for (int ni = 0; ni < NI; ++ni) {
         double cm2[2] = {0.0, 0.0};
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
@@ -541,6 +552,10 @@ int refine_check_launch(double *words, int64_t m, double tol, int max_iters, cud
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
+// Tile of a residual with m right-hand sides.
+static int res_rows(int64_t m) { return m <= 32 ? ResTile<4, 1>::kRows : ResTile<4, 2>::kRows; }
+static int res_cols(int64_t m) { return m <= 8 ? 8 : (m <= 16 ? 16 : (m <= 32 ? 32 : 64)); }
+
 int residual_splits(int64_t n, int64_t m) {
     static int sms = 0;
     if (!sms) {
@@ -549,7 +564,7 @@ int residual_splits(int64_t n, int64_t m) {
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         if (sms <= 0) sms = 1;
     }
-    const int64_t tiles = (int64_t)gx(n, kResRows) * gx(m, kResCols);
+    const int64_t tiles = (int64_t)gx(n, res_rows(m)) * gx(m, res_cols(m));
     // smallest split giving at least four waves of CTAs (at most 8)
     int s = 1;
     while (s < 8 && tiles * s < 4 * (int64_t)sms && n / (kResK * (s + 1)) >= 4) ++s;
@@ -563,8 +578,12 @@ int residual_launch(const double *A, int64_t lda, int64_t n, const double *X, in
     {
         // algorithmic work: 2 n^2 m flops
         LaunchScope ls(K_RESIDUAL, st, 2.0 * n * n * m);
-        residual_dmma_kernel<<<dim3(gx(n, kResRows), gx(m, kResCols), splits), 128, 0, st>>>(
-            A, lda, n, X, ldx, B, ldb, R, ldr, m, colmax_r, splits, P, state);
+        const dim3 grid(gx(n, res_rows(m)), gx(m, res_cols(m)), splits);
+        auto kern = m <= 8    ? residual_dmma_kernel<1, 1>
+                    : m <= 16 ? residual_dmma_kernel<2, 1>
+                    : m <= 32 ? residual_dmma_kernel<4, 1>
+                              : residual_dmma_kernel<4, 2>;
+        kern<<<grid, 128, 0, st>>>(A, lda, n, X, ldx, B, ldb, R, ldr, m, colmax_r, splits, P, state);
     }
     if (splits > 1) {
         LaunchScope ls(K_REFINE, st, 8.0 * n * m * (splits + 2));

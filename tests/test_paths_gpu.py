@@ -239,3 +239,20 @@ def test_exact_factor_matches_the_oracle(gpu_lla, dtype, n, kind):
         gpu_lla.set_algorithm(prev)
     assert (fail >= 0) == (st["code"] != 0) and (fail < 0 or fail == st["index"])
     assert ((got == want) | (np.isnan(got) & np.isnan(want))).all()
+
+
+@pytest.mark.parametrize("n", [1, 33, 64, 65, 200, 1000])
+@pytest.mark.parametrize("m", [1, 8, 9, 16, 17, 32, 33, 65])
+def test_fp64_residual_tiles(gpu_lla, n, m):
+    """FP64 residual on each of its tile widths, against an FP64 product of the same operands:
+    two sums of n products in different orders differ by at most 2 n eps |A| |x|."""
+    torch = _torch()
+    A, g = _spd(torch, n, 1.0, n + m)
+    X = torch.randn(m, n, dtype=torch.float64, device="cuda", generator=g).T
+    B = torch.randn(m, n, dtype=torch.float64, device="cuda", generator=g).T
+    R = torch.empty(m, n, dtype=torch.float64, device="cuda").T
+    low = torch.tril(A).T.contiguous().T  # only the lower triangle is read
+    gpu_lla.residual_device(low, X, B, R, "fp64")
+    torch.cuda.synchronize()
+    tol = 2 * (n + 2) * 2.2e-16 * (A.abs() @ X.abs() + B.abs())
+    assert bool(((R - (B - A @ X)).abs() <= tol).all())
