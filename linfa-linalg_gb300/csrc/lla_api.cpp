@@ -696,8 +696,7 @@ int orthonormalize_impl(const T *v, int64_t rows, int64_t cols, int64_t rs, int6
     LLA_TRY_CUDA(c->work_a.ensure(sizeof(T) * k * k));
     LLA_TRY_CUDA(c->lob_g.ensure(sizeof(T) * k * k));
     LLA_TRY_CUDA(c->lob_p.ensure(sizeof(T) * atb_ws_elems(n, k, k)));
-    LLA_TRY_CUDA(c->lob_t.ensure(sizeof(T) * k * (n > 0 ? n : 1)));
-    T *WV = (T *)c->work_b.p, *G = (T *)c->work_a.p, *Gc = (T *)c->lob_g.p, *VT = (T *)c->lob_t.p;
+    T *WV = (T *)c->work_b.p, *G = (T *)c->work_a.p, *Gc = (T *)c->lob_g.p;
     LLA_TRY_CUDA(launch_status(import_launch<T>((const T *)c->raw_a.p, drs, dcs, n, k, WV, n, c->stream)));
     LLA_TRY_CUDA(launch_status(atb_launch<T>(WV, n, WV, n, n, k, k, G, k, (T *)c->lob_p.p, 1, c->stream)));
     LLA_TRY_CUDA(cudaMemcpyAsync(Gc, G, sizeof(T) * k * k, cudaMemcpyDeviceToDevice, c->stream));
@@ -713,11 +712,17 @@ int orthonormalize_impl(const T *v, int64_t rows, int64_t cols, int64_t rs, int6
     LLA_TRY_CUDA(launch_status(export_launch<T>(G, k, (T *)c->raw_c.p, lrs_d, lcs_d, k, k, EXPORT_LOWER_ZERO_UPPER,
                                                 -1, c->stream)));
     if (n > 0) {
-        // V^T (k x n), L Z = V^T, U = Z^T
-        LLA_TRY_CUDA(launch_status(import_launch<T>(WV, n, 1, k, n, VT, k, c->stream)));
-        LLA_TRY_CUDA(trsm_on_device<T>(*c, G, k, k, /*lower=*/1, /*trans=*/0, nullptr, VT, k, n, use_exact(k), &to));
-        if (to) return lla__set_status(err, LLA_ERR_TIMEOUT);
-        LLA_TRY_CUDA(launch_status(import_launch<T>(VT, k, 1, n, k, WV, n, c->stream)));
+        if (k <= kSolveRowsMax) {  // U = V L^-T row by row, where V lies
+            LLA_TRY_CUDA(launch_status(solve_rows_launch<T>(G, k, k, WV, n, n, use_exact(k), c->stream)));
+        } else {  // V^T (k x n), L Z = V^T, U = Z^T
+            LLA_TRY_CUDA(c->lob_t.ensure(sizeof(T) * k * n));
+            T *VT = (T *)c->lob_t.p;
+            LLA_TRY_CUDA(launch_status(import_launch<T>(WV, n, 1, k, n, VT, k, c->stream)));
+            LLA_TRY_CUDA(
+                trsm_on_device<T>(*c, G, k, k, /*lower=*/1, /*trans=*/0, nullptr, VT, k, n, use_exact(k), &to));
+            if (to) return lla__set_status(err, LLA_ERR_TIMEOUT);
+            LLA_TRY_CUDA(launch_status(import_launch<T>(VT, k, 1, n, k, WV, n, c->stream)));
+        }
         View vu{(char *)u, n, k, urs, ucs, sizeof(T)};
         int64_t urs_d, ucs_d;
         LLA_TRY_CUDA(prepare_out(vu, c->raw_b, urs_d, ucs_d));

@@ -112,6 +112,10 @@ size_t atb_ws_elems(int64_t n, int64_t ka, int64_t kb);
 template <typename T>
 int atb_launch(const T *A, int64_t lda, const T *B, int64_t ldb, int64_t n, int64_t ka, int64_t kb, T *C,
                int64_t ldc, T *P, int symmetric, cudaStream_t st);
+// X (n x k) <- X L^-T, one row of X a thread (k <= kSolveRowsMax, n >= 2 k rows pay).
+constexpr int64_t kSolveRowsMax = 48;
+template <typename T>
+int solve_rows_launch(const T *L, int64_t ldl, int64_t k, T *X, int64_t ldx, int64_t n, bool exact, cudaStream_t st);
 // V (n x k) -= Y (n x ky) U (ky x k).
 template <typename T>
 int sub_tall_launch(T *V, int64_t ldv, const T *Y, int64_t ldy, const T *U, int64_t ldu, int64_t n, int64_t ky,

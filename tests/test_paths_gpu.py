@@ -256,3 +256,31 @@ def test_fp64_residual_tiles(gpu_lla, n, m):
     torch.cuda.synchronize()
     tol = 2 * (n + 2) * 2.2e-16 * (A.abs() @ X.abs() + B.abs())
     assert bool(((R - (B - A @ X)).abs() <= tol).all())
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("k", [1, 2, 15, 16, 17, 32, 33, 45, 48, 49, 63, 64, 80])
+@pytest.mark.parametrize("n", [100, 129, 5000])
+def test_cholesky_qr_forms(gpu_lla, dtype, k, n):
+    """Gram products dealt out one by one or in tiles, and substitutions row by row or through
+    the transposed block: L against the Gram matrix (n products summed in any order: n eps
+    sum |v||v|, plus the factor's k eps), U bit-identical to the oracle's solve with that L."""
+    from oracle import oracle as ora
+    rng = np.random.default_rng(k + n)
+    v = np.asfortranarray((rng.standard_normal((n, k)) * 10.0 ** rng.uniform(-1, 1, k)).astype(dtype))
+    u, l = gpu_lla.orthonormalize(v)
+    w = v.astype(np.float64)
+    low = l.astype(np.float64)
+    err = np.abs(low @ low.T - w.T @ w)
+    norms = np.sqrt((w * w).sum(0))
+    assert (err <= (n + 2 * k + 2) * np.finfo(dtype).eps * norms[:, None] * norms[None, :]).all()
+    vt = np.array(v.T, order="C")
+    assert ora.solve_triangular_inplace(np.array(l, order="C"), vt, "lower")["code"] == 0
+    assert np.array_equal(u, vt.T)
+    y = np.asfortranarray(rng.standard_normal((n, 7)).astype(dtype))
+    lyy = np.linalg.cholesky((y.astype(np.float64).T @ y.astype(np.float64))).astype(dtype)
+    x = v.copy()
+    gpu_lla.apply_constraints(x, lyy, y)
+    g = y.astype(np.float64).T @ w
+    want = w - y.astype(np.float64) @ np.linalg.solve(lyy.astype(np.float64), g)
+    assert np.abs(x - want).max() <= 1e3 * np.finfo(dtype).eps * np.sqrt(n) * np.abs(w).max()
