@@ -304,18 +304,51 @@ cudaError_t download(Ctx &c, const View &v, DevBuf &raw, HostBuf &stage) {
     return cudaSuccess;
 }
 
+// A download in two halves around one synchronisation of the stream, so that a
+// call with several results waits once: begin() copies a strided view, or a small
+// contiguous one, into its pinned staging buffer; finish(), after the caller has
+// synchronised and decided that the results stand, moves them into the view (a
+// large contiguous view is copied there directly and waited for: above 128 KiB
+// the driver's own staging beats a copy on this thread, invc of n = 300 948 us
+// against 1008).
+constexpr size_t kStageBytes = 1u << 17;
+
+bool staged_download(const View &v) {
+    const size_t bytes = (size_t)(v.rows * v.cols) * v.esz;
+    return !(colmajor_contig(v) || rowmajor_contig(v)) || bytes <= kStageBytes;
+}
+cudaError_t begin_download(Ctx &c, const View &v, DevBuf &raw, HostBuf &stage) {
+    const size_t bytes = (size_t)(v.rows * v.cols) * v.esz;
+    if (bytes == 0 || !staged_download(v)) return cudaSuccess;
+    cudaError_t e = stage.ensure(bytes);
+    if (e != cudaSuccess) return e;
+    return cudaMemcpyAsync(stage.p, raw.p, bytes, cudaMemcpyDeviceToHost, c.stream);
+}
+cudaError_t finish_download(Ctx &c, const View &v, DevBuf &raw, HostBuf &stage) {
+    const size_t bytes = (size_t)(v.rows * v.cols) * v.esz;
+    if (bytes == 0) return cudaSuccess;
+    if (!staged_download(v)) return download(c, v, raw, stage);
+    if (colmajor_contig(v) || rowmajor_contig(v))
+        std::memcpy(v.p, stage.p, bytes);
+    else
+        gather_scatter(v, (char *)stage.p, false);
+    return cudaSuccess;
+}
+
 cudaError_t launch_status(int rc) {
     if (rc == 0) return cudaSuccess;
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? cudaErrorUnknown : e;
 }
 
-// Small device/host words: [0] int64 info, [1] double min_ratio, [2] int err_word.
+// Small device/host words: the factorisation's info, smallest relative pivot and
+// status (a bounded wait that gave up), the solves' status, the predicate's flag.
 struct Words {
     int64_t info;
     double min_ratio;
     int32_t err_word;
     int32_t flag;
+    int32_t factor_err;
 };
 
 cudaError_t reset_words(Ctx &c) {
@@ -324,6 +357,7 @@ cudaError_t reset_words(Ctx &c) {
     h->min_ratio = 1e300;
     h->err_word = 0;
     h->flag = 1;
+    h->factor_err = 0;
     return cudaMemcpyAsync(c.small_dev.p, h, sizeof(Words), cudaMemcpyHostToDevice, c.stream);
 }
 
@@ -341,6 +375,21 @@ Words *dev_words(Ctx &c) { return (Words *)c.small_dev.p; }
 
 namespace lla {
 
+// Enqueues the factorisation of the column-major n x n W (words reset before).
+template <typename T>
+static cudaError_t factor_enqueue(Ctx &c, T *W, int64_t n, int64_t ld, bool exact) {
+    cudaError_t e;
+    if ((e = c.aux_d.ensure(sizeof(T) * n)) != cudaSuccess) return e;
+    if (!exact)
+        return launch_status(potrf_fast_launch<T>(W, n, ld, &dev_words(c)->info, (T *)c.aux_d.p,
+                                                  &dev_words(c)->min_ratio, &dev_words(c)->factor_err, nullptr, c.stream));
+    if ((e = c.aux_s.ensure(sizeof(T) * ld * n)) != cudaSuccess) return e;
+    return launch_status(potrf_exact_launch<T>(W, (T *)c.aux_s.p, (T *)c.aux_d.p, n, ld, &dev_words(c)->info, c.stream));
+}
+
+// Whether a FAST factorisation's outcome has to be decided in EXACT order.
+static bool fast_undecided(const Words &w) { return w.info >= 0 || w.min_ratio < kPivotGuard; }
+
 // Factor the column-major n x n W in place.  On a FAST failure or a
 // near-singular FAST factorisation, W is re-imported from (R, drs, dcs) and
 // factored in EXACT order, whose verdict stands.  *fail receives the failing
@@ -353,13 +402,10 @@ cudaError_t factor_on_device(Ctx &c, T *W, int64_t n, int64_t ld, bool exact, co
     Words w;
     if ((e = reset_words(c)) != cudaSuccess) return e;
     if (!exact) {
-        if ((e = c.aux_d.ensure(sizeof(T) * n)) != cudaSuccess) return e;
-        e = launch_status(potrf_fast_launch<T>(W, n, ld, &dev_words(c)->info, (T *)c.aux_d.p,
-                                               &dev_words(c)->min_ratio, &dev_words(c)->err_word, nullptr, c.stream));
-        if (e != cudaSuccess) return e;
+        if ((e = factor_enqueue<T>(c, W, n, ld, false)) != cudaSuccess) return e;
         if ((e = read_words(c, w)) != cudaSuccess) return e;
-        if ((*timed_out = (w.err_word == LLA_ERR_TIMEOUT))) return cudaSuccess;
-        if (w.info < 0 && !(w.min_ratio < kPivotGuard)) {
+        if ((*timed_out = (w.factor_err == LLA_ERR_TIMEOUT))) return cudaSuccess;
+        if (!fast_undecided(w)) {
             *fail = -1;
             return cudaSuccess;
         }
@@ -368,25 +414,28 @@ cudaError_t factor_on_device(Ctx &c, T *W, int64_t n, int64_t ld, bool exact, co
             return e;
         if ((e = reset_words(c)) != cudaSuccess) return e;
     }
-    if ((e = c.aux_s.ensure(sizeof(T) * ld * n)) != cudaSuccess) return e;
-    if ((e = c.aux_d.ensure(sizeof(T) * n)) != cudaSuccess) return e;
-    e = launch_status(potrf_exact_launch<T>(W, (T *)c.aux_s.p, (T *)c.aux_d.p, n, ld,
-                                            &dev_words(c)->info, c.stream));
-    if (e != cudaSuccess) return e;
+    if ((e = factor_enqueue<T>(c, W, n, ld, true)) != cudaSuccess) return e;
     if ((e = read_words(c, w)) != cudaSuccess) return e;
     *fail = w.info;
     return cudaSuccess;
+}
+
+// Enqueues a triangular solve (words reset before; err_word collects a timeout).
+template <typename T>
+static cudaError_t trsm_enqueue(Ctx &c, const T *M, int64_t ld, int64_t n, int lower, int trans, const T *diag, T *B,
+                                int64_t ldb, int64_t m, bool exact) {
+    cudaError_t e = c.ws.ensure(sizeof(int) * trsm_ws_ints(n, m));
+    if (e != cudaSuccess) return e;
+    return launch_status(trsm_launch<T>(M, ld, n, lower, trans, diag, B, ldb, m, exact, (int *)c.ws.p,
+                                        &dev_words(c)->err_word, c.stream));
 }
 
 template <typename T>
 cudaError_t trsm_on_device(Ctx &c, const T *M, int64_t ld, int64_t n, int lower, int trans,
                            const T *diag, T *B, int64_t ldb, int64_t m, bool exact, int *timed_out) {
     cudaError_t e;
-    if ((e = c.ws.ensure(sizeof(int) * trsm_ws_ints(n, m))) != cudaSuccess) return e;
     if ((e = reset_words(c)) != cudaSuccess) return e;
-    e = launch_status(trsm_launch<T>(M, ld, n, lower, trans, diag, B, ldb, m, exact, (int *)c.ws.p,
-                                     &dev_words(c)->err_word, c.stream));
-    if (e != cudaSuccess) return e;
+    if ((e = trsm_enqueue<T>(c, M, ld, n, lower, trans, diag, B, ldb, m, exact)) != cudaSuccess) return e;
     Words w;
     if ((e = read_words(c, w)) != cudaSuccess) return e;
     *timed_out = (w.err_word == LLA_ERR_TIMEOUT);
@@ -419,6 +468,57 @@ bool bad_view(const void *p, int64_t rows, int64_t cols) {
     return rows < 0 || cols < 0 || (p == nullptr && rows * cols > 0);
 }
 
+// The part that the factoring calls share, with one synchronisation where the
+// outcome is the usual one: the factor of W (imported from the raw copy of view v,
+// (R, drs, dcs)), then whatever the caller enqueues behind it, the factor's export
+// with mode `good` and the downloads; the outcome is read together with the
+// results, and only if it is not a success are they dropped and the rest done
+// step by step: a FAST outcome that the reference's arithmetic has to decide, and
+// a failure, which exports only the rows the reference would have written.
+// `then` enqueues the work behind a factor in W (again after an EXACT re-run) and
+// its downloads' first half; `keep` moves its results to the caller once they stand.
+template <typename T, typename Then, typename Keep>
+int factor_export(Ctx *c, const View &v, T *W, const T *R, int64_t drs, int64_t dcs, int good, Then then, Keep keep,
+                  bool &failed, lla_error *err) {
+    const int64_t n = v.rows;
+    const bool exact = use_exact(n);
+    Words w;
+    failed = false;
+    LLA_TRY_CUDA(reset_words(*c));
+    LLA_TRY_CUDA(factor_enqueue<T>(*c, W, n, n, exact));
+    LLA_TRY_CUDA(then());
+    LLA_TRY_CUDA(launch_status(export_launch<T>(W, n, (T *)c->raw_a.p, drs, dcs, n, n, good, -1, c->stream)));
+    LLA_TRY_CUDA(begin_download(*c, v, c->raw_a, c->stage_a));
+    LLA_TRY_CUDA(read_words(*c, w));
+    if (w.factor_err == LLA_ERR_TIMEOUT) return lla__set_status(err, LLA_ERR_TIMEOUT);
+    if (w.info >= 0 || (!exact && fast_undecided(w))) {
+        // the raw copy has been written to: the caller's view still holds the original
+        LLA_TRY_CUDA(upload(*c, v, c->raw_a, c->stage_a, drs, dcs));
+        if (!exact) {
+            LLA_TRY_CUDA(launch_status(import_launch<T>(R, drs, dcs, n, n, W, n, c->stream)));
+            LLA_TRY_CUDA(reset_words(*c));
+            LLA_TRY_CUDA(factor_enqueue<T>(*c, W, n, n, true));
+            LLA_TRY_CUDA(read_words(*c, w));
+        }
+        failed = w.info >= 0;
+        if (!failed) LLA_TRY_CUDA(then());
+        LLA_TRY_CUDA(launch_status(export_launch<T>(W, n, (T *)c->raw_a.p, drs, dcs, n, n,
+                                                    failed ? EXPORT_FAIL : good, w.info, c->stream)));
+        LLA_TRY_CUDA(begin_download(*c, v, c->raw_a, c->stage_a));
+        const int64_t row = w.info;
+        LLA_TRY_CUDA(read_words(*c, w));
+        if (failed) {
+            LLA_TRY_CUDA(finish_download(*c, v, c->raw_a, c->stage_a));
+            return not_pd(err, row);
+        }
+    }
+    // (a solve's timeout leaves the factor in the caller's view, and its result nowhere)
+    LLA_TRY_CUDA(finish_download(*c, v, c->raw_a, c->stage_a));
+    if (w.err_word == LLA_ERR_TIMEOUT) return lla__set_status(err, LLA_ERR_TIMEOUT);
+    LLA_TRY_CUDA(keep());
+    return LLA_OK;
+}
+
 template <typename T>
 int cholesky_impl(T *a, int64_t rows, int64_t cols, int64_t rs, int64_t cs, int dirty,
                   lla_error *err) {
@@ -436,54 +536,30 @@ int cholesky_impl(T *a, int64_t rows, int64_t cols, int64_t rs, int64_t cs, int 
     T *W = (T *)c->work_a.p;
     const T *R = (const T *)c->raw_a.p;
     LLA_TRY_CUDA(launch_status(import_launch<T>(R, drs, dcs, n, n, W, n, c->stream)));
-    int64_t fail = -1;
-    int to = 0;
-    LLA_TRY_CUDA(factor_on_device<T>(*c, W, n, n, use_exact(n), R, drs, dcs, &fail, &to));
-    if (to) return lla__set_status(err, LLA_ERR_TIMEOUT);
-    const int mode = fail >= 0 ? EXPORT_FAIL : (dirty ? EXPORT_LOWER : EXPORT_LOWER_ZERO_UPPER);
-    LLA_TRY_CUDA(launch_status(export_launch<T>(W, n, (T *)c->raw_a.p, drs, dcs, n, n, mode, fail,
-                                                c->stream)));
-    LLA_TRY_CUDA(download(*c, v, c->raw_a, c->stage_a));
-    if (fail >= 0) return not_pd(err, fail);
-    return LLA_OK;
+    const int good = dirty ? EXPORT_LOWER : EXPORT_LOWER_ZERO_UPPER;
+    bool failed = false;
+    return factor_export<T>(c, v, W, R, drs, dcs, good, []() { return cudaSuccess; }, []() { return cudaSuccess; },
+                            failed, err);
 }
 
-// Shared by solvec_inplace and invc_inplace: factor `a` (dirty, written back),
-// then solve with B held in the working buffer work_b (n x m, ld n).
+// Shared by solvec_inplace and invc_inplace: `a` on the device and in W.
 template <typename T>
-int factor_then(Ctx *c, T *a, int64_t n, int64_t rs, int64_t cs, bool &failed, lla_error *err) {
-    View v{(char *)a, n, n, rs, cs, sizeof(T)};
-    int64_t drs, dcs;
-    LLA_TRY_CUDA(upload(*c, v, c->raw_a, c->stage_a, drs, dcs));
-    LLA_TRY_CUDA(c->work_a.ensure(sizeof(T) * n * n));
-    T *W = (T *)c->work_a.p;
-    const T *R = (const T *)c->raw_a.p;
-    LLA_TRY_CUDA(launch_status(import_launch<T>(R, drs, dcs, n, n, W, n, c->stream)));
-    int64_t fail = -1;
-    int to = 0;
-    LLA_TRY_CUDA(factor_on_device<T>(*c, W, n, n, use_exact(n), R, drs, dcs, &fail, &to));
-    if (to) return lla__set_status(err, LLA_ERR_TIMEOUT);
-    const int mode = fail >= 0 ? EXPORT_FAIL : EXPORT_LOWER;  // self keeps the dirty factor (:140)
-    LLA_TRY_CUDA(launch_status(export_launch<T>(W, n, (T *)c->raw_a.p, drs, dcs, n, n, mode, fail,
-                                                c->stream)));
-    LLA_TRY_CUDA(download(*c, v, c->raw_a, c->stage_a));
-    failed = fail >= 0;
-    if (failed) return not_pd(err, fail);
-    return LLA_OK;
+cudaError_t import_square(Ctx *c, const View &v, int64_t &drs, int64_t &dcs) {
+    const int64_t n = v.rows;
+    cudaError_t e = upload(*c, v, c->raw_a, c->stage_a, drs, dcs);
+    if (e == cudaSuccess) e = c->work_a.ensure(sizeof(T) * n * n);
+    if (e != cudaSuccess) return e;
+    return launch_status(import_launch<T>((const T *)c->raw_a.p, drs, dcs, n, n, (T *)c->work_a.p, n, c->stream));
 }
 
-// X = L^{-T} L^{-1} B for the factor in work_a (src/cholesky.rs:141-142).
+// Enqueues X = L^{-T} L^{-1} B for the factor in work_a (src/cholesky.rs:141-142).
 template <typename T>
-int cholesky_solve_work(Ctx *c, int64_t n, T *WB, int64_t m, lla_error *err) {
+cudaError_t cholesky_solve_work(Ctx *c, int64_t n, T *WB, int64_t m) {
     const T *L = (const T *)c->work_a.p;
     const bool exact = use_exact(n);
-    int to1 = 0, to2 = 0;
-    LLA_TRY_CUDA(trsm_on_device<T>(*c, L, n, n, /*lower=*/1, /*trans=*/0, nullptr, WB, n, m, exact,
-                                   &to1));
-    LLA_TRY_CUDA(trsm_on_device<T>(*c, L, n, n, /*lower=*/0, /*trans=*/1, nullptr, WB, n, m, exact,
-                                   &to2));
-    if (to1 || to2) return lla__set_status(err, LLA_ERR_TIMEOUT);
-    return LLA_OK;
+    cudaError_t e = trsm_enqueue<T>(*c, L, n, n, /*lower=*/1, /*trans=*/0, nullptr, WB, n, m, exact);
+    if (e == cudaSuccess) e = trsm_enqueue<T>(*c, L, n, n, /*lower=*/0, /*trans=*/1, nullptr, WB, n, m, exact);
+    return e;
 }
 
 template <typename T>
@@ -500,24 +576,35 @@ int solvec_impl(T *a, int64_t rows, int64_t cols, int64_t rs, int64_t cs, T *b, 
     }
     Ctx *c = get_ctx(err);
     if (!c) return err ? err->code : LLA_ERR_NO_DEVICE;
+    View va{(char *)a, n, n, rs, cs, sizeof(T)}, vb{(char *)b, brows, bcols, brs, bcs, sizeof(T)};
+    int64_t ars, acs, drs, dcs;
+    LLA_TRY_CUDA(import_square<T>(c, va, ars, acs));
     bool failed = false;
-    int st = factor_then<T>(c, a, n, rs, cs, failed, err);
-    if (st != LLA_OK) return st;
-    if (brows != n) return wrong_rows(err, n, brows);  // src/triangular.rs:103-108, after the factor
-    if (bcols == 0) return LLA_OK;
-    View vb{(char *)b, brows, bcols, brs, bcs, sizeof(T)};
-    int64_t drs, dcs;
+    T *W = (T *)c->work_a.p;
+    const T *R = (const T *)c->raw_a.p;
+    if (brows != n || bcols == 0) {
+        // `a` is factored before b is looked at (src/triangular.rs:103-108, after the factor)
+        const int st = factor_export<T>(c, va, W, R, ars, acs, EXPORT_LOWER, []() { return cudaSuccess; },
+                                        []() { return cudaSuccess; }, failed, err);
+        if (st != LLA_OK) return st;
+        return brows != n ? wrong_rows(err, n, brows) : LLA_OK;
+    }
     LLA_TRY_CUDA(upload(*c, vb, c->raw_b, c->stage_b, drs, dcs));
     LLA_TRY_CUDA(c->work_b.ensure(sizeof(T) * n * bcols));
-    T *WB = (T *)c->work_b.p;
-    LLA_TRY_CUDA(launch_status(import_launch<T>((const T *)c->raw_b.p, drs, dcs, n, bcols, WB, n,
-                                                c->stream)));
-    st = cholesky_solve_work<T>(c, n, WB, bcols, err);
-    if (st != LLA_OK) return st;
-    LLA_TRY_CUDA(launch_status(export_launch<T>(WB, n, (T *)c->raw_b.p, drs, dcs, n, bcols,
-                                                EXPORT_FULL, -1, c->stream)));
-    LLA_TRY_CUDA(download(*c, vb, c->raw_b, c->stage_b));
-    return LLA_OK;
+    T *WB = (T *)c->work_b.p, *RB = (T *)c->raw_b.p;
+    bool again = false;
+    auto then = [&]() -> cudaError_t {  // solve, export, first half of the download
+        cudaError_t e = cudaSuccess;
+        if (again) e = upload(*c, vb, c->raw_b, c->stage_b, drs, dcs);  // raw_b has been written to
+        again = true;
+        if (e == cudaSuccess) e = launch_status(import_launch<T>(RB, drs, dcs, n, bcols, WB, n, c->stream));
+        if (e == cudaSuccess) e = cholesky_solve_work<T>(c, n, WB, bcols);
+        if (e == cudaSuccess)
+            e = launch_status(export_launch<T>(WB, n, RB, drs, dcs, n, bcols, EXPORT_FULL, -1, c->stream));
+        return e == cudaSuccess ? begin_download(*c, vb, c->raw_b, c->stage_b) : e;
+    };
+    return factor_export<T>(c, va, W, R, ars, acs, EXPORT_LOWER, then,
+                            [&]() { return finish_download(*c, vb, c->raw_b, c->stage_b); }, failed, err);
 }
 
 template <typename T>
@@ -531,43 +618,43 @@ int invc_impl(T *a, int64_t rows, int64_t cols, int64_t rs, int64_t cs, T *out, 
     if (n == 0) return LLA_OK;
     Ctx *c = get_ctx(err);
     if (!c) return err ? err->code : LLA_ERR_NO_DEVICE;
-    bool failed = false;
-    int st = factor_then<T>(c, a, n, rs, cs, failed, err);
-    if (st != LLA_OK) return st;
-    // solvec_into(Array2::eye(n)) (src/cholesky.rs:178-181)
+    View va{(char *)a, n, n, rs, cs, sizeof(T)}, vo{(char *)out, n, n, ors, ocs, sizeof(T)};
+    int64_t ars, acs;
+    LLA_TRY_CUDA(import_square<T>(c, va, ars, acs));
     LLA_TRY_CUDA(c->work_b.ensure(sizeof(T) * n * n));
-    T *WB = (T *)c->work_b.p;
-    LLA_TRY_CUDA(launch_status(eye_launch<T>(WB, n, n, c->stream)));
-    if (use_exact(n)) {
-        st = cholesky_solve_work<T>(c, n, WB, n, err);
-        if (st != LLA_OK) return st;
-    } else {
-        // POTRI-style: column panel [c0, c0 + w) of L^-1 is zero above row c0, and
-        // rows >= c0 of L^-T L^-1 there need only the trailing triangle L[c0:, c0:];
-        // the strict upper part is then mirrored from the lower one.  About n^3
-        // flops instead of n^3/3 + 2n^3 (the result is symmetric by construction).
-        const T *L = (const T *)c->work_a.p;
-        constexpr int64_t kPanel = 1024;
-        for (int64_t c0 = 0; c0 < n; c0 += kPanel) {
-            const int64_t w = std::min<int64_t>(kPanel, n - c0), nt = n - c0;
-            const T *Ls = L + c0 + c0 * n;
-            T *Bp = WB + c0 + c0 * n;
-            int to1 = 0, to2 = 0;
-            LLA_TRY_CUDA(trsm_on_device<T>(*c, Ls, n, nt, /*lower=*/1, /*trans=*/0, nullptr, Bp, n, w, false, &to1));
-            LLA_TRY_CUDA(trsm_on_device<T>(*c, Ls, n, nt, /*lower=*/0, /*trans=*/1, nullptr, Bp, n, w, false, &to2));
-            if (to1 || to2) return lla__set_status(err, LLA_ERR_TIMEOUT);
-        }
-        LLA_TRY_CUDA(launch_status(symmetrize_launch<T>(WB, n, n, c->stream)));
-    }
-    View vo{(char *)out, n, n, ors, ocs, sizeof(T)};
+    LLA_TRY_CUDA(c->raw_b.ensure(sizeof(T) * n * n));
+    T *W = (T *)c->work_a.p, *WB = (T *)c->work_b.p;
     const bool contig = colmajor_contig(vo) || rowmajor_contig(vo);
     const int64_t drs = (contig && !colmajor_contig(vo)) ? n : 1;
     const int64_t dcs = (contig && !colmajor_contig(vo)) ? 1 : n;
-    LLA_TRY_CUDA(c->raw_b.ensure(sizeof(T) * n * n));
-    LLA_TRY_CUDA(launch_status(
-        export_launch<T>(WB, n, (T *)c->raw_b.p, drs, dcs, n, n, EXPORT_FULL, -1, c->stream)));
-    LLA_TRY_CUDA(download(*c, vo, c->raw_b, c->stage_b));
-    return LLA_OK;
+    auto then = [&]() -> cudaError_t {  // solvec_into(Array2::eye(n)) (src/cholesky.rs:178-181)
+        cudaError_t e = launch_status(eye_launch<T>(WB, n, n, c->stream));
+        if (use_exact(n)) {
+            if (e == cudaSuccess) e = cholesky_solve_work<T>(c, n, WB, n);
+        } else {
+            // POTRI-style: column panel [c0, c0 + w) of L^-1 is zero above row c0, and
+            // rows >= c0 of L^-T L^-1 there need only the trailing triangle L[c0:, c0:];
+            // the strict upper part is then mirrored from the lower one.  About n^3
+            // flops instead of n^3/3 + 2n^3 (the result is symmetric by construction).
+            constexpr int64_t kPanel = 1024;
+            for (int64_t c0 = 0; c0 < n && e == cudaSuccess; c0 += kPanel) {
+                const int64_t w = std::min<int64_t>(kPanel, n - c0), nt = n - c0;
+                const T *Ls = W + c0 + c0 * n;
+                T *Bp = WB + c0 + c0 * n;
+                e = trsm_enqueue<T>(*c, Ls, n, nt, /*lower=*/1, /*trans=*/0, nullptr, Bp, n, w, false);
+                if (e == cudaSuccess)
+                    e = trsm_enqueue<T>(*c, Ls, n, nt, /*lower=*/0, /*trans=*/1, nullptr, Bp, n, w, false);
+            }
+            if (e == cudaSuccess) e = launch_status(symmetrize_launch<T>(WB, n, n, c->stream));
+        }
+        if (e == cudaSuccess)
+            e = launch_status(
+                export_launch<T>(WB, n, (T *)c->raw_b.p, drs, dcs, n, n, EXPORT_FULL, -1, c->stream));
+        return e == cudaSuccess ? begin_download(*c, vo, c->raw_b, c->stage_b) : e;
+    };
+    bool failed = false;
+    return factor_export<T>(c, va, W, (const T *)c->raw_a.p, ars, acs, EXPORT_LOWER, then,
+                            [&]() { return finish_download(*c, vo, c->raw_b, c->stage_b); }, failed, err);
 }
 
 template <typename T>
@@ -605,13 +692,15 @@ int trsm_impl(const T *a, int64_t rows, int64_t cols, int64_t rs, int64_t cs, co
     T *WB = (T *)c->work_b.p;
     LLA_TRY_CUDA(launch_status(import_launch<T>((const T *)c->raw_b.p, drs, dcs, n, bcols, WB, n,
                                                 c->stream)));
-    int to = 0;
-    LLA_TRY_CUDA(trsm_on_device<T>(*c, W, n, n, uplo == LLA_LOWER ? 1 : 0, 0, ddiag, WB, n, bcols,
-                                   use_exact(n), &to));
-    if (to) return lla__set_status(err, LLA_ERR_TIMEOUT);
+    Words w;
+    LLA_TRY_CUDA(reset_words(*c));
+    LLA_TRY_CUDA(trsm_enqueue<T>(*c, W, n, n, uplo == LLA_LOWER ? 1 : 0, 0, ddiag, WB, n, bcols, use_exact(n)));
     LLA_TRY_CUDA(launch_status(export_launch<T>(WB, n, (T *)c->raw_b.p, drs, dcs, n, bcols,
                                                 EXPORT_FULL, -1, c->stream)));
-    LLA_TRY_CUDA(download(*c, vb, c->raw_b, c->stage_b));
+    LLA_TRY_CUDA(begin_download(*c, vb, c->raw_b, c->stage_b));
+    LLA_TRY_CUDA(read_words(*c, w));
+    if (w.err_word == LLA_ERR_TIMEOUT) return lla__set_status(err, LLA_ERR_TIMEOUT);
+    LLA_TRY_CUDA(finish_download(*c, vb, c->raw_b, c->stage_b));
     return LLA_OK;
 }
 
