@@ -7,13 +7,19 @@
 // decreasing cost (n^3/3 + 2 n^2 m) into a device work list; a persistent
 // kernel of (CTAs per SM) x (#SMs) blocks takes items from an atomic counter
 // (largest first, so the tail is short) and, inside one CTA per system:
-//   * factors A_i in place, right-looking with 32-column blocks: one warp
-//     factors the diagonal block with register shuffles, one thread per row
-//     solves the rows below it into a shared-memory panel, all threads update
-//     the trailing lower triangle from that panel (L2-resident);
-//   * solves L L^T X = B in place, 32-row blocks: one warp per right-hand side
-//     solves each diagonal block with shuffles, all threads update the rows
-//     below (above) from it.
+//   * factors A_i in place, right-looking with 32-column (FP32) or 16-column
+//     (FP64) blocks, the right-hand sides carried along as rows below A_i: the
+//     diagonal block is shared out to the CTA's warps, the rows below it are
+//     solved against it (a thread, or in short FP64 panels four, per row), and
+//     the trailing lower triangle is updated in FP32 register tiles, or for FP64
+//     on the tensor cores from 8-bit digits;
+//   * solves L^T X = Y, last block first: one warp per right-hand side in the
+//     block, one thread per remaining column after it.
+// A small system is a chain of latencies, so four CTAs of 128 threads share an SM
+// by default; a large FP64 one is bound by the FP64 pipe and the digits' integer
+// work.  10,000 systems of n 16-256 (before: one-warp diagonal blocks with library
+// divisions, FP64 updates on the FP64 pipe, two substitution passes): f64 20.1 ->
+// 5.9 ms, f32 5.4 -> 1.4 ms; 3,000 of n 16-64 1.60 -> 0.33 and 0.46 -> 0.15 ms.
 // A non-positive pivot stops that system only: info[i] = first failing row
 // (-1 when the system solved).  The (CTAs per SM, threads) shape is chosen per
 // batch by lla_batch_autotune and cached on disk.
@@ -39,7 +45,7 @@
 
 namespace lla {
 
-constexpr int kBNb = 32;                // block width
+constexpr int kBNb = 32;                // block width of the FP32 solves of the refined mode
 constexpr int kBMaxN = kBatchMaxN;      // largest order a batch system may have
 constexpr int kBMaxRhs = kBatchMaxRhs;  // right-hand sides per system
 
@@ -48,28 +54,40 @@ __device__ __forceinline__ T shfl(T v, int src) {
     return __shfl_sync(0xffffffffu, v, src);
 }
 
+// Block width.  FP32: 32 columns a step.  FP64: 16, because an FP64 instruction
+// takes 64 cycles of its sub-partition: half the columns leave half the panel's
+// substitution (the rest of it goes to the tensor cores with the update), a
+// quarter of the diagonal block, and shared memory and registers for a third CTA.
+template <typename T>
+constexpr int kBN = sizeof(T) == 4 ? 32 : 16;
+
 // Shared memory of one CTA.
 //  dg   : diagonal block, dg[c * kBDs + r] = L[r][c] while factoring (and its
 //         transpose in the backward pass), identity-padded;
 //  rinv : reciprocals of L's diagonal, all n;
 //  rhs  : right-hand sides as extra rows, rhs[k * kBMaxN + i];
-//  panel: FP32: the finished panel rows, panel[c * kBPs + r]; FP64: their digits,
-//         panel[(d * kBRows + r) * 32 + k], and expo[r], the rows' exponents.
-constexpr int kBDs = 36;                     // 16-byte rows in both types
-constexpr int kBRows = kBMaxN - kBNb + 16;   // FP64 panel rows: trailing and right-hand sides, to whole 16-row tiles
-constexpr int kBPs = kBMaxN + 4;             // FP32: to whole 32-row tiles
-static_assert(kBMaxN - kBNb + kBMaxRhs <= kBRows && kBRows <= kBMaxN, "panel rows");
+//  panel: the finished panel rows: FP32 panel[c * kBPs + r]; FP64 their digits,
+//         panel[(d * kBMaxN + r) * 16 + position of k], and expo[r], the rows'
+//         exponents.  The right-hand sides' rows follow the matrix rows from the
+//         next whole tile on (rhs_row).
+constexpr int kBPs = kBMaxN + 4;
 constexpr int kBNonFinite = 1 << 20;
 template <typename T>
 struct BatchSmem {
-    T dg[kBNb * kBDs];
+    static constexpr int kBDs = kBN<T> + 4;  // 16-byte rows in both types
+    T dg[kBN<T> * kBDs];
     T rinv[kBMaxN];
     T rhs[kBMaxRhs * kBMaxN];
-    T piv[kBNb];
-    int expo[kBRows];
+    T piv[kBN<T>];
+    int expo[kBMaxN];
     int fail;
-    alignas(16) unsigned char panel[sizeof(T) == 4 ? 4 * kBNb * kBPs : kOzBal * kBRows * kBNb];
+    alignas(16) unsigned char panel[sizeof(T) == 4 ? 4 * kBN<T> * kBPs : kOzBal * kBMaxN * kBN<T>];
 };
+template <typename T>
+__device__ __forceinline__ int rhs_row(int rows) {
+    return (rows + kBN<T> - 1) / kBN<T> * kBN<T>;
+}
+static_assert(kBMaxN - 32 + kBMaxRhs <= kBPs && kBMaxN - 16 + kBMaxRhs <= kBMaxN, "panel rows");
 
 // 1 / sqrt(d), d positive and normal: FP32 approximation and one Newton step;
 // FP64 in fixed point (lla_int_math.h).
@@ -77,155 +95,138 @@ __device__ __forceinline__ float batch_rsqrt(float d) {
     const float y = im_rsqrt_seed(d);
     return fmaf(0.5f * y, fmaf(-d * y, y, 1.f), y);
 }
-__device__ __forceinline__ bool batch_normal(float d) { return d >= 1.1754944e-38f && d <= 3.4028235e38f; }
+__device__ __forceinline__ double batch_rsqrt(double d) { return im_rsqrt(d); }
+__device__ __forceinline__ bool batch_normal(float d) { return __float_as_uint(d) - 0x800000u < 0x7f000000u; }
+__device__ __forceinline__ bool batch_normal(double d) { return im_positive_normal(im_bits(d)); }
 
-// Factors the identity-padded 32 x 32 block in sm.dg; sm.rinv[kb ..] receives the
-// reciprocal pivots, the block L with its exact roots.  sm.fail: failing column.
-// FP32: one warp, a row a lane, shuffles.
-__device__ void batch_diag(BatchSmem<float> &sm, int kb, int bs) {
-    const int lane = threadIdx.x & 31;
-    if (threadIdx.x < 32) {
-        float v[32], dk = 1.f;
-#pragma unroll
-        for (int c = 0; c < 32; ++c) v[c] = sm.dg[c * kBDs + lane];
-        int fail = -1;
-#pragma unroll
-        for (int c = 0; c < 32; ++c) {
-            const float d = shfl(v[c], c);
-            float y = batch_rsqrt(d);
-            if (!batch_normal(d)) {  // (uniform) not positive (NaN does not fail, as in the reference: `d <= 0`), or special
-                if (d <= 0.f && fail < 0) fail = c;
-                y = 1.f / sqrtf(d);
-            }
-            if (lane == c) {
-                dk = d;
-                sm.rinv[kb + c] = y;
-            }
-            v[c] *= y;
-#pragma unroll
-            for (int c2 = c + 1; c2 < 32; ++c2) v[c2] = fmaf(-v[c], shfl(v[c], c2), v[c2]);
-        }
-#pragma unroll
-        for (int c = 0; c < 32; ++c)
-            if (c <= lane) sm.dg[c * kBDs + lane] = c == lane ? sqrtf(dk) : v[c];
-        if (lane == 0 && fail >= 0) sm.fail = kb + fail;
-    }
-    __syncthreads();
-}
-
-// FP64: an FP64 instruction takes 64 cycles of its sub-partition, so the block is
-// shared out: warp 0 walks the pivots, a pair of columns at a time and one pair
-// ahead, and the warps of the other sub-partitions apply the finished pairs to the
-// rest in patches of 16 rows x 2 columns.
-__device__ void batch_diag(BatchSmem<double> &sm, int kb, int bs) {
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    double *a = sm.dg;
+// Factors the identity-padded diagonal block in sm.dg; sm.rinv[kb ..] receives
+// the reciprocal pivots, the block L with its exact roots.  sm.fail: failing row.
+// Warp 0 walks the pivots, a pair of columns at a time and one pair ahead, and the
+// warps of the other sub-partitions apply the finished pairs to the rest in
+// patches of 16 rows x 2 columns.
+template <typename T>
+__device__ void batch_diag(BatchSmem<T> &sm, int kb) {
+    constexpr int NB = kBN<T>, DS = BatchSmem<T>::kBDs, NP = NB / 2;
+    constexpr int kPatches = NB == 32 ? 24 : 8;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & (NB - 1);  // (FP64: both half-warps do the same)
+    T *a = sm.dg;
     auto pivots = [&](int c) {
-        double u = a[c * kBDs + lane], v = a[(c + 1) * kBDs + lane];
+        T u = a[c * DS + lane], v = a[(c + 1) * DS + lane];
         if (c > 0) {
-            const double *x0 = a + (c - 2) * kBDs, *x1 = a + (c - 1) * kBDs;
+            const T *x0 = a + (c - 2) * DS, *x1 = a + (c - 1) * DS;
             u = fma(-x1[lane], x1[c], fma(-x0[lane], x0[c], u));
             v = fma(-x1[lane], x1[c + 1], fma(-x0[lane], x0[c + 1], v));
         }
-        const double su = u, sv = v;
-        const double d0 = shfl(u, c);
-        double y0 = im_rsqrt(d0);
+        const T su = u, sv = v;
+        const T d0 = shfl(u, c);
+        T y0 = batch_rsqrt(d0);
         u *= y0;
         v = fma(-u, shfl(u, c + 1), v);
-        double d1 = shfl(v, c + 1);
-        double y1 = im_rsqrt(d1);
+        T d1 = shfl(v, c + 1);
+        T y1 = batch_rsqrt(d1);
         v *= y1;
-        if (!im_positive_normal(im_bits(d0)) || !im_positive_normal(im_bits(d1))) {  // not positive, or special
-            int fail = d0 <= 0.0 ? c : -1;
-            y0 = 1.0 / sqrt(d0);
+        // not positive (NaN does not fail, as in the reference: `d <= 0`), or special
+        if (!batch_normal(d0) || !batch_normal(d1)) {
+            int fail = d0 <= T(0) ? c : -1;
+            y0 = T(1) / sqrt(d0);
             u = su * y0;
             v = fma(-u, shfl(u, c + 1), sv);
             d1 = shfl(v, c + 1);
-            if (d1 <= 0.0 && fail < 0) fail = c + 1;
-            y1 = 1.0 / sqrt(d1);
+            if (d1 <= T(0) && fail < 0) fail = c + 1;
+            y1 = T(1) / sqrt(d1);
             v *= y1;
-            if (lane == 0 && fail >= 0 && sm.fail < 0) sm.fail = kb + fail;
+            if (tid == 0 && fail >= 0 && sm.fail < 0) sm.fail = kb + fail;
         }
         sm.piv[c] = d0;  // (every lane writes the same value)
         sm.piv[c + 1] = d1;
         sm.rinv[kb + c] = y0;
         sm.rinv[kb + c + 1] = y1;
-        a[c * kBDs + lane] = u;
-        a[(c + 1) * kBDs + lane] = v;
+        __syncwarp();
+        a[c * DS + lane] = u;
+        a[(c + 1) * DS + lane] = v;
     };
     if (warp == 0) pivots(0);
     const int npw = (blockDim.x >> 7) * 3, pw = warp - 1 - (warp >> 2);
-    for (int k = 0; k < 15; ++k) {
+    for (int k = 0; k < NP - 1; ++k) {
         __syncthreads();  // pair k is final
         if (warp == 0) {
             pivots(2 * k + 2);
         } else if (warp & 3) {
-            const double *x0 = a + 2 * k * kBDs, *x1 = x0 + kBDs;
-            for (int t = pw; t < 24; t += npw) {  // rightmost pairs first
-                const int j = t < 8 ? 15 - t : 7 - (t - 8) / 2, g = t < 8 ? 1 : 1 - (t & 1);
+            const T *x0 = a + 2 * k * DS, *x1 = x0 + DS;
+            for (int t = pw; t < kPatches; t += npw) {  // rightmost pairs first
+                const int j = t < 8 ? NP - 1 - t : 7 - (t - 8) / 2, g = NB == 16 ? 0 : (t < 8 ? 1 : 1 - (t & 1));
                 if (j < k + 2) break;
-                const int r = 16 * g + (lane & 15), c = 2 * j + (lane >> 4);
-                a[c * kBDs + r] = fma(-x1[r], x1[c], fma(-x0[r], x0[c], a[c * kBDs + r]));
+                const int r = 16 * g + (tid & 15), c = 2 * j + ((tid >> 4) & 1);
+                a[c * DS + r] = fma(-x1[r], x1[c], fma(-x0[r], x0[c], a[c * DS + r]));
             }
         }
     }
     __syncthreads();
-    if (tid < 32) a[tid * kBDs + tid] = sqrt(sm.piv[tid]);
+    if (tid < NB) a[tid * DS + tid] = sqrt(sm.piv[tid]);
     __syncthreads();
 }
 
-// Trailing update of rows rr (0 .. rows - 1: trailing rows q + rr; rows .. rows +
-// m - 1: right-hand sides) and columns j < rows, j <= rr, from the panel.
-// FP32: warp tiles of 32 x 32, a thread 4 rows (stride 8) x 8 columns.
+// Trailing update of the lower triangle of the rows q + i, i < rows, and of the
+// right-hand sides' rows, from the panel.  FP32: warp tiles of 32 x 32, a thread 4
+// rows (stride 8) x 8 columns.
+template <bool EDGE>
+__device__ __forceinline__ void batch_tile(const float *P, float *Aq, int n, int i0, int j0, int rows) {
+    float acc[4][8];
+#pragma unroll
+    for (int w = 0; w < 8; ++w)
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            acc[u][w] = !EDGE || (i0 + 8 * u < rows && j0 + w <= i0 + 8 * u) ? Aq[8 * u + w * n] : 0.f;
+#pragma unroll 4
+    for (int k = 0; k < 32; ++k) {
+        float xr[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) xr[u] = P[k * kBPs + i0 + 8 * u];
+        const float4 c0 = *reinterpret_cast<const float4 *>(P + k * kBPs + j0);
+        const float4 c1 = *reinterpret_cast<const float4 *>(P + k * kBPs + j0 + 4);
+        const float xc[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+#pragma unroll
+            for (int w = 0; w < 8; ++w) acc[u][w] = fmaf(-xr[u], xc[w], acc[u][w]);
+    }
+#pragma unroll
+    for (int w = 0; w < 8; ++w)
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (!EDGE || (i0 + 8 * u < rows && j0 + w <= i0 + 8 * u)) Aq[8 * u + w * n] = acc[u][w];
+}
+
 __device__ void batch_update(BatchSmem<float> &sm, float *A, int n, int q, int kb, int rows, int m) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
     const float *P = reinterpret_cast<const float *>(sm.panel);
-    const int R = (rows + m + 31) / 32, C = (rows + 31) / 32;
-    const int lr = lane & 7, lc = (lane >> 3) * 8;
-    for (int t = warp; t < R * C; t += nw) {
-        const int I = t / C, J = t % C;
-        if (J > I) continue;
-        const int i0 = 32 * I + lr, j0 = 32 * J + lc;
-        float acc[4][8];
-        float *const Aq = A + q + (int64_t)(q + j0) * n;
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-#pragma unroll
-            for (int w = 0; w < 8; ++w) {
-                const int i = i0 + 8 * u, j = j0 + w;
-                acc[u][w] = 0.f;
-                if (j < rows && j <= i) {
-                    if (i < rows)
-                        acc[u][w] = Aq[i + w * n];
-                    else if (i < rows + m)
-                        acc[u][w] = sm.rhs[(i - rows) * kBMaxN + q + j];
-                }
-            }
-#pragma unroll 4
-        for (int k = 0; k < kBNb; ++k) {
-            float xr[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) xr[u] = P[k * kBPs + i0 + 8 * u];
-            const float4 c0 = *reinterpret_cast<const float4 *>(P + k * kBPs + j0);
-            const float4 c1 = *reinterpret_cast<const float4 *>(P + k * kBPs + j0 + 4);
-            const float xc[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-#pragma unroll
-                for (int w = 0; w < 8; ++w) acc[u][w] = fmaf(-xr[u], xc[w], acc[u][w]);
+    const int R = (rows + 31) / 32, lr = lane & 7, lc = (lane >> 3) * 8;
+    int I = 0, J = warp;  // lower tiles, row by row
+    for (;;) {
+        while (J > I) {
+            J -= I + 1;
+            ++I;
         }
+        if (I >= R) break;
+        const int i0 = 32 * I + lr, j0 = 32 * J + lc;
+        float *Aq = A + q + i0 + (int64_t)(q + j0) * n;
+        if (J < I && 32 * I + 32 <= rows)
+            batch_tile<false>(P, Aq, n, i0, j0, rows);
+        else
+            batch_tile<true>(P, Aq, n, i0, j0, rows);
+        J += nw;
+    }
+    const int b0 = rhs_row<float>(rows);
+    for (int j = threadIdx.x; j < rows; j += blockDim.x) {
+        float x[32];
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
+        for (int c = 0; c < 32; ++c) x[c] = P[c * kBPs + j];
+        for (int k = 0; k < m; ++k) {
+            float s = sm.rhs[k * kBMaxN + q + j];
 #pragma unroll
-            for (int w = 0; w < 8; ++w) {
-                const int i = i0 + 8 * u, j = j0 + w;
-                if (j < rows && j <= i) {
-                    if (i < rows)
-                        Aq[i + w * n] = acc[u][w];
-                    else if (i < rows + m)
-                        sm.rhs[(i - rows) * kBMaxN + q + j] = acc[u][w];
-                }
-            }
+            for (int c = 0; c < 32; ++c) s = fmaf(-P[c * kBPs + b0 + k], x[c], s);
+            sm.rhs[k * kBMaxN + q + j] = s;
+        }
     }
     __syncthreads();
 }
@@ -245,77 +246,112 @@ __device__ __forceinline__ void batch_digits(uint32_t w, uint32_t &lo, uint32_t 
     asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(hi) : "r"(b), "r"(bias));
 }
 
-// FP64: the product of the 32 panel columns on the tensor cores, from seven
+// FP64: the product of the 16 panel columns on the tensor cores, from seven
 // balanced 8-bit digits per entry (exact in FP16, their products' sums exact in
 // the FP32 accumulators), one 64-bit integer per entry and one FP64 subtraction,
-// where FMAs would spend 32 FP64 instructions per entry (lla_fast_chol.cu has the
-// scheme and its error).  Warp tiles of 16 x 8, K = 32 in two steps; the digits'
-// k order is permuted alike in both operands so that a thread's four are one word.
+// where FMAs would spend 16 FP64 instructions per entry (lla_fast_chol.cu has the
+// scheme and its error).  Warp tiles of 16 x 8; the digits' k order is permuted
+// alike in both operands so that a thread's four are one word.
 __device__ void batch_update(BatchSmem<double> &sm, double *A, int n, int q, int kb, int rows, int m) {
+    constexpr int NB = 16;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
     const int g = lane >> 2, t4 = lane & 3;
-    const int R = (rows + m + 15) / 16, C = (rows + 7) / 8;
-    for (int t = warp; t < R * C; t += nw) {
-        const int I = t / C, J = t % C;
-        if (8 * J > 16 * I + 15) continue;
-        const int i0 = 16 * I, j0 = 8 * J;
+    const int R = (rows + 15) / 16, C = (rows + 7) / 8;  // (row R: the right-hand sides)
+    int I = 0, J = warp;                                  // tiles of row I: J <= 2 I + 1, J < C
+    for (;;) {
+        for (int w = min(2 * I + 2, C); I <= R && J >= w; w = min(2 * I + 2, C)) {
+            J -= w;
+            ++I;
+        }
+        if (I > R) break;
+        const bool isb = I == R;
+        // this thread's entries, fetched before the products
+        double *wp[4], w[4];
+        int use = 0;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int i = 16 * I + g + 8 * (u >> 1), j = 8 * J + 2 * t4 + (u & 1);
+            const bool in = j < rows && (isb ? i - 16 * R < m : i < rows && j <= i);
+            wp[u] = isb ? &sm.rhs[(in ? i - 16 * R : 0) * kBMaxN + q + (in ? j : 0)]
+                        : &A[in ? (q + i) + (int64_t)(q + j) * n : 0];
+            w[u] = in ? *wp[u] : 0.0;
+            use |= in ? 1 << u : 0;
+        }
         float acc[kOzBal][4];
 #pragma unroll
         for (int l = 0; l < kOzBal; ++l)
 #pragma unroll
             for (int u = 0; u < 4; ++u) acc[l][u] = 0.f;
+        uint32_t fb[kOzBal][2];
 #pragma unroll
-        for (int ks = 0; ks < 2; ++ks) {
-            uint32_t fb[kOzBal][2];
+        for (int d = 0; d < kOzBal; ++d)
+            batch_digits(*reinterpret_cast<const uint32_t *>(sm.panel + (d * kBMaxN + 8 * J + g) * NB + 4 * t4), fb[d][0],
+                         fb[d][1]);
 #pragma unroll
-            for (int d = 0; d < kOzBal; ++d)
-                batch_digits(*reinterpret_cast<const uint32_t *>(sm.panel + (d * kBRows + j0 + g) * kBNb + 8 * t4 + 4 * ks),
-                             fb[d][0], fb[d][1]);
+        for (int d = 0; d < kOzBal; ++d) {
+            uint32_t fa[4];
+            const unsigned char *pa = sm.panel + (d * kBMaxN + 16 * I + g) * NB + 4 * t4;
+            batch_digits(*reinterpret_cast<const uint32_t *>(pa), fa[0], fa[2]);
+            batch_digits(*reinterpret_cast<const uint32_t *>(pa + 8 * NB), fa[1], fa[3]);
 #pragma unroll
-            for (int d = 0; d < kOzBal; ++d) {
-                uint32_t fa[4];
-                const unsigned char *pa = sm.panel + (d * kBRows + i0 + g) * kBNb + 8 * t4 + 4 * ks;
-                batch_digits(*reinterpret_cast<const uint32_t *>(pa), fa[0], fa[2]);
-                batch_digits(*reinterpret_cast<const uint32_t *>(pa + 8 * kBNb), fa[1], fa[3]);
-#pragma unroll
-                for (int e = 0; e < kOzBal - d; ++e) batch_mma(acc[d + e], fa, fb[e]);
-            }
+            for (int e = 0; e < kOzBal - d; ++e) batch_mma(acc[d + e], fa, fb[e]);
         }
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
-            const int i = i0 + g + 8 * (u >> 1), j = j0 + 2 * t4 + (u & 1);
-            if (j >= rows || j > i || i >= rows + m) continue;
-            double *w = i < rows ? &A[(q + i) + (int64_t)(q + j) * n] : &sm.rhs[(i - rows) * kBMaxN + q + j];
-            const int ei = sm.expo[i], ej = sm.expo[j];
-            if (ei == kBNonFinite || ej == kBNonFinite) {  // no digits: the FMA chain on the factor itself
-                double s = *w;
-                for (int k = 0; k < kBNb; ++k)
-                    s = fma(-(i < rows ? A[(q + i) + (int64_t)(kb + k) * n] : sm.rhs[(i - rows) * kBMaxN + kb + k]),
-                            A[(q + j) + (int64_t)(kb + k) * n], s);
-                *w = s;
-                continue;
-            }
+            const int ei = sm.expo[16 * I + g + 8 * (u >> 1)], ej = sm.expo[8 * J + 2 * t4 + (u & 1)];
             long long lo = 128, hi = 0;
 #pragma unroll
             for (int l = 4; l < kOzBal; ++l) lo += (long long)__float2int_rn(acc[l][u]) * (1 << (8 * (6 - l)));
 #pragma unroll
             for (int l = 0; l < 4; ++l) hi += (long long)__float2int_rn(acc[l][u]) * (1 << (8 * (3 - l)));
-            *w -= oz_scaled_double(hi * 65536 + (lo >> 8), ei + ej - 54);
+            if (use >> u & 1) {
+                if (ei != kBNonFinite && ej != kBNonFinite) {
+                    *wp[u] = w[u] - oz_scaled_double(hi * 65536 + (lo >> 8), ei + ej - 54);
+                } else {  // no digits: the FMA chain on the factor itself
+                    const int i = 16 * I + g + 8 * (u >> 1), j = 8 * J + 2 * t4 + (u & 1);
+                    double s = w[u];
+                    for (int k = 0; k < NB; ++k)
+                        s = fma(-(isb ? sm.rhs[(i - 16 * R) * kBMaxN + kb + k] : A[(q + i) + (int64_t)(kb + k) * n]),
+                                A[(q + j) + (int64_t)(kb + k) * n], s);
+                    *wp[u] = s;
+                }
+            }
         }
+        J += nw;
     }
     __syncthreads();
 }
 
-// Keeps a finished panel row (thread rr) for the update.
-__device__ __forceinline__ void batch_keep_row(BatchSmem<float> &sm, int rr, const float (&v)[kBNb]) {
+// Word t of the digits of panel row rr: columns t, t + 4, t + 8, t + 12.
+__device__ __forceinline__ void batch_keep_word(BatchSmem<double> &sm, int rr, int t, const double (&w)[4], int e) {
+    uint64_t x[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+        x[u] = (e != kBNonFinite ? (uint64_t)oz_fixed55((int64_t)im_bits(w[u]), e) : 0ull) + 0x0080808080808080ull;
+    // the four values' bytes 0-3 and 4-6, transposed: byte s of all four in one word
+    const uint32_t l0 = (uint32_t)x[0], l1 = (uint32_t)x[1], l2 = (uint32_t)x[2], l3 = (uint32_t)x[3];
+    const uint32_t h0 = (uint32_t)(x[0] >> 32), h1 = (uint32_t)(x[1] >> 32), h2 = (uint32_t)(x[2] >> 32),
+                   h3 = (uint32_t)(x[3] >> 32);
+#pragma unroll
+    for (int d = 0; d < kOzBal; ++d) {
+        const int b = kOzBal - 1 - d;  // byte of the value
+        const uint32_t sel = (uint32_t)(b & 3) | (uint32_t)((b & 3) + 4) << 4;
+        const uint32_t p01 = b < 4 ? __byte_perm(l0, l1, sel) : __byte_perm(h0, h1, sel);
+        const uint32_t p23 = b < 4 ? __byte_perm(l2, l3, sel) : __byte_perm(h2, h3, sel);
+        *reinterpret_cast<uint32_t *>(sm.panel + (d * kBMaxN + rr) * 16 + 4 * t) = __byte_perm(p01, p23, 0x5410);
+    }
+}
+
+// Keeps a finished panel row (row rr of the panel) for the update.
+__device__ __forceinline__ void batch_keep_row(BatchSmem<float> &sm, int rr, const float (&v)[32]) {
     float *P = reinterpret_cast<float *>(sm.panel);
 #pragma unroll
-    for (int c = 0; c < kBNb; ++c) P[c * kBPs + rr] = v[c];
+    for (int c = 0; c < 32; ++c) P[c * kBPs + rr] = v[c];
 }
-__device__ __forceinline__ void batch_keep_row(BatchSmem<double> &sm, int rr, const double (&v)[kBNb]) {
+__device__ __forceinline__ void batch_keep_row(BatchSmem<double> &sm, int rr, const double (&v)[16]) {
     uint64_t mx = 0;
 #pragma unroll
-    for (int c = 0; c < kBNb; ++c) {
+    for (int c = 0; c < 16; ++c) {
         const uint64_t b = im_bits(v[c]) & 0x7fffffffffffffffull;
         mx = b > mx ? b : mx;
     }
@@ -323,81 +359,125 @@ __device__ __forceinline__ void batch_keep_row(BatchSmem<double> &sm, int rr, co
     const bool fin = mx < 0x7ff0000000000000ull;
     const int e = fin ? oz_bits_exponent(mx) + 1 : kBNonFinite;
     sm.expo[rr] = e;
-    // words of four digits: k = 2 t, 2 t + 1, 2 t + 8, 2 t + 9 of step ks at byte 8 t + 4 ks
 #pragma unroll
     for (int t = 0; t < 4; ++t) {
-        uint32_t w[2][kOzBal];
+        const double w[4] = {v[t], v[t + 4], v[t + 8], v[t + 12]};
+        batch_keep_word(sm, rr, t, w, e);
+    }
+}
+
+// FP64 panel of at most blockDim / 4 rows: four threads a row (eight rows a warp),
+// thread t of a row its columns t, t + 4, t + 8, t + 12, so that a short panel
+// uses every sub-partition's FP64 pipe and a row's digits are formed four ways.
+__device__ void batch_panel_split(double *A, int n, int kb, int bs, int q, int rows, int m, BatchSmem<double> &sm) {
+    constexpr int DS = BatchSmem<double>::kBDs;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, r8 = lane & 7, t = lane >> 3;
+    const int rr = warp * 8 + r8;
+    if (warp * 8 >= rows + m) return;  // (uniform for the warp)
+    const bool in = rr < rows + m, isb = rr >= rows;
+    double v[4];
 #pragma unroll
-        for (int ks = 0; ks < 2; ++ks) {
-            uint64_t x[4];
+    for (int u = 0; u < 4; ++u) {
+        const int c = 4 * u + t;
+        v[u] = in && c < bs ? (isb ? sm.rhs[(rr - rows) * kBMaxN + kb + c] : A[(q + rr) + (int64_t)(kb + c) * n]) : 0.0;
+    }
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const int k = 16 * ks + 2 * t + (u & 1) + 8 * (u >> 1);
-                x[u] = (fin ? (uint64_t)oz_fixed55((int64_t)im_bits(v[k]), e) : 0ull) + 0x0080808080808080ull;
-            }
+    for (int c = 0; c < 16; ++c) {
+        const double x = shfl(v[c >> 2] * sm.rinv[kb + c], (c & 3) * 8 + r8);
+        if (t == (c & 3)) v[c >> 2] = x;
 #pragma unroll
-            for (int d = 0; d < kOzBal; ++d) {
-                const int s = 8 * (kOzBal - 1 - d);
-                w[ks][d] = (uint32_t)(x[0] >> s & 255) | (uint32_t)(x[1] >> s & 255) << 8 |
-                           (uint32_t)(x[2] >> s & 255) << 16 | (uint32_t)(x[3] >> s & 255) << 24;
+        for (int u = c >> 2; u < 4; ++u) {
+            const double w = fma(-x, sm.dg[c * DS + 4 * u + t], v[u]);
+            if (4 * u + t > c) v[u] = w;
+        }
+    }
+    if (in) {
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int c = 4 * u + t;
+            if (c < bs) {
+                if (isb)
+                    sm.rhs[(rr - rows) * kBMaxN + kb + c] = v[u];
+                else
+                    A[(q + rr) + (int64_t)(kb + c) * n] = v[u];
             }
         }
+    }
+    if (rows == 0) return;
+    uint64_t mx = 0;
 #pragma unroll
-        for (int d = 0; d < kOzBal; ++d)
-            *reinterpret_cast<uint2 *>(sm.panel + (d * kBRows + rr) * kBNb + 8 * t) = make_uint2(w[0][d], w[1][d]);
+    for (int u = 0; u < 4; ++u) {
+        const uint64_t b = im_bits(v[u]) & 0x7fffffffffffffffull;
+        mx = b > mx ? b : mx;
+    }
+#pragma unroll
+    for (int o = 8; o < 32; o *= 2) {
+        const uint64_t b = __shfl_xor_sync(0xffffffffu, (unsigned long long)mx, o);
+        mx = b > mx ? b : mx;
+    }
+    const int e = mx < 0x7ff0000000000000ull ? oz_bits_exponent(mx) + 1 : kBNonFinite;
+    if (in) {
+        const int p = isb ? rhs_row<double>(rows) + rr - rows : rr;
+        if (t == 0) sm.expo[p] = e;
+        batch_keep_word(sm, p, t, v, e);
     }
 }
 
 // Factor of one system by the whole CTA: A (n x n, column-major, ld = n) in
-// place (L in the lower triangle), right-looking with 32-column blocks; the m
-// right-hand sides in sm.rhs are carried along as rows below A, which makes them
-// L^-1 B.  Returns the first failing row (non-positive pivot) or -1; every thread
-// returns the same value.
+// place (L in the lower triangle), right-looking; the m right-hand sides in
+// sm.rhs are carried along as rows below A, which makes them L^-1 B.  Returns the
+// first failing row (non-positive pivot) or -1; every thread returns the same
+// value.
 template <typename T>
 __device__ int batch_factor(T *A, int n, int m, BatchSmem<T> &sm) {
+    constexpr int NB = kBN<T>, DS = BatchSmem<T>::kBDs;
     const int tid = threadIdx.x, nthr = blockDim.x;
     if (tid == 0) sm.fail = -1;
     __syncthreads();
-    for (int kb = 0; kb < n; kb += kBNb) {
-        const int bs = min(kBNb, n - kb), q = kb + bs, rows = n - q;
-        for (int e = tid; e < kBNb * kBNb; e += nthr) {
-            const int r = e % kBNb, c = e / kBNb;
-            sm.dg[c * kBDs + r] = (r < bs && c <= r) ? A[(kb + r) + (int64_t)(kb + c) * n] : T(r == c ? 1 : 0);
+    for (int kb = 0; kb < n; kb += NB) {
+        const int bs = min(NB, n - kb), q = kb + bs, rows = n - q;
+        for (int e = tid; e < NB * NB; e += nthr) {
+            const int r = e % NB, c = e / NB;
+            sm.dg[c * DS + r] = (r < bs && c <= r) ? A[(kb + r) + (int64_t)(kb + c) * n] : T(r == c ? 1 : 0);
         }
         // the rows below the block, one a thread, fetched while the block is factored
         const int total = rows + m;
-        T v[kBNb];
+        T v[NB];
         auto fetch = [&](int rr) {
 #pragma unroll
-            for (int c = 0; c < kBNb; ++c)
+            for (int c = 0; c < NB; ++c)
                 v[c] = c < bs ? (rr < rows ? A[(q + rr) + (int64_t)(kb + c) * n] : sm.rhs[(rr - rows) * kBMaxN + kb + c])
                               : T(0);
         };
-        if (tid < total) fetch(tid);
+        const bool split = sizeof(T) == 8 && 4 * total <= nthr;
+        if (tid < total && !split) fetch(tid);
         __syncthreads();
-        batch_diag(sm, kb, bs);
+        batch_diag<T>(sm, kb);
         if (sm.fail >= 0) break;
-        for (int e = tid; e < kBNb * kBNb; e += nthr) {
-            const int r = e % kBNb, c = e / kBNb;
-            if (r < bs && c <= r) A[(kb + r) + (int64_t)(kb + c) * n] = sm.dg[c * kBDs + r];
+        for (int e = tid; e < NB * NB; e += nthr) {
+            const int r = e % NB, c = e / NB;
+            if (r < bs && c <= r) A[(kb + r) + (int64_t)(kb + c) * n] = sm.dg[c * DS + r];
         }
-        for (int rr = tid; rr < total; rr += nthr) {
+        if constexpr (sizeof(T) == 8) {
+            if (split) batch_panel_split(A, n, kb, bs, q, rows, m, sm);
+        }
+        for (int rr = split ? total : tid; rr < total; rr += nthr) {
             if (rr != tid) fetch(rr);
 #pragma unroll
-            for (int c = 0; c < kBNb; ++c) {
-                v[c] *= c < bs ? sm.rinv[kb + c] : T(1);
+            for (int c = 0; c < NB; ++c) {
+                v[c] *= sm.rinv[kb + c];  // (1 past the matrix: identity padding)
 #pragma unroll
-                for (int c2 = c + 1; c2 < kBNb; ++c2) v[c2] = fma(-v[c], sm.dg[c * kBDs + c2], v[c2]);
+                for (int c2 = c + 1; c2 < NB; ++c2) v[c2] = fma(-v[c], sm.dg[c * DS + c2], v[c2]);
             }
 #pragma unroll
-            for (int c = 0; c < kBNb; ++c)
+            for (int c = 0; c < NB; ++c)
                 if (c < bs) {
                     if (rr < rows)
                         A[(q + rr) + (int64_t)(kb + c) * n] = v[c];
                     else
                         sm.rhs[(rr - rows) * kBMaxN + kb + c] = v[c];
                 }
-            if (rows > 0) batch_keep_row(sm, rr, v);
+            if (rows > 0) batch_keep_row(sm, rr < rows ? rr : rhs_row<T>(rows) + rr - rows, v);
         }
         __syncthreads();
         if (rows > 0) batch_update(sm, A, n, q, kb, rows, m);
@@ -412,18 +492,20 @@ __device__ int batch_factor(T *A, int n, int m, BatchSmem<T> &sm) {
 // one thread per remaining column after it.
 template <typename T>
 __device__ void batch_backward(const T *A, int n, int m, BatchSmem<T> &sm) {
-    const int tid = threadIdx.x, nthr = blockDim.x, warp = tid >> 5, lane = tid & 31, nw = nthr >> 5;
-    for (int kb = (n - 1) / kBNb * kBNb; kb >= 0; kb -= kBNb) {
-        const int bs = min(kBNb, n - kb);
-        for (int e = tid; e < kBNb * kBNb; e += nthr) {
-            const int r = e % kBNb, c = e / kBNb;
-            sm.dg[r * kBDs + c] = (r < bs && c < r) ? A[(kb + r) + (int64_t)(kb + c) * n] : T(0);
+    constexpr int NB = kBN<T>, DS = BatchSmem<T>::kBDs;
+    const int tid = threadIdx.x, nthr = blockDim.x, warp = tid >> 5, nw = nthr >> 5;
+    const int lane = tid & (NB - 1);  // (FP64: both half-warps do the same)
+    for (int kb = (n - 1) / NB * NB; kb >= 0; kb -= NB) {
+        const int bs = min(NB, n - kb);
+        for (int e = tid; e < NB * NB; e += nthr) {
+            const int r = e % NB, c = e / NB;
+            sm.dg[r * DS + c] = (r < bs && c < r) ? A[(kb + r) + (int64_t)(kb + c) * n] : T(0);
         }
         // the block's rows of column tid, fetched while the block is solved
-        T v[kBNb];
+        T v[NB];
         auto fetch = [&](int j) {
 #pragma unroll
-            for (int t = 0; t < kBNb; ++t) v[t] = t < bs ? A[(kb + t) + (int64_t)j * n] : T(0);
+            for (int t = 0; t < NB; ++t) v[t] = t < bs ? A[(kb + t) + (int64_t)j * n] : T(0);
         };
         if (tid < kb) fetch(tid);
         __syncthreads();
@@ -431,11 +513,12 @@ __device__ void batch_backward(const T *A, int n, int m, BatchSmem<T> &sm) {
             T z = lane < bs ? sm.rhs[k * kBMaxN + kb + lane] : T(0);
             const T ri = lane < bs ? sm.rinv[kb + lane] : T(0);
 #pragma unroll
-            for (int c = kBNb - 1; c >= 0; --c) {
+            for (int c = NB - 1; c >= 0; --c) {
                 const T x = shfl(z * ri, c);
-                const T w = fma(-x, sm.dg[c * kBDs + lane], z);
+                const T w = fma(-x, sm.dg[c * DS + lane], z);
                 z = lane == c ? x : (lane < c ? w : z);
             }
+            __syncwarp();
             if (lane < bs) sm.rhs[k * kBMaxN + kb + lane] = z;
         }
         __syncthreads();
@@ -444,7 +527,7 @@ __device__ void batch_backward(const T *A, int n, int m, BatchSmem<T> &sm) {
             for (int k = 0; k < m; ++k) {
                 T s = sm.rhs[k * kBMaxN + j];
 #pragma unroll
-                for (int t = 0; t < kBNb; ++t)
+                for (int t = 0; t < NB; ++t)
                     if (t < bs) s = fma(-v[t], sm.rhs[k * kBMaxN + kb + t], s);
                 sm.rhs[k * kBMaxN + j] = s;
             }
@@ -924,8 +1007,8 @@ struct lla_batch_plan {
     double flops = 0.0;
     BatchItem *d_items = nullptr;
     int *d_counter = nullptr;
-    int ctas_per_sm = 2, threads = 256;
-    bool tuned = false;
+    int ctas_per_sm = 4, threads = 128;  // four latency chains a SM; measured best or equal at every order
+    bool tuned = false;     // the shape comes from the cache, the autotuner or the caller
     bool refined = false;   // f64 systems through an FP32 factor + FP64 refinement (A read only)
     char *d_scratch = nullptr;  // per-CTA scratch of the refined mode
     std::string key;
@@ -1103,6 +1186,7 @@ int lla_batch_plan_info(const lla_batch_plan *p, int64_t *a_elems, int64_t *b_el
 int lla_batch_set_shape(lla_batch_plan *p, int ctas_per_sm, int threads) {
     if (!p || ctas_per_sm < 1 || ctas_per_sm > 8 || (threads != 128 && threads != 256))
         return LLA_ERR_INVALID_ARG;
+    p->tuned = true;
     if (p->ctas_per_sm != ctas_per_sm || p->threads != threads) {
         p->ctas_per_sm = ctas_per_sm;
         p->threads = threads;
@@ -1149,6 +1233,9 @@ int lla_batch_set_refined(lla_batch_plan *p, int refined, lla_error *err) {
         if (cache_lookup(p->key, cps, thr)) {
             p->ctas_per_sm = cps;
             p->threads = thr;
+        } else if (!p->tuned) {  // two CTAs of the refined kernel fit an SM
+            p->ctas_per_sm = want ? 2 : 4;
+            p->threads = want ? 256 : 128;
         }
     }
     return LLA_OK;

@@ -190,26 +190,37 @@ __host__ __device__ __forceinline__ void oz_balanced_pair(int64_t va, int64_t vb
     }
 }
 
+// T 2^s outside the normal range; out of line, or the compiler evaluates its FP64
+// conversion (64 cycles of the pipe) for every element and selects.
+#ifdef __CUDACC__
+static __device__ __noinline__ double oz_scaled_rare(int64_t T, int s) { return ldexp((double)T, s); }
+#else
+static double oz_scaled_rare(int64_t T, int s) { return std::ldexp((double)T, s); }
+#endif
+
 // The double nearest to T 2^s, |T| < 2^63 (ties to even): integer operations
-// only for results in the normal range, the plain product otherwise.
+// only for results in the normal range.
 __host__ __device__ __forceinline__ double oz_scaled_double(int64_t T, int s) {
-    if (T == 0) return 0.0;
     const uint64_t u = T < 0 ? 0ull - (uint64_t)T : (uint64_t)T;
 #ifdef __CUDA_ARCH__
-    const int lz = __clzll((long long)u);
+    const int lz = __clzll((long long)(u | 1));
 #else
-    const int lz = __builtin_clzll(u);
+    const int lz = __builtin_clzll(u | 1);
 #endif
     const uint64_t v = u << lz;
     uint64_t m = v >> 11;  // 53 bits, the leading one at bit 52
     const uint32_t rem = (uint32_t)v & 0x7ffu;
-    m += (rem > 0x400u || (rem == 0x400u && (m & 1))) ? 1 : 0;
+    m += rem > 0x400u - ((uint32_t)m & 1) ? 1 : 0;
     const int ex = 63 - lz + s + 1022;  // biased exponent minus one: the leading one of m adds it
-    if (ex < 0 || ex >= 0x7fd) return ldexp((double)T, s);
     const uint64_t b = ((uint64_t)T & 0x8000000000000000ull) | (((uint64_t)ex << 52) + m);
     double d;
     memcpy(&d, &b, 8);
-    return d;
+    if ((uint32_t)ex >= 0x7fdu) {
+#if defined(__CUDA_ARCH__) || !defined(__CUDACC__)
+        d = oz_scaled_rare(T, s);
+#endif
+    }
+    return T == 0 ? 0.0 : d;
 }
 
 // Smallest e with |v| < 2^e for the bit pattern of a finite |v| (0 and

@@ -284,3 +284,57 @@ def test_cholesky_qr_forms(gpu_lla, dtype, k, n):
     g = y.astype(np.float64).T @ w
     want = w - y.astype(np.float64) @ np.linalg.solve(lyy.astype(np.float64), g)
     assert np.abs(x - want).max() <= 1e3 * np.finfo(dtype).eps * np.sqrt(n) * np.abs(w).max()
+
+
+@pytest.mark.parametrize("dtype", ["f64", "f32"])
+@pytest.mark.parametrize("shape", [(4, 128), (2, 256), (1, 128)])
+def test_batch_orders_and_failures(gpu_lla, dtype, shape):
+    """Every order around the blocks, tiles and panel forms, 0-8 right-hand sides, with failing and
+    NaN systems among them: residuals within 10 n eps, first failing rows, untouched upper parts,
+    and B left alone where the factorisation fails."""
+    torch = _torch()
+    orders = [1, 2, 7, 8, 9, 15, 16, 17, 23, 24, 25, 31, 32, 33, 40, 47, 48, 49, 63, 64, 65, 95, 96, 97, 127, 128, 129,
+              160, 191, 192, 193, 223, 224, 225, 239, 240, 241, 254, 255, 256]
+    rng = np.random.default_rng(1)
+    n = np.array(orders * 3, dtype=np.int32)
+    m = np.array([(7 * i) % 9 for i in range(len(n))], dtype=np.int32)
+    bad = {i: int(rng.integers(0, n[i])) for i in range(len(orders), 2 * len(orders))}
+    nan = set(range(2 * len(orders), len(n), 5))
+    As, Bs = [], []
+    for i, k in enumerate(n):
+        g = rng.standard_normal((k, k))
+        a = g @ g.T / k + 0.5 * np.eye(k)
+        if i in bad:
+            a[bad[i], bad[i]] = -1.0
+        if i in nan:
+            a[k // 2, k // 3] = np.nan
+        As.append(a)
+        Bs.append(rng.standard_normal((k, m[i])))
+    plan = gpu_lla.BatchPlan(n, m, dtype)
+    plan.set_shape(*shape)
+    ap, bp = plan.pack(As, Bs)
+    A, B = torch.from_numpy(ap.copy()).cuda(), torch.from_numpy(bp.copy()).cuda()
+    info = torch.empty(len(n), dtype=torch.int32, device="cuda")
+    plan.solve(A, B, info)
+    torch.cuda.synchronize()
+    X, info, out = plan.unpack_x(B.cpu().numpy()), info.cpu().numpy(), A.cpu().numpy()
+    eps = np.finfo(plan.np_dtype).eps
+    b0 = plan.unpack_x(bp)
+    for i, k in enumerate(n):
+        fac = out[plan.a_off[i]:plan.a_off[i] + k * k].reshape((k, k), order="F")
+        a = ap[plan.a_off[i]:plan.a_off[i] + k * k].reshape((k, k), order="F")
+        up = np.triu(np.ones((k, k), bool), 1)
+        assert ((fac == a) | (np.isnan(fac) & np.isnan(a)))[up].all(), i
+        if i in bad:
+            assert info[i] == bad[i] and (X[i] == b0[i]).all(), (i, k)
+            continue
+        assert info[i] == -1, (i, k, info[i])
+        if i in nan:
+            continue
+        ad, x = a.astype(np.float64), X[i].astype(np.float64)
+        low = np.tril(fac).astype(np.float64)
+        assert np.abs(low @ low.T - ad).max() <= 10 * max(k, 4) * eps * np.abs(ad).sum(1).max(), (i, k)
+        r = np.abs(ad @ x - b0[i])
+        if x.size:
+            den = np.abs(ad).sum(1).max() * np.abs(x).max(0) + np.abs(b0[i]).max(0)
+            assert (r.max(0) <= 10 * max(k, 4) * eps * den).all(), (i, k)
