@@ -8,7 +8,8 @@
 // pipe take 176 ms at n = 8192 however they are tiled; the FP32 pipe's n^3/3 is
 // 1 ms at n = 6001, but its rate needs large register tiles.  Here only the
 // O(n^2) parts stay on those pipes:
-//   diag   : 64 x 64 diagonal block, one CTA;
+//   diag   : 64 x 64 diagonal block, one CTA (the update kernel's first, beside
+//            the others' tiles);
 //   panel  : L21 = A21 L11^-T, 64 columns, by substitution; the finished rows are
 //            also cut into balanced 8-bit digits (lla_oz_digits.h; seven for FP64,
 //            four for FP32) relative to each row's largest magnitude, exact in
@@ -26,8 +27,8 @@
 // the rest, so the trailing matrix is read and written once per 128 columns.
 //
 // Measured, FMA updates before -> now (error against 64 bits the same or lower):
-// f64 n = 8192 220 -> 15.1 ms, n = 2048 14.4 -> 2.25 ms; f32 n = 6001 14.6 ->
-// 4.3 ms.  There is no size at which the FMA form is faster: one 64 x 64 tile of
+// f64 n = 8192 220 -> 13.6 ms, n = 2048 14.4 -> 2.2 ms; f32 n = 6001 14.6 ->
+// 3.7 ms.  There is no size at which the FMA form is faster: one 64 x 64 tile of
 // the FP64 one took 70 us on its SM.
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -203,24 +204,32 @@ __device__ __forceinline__ bool fc_pivot_pair(T (*a)[kFcNb], T *piv, T *rv, int 
     return fail >= 0;
 }
 
+// Shared state of a diagonal block's CTA.
 template <typename T>
-__global__ void __launch_bounds__(kFcDiagThreads) fc_diag_kernel(T *W, int64_t ld, int64_t p, int b,
-                                                                 const T *diag0, T *rinv, int64_t *info,
-                                                                 double *min_ratio) {
-    __shared__ T a[kFcNb][kFcNb];  // [column][row]
-    __shared__ T piv[kFcNb], rv[kFcNb];
-    __shared__ int s_fail;
+struct FcDiagSmem {
+    T a[kFcNb][kFcNb];  // [column][row]
+    T piv[kFcNb], rv[kFcNb];
+    int fail;
+};
+
+__device__ __forceinline__ void fc_diag_sync() {
+    asm volatile("bar.sync 1, %0;" ::"n"(kFcDiagThreads) : "memory");
+}
+
+// By threads 0 .. 511 of a CTA.
+template <typename T>
+__device__ __forceinline__ void fc_diag_block(FcDiagSmem<T> &sm, T *W, int64_t ld, int64_t p, int b, const T *diag0,
+                                              T *rinv, int64_t *info, double *min_ratio) {
+    T(*a)[kFcNb] = sm.a;
+    T *piv = sm.piv, *rv = sm.rv;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    pdl_wait();
-    pdl_trigger();
-    if (*(volatile int64_t *)info >= 0) return;  // an earlier panel failed
     for (int e = tid; e < kFcNb * kFcNb; e += kFcDiagThreads) {
         const int r = e % kFcNb, c = e / kFcNb;
         // a short block is padded with the identity
         a[c][r] = (r < b && c <= r) ? cm(W, ld, p + r, p + c) : T(r == c ? 1 : 0);
     }
-    if (tid == 0) s_fail = -1;
-    __syncthreads();
+    if (tid == 0) sm.fail = -1;
+    fc_diag_sync();
     const bool upd = (warp & 3) != 0;  // a patch warp (warps 4, 8 and 12 only load and store)
     T acc[kFcSlots];
     int row[kFcSlots], col[kFcSlots];  // col < 0: no patch
@@ -236,17 +245,17 @@ __global__ void __launch_bounds__(kFcDiagThreads) fc_diag_kernel(T *W, int64_t l
         }
     }
     bool bad = false;
-    if (warp == 0) bad = fc_pivot_pair<T, true>(a, piv, rv, &s_fail, 0, lane);
+    if (warp == 0) bad = fc_pivot_pair<T, true>(a, piv, rv, &sm.fail, 0, lane);
     for (int k = 0;; ++k) {
-        __syncthreads();  // pair k is final
+        fc_diag_sync();  // pair k is final
         // A pivot failure of pair k ends the loop for everyone here.  Warp 0 may already have
         // recorded one of pair k + 1 by the time another warp reads the word: that one ends the
         // loop after the next barrier.
-        if (warp > 0) bad = (unsigned)*(volatile int *)&s_fail <= (unsigned)(2 * k + 1);
+        if (warp > 0) bad = (unsigned)*(volatile int *)&sm.fail <= (unsigned)(2 * k + 1);
         if (bad || k == kFcNb / 2 - 1) break;
         if (warp == 0) {
-            bad = k < 15 ? fc_pivot_pair<T, true>(a, piv, rv, &s_fail, 2 * k + 2, lane)
-                         : fc_pivot_pair<T, false>(a, piv, rv, &s_fail, 2 * k + 2, lane);
+            bad = k < 15 ? fc_pivot_pair<T, true>(a, piv, rv, &sm.fail, 2 * k + 2, lane)
+                         : fc_pivot_pair<T, false>(a, piv, rv, &sm.fail, 2 * k + 2, lane);
         } else if (upd) {
 #pragma unroll
             for (int s = 0; s < kFcSlots; ++s) {
@@ -257,7 +266,7 @@ __global__ void __launch_bounds__(kFcDiagThreads) fc_diag_kernel(T *W, int64_t l
             }
         }
     }
-    const int fail = bad ? s_fail : -1;
+    const int fail = bad ? sm.fail : -1;
     const int done = fail >= 0 ? fail : kFcNb;
     if (bad && upd) {  // the columns right of the failing pair, up to date with what was finished
 #pragma unroll
@@ -285,11 +294,22 @@ __global__ void __launch_bounds__(kFcDiagThreads) fc_diag_kernel(T *W, int64_t l
         }
     }
     if (tid == 0 && fail >= 0) *info = p + fail;
-    __syncthreads();
+    fc_diag_sync();
     for (int e = tid; e < kFcNb * kFcNb; e += kFcDiagThreads) {
         const int r = e % kFcNb, c = e / kFcNb;
         if (r < b && c <= r) cm(W, ld, p + r, p + c) = a[c][r];
     }
+}
+
+// The first block; the others follow their trailing update in its kernel.
+template <typename T>
+__global__ void __launch_bounds__(kFcDiagThreads) fc_diag_kernel(T *W, int64_t ld, int64_t p, int b,
+                                                                 const T *diag0, T *rinv, int64_t *info,
+                                                                 double *min_ratio) {
+    __shared__ FcDiagSmem<T> sm;
+    pdl_wait();
+    pdl_trigger();
+    fc_diag_block(sm, W, ld, p, b, diag0, rinv, info, min_ratio);
 }
 
 // Panel rows [q, n), q = p + 64: L21 = A21 L11^-T by substitution (multiplying
@@ -441,7 +461,8 @@ template <typename T>
 constexpr int kFuBSet = Fc<T>::kDigits *kFuBTile;
 template <typename T>
 constexpr int kFuSmem = 1024 + kFuRing * kFuATile + 2 * kFuBSet<T> + 256;
-constexpr int kFuEpi = 512;                        // 16 epilogue warps
+constexpr int kFuEpi = 512;                        // 16 epilogue warps (and the next diagonal block's)
+static_assert(kFuEpi == kFcDiagThreads && sizeof(FcDiagSmem<double>) <= kFuRing * kFuATile, "");
 constexpr int kFuThreads = kFuEpi + 64;            // and the producer's and the MMA issuer's
 // Tensor memory: all 512 columns; FP64's seven levels fill 448 of them, FP32's
 // four levels leave room for a second set.
@@ -485,7 +506,7 @@ template <typename T>
 __global__ void __launch_bounds__(kFuThreads, 1) fc_update_kernel(
     const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, T *W, int64_t ld,
     int64_t q, int64_t n, int64_t p0, int kchunks, int ntiles, int narrow, const int *__restrict__ expo,
-    const int64_t *info, int *err_word, int *sticky) {
+    const T *diag0, T *rinv, int64_t *info, double *min_ratio, int *err_word, int *sticky) {
     constexpr int ND = Fc<T>::kDigits, SETS = kFuSets<T>, BSET = kFuBSet<T>;
     extern __shared__ uint8_t smem_raw[];
     __shared__ int s_abort, s_skip;
@@ -526,22 +547,27 @@ __global__ void __launch_bounds__(kFuThreads, 1) fc_update_kernel(
     tc_fence_after();
     const uint32_t tmem = *tslot;
     pdl_wait();
-    pdl_trigger();
-    // one reader decides for the whole CTA (another CTA may report meanwhile)
-    if (tid == 0) s_skip = (*(volatile const int64_t *)info >= 0 || *(volatile const int *)err_word != 0);
+    // One reader decides for the whole CTA (another CTA may report meanwhile; rows from q on are
+    // CTA 0's own report on the next block, which stops nobody here).
+    if (tid == 0) {
+        const int64_t f = *(volatile const int64_t *)info;
+        s_skip = (f >= 0 && f < q) || *(volatile const int *)err_word != 0;
+    }
     __syncthreads();
     if (s_skip) {
         if (warp == 0)
             asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kFuTmem) : "memory");
         return;
     }
+    // CTA 0 takes the first tile alone, the others share the rest
+    const int tstep = blockIdx.x ? (int)gridDim.x - 1 : (gridDim.x > 1 ? ntiles : 1);
     // instruction descriptor without N: D F32, A/B BF16, K-major, M = 128
     const uint32_t idesc0 = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kFuM >> 4) << 24);
 
     if (warp == kFuEpi / 32) {
         if (lane == 0) {  // TMA producer
             uint32_t ga = 0, gb = 0;
-            for (int t = blockIdx.x; t < ntiles && !*(volatile int *)&s_abort; t += gridDim.x) {
+            for (int t = blockIdx.x; t < ntiles && !*(volatile int *)&s_abort; t += tstep) {
                 int I, J;
                 fu_tile(t, narrow, I, J);
                 const int ra = (int)(q + (int64_t)I * kFuM), rb = (int)(q + (int64_t)J * kFuN);
@@ -568,7 +594,7 @@ __global__ void __launch_bounds__(kFuThreads, 1) fc_update_kernel(
     } else if (warp == kFuEpi / 32 + 1) {
         if (lane == 0) {  // MMA issuer
             uint32_t ga = 0, gb = 0, lt = 0;
-            for (int t = blockIdx.x; t < ntiles && !*(volatile int *)&s_abort; t += gridDim.x, ++lt) {
+            for (int t = blockIdx.x; t < ntiles && !*(volatile int *)&s_abort; t += tstep, ++lt) {
                 const uint32_t set = lt % SETS, use = lt / SETS;
                 if (use > 0 && !mbar_wait(tempty + 8 * set, (use - 1) & 1, err_word)) {
                     s_abort = 1;
@@ -613,7 +639,7 @@ __global__ void __launch_bounds__(kFuThreads, 1) fc_update_kernel(
         const int r = qw * 32 + lane;
         const uint32_t tcol0 = tmem + ((uint32_t)(qw * 32) << 16) + (uint32_t)(cq * 16);
         uint32_t lt = 0;
-        for (int t = blockIdx.x; t < ntiles; t += gridDim.x, ++lt) {
+        for (int t = blockIdx.x; t < ntiles; t += tstep, ++lt) {
             const uint32_t set = lt % SETS, use = lt / SETS, tcol = tcol0 + set * (kFuTmem / SETS);
             int I, J;
             fu_tile(t, narrow, I, J);
@@ -699,6 +725,16 @@ __global__ void __launch_bounds__(kFuThreads, 1) fc_update_kernel(
     tc_fence_after();
     if (warp == 0)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kFuTmem) : "memory");
+    // The panel kernel may start here and no earlier: its blocks would crowd onto the SMs that this
+    // one leaves first (f64 n = 8192: 15.1 ms against 13.6).
+    pdl_trigger();
+    // The first tile holds the next diagonal block: factored here, in the ring's space (every MMA
+    // has read its stages: the epilogue waited for the last one), while the other CTAs go on.  As a
+    // kernel of its own between update and panel it left the other SMs idle (f64 n = 8192 15.0 ->
+    // 13.6 ms, n = 2048 2.24 -> 2.22; f32 n = 6001 4.26 -> 3.73 ms).
+    if (blockIdx.x == 0 && tid < kFcDiagThreads && !s_abort)
+        fc_diag_block(*reinterpret_cast<FcDiagSmem<T> *>(smem), W, ld, q, (int)min((int64_t)kFcNb, n - q), diag0, rinv,
+                      info, min_ratio);
 }
 
 // Saves the input diagonal (for the pivot-ratio guard) and clears the status word.
@@ -766,21 +802,11 @@ int potrf_fast_launch(T *W, int64_t n, int64_t ld, int64_t *d_info, T *diag0, do
         LaunchScope ls(K_MISC, st);
         fc_begin_kernel<T><<<(unsigned)ceil_div(n, 256), 256, 0, st>>>(W, ld, n, diag0, err_word ? nullptr : own_err);
     }
-    auto diag_panel = [&](int64_t p, int second) -> int64_t {  // rows left below the block
-        const int b = (int)std::min<int64_t>(kFcNb, n - p);
-        {
-            LaunchScope ls(K_POTRF_FAST_DIAG, st, (double)b * b * b / 3.0);
-            launch_maybe_pdl(true, fc_diag_kernel<T>, dim3(1), dim3(kFcDiagThreads), 0, st, W, ld, p, b,
-                             (const T *)diag0, rinv, d_info, min_ratio);
-        }
-        const int64_t rest = n - p - b;
-        if (rest > 0) {
-            LaunchScope ls(K_POTRF_FAST_PANEL, st, (double)rest * b * b);
-            launch_maybe_pdl(true, fc_panel_kernel<T>, dim3((unsigned)ceil_div(rest, kFcRows)), dim3(kFcPanelThreads), 0,
-                             st, W, ld, n, p, second, (const T *)rinv, planes, pstride, expo,
-                             (const int64_t *)d_info);
-        }
-        return rest;
+    const auto panel = [&](int64_t p, int second) {
+        const int64_t rest = n - p - kFcNb;
+        LaunchScope ls(K_POTRF_FAST_PANEL, st, (double)rest * kFcNb * kFcNb);
+        launch_maybe_pdl(true, fc_panel_kernel<T>, dim3((unsigned)ceil_div(rest, kFcRows)), dim3(kFcPanelThreads), 0,
+                         st, W, ld, n, p, second, (const T *)rinv, planes, pstride, expo, (const int64_t *)d_info);
     };
     auto update = [&](int64_t q, int64_t p0, int kchunks, int narrow) {
         const int64_t m = n - q, R = ceil_div(m, kFuM);
@@ -793,12 +819,19 @@ int potrf_fast_launch(T *W, int64_t n, int64_t ld, int64_t *d_info, T *diag0, do
                        ((double)m * cols - (double)cols * (cols - 1) / 2) * 2.0 * kchunks * kFuK);
         launch_maybe_pdl(true, fc_update_kernel<T>, dim3((unsigned)std::min<int64_t>(tiles, fc_sms())), dim3(kFuThreads),
                          (size_t)kFuSmem<T>, st, tmA, tmB, W, ld, q, n, p0, kchunks, (int)tiles, narrow,
-                         (const int *)expo, (const int64_t *)d_info, ew, sticky);
+                         (const int *)expo, (const T *)diag0, rinv, d_info, min_ratio, ew, sticky);
     };
-    for (int64_t p = 0; p < n; p += kFcPair) {
-        if (diag_panel(p, 0) <= 0) break;
+    {
+        const int b = (int)std::min<int64_t>(kFcNb, n);
+        LaunchScope ls(K_POTRF_FAST_DIAG, st, (double)b * b * b / 3.0);
+        launch_maybe_pdl(true, fc_diag_kernel<T>, dim3(1), dim3(kFcDiagThreads), 0, st, W, ld, (int64_t)0, b,
+                         (const T *)diag0, rinv, d_info, min_ratio);
+    }
+    for (int64_t p = 0; p + kFcNb < n; p += kFcPair) {
+        panel(p, 0);
         update(p + kFcNb, p, 1, 1);
-        if (diag_panel(p + kFcNb, 1) <= 0) break;
+        if (p + kFcPair >= n) break;
+        panel(p + kFcNb, 1);
         update(p + kFcPair, p, 2, 0);
     }
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
