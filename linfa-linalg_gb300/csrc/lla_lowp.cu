@@ -3,11 +3,9 @@
 //
 // Right-looking with panels of nb = 128 columns:
 //   diag   : one CTA factors the 128 x 128 diagonal block in FP32 (32-column
-//            sub-blocks: an unpredicated one-warp shuffle Cholesky without
-//            square roots on its pivot chain, a row-parallel solve of the
-//            rows below it, a shared-memory update of the next sub-block's
-//            columns first and of the rest while the next pivots run; a
-//            short last block is padded with the identity);
+//            sub-blocks: four warps walk the pivots in pairs while the others
+//            update what lies right of the block; two threads a row solve the
+//            rows below it; a short last block is padded with the identity);
 //   panel  : L21 = A21 L11^-T in FP32 by 32-column blocks (products with the
 //            inverted 32 x 32 diagonal blocks of L11), and the operand
 //            planes of L21 for the tensor cores: a one-, two- or three-term
@@ -57,8 +55,10 @@ __device__ __forceinline__ void lp_cp_wait_all() { asm volatile("cp.async.wait_a
 
 constexpr int kDgThreads = 512;
 constexpr int kDgLd = kLpNb + 4;  // column stride of the block in shared memory (16-byte columns)
-constexpr int kDgLt = 36;         // row stride of a transposed 32 x 32 factor (16-byte rows)
-constexpr size_t kDgSmem = sizeof(float) * (kLpNb * kDgLd + 32 * kDgLt + 5 * 32);
+constexpr int kDgLt = 36;         // column stride of the 32 x 32 factor (16-byte columns)
+constexpr int kDgCb = 2 * 32;     // a pair of column buffers
+constexpr int kDgWt = 33;         // row stride of W_JJ on its way out
+constexpr size_t kDgSmem = sizeof(float) * (kLpNb * kDgLd + 32 * kDgLt + 3 * kDgCb + 32 * kDgWt);
 
 __device__ __forceinline__ float dg_rcp(float x) {
     float r;
@@ -105,21 +105,53 @@ __device__ __forceinline__ void dg_syrk(float *sa, int k0, int r0, int c0, int c
     }
 }
 
-// Right-looking by 32-column blocks J with a look-ahead inside the block:
-//   (1) warp 0 factors the 32 x 32 diagonal block (lane i holds row i in
-//       registers) without square roots on the pivot chain: with d_c the
-//       pivot, a_ij -= (a_ic / d_c) a_jc.  Columns go through shared memory
-//       two at a time (one store, four-wide broadcast loads) and every lane
-//       forms the second pivot of the pair itself, so one store, barrier and
-//       load serve two pivots; the columns are scaled by 1/sqrt(d_c)
-//       afterwards.  Meanwhile
-//       warps 1-15 subtract the previous block's panel from the columns right
-//       of the next block;
-//   (2) the rows below solve x L_JJ^T = a, and 32 more threads solve the rows
-//       of the identity, giving W_JJ = L_JJ^-1 for the panel kernel (products
-//       with a transposed copy of L_JJ, read four entries at a time);
-//   (3) the panel is subtracted from the next block's 32 columns only, and
-//       the finished column block goes back to HBM.
+// The same for the 32 x 32 block at r0 alone, in 2 x 2 tiles by threads 0 .. 255.
+__device__ __forceinline__ void dg_syrk_block(float *sa, int k0, int r0, int tid) {
+    const int rr = r0 + 2 * (tid % 16), cc = r0 + 2 * (tid / 16);
+    if (tid >= 256 || cc > rr) return;
+    float2 u = *reinterpret_cast<const float2 *>(&sa[cc * kDgLd + rr]);
+    float2 v = *reinterpret_cast<const float2 *>(&sa[(cc + 1) * kDgLd + rr]);
+#pragma unroll 16
+    for (int t = 0; t < 32; ++t) {
+        const float2 a2 = *reinterpret_cast<const float2 *>(&sa[(k0 + t) * kDgLd + rr]);
+        const float2 b2 = *reinterpret_cast<const float2 *>(&sa[(k0 + t) * kDgLd + cc]);
+        u.x = fmaf(-a2.x, b2.x, u.x);
+        u.y = fmaf(-a2.y, b2.x, u.y);
+        v.x = fmaf(-a2.x, b2.y, v.x);
+        v.y = fmaf(-a2.y, b2.y, v.y);
+    }
+    // (the entry above the diagonal is not read by anything)
+    *reinterpret_cast<float2 *>(&sa[cc * kDgLd + rr]) = u;
+    *reinterpret_cast<float2 *>(&sa[(cc + 1) * kDgLd + rr]) = v;
+}
+
+// The finished columns kb .. kb + 31 of the lower triangle to memory, a warp per column.
+__device__ __forceinline__ void dg_store(const float *sa, float *L, int64_t ld, int64_t p, int b, int kb, int w, int nw,
+                                         int lane) {
+    for (int c = kb + w; c < kb + 32; c += nw) {
+        float *dst = L + p + (p + c) * ld;
+        for (int r = kb + lane; r < b; r += 32)
+            if (r >= c) dst[r] = sa[c * kDgLd + r];
+    }
+}
+
+// Right-looking by 32-column blocks J with a look-ahead inside the block.  What
+// bounds it is the chain of pivots and, on one SM, the issue of FP32 FMAs (one
+// warp: 2.1 cycles each), so every step is spread over the SM's sub-partitions:
+//   (1) warps 0-3 factor the 32 x 32 diagonal block (2 rows x 4 columns a
+//       thread) without square roots on the pivot chain: with d_c the pivot,
+//       a_ij -= (a_ic / d_c) a_jc.  Columns go through shared memory two at a
+//       time and every thread forms the inverse of the pair's 2 x 2 pivot block
+//       itself, so one store, barrier and load serve two pivots (256 cycles);
+//       the next pair is brought up to date and stored before the columns right
+//       of it.  Meanwhile warps 4-15 subtract the previous block's panel from
+//       everything below and right of this block and store that panel;
+//   (2) the rows below solve x L_JJ^T = a, and 32 more rows are those of the
+//       identity, giving W_JJ = L_JJ^-1 for the panel kernel; two threads a row,
+//       a shuffle a column;
+//   (3) the panel is subtracted from the next 32 x 32 block.
+// With one warp for the pivots and one thread a row, and the finished panel
+// stored in step 3, a block took 26 us from its load to its last store; now 19.
 // The block is column-major in shared memory, copied in 16-byte pieces
 // (4-byte pieces for an unaligned matrix or a short last block, which is
 // padded with the identity: blockdiag(A11, I) factors as blockdiag(L11, I),
@@ -129,13 +161,14 @@ __device__ __forceinline__ void dg_syrk(float *sa, int k0, int r0, int c0, int c
 // step loop (J = -1) runs on the uninitialised shared memory, with every
 // global store off, while the previous kernel still finishes (before
 // pdl_wait), so the real passes run from a warm cache; its phases run side
-// by side without barriers (warp 0 the pivots, the others the solves and
-// updates), so it takes about as long as its longest phase.
+// by side without barriers (but the pivots' own), so it takes about as long as
+// its longest phase.
 __global__ void __launch_bounds__(kDgThreads) lowp_diag_kernel(float *L, int64_t ld, int64_t p, int b,
                                                                int64_t *info, double *min_ratio, float *Wd) {
     extern __shared__ __align__(16) float sa[];  // sa[c * kDgLd + r] = A11[r][c]
-    float *slt = sa + kLpNb * kDgLd;              // slt[c * kDgLt + c2] = L_JJ[c2][c] for c2 > c, else 0
-    float *colb = slt + 32 * kDgLt;               // two pairs of column buffers, then 1/sqrt(d)
+    float *slt = sa + kLpNb * kDgLd;              // slt[c * kDgLt + r] = L_JJ[r][c], r >= c
+    float *colb = slt + 32 * kDgLt;               // three pairs of column buffers
+    float *sw = colb + 3 * kDgCb;                 // sw[k * kDgWt + c] = W_JJ[c][k]
     __shared__ __align__(16) float rdiag[32];     // 1 / L_JJ[c][c]
     __shared__ int failed, skip;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -183,127 +216,130 @@ __global__ void __launch_bounds__(kDgThreads) lowp_diag_kernel(float *L, int64_t
             ratio = 1e30f;  // forget the warm-up pass's pivots
         }
         const int kb = dry ? 32 : 32 * J;
-        if (warp == 0) {
-            // (1) sqrt-free Cholesky of the 32 x 32 block
-            float v[32];
+        if (warp < 4) {
+            const int lr = 2 * (tid & 15), lc = 4 * (tid >> 4);
+            float v[4][2];  // column lc + j, row lr + i (above the diagonal: anything)
 #pragma unroll
-            for (int c = 0; c < 32; ++c) v[c] = (c <= lane) ? sa[(kb + c) * kDgLd + kb + lane] : 0.f;
+            for (int j = 0; j < 4; ++j) {
+                const float2 t = *reinterpret_cast<const float2 *>(&sa[(kb + lc + j) * kDgLd + kb + lr]);
+                v[j][0] = t.x, v[j][1] = t.y;
+            }
             bool bad = false;
-            float myd = 1.f;  // this lane's pivot d_lane
-            // Two columns per round: both go to shared memory together, every lane
-            // forms the 2 x 2 pivot block's recurrence itself (d_{c+1} after column
-            // c's update) and the column c + 1 entries it needs, so one store,
-            // barrier and load serve two pivots.
+            float *cb = colb;
+            // columns c and c + 1 of the block to a buffer pair, by the threads that hold them
+            const auto put = [&](float *to, int c, const float (&x)[2], const float (&y)[2]) {
+                if (lc == (c & ~3)) {
+                    *reinterpret_cast<float2 *>(to + lr) = make_float2(x[0], x[1]);
+                    *reinterpret_cast<float2 *>(to + 32 + lr) = make_float2(y[0], y[1]);
+                }
+                asm volatile("bar.sync 1, 128;" ::: "memory");
+            };
+            // finished columns: threads 0-31 to the block, 32-63 to the copy for step 2
+            float *const out = warp == 0 ? &sa[(kb + (tid >> 4)) * kDgLd + kb + lr] : &slt[((tid >> 4) & 1) * kDgLt + lr];
+            const int ostep = warp == 0 ? kDgLd : kDgLt;
+            put(cb, 0, v[0], v[1]);
+#pragma unroll 1
+            for (int c4 = 0; c4 < 32; c4 += 4)
 #pragma unroll
-            for (int c = 0; c < 32; c += 2) {
-                float *cb0 = colb + ((c >> 1) & 1) * 64, *cb1 = cb0 + 32;  // two buffer pairs: no reuse hazard
-                cb0[lane] = v[c];
-                cb1[lane] = v[c + 1];
-                __syncwarp();
-                const float a00 = cb0[c], a10 = cb0[c + 1], a11 = cb1[c + 1];
-                const float r0 = dg_rcp(a00);
-                const float d1 = fmaf(-(a10 * r0), a10, a11);  // pivot c + 1 after column c's update
-                const float r1 = dg_rcp(d1);
-                bad |= !(a00 > 0.f) || !(d1 > 0.f);  // non-positive (or NaN) pivot: breakdown
-                myd = (lane == c) ? a00 : ((lane == c + 1) ? d1 : myd);
-                const float s0 = v[c] * r0;                // l_{lane,c}
-                const float u = fmaf(-s0, a10, v[c + 1]);  // a_{lane,c+1} after column c
-                v[c + 1] = u;
-                const float s1 = u * r1;  // l_{lane,c+1}
+                for (int j0 = 0; j0 < 4; j0 += 2) {
+                    const int c = c4 + j0, jn = (j0 + 2) & 3;
+                    // three buffer pairs: a pair's last readers are two barriers before its reuse
+                    float *nb = cb == colb + 2 * kDgCb ? colb : cb + kDgCb;
+                    const float2 a0 = *reinterpret_cast<const float2 *>(cb + c);  // a_cc, a_{c+1,c}
+                    const float a11 = cb[32 + c + 1];
+                    const float2 x2 = *reinterpret_cast<const float2 *>(cb + lr);
+                    const float2 y2 = *reinterpret_cast<const float2 *>(cb + 32 + lr);
+                    const float4 t4 = *reinterpret_cast<const float4 *>(cb + lc);
+                    const float4 u4 = *reinterpret_cast<const float4 *>(cb + 32 + lc);
+                    const float t[4] = {t4.x, t4.y, t4.z, t4.w}, u[4] = {u4.x, u4.y, u4.z, u4.w};
+                    const float r0 = dg_rcp(a0.x), g = a0.y * r0;
+                    const float d0 = a0.x, d1 = fmaf(-g, a0.y, a11);  // pivot c + 1 after column c's update
+                    const float r1 = dg_rcp(d1);
+                    const float x0[2] = {x2.x, x2.y};  // columns c and c + 1, unscaled
+                    float x1[2] = {y2.x, y2.y}, s0[2], s1[2];
 #pragma unroll
-                for (int g = (c + 2) / 4; g < 8; ++g) {
-                    const float4 t0 = *reinterpret_cast<const float4 *>(&cb0[4 * g]);
-                    const float4 t1 = *reinterpret_cast<const float4 *>(&cb1[4 * g]);
-                    const float tv0[4] = {t0.x, t0.y, t0.z, t0.w}, tv1[4] = {t1.x, t1.y, t1.z, t1.w};
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        const int c2 = 4 * g + i;
-                        if (c2 > c + 1) {
-                            const float w1 = fmaf(-(tv0[i] * r0), a10, tv1[i]);  // a_{c2,c+1} after column c
-                            v[c2] = fmaf(-s1, w1, fmaf(-s0, tv0[i], v[c2]));
-                        }
+                    for (int i = 0; i < 2; ++i) {
+                        x1[i] = fmaf(-g, x0[i], x1[i]);
+                        s1[i] = x1[i] * r1;
+                        s0[i] = fmaf(-s1[i], g, x0[i] * r0);
                     }
+                    const auto apply = [&](int j) {
+#pragma unroll
+                        for (int i = 0; i < 2; ++i) v[j][i] = fmaf(-s1[i], u[j], fmaf(-s0[i], t[j], v[j][i]));
+                    };
+                    apply(jn);
+                    apply(jn + 1);
+                    put(nb, c + 2, v[jn], v[jn + 1]);  // (c + 2 = 32: nobody's)
+                    apply(j0);
+                    apply(j0 + 1);
+                    // the finished pair
+                    bad |= !(d0 > 0.f) || !(d1 > 0.f);  // non-positive (or NaN) pivot: breakdown
+                    if (kb + c < b) ratio = fminf(ratio, d0);
+                    if (kb + c + 1 < b) ratio = fminf(ratio, d1);
+                    if (warp < 2) {
+                        const float q0 = rsqrtf(d0), q1 = rsqrtf(d1);
+                        const bool second = tid & 16;
+                        const float q = second ? q1 : q0;
+                        *reinterpret_cast<float2 *>(out + c * ostep) =
+                            make_float2((second ? x1[0] : x0[0]) * q, (second ? x1[1] : x0[1]) * q);
+                        if (tid == 0) *reinterpret_cast<float2 *>(&rdiag[c]) = make_float2(q0, q1);
+                    }
+                    cb = nb;
                 }
-            }
-            // L[lane][c] = a_{lane,c} / sqrt(d_c) (c < lane), L[lane][lane] = sqrt(d_lane)
-            const float rs_me = rsqrtf(myd);
-            colb[128 + lane] = rs_me;
-            __syncwarp();
-#pragma unroll
-            for (int g = 0; g < 8; ++g) {
-                const float4 r4 = *reinterpret_cast<const float4 *>(&colb[128 + 4 * g]);
-                const float rv[4] = {r4.x, r4.y, r4.z, r4.w};
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const int c = 4 * g + i;
-                    v[c] = (c < lane) ? v[c] * rv[i] : (c == lane ? myd * rs_me : 0.f);
-                }
-            }
-            if (kb + lane < b) ratio = fminf(ratio, myd);
-            if (lane == 0 && bad && !dry) failed = 1;
-#pragma unroll
-            for (int c = 0; c < 32; ++c) {
-                if (c <= lane) sa[(kb + c) * kDgLd + kb + lane] = v[c];
-                slt[c * kDgLt + lane] = (lane > c) ? v[c] : 0.f;
-            }
-            rdiag[lane] = rs_me;
+            if (tid == 0 && bad && !dry) failed = 1;
         } else if (J != 0) {
             // the previous panel's product for the columns right of this block
-            dg_syrk(sa, kb - 32, kb + 32, kb + 32, kLpNb, tid - 32, kDgThreads - 32);
+            dg_syrk(sa, kb - 32, kb + 32, kb, kLpNb, tid - 128, kDgThreads - 128);
+            if (!dry) dg_store(sa, L, ld, p, b, kb - 32, warp - 4, kDgThreads / 32 - 4, lane);
         }
         if (J == 0) asm volatile("cp.async.wait_group 0;" ::: "memory");  // this thread's copies, columns 32-127
         if (!dry) __syncthreads();  // (the warm-up pass runs its phases side by side: its data is discarded)
         if (failed && !dry) break;  // (`failed` is set at the first real step)
         const int w = kLpNb - kb - 32;  // rows below the diagonal block
         // (2) rows below: x L_JJ^T = a; rows of the identity: W_JJ
-        if (tid < w + 32) {
-            const int ie = tid - w;                  // identity row, when >= 0
-            const int r = ie < 0 ? kb + 32 + tid : 0;  // (row 0: any in-bounds address)
-            float v[32], rd[32];
+        // two threads a row: the even groups of four columns and the odd ones
+        if (tid < 2 * (w + 32)) {
+            const int t = tid >> 1, h = tid & 1, ie = t - w;  // ie: identity row, when >= 0
+            float *const dst = ie < 0 ? &sa[kb * kDgLd + kb + 32 + t] : &sw[ie * kDgWt];
+            const int step = ie < 0 ? kDgLd : 1;
+            float v[4][4];  // group 2 l + h
 #pragma unroll
-            for (int c = 0; c < 32; ++c) v[c] = (ie < 0) ? sa[(kb + c) * kDgLd + r] : (c == ie ? 1.f : 0.f);
+            for (int l = 0; l < 4; ++l)
 #pragma unroll
-            for (int g = 0; g < 8; ++g) {  // the reciprocal diagonal in registers: off the chain
-                const float4 r4 = *reinterpret_cast<const float4 *>(&rdiag[4 * g]);
-                rd[4 * g] = r4.x, rd[4 * g + 1] = r4.y, rd[4 * g + 2] = r4.z, rd[4 * g + 3] = r4.w;
-            }
+                for (int i = 0; i < 4; ++i) {
+                    const int c = 4 * (2 * l + h) + i;
+                    v[l][i] = ie < 0 ? dst[c * step] : (c == ie ? 1.f : 0.f);
+                }
 #pragma unroll
             for (int c = 0; c < 32; ++c) {
-                v[c] *= rd[c];
+                const int g = c / 4;
+                const float own = v[g / 2][c % 4] * rdiag[c];
+                const float x = __shfl_sync(0xffffffffu, own, (lane & ~1) | (g & 1));
+                if (h == (g & 1)) dst[c * step] = own;
+                // (finished entries are updated too: nothing reads them)
 #pragma unroll
-                for (int g = (c + 1) / 4; g < 8; ++g) {
-                    const float4 l4 = *reinterpret_cast<const float4 *>(&slt[c * kDgLt + 4 * g]);
-                    const float lv[4] = {l4.x, l4.y, l4.z, l4.w};
-#pragma unroll
-                    for (int i = 0; i < 4; ++i)
-                        if (4 * g + i > c) v[4 * g + i] = fmaf(-v[c], lv[i], v[4 * g + i]);
+                for (int l = g / 2; l < 4; ++l) {
+                    const float4 l4 = *reinterpret_cast<const float4 *>(&slt[c * kDgLt + 4 * (2 * l + h)]);
+                    v[l][0] = fmaf(-x, l4.x, v[l][0]);
+                    v[l][1] = fmaf(-x, l4.y, v[l][1]);
+                    v[l][2] = fmaf(-x, l4.z, v[l][2]);
+                    v[l][3] = fmaf(-x, l4.w, v[l][3]);
                 }
-            }
-            if (ie < 0) {
-#pragma unroll
-                for (int c = 0; c < 32; ++c) sa[(kb + c) * kDgLd + r] = v[c];
-            } else {
-#pragma unroll
-                for (int c = 0; c < 32; ++c)
-                    if (!dry) Wd[kb * 32 + ie * 32 + c] = v[c];  // W[c][ie] at [J][ie][c]
             }
         }
         if (!dry) __syncthreads();
-        // (3) the next block's columns; the finished column block to HBM
-        if (tid < 256) {
-            if (w > 0) dg_syrk(sa, kb, kb + 32, kb + 32, kb + 64, tid, 256);
-        } else {
-            for (int e = tid - 256; e < (dry ? 0 : (kLpNb - kb) * 32); e += kDgThreads - 256) {
-                const int r = kb + e % (kLpNb - kb), c = kb + e / (kLpNb - kb);
-                if (r < b && c <= r) L[(p + r) + (p + c) * ld] = sa[c * kDgLd + r];
-            }
-        }
+        // (3) the next diagonal block; W_JJ to memory
+        if (!dry)
+            for (int e = tid; e < 32 * 32; e += kDgThreads)  // W[c][ie] at [J][ie][c]
+                Wd[kb * 32 + e] = sw[(e >> 5) * kDgWt + (e & 31)];
+        if (w > 0) dg_syrk_block(sa, kb, kb + 32, tid);
         if (!dry) __syncthreads();
     }
     if (failed) {
         if (tid == 0) *info = p;  // the low-precision factorisation broke down in this panel
         return;
     }
+    dg_store(sa, L, ld, p, b, kLpNb - 32, warp, kDgThreads / 32, lane);
     if (warp == 0) {
         // smallest pivot of this block relative to the unit-ish equilibrated diagonal
         float rmin = ratio;

@@ -338,3 +338,30 @@ def test_batch_orders_and_failures(gpu_lla, dtype, shape):
         if x.size:
             den = np.abs(ad).sum(1).max() * np.abs(x).max(0) + np.abs(b0[i]).max(0)
             assert (r.max(0) <= 10 * max(k, 4) * eps * den).all(), (i, k)
+
+
+@pytest.mark.parametrize("n", [1, 2, 31, 32, 33, 63, 65, 96, 97, 127, 128, 129, 160, 255, 257, 385])
+@pytest.mark.parametrize("pad", [0, 4, 3])
+def test_mixed_factor_blocks(gpu_lla, n, pad):
+    """The mixed solve's diagonal blocks: edges of the 32-column steps and the 128-column blocks,
+    16-byte aligned columns and not: ||L L^T - A|| <= 10 n eps ||A||, nothing else written, and a
+    negative pivot reported in its block."""
+    torch = _torch()
+    A, _ = _spd(torch, n, 0.5, n)
+    A = A.float()
+    for row in (None, n - 1):
+        M = A.clone()
+        if row is not None:
+            M[row, row] = -1.0
+        buf = torch.full((n, n + pad), -7.0, dtype=torch.float32, device="cuda")
+        buf[:, :n] = M.T
+        L = buf.T[:n]
+        info = gpu_lla.spotrf_mixed_device(L, update="bf16x6")
+        torch.cuda.synchronize()
+        assert bool((buf[:, n:] == -7.0).all())
+        if row is not None:
+            assert int(info.item()) == row // 128 * 128
+            continue
+        assert int(info.item()) == -1
+        low = torch.tril(L).double()
+        assert float((low @ low.T - A.double()).norm() / A.double().norm()) <= 10 * n * torch.finfo(torch.float32).eps
