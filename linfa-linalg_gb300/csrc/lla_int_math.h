@@ -1,4 +1,5 @@
-// lla_int_math.h -- double-precision roots and quotients in integer arithmetic.
+// lla_int_math.h -- double-precision roots and quotients in integer arithmetic,
+// single-precision quotients by FMAs.
 // Host and device code; a host test checks them against the compiler's.
 //
 // On GB300 an FP64 instruction takes 64 cycles and occupies its sub-partition
@@ -158,6 +159,42 @@ __host__ __device__ __forceinline__ double im_div(double a, const ImDivisor &d, 
     const bool undecided = (spare == -1 && top == -1) || (spare == 0 && top == 0);
     ok = d.ok && (zero || (ea != 0 && ea != 0x7ff && q > -1020 && q < 1020 && !undecided));
     return im_double(zero ? sign : sign | (e + m));
+}
+
+// The same for FP32, where a chain of FMAs is short (4 cycles each; the general
+// division's is some 78): the reciprocal rounded to nearest, then Markstein's
+// theorem (IBM J. Res. Dev. 34, 1990): a quotient within one unit in the last
+// place, its exact remainder and that reciprocal give the rounded quotient.  The
+// first of the two corrections brings the quotient within the unit.
+struct FloatDivisor {
+    float d, y;
+    bool ok;
+};
+
+// Magnitudes 2^-lo .. 2^hi (a range of bit patterns: false for NaN and infinity).
+__host__ __device__ __forceinline__ bool float_within(float v, int lo, int hi) {
+    uint32_t b;
+    memcpy(&b, &v, 4);
+    const uint32_t first = (uint32_t)(127 - lo) << 23, last = (uint32_t)(127 + hi) << 23;
+    return (b & 0x7fffffffu) - first <= last - first;
+}
+
+__host__ __device__ __forceinline__ FloatDivisor float_divisor(float d) {
+    return {d, 1.0f / d, float_within(d, 100, 100)};
+}
+
+// a / d ..
+__host__ __device__ __forceinline__ float float_div(float a, const FloatDivisor &v) {
+    const float q0 = a * v.y;
+    const float q1 = fmaf(fmaf(-v.d, q0, a), v.y, q0);
+    const float q = fmaf(fmaf(-v.d, q1, a), v.y, q1);
+    return a == 0.0f ? q0 : q;  // (the corrections would lose a zero's sign)
+}
+
+// .. and whether that is IEEE division's result: a zero, or far enough from the
+// ends of the exponent range that the remainders are exact.
+__host__ __device__ __forceinline__ bool float_div_ok(float a, float q, const FloatDivisor &v) {
+    return v.ok && (a == 0.0f || (float_within(a, 100, 100) && float_within(q, 120, 120)));
 }
 
 // sqrt(d), correctly rounded, and the divisor it becomes; d positive and normal.

@@ -28,10 +28,10 @@
 // buffers, and the diagonal block, which is loaded and prepared before the
 // first wait.  An FP64 instruction takes 64 cycles of its sub-partition, so the
 // solve of a block keeps few of them in its chain: in EXACT mode the division by
-// the diagonal is done in integers (lla_int_math.h), in FAST mode the rows are divided by their diagonal beforehand and
-// a step is one FMA.  Four right-hand sides a CTA: one warp per sub-partition.
-// Per row block, before -> now: EXACT f64 25 -> 11 us (n = 512), EXACT f32 7.1 ->
-// 3.7 us (n = 1000, 8 right-hand sides), FAST f64 30 -> 7.3 us (n = 8192, 16
+// the diagonal is done in integers, for FP32 by FMAs (lla_int_math.h); in FAST mode
+// the rows are divided by their diagonal beforehand and a step is one FMA.  Four right-hand sides a CTA: one warp per sub-partition.
+// Per row block, before -> now: EXACT f64 25 -> 9.9 us (n = 512), EXACT f32 7.1 ->
+// 2.9 us (n = 1000, 8 right-hand sides), FAST f64 30 -> 7.3 us (n = 8192, 16
 // right-hand sides; 1.03 ms of the 1.9 ms solve is the FP64 pipe's share), FAST
 // f32 9.4 -> 2.0 us (n = 6001, 3 right-hand sides).
 //
@@ -70,25 +70,33 @@ __device__ __forceinline__ void cp_async_elem(T *dst, const T *src) {
 // Warps of a CTA: one per right-hand side; at least four copy the tiles.
 static int trsm_warps(int mc) { return std::max(mc, kTrsmMc); }
 
-// The division of the reference's substitution by a divisor that is known early;
-// ok says, off the chain, whether the quotient is IEEE division's, and the solve
-// repeats a block with IEEE division if one was not.
+// The division of the reference's substitution by a divisor that is known early,
+// without a test on its chain; ok says afterwards whether x is IEEE division's
+// num / d, and the solve repeats a block with IEEE division if one was not.
+// (Tested in every step: EXACT f64 n = 512 190 us a solve, now 165; EXACT f32
+// n = 1000, with the general division 123 us, with the test 137, now 99.)
 template <typename T>
 struct TrsmDivisor;
 template <>
 struct TrsmDivisor<float> {
-    float d;
-    __device__ __forceinline__ explicit TrsmDivisor(float v) { d = v; }
-    __device__ __forceinline__ float divide(float b, bool &ok) const {
-        ok = true;
-        return __fdiv_rn(b, d);
-    }
+    FloatDivisor q;
+    __device__ __forceinline__ explicit TrsmDivisor(float v) { q = float_divisor(v); }
+    __device__ __forceinline__ float divide(float b) const { return float_div(b, q); }
+    __device__ __forceinline__ bool ok(float num, float x) const { return float_div_ok(num, x, q); }
 };
 template <>
 struct TrsmDivisor<double> {
     ImDivisor q;
     __device__ __forceinline__ explicit TrsmDivisor(double v) { q = im_divisor(v); }
-    __device__ __forceinline__ double divide(double b, bool &ok) const { return im_div(b, q, ok); }
+    __device__ __forceinline__ double divide(double b) const {
+        bool unused;
+        return im_div(b, q, unused);
+    }
+    __device__ __forceinline__ bool ok(double num, double) const {
+        bool good;
+        im_div(num, q, good);
+        return good;
+    }
 };
 
 template <typename T, bool kExact>
@@ -222,15 +230,15 @@ __global__ void __launch_bounds__(kTrsmNb *kTrsmMaxMc) trsm_lookback(const T *__
             }
         } else {
             const T b0 = bv;
-            bool ok = true;
+            T num = bv;  // what this lane's row was divided from
 #pragma unroll 4
             for (int y = 0; y < bs; ++y) {
-                bool quot_ok;
-                const T xy = __shfl_sync(0xffffffffu, dq.divide(bv, quot_ok), y);  // coeff = b[i,k] / diag  (:117-119)
-                ok = ok && (tx != y || quot_ok);
+                const T xy = __shfl_sync(0xffffffffu, dq.divide(bv), y);  // coeff = b[i,k] / diag  (:117-119)
                 const T nb = kExact ? Ar::sub(bv, Ar::mul(xy, td[y][tx])) : Ar::fma_(-xy, td[y][tx], bv);
+                num = tx == y ? bv : num;
                 bv = tx == y ? xy : (tx > y ? nb : bv);
             }
+            const bool ok = tx >= bs || dq.ok(num, bv);
             if (!__all_sync(0xffffffffu, ok)) {
                 bv = b0;
 #pragma unroll 1

@@ -171,3 +171,64 @@ def test_integer_math_on_host(seed_error):
                         src, "-o", exe], check=True)
         r = subprocess.run([exe], capture_output=True, text=True)
         assert r.returncode == 0, r.stdout
+
+
+DIVISION = r"""
+#include <cmath>
+#include <cstdio>
+#include <cstring>
+#include <random>
+#include "lla_int_math.h"
+using namespace lla;
+static float bits(uint32_t b) { float f; std::memcpy(&f, &b, 4); return f; }
+static uint32_t ubits(float f) { uint32_t b; std::memcpy(&b, &f, 4); return b; }
+int main() {
+    std::mt19937_64 g(11);
+    long long bad = 0, taken = 0, asked = 0;
+    auto check = [&](float a, const FloatDivisor &v, bool want) {
+        const float q = float_div(a, v), w = a / v.d;
+        const bool ok = float_div_ok(a, q, v);
+        if (ok && ubits(q) != ubits(w) && bad++ < 5) std::printf("%a / %a = %a, %a\n", a, v.d, q, w);
+        if (want) ++asked, taken += ok;
+    };
+    for (long t = 0; t < 1500000; ++t) {
+        uint32_t db = (uint32_t)g();
+        if (t % 2) db = (db & 0x807fffffu) | ((100u + (uint32_t)(g() % 54)) << 23);
+        if (t % 5 == 0) db |= 0x7fff00u;            // mantissas near the ends
+        if (t % 7 == 0) db &= ~0x7fff00u;
+        if (t % 11 == 0) db |= 0x7fffffu;
+        const FloatDivisor v = float_divisor(bits(db));
+        for (int k = 0; k < 8; ++k) {
+            uint32_t ab = (uint32_t)g();
+            if (k & 1) ab = (ab & 0x807fffffu) | ((100u + (uint32_t)(g() % 54)) << 23);
+            if (k == 1) ab |= 0x7ffff0u;
+            if (k == 3) ab &= ~0x7ffff0u;
+            // next to a quotient, and next to the midpoint of two quotients
+            if (k == 4) ab = ubits(bits((uint32_t)(g() & 0x7fffffu) | 0x3f800000u) * v.d) + (uint32_t)(g() % 3) - 1u;
+            if (k == 6) ab = ubits((float)(((double)((g() & 0xffffffu) | 0x800000u) + 0.5) * (double)v.d * 0x1p-23));
+            if (k == 2) ab &= 0x80000000u;
+            check(bits(ab), v, k == 5 && t % 2);
+        }
+    }
+    // every mantissa by a few divisors
+    for (uint32_t db : {0x3f800001u, 0x3fffffffu, 0x3f7fffffu, 0xbfaaaaabu, 0x3fb504f3u})
+        for (uint32_t m = 0; m < 1u << 23; ++m) check(bits(0x3f800000u | m), float_divisor(bits(db)), false);
+    std::printf("bad %lld, taken %lld of %lld\n", bad, taken, asked);
+    return bad != 0 || taken != asked;
+}
+"""
+
+
+def test_float_division_on_host():
+    """FP32 quotients by Markstein's corrections: IEEE division's wherever they say so, and always
+    for exponents well inside the range."""
+    cxx = shutil.which("g++") or shutil.which("c++")
+    if cxx is None:
+        pytest.skip("no host C++ compiler")
+    with tempfile.TemporaryDirectory() as d:
+        src, exe = os.path.join(d, "t.cpp"), os.path.join(d, "t")
+        with open(src, "w") as f:
+            f.write(DIVISION)
+        subprocess.run([cxx, "-O2", "-std=c++17", "-ffp-contract=off", "-I", CSRC, src, "-o", exe], check=True)
+        r = subprocess.run([exe], capture_output=True, text=True)
+        assert r.returncode == 0, r.stdout
