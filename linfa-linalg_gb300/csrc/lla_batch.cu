@@ -40,7 +40,7 @@
 #include "lla_common.cuh"
 #include "lla_int_math.h"
 #include "lla_kernels.h"
-#include "lla_oz_digits.h"
+#include "lla_oz_mma.cuh"
 #include "lla_prof.h"
 
 namespace lla {
@@ -231,21 +231,6 @@ __device__ void batch_update(BatchSmem<float> &sm, float *A, int n, int q, int k
     __syncthreads();
 }
 
-// D (16 x 8, FP32) += A (16 x 16) B (16 x 8), FP16 operands.
-__device__ __forceinline__ void batch_mma(float (&d)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
-    asm volatile(
-        "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
-        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
-}
-// Four digits (bytes, biased by 128) as two pairs of FP16: 0x64xx is 1024 + xx.
-__device__ __forceinline__ void batch_digits(uint32_t w, uint32_t &lo, uint32_t &hi) {
-    const uint32_t a = __byte_perm(w, 0x64646464u, 0x4140), b = __byte_perm(w, 0x64646464u, 0x4342);
-    const uint32_t bias = 0x64806480u;  // 1152, 1152
-    asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(lo) : "r"(a), "r"(bias));
-    asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(hi) : "r"(b), "r"(bias));
-}
-
 // FP64: the product of the 16 panel columns on the tensor cores, from seven
 // balanced 8-bit digits per entry (exact in FP16, their products' sums exact in
 // the FP32 accumulators), one 64-bit integer per entry and one FP64 subtraction,
@@ -285,28 +270,24 @@ __device__ void batch_update(BatchSmem<double> &sm, double *A, int n, int q, int
         uint32_t fb[kOzBal][2];
 #pragma unroll
         for (int d = 0; d < kOzBal; ++d)
-            batch_digits(*reinterpret_cast<const uint32_t *>(sm.panel + (d * kBMaxN + 8 * J + g) * NB + 4 * t4), fb[d][0],
+            oz_byte_digits(*reinterpret_cast<const uint32_t *>(sm.panel + (d * kBMaxN + 8 * J + g) * NB + 4 * t4), fb[d][0],
                          fb[d][1]);
 #pragma unroll
         for (int d = 0; d < kOzBal; ++d) {
             uint32_t fa[4];
             const unsigned char *pa = sm.panel + (d * kBMaxN + 16 * I + g) * NB + 4 * t4;
-            batch_digits(*reinterpret_cast<const uint32_t *>(pa), fa[0], fa[2]);
-            batch_digits(*reinterpret_cast<const uint32_t *>(pa + 8 * NB), fa[1], fa[3]);
+            oz_byte_digits(*reinterpret_cast<const uint32_t *>(pa), fa[0], fa[2]);
+            oz_byte_digits(*reinterpret_cast<const uint32_t *>(pa + 8 * NB), fa[1], fa[3]);
 #pragma unroll
-            for (int e = 0; e < kOzBal - d; ++e) batch_mma(acc[d + e], fa, fb[e]);
+            for (int e = 0; e < kOzBal - d; ++e) oz_mma(acc[d + e], fa, fb[e]);
         }
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
             const int ei = sm.expo[16 * I + g + 8 * (u >> 1)], ej = sm.expo[8 * J + 2 * t4 + (u & 1)];
-            long long lo = 128, hi = 0;
-#pragma unroll
-            for (int l = 4; l < kOzBal; ++l) lo += (long long)__float2int_rn(acc[l][u]) * (1 << (8 * (6 - l)));
-#pragma unroll
-            for (int l = 0; l < 4; ++l) hi += (long long)__float2int_rn(acc[l][u]) * (1 << (8 * (3 - l)));
+            const int64_t sum = oz_byte_sum(acc, u);
             if (use >> u & 1) {
                 if (ei != kBNonFinite && ej != kBNonFinite) {
-                    *wp[u] = w[u] - oz_scaled_double(hi * 65536 + (lo >> 8), ei + ej - 54);
+                    *wp[u] = w[u] - oz_scaled_double(sum, ei + ej - 54);
                 } else {  // no digits: the FMA chain on the factor itself
                     const int i = 16 * I + g + 8 * (u >> 1), j = 8 * J + 2 * t4 + (u & 1);
                     double s = w[u];
@@ -324,22 +305,10 @@ __device__ void batch_update(BatchSmem<double> &sm, double *A, int n, int q, int
 
 // Word t of the digits of panel row rr: columns t, t + 4, t + 8, t + 12.
 __device__ __forceinline__ void batch_keep_word(BatchSmem<double> &sm, int rr, int t, const double (&w)[4], int e) {
-    uint64_t x[4];
+    uint32_t word[kOzBal];
+    oz_byte_words(w, e, e != kBNonFinite, word);
 #pragma unroll
-    for (int u = 0; u < 4; ++u)
-        x[u] = (e != kBNonFinite ? (uint64_t)oz_fixed55((int64_t)im_bits(w[u]), e) : 0ull) + 0x0080808080808080ull;
-    // the four values' bytes 0-3 and 4-6, transposed: byte s of all four in one word
-    const uint32_t l0 = (uint32_t)x[0], l1 = (uint32_t)x[1], l2 = (uint32_t)x[2], l3 = (uint32_t)x[3];
-    const uint32_t h0 = (uint32_t)(x[0] >> 32), h1 = (uint32_t)(x[1] >> 32), h2 = (uint32_t)(x[2] >> 32),
-                   h3 = (uint32_t)(x[3] >> 32);
-#pragma unroll
-    for (int d = 0; d < kOzBal; ++d) {
-        const int b = kOzBal - 1 - d;  // byte of the value
-        const uint32_t sel = (uint32_t)(b & 3) | (uint32_t)((b & 3) + 4) << 4;
-        const uint32_t p01 = b < 4 ? __byte_perm(l0, l1, sel) : __byte_perm(h0, h1, sel);
-        const uint32_t p23 = b < 4 ? __byte_perm(l2, l3, sel) : __byte_perm(h2, h3, sel);
-        *reinterpret_cast<uint32_t *>(sm.panel + (d * kBMaxN + rr) * 16 + 4 * t) = __byte_perm(p01, p23, 0x5410);
-    }
+    for (int d = 0; d < kOzBal; ++d) *reinterpret_cast<uint32_t *>(sm.panel + (d * kBMaxN + rr) * 16 + 4 * t) = word[d];
 }
 
 // Keeps a finished panel row (row rr of the panel) for the update.
@@ -355,9 +324,7 @@ __device__ __forceinline__ void batch_keep_row(BatchSmem<double> &sm, int rr, co
         const uint64_t b = im_bits(v[c]) & 0x7fffffffffffffffull;
         mx = b > mx ? b : mx;
     }
-    // one bit of headroom, so that the leading digit fits a byte as well
-    const bool fin = mx < 0x7ff0000000000000ull;
-    const int e = fin ? oz_bits_exponent(mx) + 1 : kBNonFinite;
+    const int e = mx < 0x7ff0000000000000ull ? oz_byte_exponent(mx) : kBNonFinite;
     sm.expo[rr] = e;
 #pragma unroll
     for (int t = 0; t < 4; ++t) {
@@ -415,7 +382,7 @@ __device__ void batch_panel_split(double *A, int n, int kb, int bs, int q, int r
         const uint64_t b = __shfl_xor_sync(0xffffffffu, (unsigned long long)mx, o);
         mx = b > mx ? b : mx;
     }
-    const int e = mx < 0x7ff0000000000000ull ? oz_bits_exponent(mx) + 1 : kBNonFinite;
+    const int e = mx < 0x7ff0000000000000ull ? oz_byte_exponent(mx) : kBNonFinite;
     if (in) {
         const int p = isb ? rhs_row<double>(rows) + rr - rows : rr;
         if (t == 0) sm.expo[p] = e;

@@ -27,7 +27,7 @@
 // the rest, so the trailing matrix is read and written once per 128 columns.
 //
 // Measured, FMA updates before -> now (error against 64 bits the same or lower):
-// f64 n = 8192 220 -> 13.6 ms, n = 2048 14.4 -> 2.2 ms; f32 n = 6001 14.6 ->
+// f64 n = 8192 220 -> 12.9 ms, n = 2048 14.4 -> 2.2 ms; f32 n = 6001 14.6 ->
 // 3.7 ms.  There is no size at which the FMA form is faster: one 64 x 64 tile of
 // the FP64 one took 70 us on its SM.
 #include <cuda.h>
@@ -40,7 +40,7 @@
 #include "lla_common.cuh"
 #include "lla_int_math.h"
 #include "lla_kernels.h"
-#include "lla_oz_digits.h"
+#include "lla_oz_mma.cuh"
 #include "lla_prof.h"
 #include "lla_scratch.h"
 #include "lla_tcgen05.cuh"
@@ -312,6 +312,88 @@ __global__ void __launch_bounds__(kFcDiagThreads) fc_diag_kernel(T *W, int64_t l
     fc_diag_block(sm, W, ld, p, b, diag0, rinv, info, min_ratio);
 }
 
+// FP64 panel, between its halves: x[32 + c][r] = sum_k x[k][r] L11[32 + c][k] over
+// the 32 finished columns, from byte digits of the 16 rows (wx) and of L11's rows
+// (wl, in the space of l11's upper triangle: row 32 + c's at column 32 + c).  By
+// 256 threads; ex, el: scale exponents.  Word q of a row and digit: columns q, q +
+// 8, q + 16, q + 24; words are swizzled by the row so that a fragment's loads meet
+// no bank twice.
+__device__ __forceinline__ uint32_t &fc_half_word(uint32_t *row, int i, int d, int q) {
+    return row[(d * 8 + q) ^ (4 * (i & 7))];
+}
+
+__device__ __forceinline__ int fc_half_digits(uint32_t *row, int i, int q, const double (&v)[4]) {
+    unsigned long long mx = 0;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        const unsigned long long b = Fc<double>::abs_bits(v[u]);
+        mx = b > mx ? b : mx;
+    }
+#pragma unroll
+    for (int o = 1; o < 8; o *= 2) {
+        const unsigned long long b = __shfl_xor_sync(0xffffffffu, mx, o);
+        mx = b > mx ? b : mx;
+    }
+    const bool finite = mx < 0x7ff0000000000000ull;
+    const int e = finite ? oz_byte_exponent(mx) : kFcNonFinite;
+    uint32_t w[kOzBal];
+    oz_byte_words(v, e, finite, w);
+#pragma unroll
+    for (int d = 0; d < kOzBal; ++d) fc_half_word(row, i, d, q) = w[d];
+    return e;
+}
+
+// Rows that hold inf or NaN have no digits: the FMA chain.
+__device__ __noinline__ double fc_half_plain(double v, const double *x, const double *l) {
+    for (int k = 0; k < kFcNb / 2; ++k) v = fma(-x[k * (16 + 1)], l[k * kFcNb], v);
+    return v;
+}
+
+__device__ __forceinline__ void fc_half_product(double (*l11)[kFcNb], double (*x)[16 + 1], uint32_t *wx, int *ex,
+                                                int *el) {
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
+    {
+        const int i = tid >> 3, q = tid & 7;
+        const double v[4] = {l11[q][32 + i], l11[q + 8][32 + i], l11[q + 16][32 + i], l11[q + 24][32 + i]};
+        const int e = fc_half_digits(reinterpret_cast<uint32_t *>(l11[32 + i]), i, q, v);
+        if (q == 0) el[i] = e;
+        if (tid < 128) {
+            const double u[4] = {x[q][i], x[q + 8][i], x[q + 16][i], x[q + 24][i]};
+            const int f = fc_half_digits(wx + i * 64, i, q, u);
+            if (q == 0) ex[i] = f;
+        }
+    }
+    __syncthreads();
+    if (warp < 4) {  // 8 columns a warp
+        float acc[kOzBal][4];
+#pragma unroll
+        for (int l = 0; l < kOzBal; ++l)
+#pragma unroll
+            for (int u = 0; u < 4; ++u) acc[l][u] = 0.f;
+        uint32_t *lrow = reinterpret_cast<uint32_t *>(l11[32 + 8 * warp + g]);
+#pragma unroll
+        for (int q = t4; q < 8; q += 4) {
+            uint32_t fb[kOzBal][2];
+#pragma unroll
+            for (int d = 0; d < kOzBal; ++d) oz_byte_digits(fc_half_word(lrow, g, d, q), fb[d][0], fb[d][1]);
+#pragma unroll
+            for (int d = 0; d < kOzBal; ++d) {
+                uint32_t fa[4];
+                oz_byte_digits(fc_half_word(wx + g * 64, g, d, q), fa[0], fa[2]);
+                oz_byte_digits(fc_half_word(wx + (g + 8) * 64, g, d, q), fa[1], fa[3]);
+#pragma unroll
+                for (int e = 0; e < kOzBal - d; ++e) oz_mma(acc[d + e], fa, fb[e]);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int r = g + 8 * (u >> 1), c = 8 * warp + 2 * t4 + (u & 1);
+            x[32 + c][r] = oz_scaled_double(oz_byte_sum(acc, u), ex[r] + el[c] - 54);
+        }
+    }
+    __syncthreads();
+}
+
 // Panel rows [q, n), q = p + 64: L21 = A21 L11^-T by substitution (multiplying
 // by the reciprocal pivots), 16 rows per CTA so that a trailing matrix of 2400
 // rows still covers the chip, and the digits of the finished rows.  The rows
@@ -319,10 +401,13 @@ __global__ void __launch_bounds__(kFcDiagThreads) fc_diag_kernel(T *W, int64_t l
 // column pairs w, w + 8, w + 16, w + 24).  Pairs are finished in turn: the
 // owner solves its two columns and publishes them, one barrier, every warp
 // applies both to its pairs right of them; the next owner updates and solves
-// its own pair before the others, so a step's chain is two updates, two
-// scalings and one exchange (n = 8192: 172 -> 33 us a panel on average).  second: the pair of panels' second one -- the
-// rows' first-panel entries are read back and the digits of all 128 columns are
-// formed with a common exponent.
+// its own pair before the others, so a step's chain is two updates, two scalings
+// and one exchange.  In FP64 the pipe bounds a panel with more than one CTA an SM,
+// so the right half takes the left half's columns from the tensor cores instead of
+// by substitution, which halves the FP64 instructions (n = 8192: 172 us a panel on
+// average before, 32 by substitution alone, 27 now; n = 2048 21.9 -> 21.1).
+// second: the pair of panels' second one -- the rows' first-panel entries are read
+// back and the digits of all 128 columns are formed with a common exponent.
 constexpr int kFcRows = 16;
 constexpr int kFcPanelThreads = 256;
 
@@ -338,6 +423,9 @@ __global__ void __launch_bounds__(kFcPanelThreads) fc_panel_kernel(T *W, int64_t
     __shared__ T rv[kFcNb];
     __shared__ Bits s_max[kFcPanelThreads / 16][kFcRows];
     __shared__ int s_e[kFcRows];
+    constexpr bool kHalves = sizeof(T) == 8;
+    __shared__ uint32_t wx[kHalves ? kFcRows * 64 : 1];
+    __shared__ int el[kFcNb / 2];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int r16 = lane & 15, cc = lane >> 4;
     const int64_t j0 = p + kFcNb + (int64_t)blockIdx.x * kFcRows;
@@ -366,13 +454,30 @@ __global__ void __launch_bounds__(kFcPanelThreads) fc_panel_kernel(T *W, int64_t
     __syncthreads();
 #pragma unroll
     for (int s0 = 0; s0 < 4; ++s0) {
+        const int send = kHalves && s0 < 2 ? 2 : 4;
+        if constexpr (kHalves) {
+            if (s0 == 2) {
+                fc_half_product(l11, x, wx, s_e, el);
+#pragma unroll
+                for (int s = 2; s < 4; ++s) {
+                    const int c = 2 * (warp + 8 * s) + cc;
+                    if (s_e[r16] != kFcNonFinite && el[c - 32] != kFcNonFinite)
+                        acc[s] -= x[c][r16];
+                    else
+                        acc[s] = fc_half_plain(acc[s], &x[0][r16], &l11[0][c]);
+                }
+                __syncthreads();  // the products have been read
+                if (warp == 0) solve(16, acc[2]);
+                __syncthreads();
+            }
+        }
 #pragma unroll 1
         for (int w0 = 0; w0 < 8; ++w0) {
             const int j = 8 * s0 + w0;  // pair j is finished: apply it to the pairs right of it
-            if (j == kFcNb / 2 - 1) break;
+            if (j == kFcNb / 2 - 1 || (kHalves && j == kFcNb / 4 - 1)) break;
             const T x0 = x[2 * j][r16], x1 = x[2 * j + 1][r16];
 #pragma unroll
-            for (int s = s0; s < 4; ++s) {
+            for (int s = s0; s < send; ++s) {
                 const int jj = 8 * s + warp;
                 if (jj <= j) continue;
                 const int c = 2 * jj + cc;

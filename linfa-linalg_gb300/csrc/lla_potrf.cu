@@ -1,8 +1,6 @@
 // lla_potrf.cu -- blocked Cholesky factorisation kernels (lower triangle,
-// column-major device matrices) in two arithmetic modes.
-//
-// EXACT mode keeps the reference's per-element operation order
-// (src/cholesky.rs:54-74): for every pair j > k the sum
+// column-major device matrices), EXACT mode.  It keeps the reference's
+// per-element operation order (src/cholesky.rs:54-74): for every pair j > k the sum
 //     s_jk = sum_{i<k} L[k,i] * L[j,i]
 // is accumulated from zero in ascending i, then
 //     L[j,k] = (A[j,k] - s_jk) / L[k,k],      d_j += L[j,k]^2   (ascending k),
@@ -13,8 +11,7 @@
 // exactly the same products in exactly the same order, each multiply and add
 // rounded separately, so the factor is bit-identical to the reference's.
 //
-// FAST mode is LAPACK-style right-looking (A22 -= L21 L21^T in place) with
-// fused multiply-add; this file holds the FP32 form, lla_fp64_chol.cu the FP64 one.
+// FAST mode is in lla_fast_chol.cu.
 #include "lla_common.cuh"
 #include "lla_int_math.h"
 #include "lla_kernels.h"
