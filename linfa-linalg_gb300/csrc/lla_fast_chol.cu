@@ -27,8 +27,8 @@
 // the rest, so the trailing matrix is read and written once per 128 columns.
 //
 // Measured, FMA updates before -> now (error against 64 bits the same or lower):
-// f64 n = 8192 220 -> 12.9 ms, n = 2048 14.4 -> 2.2 ms; f32 n = 6001 14.6 ->
-// 3.7 ms.  There is no size at which the FMA form is faster: one 64 x 64 tile of
+// f64 n = 8192 220 -> 12.4 ms, n = 2048 14.4 -> 2.0 ms; f32 n = 6001 14.6 ->
+// 3.1 ms.  There is no size at which the FMA form is faster: one 64 x 64 tile of
 // the FP64 one took 70 us on its SM.
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -89,6 +89,12 @@ struct Fc<float> {
     static __device__ __forceinline__ bool normal(float d) { return __float_as_uint(d) - 0x800000u < 0x7f000000u; }
 };
 
+// Asynchronous copy to shared memory: all of a thread's copies are in flight at once.
+template <typename T>
+__device__ __forceinline__ void fc_copy(T *dst, const T *src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(smem_u32(dst)), "l"(src), "n"(sizeof(T)) : "memory");
+}
+
 __device__ __forceinline__ void atomic_min_pos_f64(double *addr, double v) {
     // non-negative doubles order like their bit patterns
     if (v >= 0.0) atomicMin((unsigned long long *)addr, (unsigned long long)__double_as_longlong(v));
@@ -106,7 +112,7 @@ __device__ __forceinline__ void atomic_min_pos_f64(double *addr, double v) {
 // the other three sub-partitions keep the rest in registers, in patches of 16
 // rows x 2 columns (one FP64 instruction per column applied), and hand pair
 // k + 2 to warp 0 through shared memory once pair k is in it.  One barrier per
-// pair.  160 -> 33 us a block (FP32 67 -> 14 us).
+// pair.  160 -> 31 us a block (FP32 67 -> 13 us).
 constexpr int kFcDiagThreads = 512;
 constexpr int kFcPatches = 80, kFcPatchWarps = 12, kFcSlots = 7;
 
@@ -223,12 +229,17 @@ __device__ __forceinline__ void fc_diag_block(FcDiagSmem<T> &sm, T *W, int64_t l
     T(*a)[kFcNb] = sm.a;
     T *piv = sm.piv, *rv = sm.rv;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+#pragma unroll
     for (int e = tid; e < kFcNb * kFcNb; e += kFcDiagThreads) {
         const int r = e % kFcNb, c = e / kFcNb;
         // a short block is padded with the identity
-        a[c][r] = (r < b && c <= r) ? cm(W, ld, p + r, p + c) : T(r == c ? 1 : 0);
+        if (r < b && c <= r)
+            fc_copy(&a[c][r], &cm(W, ld, p + r, p + c));
+        else
+            a[c][r] = T(r == c ? 1 : 0);
     }
     if (tid == 0) sm.fail = -1;
+    asm volatile("cp.async.wait_all;" ::: "memory");
     fc_diag_sync();
     const bool upd = (warp & 3) != 0;  // a patch warp (warps 4, 8 and 12 only load and store)
     T acc[kFcSlots];
@@ -397,15 +408,17 @@ __device__ __forceinline__ void fc_half_product(double (*l11)[kFcNb], double (*x
 // Panel rows [q, n), q = p + 64: L21 = A21 L11^-T by substitution (multiplying
 // by the reciprocal pivots), 16 rows per CTA so that a trailing matrix of 2400
 // rows still covers the chip, and the digits of the finished rows.  The rows
-// stay in registers as patches of 16 rows x 2 columns, four per warp (warp w:
-// column pairs w, w + 8, w + 16, w + 24).  Pairs are finished in turn: the
-// owner solves its two columns and publishes them, one barrier, every warp
-// applies both to its pairs right of them; the next owner updates and solves
-// its own pair before the others, so a step's chain is two updates, two scalings
-// and one exchange.  In FP64 the pipe bounds a panel with more than one CTA an SM,
-// so the right half takes the left half's columns from the tensor cores instead of
-// by substitution, which halves the FP64 instructions (n = 8192: 172 us a panel on
-// average before, 32 by substitution alone, 27 now; n = 2048 21.9 -> 21.1).
+// stay in registers as patches of 8 rows x 4 columns, four per warp (warp w: rows
+// 8 (w % 2) .., column quads w / 2 + 4 s).  Quads are finished in turn: their two
+// owners solve the four columns by shuffles and publish them, one barrier, every
+// warp applies them to its quads right of them; the next owners update and solve
+// their own quad before the others.  What bounds it is that chain: with pairs of
+// columns, twice the barriers and exchanges, n = 2048 took 21 us a panel in FP64
+// and 13 in FP32 (n = 6001), now 16 and 8; the loads, all in flight at once, take
+// 1.5 of them, 2 before.  In FP64 the pipe bounds a panel with more than one CTA an
+// SM, so the right half takes the left half's columns from the tensor cores instead
+// of by substitution, which halves the FP64 instructions.  n = 8192: 172 us a panel
+// on average at first, 32 with pairs by substitution alone, 27 in halves, now 24.
 // second: the pair of panels' second one -- the rows' first-panel entries are read
 // back and the digits of all 128 columns are formed with a common exponent.
 constexpr int kFcRows = 16;
@@ -427,30 +440,43 @@ __global__ void __launch_bounds__(kFcPanelThreads) fc_panel_kernel(T *W, int64_t
     __shared__ uint32_t wx[kHalves ? kFcRows * 64 : 1];
     __shared__ int el[kFcNb / 2];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int r16 = lane & 15, cc = lane >> 4;
+    const int row = 8 * (warp & 1) + (lane & 7), c4 = lane >> 3, wq = warp >> 1;
     const int64_t j0 = p + kFcNb + (int64_t)blockIdx.x * kFcRows;
     pdl_wait();
     pdl_trigger();
     if (*(volatile const int64_t *)info >= 0) return;
-    const bool in = j0 + r16 < n;
-    T acc[4];
+    // everything the panel reads, in flight at once: L11's lower triangle straight to shared memory
 #pragma unroll
-    for (int s = 0; s < 4; ++s) acc[s] = in ? cm(W, ld, j0 + r16, p + 2 * (warp + 8 * s) + cc) : T(0);
     for (int e = tid; e < kFcNb * kFcNb; e += kFcPanelThreads) {
         const int r = e % kFcNb, c = e / kFcNb;
-        l11[c][r] = c <= r ? cm(W, ld, p + r, p + c) : T(0);
+        if (c <= r) fc_copy(&l11[c][r], &cm(W, ld, p + r, p + c));
+    }
+    T acc[4], first[4];  // first: the pair's first panel
+#pragma unroll
+    for (int s = 0; s < 4; ++s) acc[s] = j0 + row < n ? cm(W, ld, j0 + row, p + 4 * (wq + 4 * s) + c4) : T(0);
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+        const int e = tid + s * kFcPanelThreads, r = e % kFcRows, c = e / kFcRows;
+        first[s] = second && j0 + r < n ? cm(W, ld, j0 + r, p - kFcNb + c) : T(0);
     }
     if (tid < kFcNb) rv[tid] = rinv[tid];
+    asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
-    // solves column pair j (this warp's slot value v) and publishes it
-    auto solve = [&](int j, T v) {
-        const int c = 2 * j;
-        T u = v * rv[c];
-        const T x0 = __shfl_sync(0xffffffffu, u, r16);
-        if (cc) u = fma(-x0, l11[c][c + 1], v) * rv[c + 1];
-        x[c + cc][r16] = u;
+    // solves column quad q (this warp's slot value v) and publishes it
+    auto solve = [&](int q, T v) {
+        const int c = 4 * q;
+        const T rc = rv[c + c4], l0 = l11[c][c + c4], l1 = l11[c + 1][c + c4], l2 = l11[c + 2][c + c4];
+        // (a lane's v goes on past its own column; nothing reads it there)
+        const T u0 = v * rc;
+        v = fma(-__shfl_sync(0xffffffffu, u0, lane & 7), l0, v);
+        const T u1 = v * rc;
+        v = fma(-__shfl_sync(0xffffffffu, u1, 8 + (lane & 7)), l1, v);
+        const T u2 = v * rc;
+        v = fma(-__shfl_sync(0xffffffffu, u2, 16 + (lane & 7)), l2, v);
+        const T u3 = v * rc;
+        x[c + c4][row] = c4 & 2 ? (c4 & 1 ? u3 : u2) : (c4 & 1 ? u1 : u0);
     };
-    if (warp == 0) solve(0, acc[0]);
+    if (wq == 0) solve(0, acc[0]);
     __syncthreads();
 #pragma unroll
     for (int s0 = 0; s0 < 4; ++s0) {
@@ -460,29 +486,31 @@ __global__ void __launch_bounds__(kFcPanelThreads) fc_panel_kernel(T *W, int64_t
                 fc_half_product(l11, x, wx, s_e, el);
 #pragma unroll
                 for (int s = 2; s < 4; ++s) {
-                    const int c = 2 * (warp + 8 * s) + cc;
-                    if (s_e[r16] != kFcNonFinite && el[c - 32] != kFcNonFinite)
-                        acc[s] -= x[c][r16];
+                    const int c = 4 * (wq + 4 * s) + c4;
+                    if (s_e[row] != kFcNonFinite && el[c - 32] != kFcNonFinite)
+                        acc[s] -= x[c][row];
                     else
-                        acc[s] = fc_half_plain(acc[s], &x[0][r16], &l11[0][c]);
+                        acc[s] = fc_half_plain(acc[s], &x[0][row], &l11[0][c]);
                 }
                 __syncthreads();  // the products have been read
-                if (warp == 0) solve(16, acc[2]);
+                if (wq == 0) solve(8, acc[2]);
                 __syncthreads();
             }
         }
 #pragma unroll 1
-        for (int w0 = 0; w0 < 8; ++w0) {
-            const int j = 8 * s0 + w0;  // pair j is finished: apply it to the pairs right of it
-            if (j == kFcNb / 2 - 1 || (kHalves && j == kFcNb / 4 - 1)) break;
-            const T x0 = x[2 * j][r16], x1 = x[2 * j + 1][r16];
+        for (int w0 = 0; w0 < 4; ++w0) {
+            const int j = 4 * s0 + w0;  // quad j is finished: apply it to the quads right of it
+            if (j == kFcNb / 4 - 1 || (kHalves && j == kFcNb / 8 - 1)) break;
+            T xv[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) xv[u] = x[4 * j + u][row];
 #pragma unroll
             for (int s = s0; s < send; ++s) {
-                const int jj = 8 * s + warp;
-                if (jj <= j) continue;
-                const int c = 2 * jj + cc;
-                acc[s] = fma(-x1, l11[2 * j + 1][c], fma(-x0, l11[2 * j][c], acc[s]));
-                if (jj == j + 1) solve(jj, acc[s]);
+                const int q = 4 * s + wq;
+                if (q <= j) continue;
+#pragma unroll
+                for (int u = 0; u < 4; ++u) acc[s] = fma(-xv[u], l11[4 * j + u][4 * q + c4], acc[s]);
+                if (q == j + 1) solve(q, acc[s]);
             }
             __syncthreads();
         }
@@ -494,9 +522,10 @@ __global__ void __launch_bounds__(kFcPanelThreads) fc_panel_kernel(T *W, int64_t
     // the pair's first panel, in the space of L11
     T(*x1)[kFcRows + 1] = reinterpret_cast<T(*)[kFcRows + 1]>(&l11[0][0]);
     if (second)
-        for (int e = tid; e < kFcRows * kFcNb; e += kFcPanelThreads) {
-            const int r = e % kFcRows, c = e / kFcRows;
-            x1[c][r] = j0 + r < n ? cm(W, ld, j0 + r, p - kFcNb + c) : T(0);
+#pragma unroll
+        for (int s = 0; s < 4; ++s) {
+            const int e = tid + s * kFcPanelThreads;
+            x1[e / kFcRows][e % kFcRows] = first[s];
         }
     __syncthreads();
     // row maxima over the pair's columns so far, on the bit patterns

@@ -81,7 +81,7 @@ constexpr int kExPatches = 24, kExPatchWarps = 12, kExSlots = 2;
 // *s_fail is the failing column or -1.
 template <typename T, bool LIB>
 __device__ bool exact_diag_block(const T *W, const T *S, const T *D, int64_t ld, int64_t p, int b,
-                                 T (*a)[kNbExact + 1], T (*s)[kNbExact + 1], int *s_fail) {
+                                 T (*a)[kNbExact + 1], T (*s)[kNbExact + 1], int64_t failed, int *s_fail) {
     using Ar = Arith<T>;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     for (int e = tid; e < kNbExact * kNbExact; e += kExDiagThreads) {
@@ -92,6 +92,7 @@ __device__ bool exact_diag_block(const T *W, const T *S, const T *D, int64_t ld,
     }
     if (tid == 0) *s_fail = -1;
     T d = (warp == 0 && lane < b && p > 0) ? D[p + lane] : T(0);
+    if (failed >= 0) return true;  // (the same for all threads; tested here, its load in flight with the others)
     __syncthreads();
     const bool upd = (warp & 3) != 0;
     T acc[kExSlots];
@@ -164,10 +165,11 @@ __global__ void __launch_bounds__(kExDiagThreads) potrf_exact_diag(T *W, const T
     const int tid = threadIdx.x;
     pdl_wait();
     pdl_trigger();
-    if (*(volatile int64_t *)info >= 0) return;  // an earlier panel failed
+    const int64_t failed = *(volatile int64_t *)info;  // an earlier panel failed
     constexpr bool lib = sizeof(T) == 4;  // FP32 roots and quotients are fast as they are
-    if (!exact_diag_block<T, lib>(W, S, D, ld, p, b, a, s, &s_fail) && !lib)
-        exact_diag_block<T, true>(W, S, D, ld, p, b, a, s, &s_fail);
+    if (!exact_diag_block<T, lib>(W, S, D, ld, p, b, a, s, failed, &s_fail) && !lib)
+        exact_diag_block<T, true>(W, S, D, ld, p, b, a, s, failed, &s_fail);
+    if (failed >= 0) return;
     if (s_fail >= 0 && tid == 0) *info = p + s_fail;
     // every value computed (on failure the caller keeps only rows < info and row
     // info's strict lower part)
@@ -252,11 +254,12 @@ __global__ void __launch_bounds__(kExPanelThreads) potrf_exact_panel(T *W, const
     const int64_t j0 = p + kNbExact + (int64_t)blockIdx.x * kExRows;
     pdl_wait();
     pdl_trigger();
-    if (*(volatile const int64_t *)info >= 0) return;
+    const int64_t failed = *(volatile const int64_t *)info;  // (its load in flight with the others)
     for (int e = tid; e < kNbExact * kNbExact; e += kExPanelThreads) {
         const int r = e % kNbExact, c = e / kNbExact;
         l11[c][r] = c <= r ? cm(W, ld, p + r, p + c) : T(0);
     }
+    if (failed >= 0) return;
     if (tid < kNbExact) {
         const T l = cm(W, ld, p + tid, p + tid);
         piv[tid].from_root(l);
@@ -295,7 +298,7 @@ __global__ void __launch_bounds__(128) potrf_exact_update(const T *W, T *S, int6
     __shared__ T lk[kNbExact][kExTile];
     pdl_wait();
     pdl_trigger();
-    if (*(volatile const int64_t *)info >= 0) return;
+    const int64_t failed = *(volatile const int64_t *)info;  // (its load in flight with the others)
     int64_t I, J;
     tri_tile(blockIdx.x, I, J);
     const int64_t q = p + kNbExact, j0 = q + I * kExTile, k0 = q + J * kExTile;
@@ -311,6 +314,7 @@ __global__ void __launch_bounds__(128) potrf_exact_update(const T *W, T *S, int6
         lj[k][r] = (j0 + r < n) ? cm(W, ld, j0 + r, p + k) : T(0);
         lk[k][r] = (k0 + r < n) ? cm(W, ld, k0 + r, p + k) : T(0);
     }
+    if (failed >= 0) return;
     __syncthreads();
 #pragma unroll 8
     for (int k = 0; k < kNbExact; ++k)
