@@ -26,9 +26,17 @@ namespace lla {
 // bit-identical to IEEE), the accumulators stay in registers as patches of 16
 // rows x 2 columns, and tiles are small, so that every SM's pipe has a share.
 // Per panel of a 512 x 512 factorisation, before -> now: diagonal block 53 ->
-// 20 us, panel 66 -> 18 us, update 82 -> 10 us (f64; the whole factor 3160 ->
-// 783 us).
+// 18 us, panel 66 -> 15 us, update 82 -> 10 us (f64; the whole factor 3160 ->
+// 730 us).
 constexpr int kNbExact = 32;
+
+// Asynchronous copy to shared memory: all of a thread's copies are in flight at once.
+template <typename T>
+__device__ __forceinline__ void exact_copy(T *dst, const T *src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src),
+                 "n"(sizeof(T))
+                 : "memory");
+}
 
 // d <= 0 as the reference tests it (src/cholesky.rs:69, false for NaN).
 template <typename T>
@@ -87,11 +95,18 @@ __device__ bool exact_diag_block(const T *W, const T *S, const T *D, int64_t ld,
     for (int e = tid; e < kNbExact * kNbExact; e += kExDiagThreads) {
         const int r = e % kNbExact, c = e / kNbExact;
         // a short block is padded with the identity
-        a[c][r] = (r < b && c <= r) ? cm(W, ld, p + r, p + c) : T(r == c ? 1 : 0);
-        s[c][r] = (r < b && c < r && p > 0) ? cm(S, ld, p + r, p + c) : T(0);
+        if (r < b && c <= r)
+            exact_copy(&a[c][r], &cm(W, ld, p + r, p + c));
+        else
+            a[c][r] = T(r == c ? 1 : 0);
+        if (r < b && c < r && p > 0)
+            exact_copy(&s[c][r], &cm(S, ld, p + r, p + c));
+        else
+            s[c][r] = T(0);
     }
     if (tid == 0) *s_fail = -1;
     T d = (warp == 0 && lane < b && p > 0) ? D[p + lane] : T(0);
+    asm volatile("cp.async.wait_all;" ::: "memory");
     if (failed >= 0) return true;  // (the same for all threads; tested here, its load in flight with the others)
     __syncthreads();
     const bool upd = (warp & 3) != 0;
@@ -180,10 +195,12 @@ __global__ void __launch_bounds__(kExDiagThreads) potrf_exact_diag(T *W, const T
 }
 
 // Rows [q, n) below the diagonal block, q = p + 32; 16 rows per CTA.  The sums
-// stay in registers as patches of 16 rows x 2 columns, two per warp (warp w:
-// column pairs w and w + 8); pairs are finished in turn by their owner, one
-// barrier each, the next owner bringing its own pair up to date first.  Warp 8
-// adds the rows' squares to D as their columns appear.
+// stay in registers as patches of 8 rows x 4 columns, two per warp (warp w: rows
+// 8 (w % 2) .., column quads w / 2 and w / 2 + 4); quads are finished in turn by
+// their two owners, one barrier each, the next owners bringing their own quad up to
+// date first.  The chain of divisions and sums bounds it; by pairs of columns, with
+// twice the barriers, a panel took 17 us (one copy of the division in a rolled loop:
+// 16, and the diagonal block so 20 instead of 18).  Warp 8 adds the rows' squares to D as their columns appear.
 constexpr int kExRows = 16;
 constexpr int kExPanelThreads = 288;
 
@@ -191,52 +208,63 @@ template <typename T, bool LIB>
 __device__ bool exact_panel_rows(const T *W, const T *S, const T *D, int64_t ld, int64_t n, int64_t p, int64_t j0,
                                  const T (*l11)[kNbExact + 1], const ExactPivot<T, LIB> *piv, T (*x)[kExRows], T &dj) {
     using Ar = Arith<T>;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, r16 = lane & 15, cc = lane >> 4;
-    const bool in = j0 + r16 < n;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, c4 = lane >> 3, wq = warp >> 1;
+    const int row = warp < 8 ? 8 * (warp & 1) + (lane & 7) : lane & 15;
+    const bool in = j0 + row < n;
     T av[2] = {T(0), T(0)}, sv[2] = {T(0), T(0)};
     if (warp < 8) {
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
-            const int64_t c = p + 2 * (warp + 8 * i) + cc;
-            av[i] = in ? cm(W, ld, j0 + r16, c) : T(0);
-            sv[i] = (in && p > 0) ? cm(S, ld, j0 + r16, c) : T(0);
+            const int64_t c = p + 4 * (wq + 4 * i) + c4;
+            av[i] = in ? cm(W, ld, j0 + row, c) : T(0);
+            sv[i] = (in && p > 0) ? cm(S, ld, j0 + row, c) : T(0);
         }
     }
-    dj = (warp == 8 && in && p > 0) ? D[j0 + r16] : T(0);
+    dj = (warp == 8 && in && p > 0) ? D[j0 + row] : T(0);
+    asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();  // l11, piv
     bool ok = true;
-    auto solve = [&](int j, T a0, T s0) {  // column pair j
-        const int c = 2 * j;
-        bool g0 = true, g1 = true;
-        const T u0 = piv[c].divide(Ar::sub(a0, s0), g0);  // (:62); the first column's lanes
-        const T x0 = __shfl_sync(0xffffffffu, u0, r16);
-        const T u1 = piv[c + 1].divide(Ar::sub(a0, Ar::add(s0, Ar::mul(l11[c][c + 1], x0))), g1);
-        ok = ok && (cc ? g1 : g0);
-        x[c + cc][r16] = cc ? u1 : u0;
+    auto solve = [&](int q, T a0, T s0) {  // column quad q
+        const int c = 4 * q;
+        const ExactPivot<T, LIB> pv = piv[c + c4];
+        const T l0 = l11[c][c + c4], l1 = l11[c + 1][c + c4], l2 = l11[c + 2][c + c4];
+        // (a lane's sum goes on past its own column; nothing reads it there)
+        bool g[4] = {true, true, true, true};
+        const T u0 = pv.divide(Ar::sub(a0, s0), g[0]);  // (:62)
+        s0 = Ar::add(s0, Ar::mul(l0, __shfl_sync(0xffffffffu, u0, lane & 7)));
+        const T u1 = pv.divide(Ar::sub(a0, s0), g[1]);
+        s0 = Ar::add(s0, Ar::mul(l1, __shfl_sync(0xffffffffu, u1, 8 + (lane & 7))));
+        const T u2 = pv.divide(Ar::sub(a0, s0), g[2]);
+        s0 = Ar::add(s0, Ar::mul(l2, __shfl_sync(0xffffffffu, u2, 16 + (lane & 7))));
+        const T u3 = pv.divide(Ar::sub(a0, s0), g[3]);
+        x[c + c4][row] = c4 & 2 ? (c4 & 1 ? u3 : u2) : (c4 & 1 ? u1 : u0);
+        ok = ok && (c4 & 2 ? (c4 & 1 ? g[3] : g[2]) : (c4 & 1 ? g[1] : g[0]));
     };
-    if (warp == 0) solve(0, av[0], sv[0]);
+    if (wq == 0) solve(0, av[0], sv[0]);
     __syncthreads();
 #pragma unroll
     for (int i0 = 0; i0 < 2; ++i0) {
 #pragma unroll 1
-        for (int w0 = 0; w0 < 8; ++w0) {
-            const int j = 8 * i0 + w0;  // pair j is finished: add its products to the pairs right of it
-            const T x0 = x[2 * j][r16], x1 = x[2 * j + 1][r16];
+        for (int w0 = 0; w0 < 4; ++w0) {
+            const int j = 4 * i0 + w0;  // quad j is finished: add its products to the quads right of it
+            T xv[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) xv[u] = x[4 * j + u][row];
             if (warp == 8) {
-                dj = Ar::add(dj, Ar::mul(x0, x0));  // (:64)
-                dj = Ar::add(dj, Ar::mul(x1, x1));
+#pragma unroll
+                for (int u = 0; u < 4; ++u) dj = Ar::add(dj, Ar::mul(xv[u], xv[u]));  // (:64)
             } else {
 #pragma unroll
                 for (int i = i0; i < 2; ++i) {
-                    const int jj = 8 * i + warp;
-                    if (jj <= j) continue;
-                    const int c = 2 * jj + cc;
-                    sv[i] = Ar::add(sv[i], Ar::mul(l11[2 * j][c], x0));  // (:59-61)
-                    sv[i] = Ar::add(sv[i], Ar::mul(l11[2 * j + 1][c], x1));
-                    if (jj == j + 1) solve(jj, av[i], sv[i]);
+                    const int q = 4 * i + wq;
+                    if (q <= j) continue;
+#pragma unroll
+                    for (int u = 0; u < 4; ++u)
+                        sv[i] = Ar::add(sv[i], Ar::mul(l11[4 * j + u][4 * q + c4], xv[u]));  // (:59-61)
+                    if (q == j + 1) solve(q, av[i], sv[i]);
                 }
             }
-            if (j < kNbExact / 2 - 1) __syncthreads();
+            if (j < kNbExact / 4 - 1) __syncthreads();
         }
     }
     return __syncthreads_and(ok) != 0;
@@ -255,15 +283,19 @@ __global__ void __launch_bounds__(kExPanelThreads) potrf_exact_panel(T *W, const
     pdl_wait();
     pdl_trigger();
     const int64_t failed = *(volatile const int64_t *)info;  // (its load in flight with the others)
+#pragma unroll
     for (int e = tid; e < kNbExact * kNbExact; e += kExPanelThreads) {
         const int r = e % kNbExact, c = e / kNbExact;
-        l11[c][r] = c <= r ? cm(W, ld, p + r, p + c) : T(0);
+        if (c <= r) exact_copy(&l11[c][r], &cm(W, ld, p + r, p + c));
     }
-    if (failed >= 0) return;
     if (tid < kNbExact) {
         const T l = cm(W, ld, p + tid, p + tid);
         piv[tid].from_root(l);
         lpiv[tid].from_root(l);
+    }
+    if (failed >= 0) {
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        return;
     }
     T dj;
     if (!exact_panel_rows<T, lib>(W, S, D, ld, n, p, j0, l11, piv, x, dj) && !lib)
@@ -309,6 +341,7 @@ __global__ void __launch_bounds__(128) potrf_exact_update(const T *W, T *S, int6
         const int64_t j = j0 + r16, k2 = k0 + c0 + 2 * i;
         acc[i] = (j < n && k2 < j && p > 0) ? cm(S, ld, j, k2) : T(0);
     }
+#pragma unroll
     for (int e = tid; e < kExTile * kNbExact; e += 128) {
         const int r = e % kExTile, k = e / kExTile;
         lj[k][r] = (j0 + r < n) ? cm(W, ld, j0 + r, p + k) : T(0);
