@@ -196,12 +196,14 @@ int atb_launch(const T *A, int64_t lda, const T *B, int64_t ldb, int64_t n, int6
 }
 
 // X (n x k, k <= KM) <- X L^-T for the lower k x k L: every row of X is a
-// right-hand side of L z = x, solved by one thread in registers with the
+// right-hand side of L z = x, solved by one thread in shared memory with the
 // reference's sequence (src/triangular.rs:113-125: divide, subtract from all later
 // entries; multiply and subtract rounded separately when EXACT).  The substitution
 // kernel's one warp per right-hand side spends a warp instruction on a term of one
 // of them; a lane each serves 32 (40000 x 20: 200 us and two transpositions ->
-// 110 us).
+// 110 us).  A row in registers needs every loop unrolled, some 60 KB of code that
+// each SM runs through a few times: it waited for instructions; a few rolled loops
+// over shared memory take 46 us (the FP64 pipe's share is 38).
 __device__ __noinline__ double rows_div_library(double a, double b) { return __ddiv_rn(a, b); }
 
 template <typename T, bool kExact, int KM>
@@ -219,35 +221,44 @@ __global__ void __launch_bounds__(64) solve_rows_kernel(const T *__restrict__ L,
     __syncthreads();
     const int64_t row = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (row >= n) return;
-    T v[KM];
+    __shared__ T vs[KM][64];  // this thread's row: vs[.][threadIdx.x]
+    T(*v)[64] = reinterpret_cast<T(*)[64]>(&vs[0][threadIdx.x]);
     bool ok = true;
     auto solve = [&](bool lib) {
-#pragma unroll
-        for (int c = 0; c < KM; ++c) v[c] = c < k ? X[row + c * ldx] : T(0);
-#pragma unroll
-        for (int c = 0; c < KM; ++c) {
-            if (c >= k) break;
+#pragma unroll 4
+        for (int c = 0; c < k; ++c) v[c][0] = X[row + c * ldx];
+#pragma unroll 1
+        for (int c = 0; c < k; ++c) {
+            const T b = v[c][0];
             T x;
             if (kInt && !lib) {
                 bool good;
-                x = (T)im_div((double)v[c], dq[c], good);
+                x = (T)im_div((double)b, dq[c], good);
                 ok = ok && good;
             } else if (kInt) {
-                x = (T)rows_div_library((double)v[c], (double)l[c][c]);
+                x = (T)rows_div_library((double)b, (double)l[c][c]);
             } else {
-                x = Ar::div(v[c], l[c][c]);
+                x = Ar::div(b, l[c][c]);
             }
-            v[c] = x;
+            v[c][0] = x;
+#pragma unroll 1
+            for (int r = c + 1; r < k; r += 4) {
+                T t[4];
 #pragma unroll
-            for (int r = c + 1; r < KM; ++r)
-                if (r < k) v[r] = kExact ? Ar::sub(v[r], Ar::mul(x, l[c][r])) : Ar::fma_(-x, l[c][r], v[r]);
+                for (int u = 0; u < 4; ++u) t[u] = r + u < k ? v[r + u][0] : T(0);
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                    if (r + u < k) t[u] = kExact ? Ar::sub(t[u], Ar::mul(x, l[c][r + u])) : Ar::fma_(-x, l[c][r + u], t[u]);
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                    if (r + u < k) v[r + u][0] = t[u];
+            }
         }
     };
     solve(false);
     if (!ok) solve(true);  // a quotient that the integer form does not take
-#pragma unroll
-    for (int c = 0; c < KM; ++c)
-        if (c < k) X[row + c * ldx] = v[c];
+#pragma unroll 4
+    for (int c = 0; c < k; ++c) X[row + c * ldx] = v[c][0];
 }
 
 template <typename T>
