@@ -723,7 +723,10 @@ def measure_batch(torch, lla, dev, count, dtname, steps, warmup, cpu_sample=0, r
         "roofline": {"kernel": "batch", "bound": "fp64-tensor" if dt == torch.float64 else "fp32-fma",
                      "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
                      "frac": achieved / peak if peak > 0 else None,
-                     "peak_source": "measured live (FP64 tensor pipe / FFMA loop on all SMs)"},
+                     "peak_source": "measured live (FP64 tensor pipe / FFMA loop on all SMs)",
+                     # above 1 is possible: the pipe bounds only the part that is left on it
+                     "note": "algorithmic flops; the plain f64 trailing updates run as exact digit products on the "
+                             "FP16 tensor cores, not on the FP64 pipe" if dt == torch.float64 and not refined else None},
         "cpu_baseline": cpu, "clocks": clk.summary(),
         "gpu_launches": launches * steps // (warmup + steps),
         "kernels": {k: {"ms": v[0], "launches": v[1]} for k, v in prof.items()},
