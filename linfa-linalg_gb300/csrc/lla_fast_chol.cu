@@ -27,8 +27,8 @@
 // the rest, so the trailing matrix is read and written once per 128 columns.
 //
 // Measured, FMA updates before -> now (error against 64 bits the same or lower):
-// f64 n = 8192 220 -> 12.4 ms, n = 2048 14.4 -> 2.0 ms; f32 n = 6001 14.6 ->
-// 3.1 ms.  There is no size at which the FMA form is faster: one 64 x 64 tile of
+// f64 n = 8192 220 -> 12.3 ms, n = 2048 14.4 -> 2.0 ms; f32 n = 6001 14.6 ->
+// 2.8 ms.  There is no size at which the FMA form is faster: one 64 x 64 tile of
 // the FP64 one took 70 us on its SM.
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -112,7 +112,7 @@ __device__ __forceinline__ void atomic_min_pos_f64(double *addr, double v) {
 // the other three sub-partitions keep the rest in registers, in patches of 16
 // rows x 2 columns (one FP64 instruction per column applied), and hand pair
 // k + 2 to warp 0 through shared memory once pair k is in it.  One barrier per
-// pair.  160 -> 31 us a block (FP32 67 -> 13 us).
+// pair.  160 -> 31 us a block (FP32, where fc_diag_quick cannot take it, 67 -> 13 us).
 constexpr int kFcDiagThreads = 512;
 constexpr int kFcPatches = 80, kFcPatchWarps = 12, kFcSlots = 7;
 
@@ -215,11 +215,100 @@ template <typename T>
 struct FcDiagSmem {
     T a[kFcNb][kFcNb];  // [column][row]
     T piv[kFcNb], rv[kFcNb];
+    float pair[3][2][kFcNb];  // FP32: column pairs in turn
     int fail;
 };
 
 __device__ __forceinline__ void fc_diag_sync() {
     asm volatile("bar.sync 1, %0;" ::"n"(kFcDiagThreads) : "memory");
+}
+
+// FP32 block with all pivots positive and normal: sm.a, sm.piv and sm.rv finished.
+// Otherwise sm.fail is set and the block spoilt.  FP32 instructions are short, so
+// the chain is exchanges: eight warps hold the block (two rows a lane, eight columns
+// a warp), a pair of columns a step goes through shared memory, every thread forms
+// the inverse of its 2 x 2 pivot block itself, and the next pair is brought up to
+// date and stored before the columns right of it.  No shuffle, one barrier a pair
+// (of warps 0 .. 7).  The factor of n = 6001: 3.12 -> 2.80 ms, of n = 1100 0.49 -> 0.40.
+__device__ __forceinline__ void fc_diag_quick(FcDiagSmem<float> &sm) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, lr = 2 * lane, lc = 8 * warp;
+    if (warp >= 8) return;
+    float v[8][2];  // column lc + j, row lr + i (above the diagonal: anything)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        const float2 t = *reinterpret_cast<const float2 *>(&sm.a[lc + j][lr]);
+        v[j][0] = t.x, v[j][1] = t.y;
+    }
+    const auto put = [&](float (*to)[kFcNb], int c, const float (&x)[2], const float (&y)[2]) {
+        if (lc == (c & ~7)) {
+            *reinterpret_cast<float2 *>(&to[0][lr]) = make_float2(x[0], x[1]);
+            *reinterpret_cast<float2 *>(&to[1][lr]) = make_float2(y[0], y[1]);
+        }
+        asm volatile("bar.sync 2, 256;" ::: "memory");
+    };
+    const auto reciprocal = [](float d) {  // FP32 approximation and one Newton step
+        float r;
+        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
+        return fmaf(r, fmaf(-d, r, 1.f), r);
+    };
+    int b = 0;
+    put(sm.pair[0], 0, v[0], v[1]);
+#pragma unroll 1
+    for (int c8 = 0; c8 < kFcNb; c8 += 8)
+#pragma unroll
+        for (int j0 = 0; j0 < 8; j0 += 2) {
+            const int c = c8 + j0, jn = (j0 + 2) & 7, nb = b == 2 ? 0 : b + 1;
+            // (three buffers: a pair's last readers are two barriers before its buffer's reuse)
+            const float(*cb)[kFcNb] = sm.pair[b];
+            const float2 a0 = *reinterpret_cast<const float2 *>(&cb[0][c]);  // a_cc, a_{c+1,c}
+            const float a11 = cb[1][c + 1];
+            const float2 x2 = *reinterpret_cast<const float2 *>(&cb[0][lr]);
+            const float2 y2 = *reinterpret_cast<const float2 *>(&cb[1][lr]);
+            const float d0 = a0.x, r0 = reciprocal(d0), g = a0.y * r0;
+            const float d1 = fmaf(-g, a0.y, a11), r1 = reciprocal(d1);
+            const float x0[2] = {x2.x, x2.y};  // columns c and c + 1, unscaled
+            const float x1[2] = {fmaf(-g, x2.x, y2.x), fmaf(-g, x2.y, y2.y)};
+            if (lc >= c8) {
+                float t[8], u[8], s0[2], s1[2];
+#pragma unroll
+                for (int h = 0; h < 8; h += 4) {
+                    const float4 t4 = *reinterpret_cast<const float4 *>(&cb[0][lc + h]);
+                    const float4 u4 = *reinterpret_cast<const float4 *>(&cb[1][lc + h]);
+                    t[h] = t4.x, t[h + 1] = t4.y, t[h + 2] = t4.z, t[h + 3] = t4.w;
+                    u[h] = u4.x, u[h + 1] = u4.y, u[h + 2] = u4.z, u[h + 3] = u4.w;
+                }
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    s1[i] = x1[i] * r1;
+                    s0[i] = fmaf(-s1[i], g, x0[i] * r0);
+                }
+                const auto apply = [&](int j) {
+#pragma unroll
+                    for (int i = 0; i < 2; ++i) v[j][i] = fmaf(-s1[i], u[j], fmaf(-s0[i], t[j], v[j][i]));
+                };
+                apply(jn);
+                apply(jn + 1);
+                put(sm.pair[nb], c + 2, v[jn], v[jn + 1]);  // (c + 2 = 64: nobody's)
+#pragma unroll
+                for (int j = 0; j < 8; ++j)
+                    if (j != jn && j != jn + 1) apply(j);
+            } else {
+                asm volatile("bar.sync 2, 256;" ::: "memory");
+            }
+            if (warp == 0) {  // the finished pair
+                const float q0 = Fc<float>::rsqrt_(d0), q1 = Fc<float>::rsqrt_(d1);
+                *reinterpret_cast<float2 *>(&sm.a[c][lr]) = make_float2(x0[0] * q0, x0[1] * q0);
+                *reinterpret_cast<float2 *>(&sm.a[c + 1][lr]) = make_float2(x1[0] * q1, x1[1] * q1);
+                if (lane == 0) {
+                    sm.piv[c] = d0;
+                    sm.piv[c + 1] = d1;
+                    sm.rv[c] = q0;
+                    sm.rv[c + 1] = q1;
+                    if (!Fc<float>::normal(d0) || !Fc<float>::normal(d1)) sm.fail = kFcNb;
+                }
+            }
+            b = nb;
+        }
 }
 
 // By threads 0 .. 511 of a CTA.
@@ -229,18 +318,31 @@ __device__ __forceinline__ void fc_diag_block(FcDiagSmem<T> &sm, T *W, int64_t l
     T(*a)[kFcNb] = sm.a;
     T *piv = sm.piv, *rv = sm.rv;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const auto load = [&]() {
 #pragma unroll
-    for (int e = tid; e < kFcNb * kFcNb; e += kFcDiagThreads) {
-        const int r = e % kFcNb, c = e / kFcNb;
-        // a short block is padded with the identity
-        if (r < b && c <= r)
-            fc_copy(&a[c][r], &cm(W, ld, p + r, p + c));
-        else
-            a[c][r] = T(r == c ? 1 : 0);
+        for (int e = tid; e < kFcNb * kFcNb; e += kFcDiagThreads) {
+            const int r = e % kFcNb, c = e / kFcNb;
+            // a short block is padded with the identity
+            if (r < b && c <= r)
+                fc_copy(&a[c][r], &cm(W, ld, p + r, p + c));
+            else
+                a[c][r] = T(r == c ? 1 : 0);
+        }
+        if (tid == 0) sm.fail = -1;
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        fc_diag_sync();
+    };
+    load();
+    bool done_quick = false;
+    if constexpr (sizeof(T) == 4) {
+        fc_diag_quick(sm);
+        fc_diag_sync();
+        done_quick = *(volatile int *)&sm.fail < 0;
+        if (!done_quick) {  // (the same for all threads)
+            fc_diag_sync();  // every thread has read the verdict
+            load();
+        }
     }
-    if (tid == 0) sm.fail = -1;
-    asm volatile("cp.async.wait_all;" ::: "memory");
-    fc_diag_sync();
     const bool upd = (warp & 3) != 0;  // a patch warp (warps 4, 8 and 12 only load and store)
     T acc[kFcSlots];
     int row[kFcSlots], col[kFcSlots];  // col < 0: no patch
@@ -256,8 +358,8 @@ __device__ __forceinline__ void fc_diag_block(FcDiagSmem<T> &sm, T *W, int64_t l
         }
     }
     bool bad = false;
-    if (warp == 0) bad = fc_pivot_pair<T, true>(a, piv, rv, &sm.fail, 0, lane);
-    for (int k = 0;; ++k) {
+    if (warp == 0 && !done_quick) bad = fc_pivot_pair<T, true>(a, piv, rv, &sm.fail, 0, lane);
+    for (int k = 0; !done_quick; ++k) {
         fc_diag_sync();  // pair k is final
         // A pivot failure of pair k ends the loop for everyone here.  Warp 0 may already have
         // recorded one of pair k + 1 by the time another warp reads the word: that one ends the
@@ -286,29 +388,28 @@ __device__ __forceinline__ void fc_diag_block(FcDiagSmem<T> &sm, T *W, int64_t l
                 a[col[s]][row[s]] =
                     (fail & 1) ? fma(-a[fail - 1][row[s]], a[fail - 1][col[s]], acc[s]) : acc[s];
     }
-    if (tid < done) rinv[tid] = rv[tid];
-    if (tid < kFcNb) {  // exact roots of the pivots, and the smallest relative pivot
-        double ratio = 1.0e300;
-        if (tid < done && tid < b) {
-            const T d = piv[tid];
-            a[tid][tid] = sqrt(d);
-            const double r0 = (double)d / (double)diag0[p + tid];
-            if (r0 < ratio) ratio = r0;
-        }
-        if (min_ratio) {
-#pragma unroll
-            for (int o = 16; o; o >>= 1) {
-                const double v = __shfl_xor_sync(0xffffffffu, ratio, o);
-                if (v < ratio) ratio = v;
-            }
-            if (lane == 0) atomic_min_pos_f64(min_ratio, ratio);
-        }
+    if (tid < done) {
+        rinv[tid] = rv[tid];
+        a[tid][tid] = sqrt(piv[tid]);  // exact roots
     }
     if (tid == 0 && fail >= 0) *info = p + fail;
     fc_diag_sync();
     for (int e = tid; e < kFcNb * kFcNb; e += kFcDiagThreads) {
         const int r = e % kFcNb, c = e / kFcNb;
         if (r < b && c <= r) cm(W, ld, p + r, p + c) = a[c][r];
+    }
+    if (tid < kFcNb && min_ratio) {  // the smallest relative pivot
+        double ratio = 1.0e300;
+        if (tid < done && tid < b) {
+            const double r0 = (double)piv[tid] / (double)diag0[p + tid];
+            if (r0 < ratio) ratio = r0;
+        }
+#pragma unroll
+        for (int o = 16; o; o >>= 1) {
+            const double v = __shfl_xor_sync(0xffffffffu, ratio, o);
+            if (v < ratio) ratio = v;
+        }
+        if (lane == 0) atomic_min_pos_f64(min_ratio, ratio);
     }
 }
 
