@@ -372,21 +372,21 @@ __device__ __forceinline__ float from_half(__half h) { return __half2float(h); }
 //     Y_J = A_J - sum_{I<J} X_I L_JI^T,   X_J = Y_J W_JJ^T,
 // W_JJ = L_JJ^-1 from the diagonal kernel (Wd[J][k][c] = W_JJ[c][k]); only the
 // blocks of L11 below its diagonal blocks are read.  Then the operand planes of L21
-// for the tensor cores (zero for k >= b).  One CTA of 256 threads per 64 rows;
-// for products, thread (rt = tid % 32, ct = tid / 32) owns rows rt, rt + 32 and
-// columns 4 ct .. 4 ct + 3 of the current block.
-constexpr int kPnRows = 64;
-constexpr int kPnXd = kPnRows + 4;  // row stride of sXT (k-major copy of the row tile)
+// for the tensor cores (zero for k >= b).  One CTA of 256 threads per 64
+// rows (32 where that leaves SMs idle); for products, thread (rt = tid % 32, ct =
+// tid / 32) owns rows rt, rt + 32 and columns 4 ct .. 4 ct + 3 of the current block.
 constexpr int kPnLd = kLpNb + 4;    // row stride of sLT (k-major copy of L11, columns k < 96)
 constexpr int kPnWd = 32 + 4;       // row stride of sWT (k-major W_JJ)
-// 103,936 bytes: two CTAs per SM
-constexpr size_t kPnSmem = sizeof(float) * (kLpNb * kPnXd + (kLpNb - 32) * kPnLd + 4 * 32 * kPnWd);
+// 103,936 bytes with 64 rows: two CTAs per SM
+template <int ROWS>
+constexpr size_t kPnSmem = sizeof(float) * (kLpNb * (ROWS + 4) + (kLpNb - 32) * kPnLd + 4 * 32 * kPnWd);
 
-template <typename H>
+template <typename H, int ROWS>
 __global__ void __launch_bounds__(256, 2) lowp_panel_kernel(float *L, int64_t ld, int64_t n, int64_t p,
                                                          const float *__restrict__ Wd, H *planes,
                                                          int64_t plane_stride, int64_t ldp, int koff, int terms,
                                                          const int64_t *info) {
+    constexpr int kPnRows = ROWS, kPnXd = ROWS + 4, U = ROWS / 32;  // kPnXd: row stride of sXT
     extern __shared__ __align__(16) float sm[];
     float *sXT = sm;                         // sXT[k * kPnXd + r] = row r, column k of the tile
     float *sLT = sXT + kLpNb * kPnXd;        // sLT[k * kPnLd + c] = L11[c][k]
@@ -452,69 +452,64 @@ __global__ void __launch_bounds__(256, 2) lowp_panel_kernel(float *L, int64_t ld
 #pragma unroll 1
     for (int J = 0; J < 4; ++J) {
         const int cj = J * 32 + 4 * ct;  // this thread's first column
-        float acc[2][4];
+        float acc[U][4];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            acc[0][u] = sXT[(cj + u) * kPnXd + rt];
-            acc[1][u] = sXT[(cj + u) * kPnXd + rt + 32];
-        }
+        for (int h = 0; h < U; ++h)
+#pragma unroll
+            for (int u = 0; u < 4; ++u) acc[h][u] = sXT[(cj + u) * kPnXd + rt + 32 * h];
         // Y_J = A_J - X_{<J} L_J,<J^T, eight k at a time: all their shared loads
         // issue before the products, so the loop is not a chain of load latencies
         for (int k0 = 0; k0 < J * 32; k0 += 8) {
-            float x0[8], x1[8];
+            float x[U][8];
             float4 l4[8];
 #pragma unroll
             for (int kk = 0; kk < 8; ++kk) {
-                x0[kk] = sXT[(k0 + kk) * kPnXd + rt];
-                x1[kk] = sXT[(k0 + kk) * kPnXd + rt + 32];
+#pragma unroll
+                for (int h = 0; h < U; ++h) x[h][kk] = sXT[(k0 + kk) * kPnXd + rt + 32 * h];
                 l4[kk] = *reinterpret_cast<const float4 *>(&sLT[(k0 + kk) * kPnLd + cj]);
             }
 #pragma unroll
             for (int kk = 0; kk < 8; ++kk) {
                 const float lv[4] = {l4[kk].x, l4[kk].y, l4[kk].z, l4[kk].w};
 #pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    acc[0][u] = fmaf(-x0[kk], lv[u], acc[0][u]);
-                    acc[1][u] = fmaf(-x1[kk], lv[u], acc[1][u]);
-                }
+                for (int u = 0; u < 4; ++u)
+#pragma unroll
+                    for (int h = 0; h < U; ++h) acc[h][u] = fmaf(-x[h][kk], lv[u], acc[h][u]);
             }
         }
         __syncthreads();  // every thread has read A_J
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            sXT[(cj + u) * kPnXd + rt] = acc[0][u];
-            sXT[(cj + u) * kPnXd + rt + 32] = acc[1][u];
-        }
+        for (int u = 0; u < 4; ++u)
+#pragma unroll
+            for (int h = 0; h < U; ++h) sXT[(cj + u) * kPnXd + rt + 32 * h] = acc[h][u];
         __syncthreads();
         // X_J = Y_J W_JJ^T
-        float x[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+        float x[U][4] = {};
 #pragma unroll
         for (int k0 = 0; k0 < 32; k0 += 8) {
-            float y0[8], y1[8];
+            float y[U][8];
             float4 w4[8];
 #pragma unroll
             for (int kk = 0; kk < 8; ++kk) {
                 const int k = J * 32 + k0 + kk;
-                y0[kk] = sXT[k * kPnXd + rt];
-                y1[kk] = sXT[k * kPnXd + rt + 32];
+#pragma unroll
+                for (int h = 0; h < U; ++h) y[h][kk] = sXT[k * kPnXd + rt + 32 * h];
                 w4[kk] = *reinterpret_cast<const float4 *>(&sWT[k * kPnWd + 4 * ct]);
             }
 #pragma unroll
             for (int kk = 0; kk < 8; ++kk) {
                 const float wv[4] = {w4[kk].x, w4[kk].y, w4[kk].z, w4[kk].w};
 #pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    x[0][u] = fmaf(y0[kk], wv[u], x[0][u]);
-                    x[1][u] = fmaf(y1[kk], wv[u], x[1][u]);
-                }
+                for (int u = 0; u < 4; ++u)
+#pragma unroll
+                    for (int h = 0; h < U; ++h) x[h][u] = fmaf(y[h][kk], wv[u], x[h][u]);
             }
         }
         __syncthreads();  // every thread has read Y_J
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            sXT[(cj + u) * kPnXd + rt] = x[0][u];
-            sXT[(cj + u) * kPnXd + rt + 32] = x[1][u];
-        }
+        for (int u = 0; u < 4; ++u)
+#pragma unroll
+            for (int h = 0; h < U; ++h) sXT[(cj + u) * kPnXd + rt + 32 * h] = x[h][u];
         __syncthreads();
     }
     // L21 back to the factor (columns contiguous)
@@ -549,6 +544,12 @@ __global__ void __launch_bounds__(256, 2) lowp_panel_kernel(float *L, int64_t ld
 
 // ---------------------------------------------------------------------------
 // host loop
+
+template <typename H, int ROWS>
+static bool panel_attrs() {  // true on failure
+    return cudaFuncSetAttribute(lowp_panel_kernel<H, ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)kPnSmem<ROWS>) != cudaSuccess;
+}
 
 int lowp_factor_launch(float *L, int64_t n, int64_t ld, const lla_refine_opts &opts, int64_t *info,
                        float *diag0, double *min_ratio, Ctx *c, cudaStream_t st) {
@@ -590,16 +591,17 @@ int lowp_factor_launch(float *L, int64_t n, int64_t ld, const lla_refine_opts &o
     unsigned sched_base = 0;
     if (cudaMemsetAsync(err_word, 0, 4 * sizeof(int), st) != cudaSuccess) return -1;
     const size_t smem_l11 = kDgSmem;
-    const size_t smem_panel = kPnSmem;
+    int sms = 1, dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        return -1;
     if (c->mixed.pinv.ensure(sizeof(float) * 4 * 32 * 32) != cudaSuccess) return -1;
     float *Wd = (float *)c->mixed.pinv.p;
     // kernel attributes are per device: set them on every call (cheap)
     if (cudaFuncSetAttribute(lowp_diag_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_l11) !=
             cudaSuccess ||
-        cudaFuncSetAttribute(lowp_panel_kernel<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)smem_panel) != cudaSuccess ||
-        cudaFuncSetAttribute(lowp_panel_kernel<__half>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)smem_panel) != cudaSuccess ||
+        panel_attrs<__nv_bfloat16, 64>() || panel_attrs<__nv_bfloat16, 32>() || panel_attrs<__half, 64>() ||
+        panel_attrs<__half, 32>() ||
         tc_update_prepare() != 0)
         return -1;
     const size_t esz = sizeof(uint16_t);
@@ -615,15 +617,20 @@ int lowp_factor_launch(float *L, int64_t n, int64_t ld, const lla_refine_opts &o
     auto panel = [&](int64_t p, int half) {
         const int64_t rest = n - p - kLpNb;
         LaunchScope ls(K_MIXED_PANEL, st, (double)rest * kLpNb * kLpNb);
-        const dim3 grid((unsigned)ceil_div(rest, kPnRows));
+        // 32 rows a CTA where each still has an SM to itself (n = 3001, 64 -> 32 rows: 11.7 -> 8.5 us
+        // a panel); with more the two are even, and 64 rows copy L11 half as often.
+        const bool half_rows = ceil_div(rest, 32) <= sms;
+        const dim3 grid((unsigned)ceil_div(rest, half_rows ? 32 : 64));
+        const size_t smem = half_rows ? kPnSmem<32> : kPnSmem<64>;
+        const auto go = [&](auto kern, auto *pl) {
+            launch_maybe_pdl(true, kern, grid, dim3(256), smem, st, L, ld, n, p, (const float *)Wd, pl, plane_stride,
+                             ldp, half * kLpNb, terms, (const int64_t *)info);
+        };
         if (fp16)
-            launch_maybe_pdl(true, lowp_panel_kernel<__half>, grid, dim3(256), smem_panel, st, L, ld, n, p,
-                             (const float *)Wd, (__half *)planes, plane_stride, ldp, half * kLpNb, terms,
-                             (const int64_t *)info);
+            go(half_rows ? lowp_panel_kernel<__half, 32> : lowp_panel_kernel<__half, 64>, (__half *)planes);
         else
-            launch_maybe_pdl(true, lowp_panel_kernel<__nv_bfloat16>, grid, dim3(256), smem_panel, st, L, ld, n,
-                             p, (const float *)Wd, (__nv_bfloat16 *)planes, plane_stride, ldp, half * kLpNb,
-                             terms, (const int64_t *)info);
+            go(half_rows ? lowp_panel_kernel<__nv_bfloat16, 32> : lowp_panel_kernel<__nv_bfloat16, 64>,
+               (__nv_bfloat16 *)planes);
     };
     // A22 -= sum of the products of K columns of the planes, rows [q, n)
     auto update = [&](int64_t q, int kext, bool narrow) -> int {
