@@ -491,7 +491,13 @@ __device__ int batch_factor(T *A, int n, int m, BatchSmem<T> &sm) {
         const int bs = min(NB, n - kb), q = kb + bs, rows = n - q;
         for (int e = tid; e < NB * NB; e += nthr) {
             const int r = e % NB, c = e / NB;
-            sm.dg[c * DS + r] = (r < bs && c <= r) ? A[(kb + r) + (int64_t)(kb + c) * n] : T(r == c ? 1 : 0);
+            if (r < bs && c <= r)
+                asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(
+                                 (uint32_t)__cvta_generic_to_shared(&sm.dg[c * DS + r])),
+                             "l"(&A[(kb + r) + (int64_t)(kb + c) * n]), "n"(sizeof(T))
+                             : "memory");
+            else
+                sm.dg[c * DS + r] = T(r == c ? 1 : 0);
         }
         // the rows below the block, one a thread, fetched while the block is factored
         const int total = rows + m;
@@ -504,6 +510,7 @@ __device__ int batch_factor(T *A, int n, int m, BatchSmem<T> &sm) {
         };
         const bool split = sizeof(T) == 8 && 4 * total <= nthr;
         if (tid < total && !split) fetch(tid);
+        asm volatile("cp.async.wait_all;" ::: "memory");
         __syncthreads();
         if constexpr (sizeof(T) == 4) {
             if (!batch_diag_quick(sm, kb)) {
