@@ -19,7 +19,7 @@
 // by default; a large FP64 one is bound by the FP64 pipe and the digits' integer
 // work.  10,000 systems of n 16-256 (before: one-warp diagonal blocks with library
 // divisions, FP64 updates on the FP64 pipe, two substitution passes): f64 20.1 ->
-// 5.9 ms, f32 5.4 -> 1.3 ms; 3,000 of n 16-64 1.60 -> 0.33 and 0.46 -> 0.13 ms.
+// 5.8 ms, f32 5.4 -> 1.2 ms; 3,000 of n 16-64 1.60 -> 0.33 and 0.46 -> 0.13 ms.
 // A non-positive pivot stops that system only: info[i] = first failing row
 // (-1 when the system solved).  The (CTAs per SM, threads) shape is chosen per
 // batch by lla_batch_autotune and cached on disk.
