@@ -194,7 +194,14 @@ __global__ void __launch_bounds__(kTrsmNb *kTrsmMaxMc) trsm_lookback(const T *__
                     abort = true;
                     break;
                 }
-                if (spins > 64) __nanosleep(64);
+                // only the block right before this one is worth polling without a pause: thousands of
+                // warps wait further back, on the same few lines (n = 8192, 16 right-hand sides:
+                // 1.98 -> 1.86 ms a solve)
+                if (q + 1 < rb) {
+                    if (spins > 2) __nanosleep(256);
+                } else if (spins > 64) {
+                    __nanosleep(64);
+                }
             }
             abort = __any_sync(0xffffffffu, abort);
             // solved block q (always a full block: q < rb), one row a lane
