@@ -41,6 +41,7 @@
 #include "lla_int_math.h"
 #include "lla_kernels.h"
 #include "lla_oz_mma.cuh"
+#include "lla_pivot_pair.cuh"
 #include "lla_prof.h"
 
 namespace lla {
@@ -181,8 +182,8 @@ __device__ void batch_diag(BatchSmem<T> &sm, int kb) {
 
 // FP32, all pivots positive and normal (false otherwise, the block spoilt): four
 // warps hold the block, 2 rows x 4 columns a thread.  Two columns a round go through
-// shared memory (the panel's space), every thread forms the inverse of their 2 x 2
-// pivot block itself, and the next pair is brought up to date and stored before the
+// shared memory (the panel's space), every thread forms their pivots itself
+// (lla_pivot_pair.cuh), and the next pair is brought up to date and stored before the
 // columns right of it: one exchange and no shuffle on a pair's chain (10,000 systems
 // of n 16-256: 1.23 -> 1.12 ms against batch_diag).
 __device__ bool batch_diag_quick(BatchSmem<float> &sm, int kb) {
@@ -226,19 +227,15 @@ __device__ bool batch_diag_quick(BatchSmem<float> &sm, int kb) {
                 const float4 t4 = *reinterpret_cast<const float4 *>(cb + lc);
                 const float4 u4 = *reinterpret_cast<const float4 *>(cb + 32 + lc);
                 const float t[4] = {t4.x, t4.y, t4.z, t4.w}, u[4] = {u4.x, u4.y, u4.z, u4.w};
-                const float d0 = a0.x, r0 = reciprocal(d0), g = a0.y * r0;
-                const float d1 = fmaf(-g, a0.y, a11), r1 = reciprocal(d1);
+                const PivotPair pp(a0.x, a0.y, a11, reciprocal);
+                const float d0 = pp.d0, d1 = pp.d1;
                 const float x0[2] = {x2.x, x2.y};  // columns c and c + 1, unscaled
-                float x1[2] = {y2.x, y2.y}, s0[2], s1[2];
-#pragma unroll
-                for (int i = 0; i < 2; ++i) {
-                    x1[i] = fmaf(-g, x0[i], x1[i]);
-                    s1[i] = x1[i] * r1;
-                    s0[i] = fmaf(-s1[i], g, x0[i] * r0);
-                }
+                const float x1[2] = {pp.second(x2.x, y2.x), pp.second(x2.y, y2.y)};
+                const float s0[2] = {x0[0] * pp.r0, x0[1] * pp.r0}, s1[2] = {x1[0] * pp.r1, x1[1] * pp.r1};
                 const auto apply = [&](int j) {
+                    const float w = pp.second(t[j], u[j]);
 #pragma unroll
-                    for (int i = 0; i < 2; ++i) v[j][i] = fmaf(-s1[i], u[j], fmaf(-s0[i], t[j], v[j][i]));
+                    for (int i = 0; i < 2; ++i) v[j][i] = pivot_pair_apply(v[j][i], s0[i], t[j], s1[i], w);
                 };
                 apply(jn);
                 apply(jn + 1);

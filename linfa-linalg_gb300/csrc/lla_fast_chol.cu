@@ -41,6 +41,7 @@
 #include "lla_int_math.h"
 #include "lla_kernels.h"
 #include "lla_oz_mma.cuh"
+#include "lla_pivot_pair.cuh"
 #include "lla_prof.h"
 #include "lla_scratch.h"
 #include "lla_tcgen05.cuh"
@@ -227,9 +228,9 @@ __device__ __forceinline__ void fc_diag_sync() {
 // Otherwise sm.fail is set and the block spoilt.  FP32 instructions are short, so
 // the chain is exchanges: eight warps hold the block (two rows a lane, eight columns
 // a warp), a pair of columns a step goes through shared memory, every thread forms
-// the inverse of its 2 x 2 pivot block itself, and the next pair is brought up to
-// date and stored before the columns right of it.  No shuffle, one barrier a pair
-// (of warps 0 .. 7).  The factor of n = 6001: 3.12 -> 2.80 ms, of n = 1100 0.49 -> 0.40.
+// its pivots itself (lla_pivot_pair.cuh), and the next pair is brought up to date and
+// stored before the columns right of it.  No shuffle, one barrier a pair (of warps
+// 0 .. 7).  The factor of n = 6001: 3.12 -> 2.80 ms, of n = 1100 0.49 -> 0.40.
 __device__ __forceinline__ void fc_diag_quick(FcDiagSmem<float> &sm) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, lr = 2 * lane, lc = 8 * warp;
     if (warp >= 8) return;
@@ -264,10 +265,10 @@ __device__ __forceinline__ void fc_diag_quick(FcDiagSmem<float> &sm) {
             const float a11 = cb[1][c + 1];
             const float2 x2 = *reinterpret_cast<const float2 *>(&cb[0][lr]);
             const float2 y2 = *reinterpret_cast<const float2 *>(&cb[1][lr]);
-            const float d0 = a0.x, r0 = reciprocal(d0), g = a0.y * r0;
-            const float d1 = fmaf(-g, a0.y, a11), r1 = reciprocal(d1);
+            const PivotPair pp(a0.x, a0.y, a11, reciprocal);
+            const float d0 = pp.d0, d1 = pp.d1;
             const float x0[2] = {x2.x, x2.y};  // columns c and c + 1, unscaled
-            const float x1[2] = {fmaf(-g, x2.x, y2.x), fmaf(-g, x2.y, y2.y)};
+            const float x1[2] = {pp.second(x2.x, y2.x), pp.second(x2.y, y2.y)};
             if (lc >= c8) {
                 float t[8], u[8], s0[2], s1[2];
 #pragma unroll
@@ -279,12 +280,13 @@ __device__ __forceinline__ void fc_diag_quick(FcDiagSmem<float> &sm) {
                 }
 #pragma unroll
                 for (int i = 0; i < 2; ++i) {
-                    s1[i] = x1[i] * r1;
-                    s0[i] = fmaf(-s1[i], g, x0[i] * r0);
+                    s0[i] = x0[i] * pp.r0;
+                    s1[i] = x1[i] * pp.r1;
                 }
                 const auto apply = [&](int j) {
+                    const float w = pp.second(t[j], u[j]);
 #pragma unroll
-                    for (int i = 0; i < 2; ++i) v[j][i] = fmaf(-s1[i], u[j], fmaf(-s0[i], t[j], v[j][i]));
+                    for (int i = 0; i < 2; ++i) v[j][i] = pivot_pair_apply(v[j][i], s0[i], t[j], s1[i], w);
                 };
                 apply(jn);
                 apply(jn + 1);

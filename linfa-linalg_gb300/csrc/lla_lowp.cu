@@ -30,6 +30,7 @@
 #include "lla_common.cuh"
 #include "lla_kernels.h"
 #include "lla_mixed.h"
+#include "lla_pivot_pair.cuh"
 #include "lla_prof.h"
 #include "lla_tc.h"
 
@@ -141,8 +142,8 @@ __device__ __forceinline__ void dg_store(const float *sa, float *L, int64_t ld, 
 //   (1) warps 0-3 factor the 32 x 32 diagonal block (2 rows x 4 columns a
 //       thread) without square roots on the pivot chain: with d_c the pivot,
 //       a_ij -= (a_ic / d_c) a_jc.  Columns go through shared memory two at a
-//       time and every thread forms the inverse of the pair's 2 x 2 pivot block
-//       itself, so one store, barrier and load serve two pivots (256 cycles);
+//       time and every thread forms the pair's pivots itself
+//       (lla_pivot_pair.cuh), so one store, barrier and load serve two pivots;
 //       the next pair is brought up to date and stored before the columns right
 //       of it.  Meanwhile warps 4-15 subtract the previous block's panel from
 //       everything below and right of this block and store that panel;
@@ -252,20 +253,15 @@ __global__ void __launch_bounds__(kDgThreads) lowp_diag_kernel(float *L, int64_t
                     const float4 t4 = *reinterpret_cast<const float4 *>(cb + lc);
                     const float4 u4 = *reinterpret_cast<const float4 *>(cb + 32 + lc);
                     const float t[4] = {t4.x, t4.y, t4.z, t4.w}, u[4] = {u4.x, u4.y, u4.z, u4.w};
-                    const float r0 = dg_rcp(a0.x), g = a0.y * r0;
-                    const float d0 = a0.x, d1 = fmaf(-g, a0.y, a11);  // pivot c + 1 after column c's update
-                    const float r1 = dg_rcp(d1);
+                    const PivotPair pp(a0.x, a0.y, a11, dg_rcp);
+                    const float d0 = pp.d0, d1 = pp.d1;
                     const float x0[2] = {x2.x, x2.y};  // columns c and c + 1, unscaled
-                    float x1[2] = {y2.x, y2.y}, s0[2], s1[2];
-#pragma unroll
-                    for (int i = 0; i < 2; ++i) {
-                        x1[i] = fmaf(-g, x0[i], x1[i]);
-                        s1[i] = x1[i] * r1;
-                        s0[i] = fmaf(-s1[i], g, x0[i] * r0);
-                    }
+                    const float x1[2] = {pp.second(x2.x, y2.x), pp.second(x2.y, y2.y)};
+                    const float s0[2] = {x0[0] * pp.r0, x0[1] * pp.r0}, s1[2] = {x1[0] * pp.r1, x1[1] * pp.r1};
                     const auto apply = [&](int j) {
+                        const float w = pp.second(t[j], u[j]);
 #pragma unroll
-                        for (int i = 0; i < 2; ++i) v[j][i] = fmaf(-s1[i], u[j], fmaf(-s0[i], t[j], v[j][i]));
+                        for (int i = 0; i < 2; ++i) v[j][i] = pivot_pair_apply(v[j][i], s0[i], t[j], s1[i], w);
                     };
                     apply(jn);
                     apply(jn + 1);

@@ -1,0 +1,63 @@
+"""FP32 diagonal blocks on matrices that are hard on the pivots: nearly collinear
+neighbouring columns, against the bound of a column-by-column factor."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _torch():
+    import torch
+    return torch
+
+
+def _collinear(n, start, gap, seed):
+    """Correlation matrix of n features: feature start + 1 is feature start plus gap times
+    another direction, the others correlate with both."""
+    rng = np.random.default_rng([n, start, seed])
+    F = rng.standard_normal((8 * n + 64, n))
+    z = rng.standard_normal(len(F))
+    F[:, start + 1] = F[:, start] + gap * z
+    for j in range(n):
+        if j not in (start, start + 1):
+            F[:, j] = 0.3 * F[:, j] + rng.standard_normal() * F[:, start] + rng.standard_normal() * z
+    F /= np.sqrt((F * F).sum(0))
+    a = (F.T @ F).astype(np.float32)
+    return np.tril(a) + np.tril(a, -1).T
+
+
+def _factor(gpu_lla, path, a):
+    torch = _torch()
+    n = len(a)
+    if path == "batch":
+        plan = gpu_lla.BatchPlan(np.array([n], np.int32), np.array([1], np.int32), "f32")
+        ap, bp = plan.pack([a], [np.ones((n, 1), np.float32)])
+        A, B = torch.from_numpy(ap.copy()).cuda(), torch.from_numpy(bp.copy()).cuda()
+        info = torch.empty(1, dtype=torch.int32, device="cuda")
+        plan.solve(A, B, info)
+        torch.cuda.synchronize()
+        return A.cpu().numpy()[:n * n].reshape((n, n), order="F"), int(info.item())
+    L = torch.from_numpy(a.copy()).cuda().T
+    if path == "device":
+        info = gpu_lla.potrf_device(L, algo=gpu_lla.ALGO_FAST)
+    else:
+        info = gpu_lla.spotrf_mixed_device(L, update="bf16x6")
+    torch.cuda.synchronize()
+    return L.cpu().numpy(), int(info.item())
+
+
+@pytest.mark.parametrize("path", ["device", "batch", "mixed"])
+@pytest.mark.parametrize("n,gap", [(4, 1e-2), (4, 3e-3), (8, 1e-2), (8, 3e-3), (16, 1e-2), (32, 1e-2), (64, 1e-2)])
+@pytest.mark.parametrize("start", [0, 1, "last"])
+def test_collinear_neighbours(gpu_lla, path, n, gap, start):
+    """|L L^T - A|_ij over sqrt(a_ii a_jj): quotients and scalings by approximate reciprocals cost
+    at most 8 eps a product, the sums (worst case n eps / 2) n eps / 8 as they add up in earnest."""
+    start = n - 4 if start == "last" else start
+    for seed in range(3):
+        a = _collinear(n, start, gap, seed)
+        fac, info = _factor(gpu_lla, path, a)
+        assert info == -1
+        low = np.tril(fac).astype(np.float64)
+        scale = np.sqrt(np.diag(a).astype(np.float64))
+        err = np.abs(low @ low.T - a) / scale[:, None] / scale[None, :]
+        assert err.max() <= (8 + n / 8) * np.finfo(np.float32).eps, (seed, err.max())
