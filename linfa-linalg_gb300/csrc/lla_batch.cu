@@ -180,7 +180,7 @@ __device__ void batch_diag(BatchSmem<T> &sm, int kb) {
     __syncthreads();
 }
 
-// FP32, all pivots positive and normal (false otherwise, the block spoilt): four
+// FP32, pivot_pair_takes() every pivot (false otherwise, the block spoilt): four
 // warps hold the block, 2 rows x 4 columns a thread.  Two columns a round go through
 // shared memory (the panel's space), every thread forms their pivots itself
 // (lla_pivot_pair.cuh), and the next pair is brought up to date and stored before the
@@ -242,7 +242,7 @@ __device__ bool batch_diag_quick(BatchSmem<float> &sm, int kb) {
                 put(nb, c + 2, v[jn], v[jn + 1]);  // (c + 2 = 32: nobody's)
                 apply(j0);
                 apply(j0 + 1);
-                ok = ok && batch_normal(d0) && batch_normal(d1);
+                ok = ok && pivot_pair_takes(d0) && pivot_pair_takes(d1);
                 if (tid < 32) {  // the finished pair, a column for each half of the warp
                     const bool second = tid & 16;
                     const float y = batch_rsqrt(second ? d1 : d0);

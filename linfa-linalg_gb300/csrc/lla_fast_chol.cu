@@ -224,7 +224,7 @@ __device__ __forceinline__ void fc_diag_sync() {
     asm volatile("bar.sync 1, %0;" ::"n"(kFcDiagThreads) : "memory");
 }
 
-// FP32 block with all pivots positive and normal: sm.a, sm.piv and sm.rv finished.
+// FP32 block whose pivots pivot_pair_takes() all: sm.a, sm.piv and sm.rv finished.
 // Otherwise sm.fail is set and the block spoilt.  FP32 instructions are short, so
 // the chain is exchanges: eight warps hold the block (two rows a lane, eight columns
 // a warp), a pair of columns a step goes through shared memory, every thread forms
@@ -306,7 +306,7 @@ __device__ __forceinline__ void fc_diag_quick(FcDiagSmem<float> &sm) {
                     sm.piv[c + 1] = d1;
                     sm.rv[c] = q0;
                     sm.rv[c + 1] = q1;
-                    if (!Fc<float>::normal(d0) || !Fc<float>::normal(d1)) sm.fail = kFcNb;
+                    if (!pivot_pair_takes(d0) || !pivot_pair_takes(d1)) sm.fail = kFcNb;
                 }
             }
             b = nb;

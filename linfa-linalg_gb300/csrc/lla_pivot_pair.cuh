@@ -13,7 +13,14 @@
 // two agree, and the entry that is stored as L's is the one the update used.
 #pragma once
 
+#include <cuda_runtime.h>
+
 namespace lla {
+
+// Whether a pivot is positive and normal with a normal reciprocal (the approximate
+// one flushes subnormal results to zero): 2^-126 <= d < 2^126.  Others take the blocks'
+// general forms, which divide by no pivot's reciprocal.
+__device__ __forceinline__ bool pivot_pair_takes(float d) { return __float_as_uint(d) - 0x800000u < 0x7e000000u; }
 
 struct PivotPair {
     float d0, r0;  // pivot of column c and its reciprocal

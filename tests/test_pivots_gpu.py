@@ -1,5 +1,5 @@
 """FP32 diagonal blocks on matrices that are hard on the pivots: nearly collinear
-neighbouring columns, against the bound of a column-by-column factor."""
+neighbouring columns, values near the ends of the exponent range, against the bound of a column-by-column factor."""
 import numpy as np
 import pytest
 
@@ -61,3 +61,20 @@ def test_collinear_neighbours(gpu_lla, path, n, gap, start):
         scale = np.sqrt(np.diag(a).astype(np.float64))
         err = np.abs(low @ low.T - a) / scale[:, None] / scale[None, :]
         assert err.max() <= (8 + n / 8) * np.finfo(np.float32).eps, (seed, err.max())
+
+
+@pytest.mark.parametrize("path", ["device", "batch"])
+@pytest.mark.parametrize("n", [1, 2, 5, 33, 65, 200])
+@pytest.mark.parametrize("scale", [2.0**126, 1.9 * 2.0**126, 2.0**-100])
+def test_pivots_near_the_ends_of_the_range(gpu_lla, path, n, scale):
+    """Pivots above 2^126, whose reciprocals are subnormal, and tiny ones: the same bound."""
+    rng = np.random.default_rng(n)
+    g = rng.standard_normal((n, 2 * n))
+    g /= np.sqrt((g * g).sum(1))[:, None]
+    a = (g @ g.T * scale).astype(np.float32)
+    a = np.tril(a) + np.tril(a, -1).T
+    fac, info = _factor(gpu_lla, path, a)
+    assert info == -1
+    low = np.tril(fac).astype(np.float64)
+    err = np.abs(low @ low.T - a) / scale
+    assert err.max() <= (8 + n / 8) * np.finfo(np.float32).eps, err.max()
