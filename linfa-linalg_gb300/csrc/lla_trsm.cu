@@ -72,7 +72,8 @@ static int trsm_warps(int mc) { return std::max(mc, kTrsmMc); }
 
 // The division of the reference's substitution by a divisor that is known early,
 // without a test on its chain; ok says afterwards whether x is IEEE division's
-// num / d, and the solve repeats a block with IEEE division if one was not.
+// num / d, and the solve repeats a block with IEEE division if one was not (so does
+// the FAST solve whose rows were divided beforehand, if a result is not finite).
 // (Tested in every step: EXACT f64 n = 512 190 us a solve, now 165; EXACT f32
 // n = 1000, with the general division 123 us, with the test 137, now 99.)
 template <typename T>
@@ -98,6 +99,9 @@ struct TrsmDivisor<double> {
         return good;
     }
 };
+
+__device__ __forceinline__ bool trsm_finite(double v) { return ((unsigned)__double2hiint(v) & 0x7ff00000u) != 0x7ff00000u; }
+__device__ __forceinline__ bool trsm_finite(float v) { return (__float_as_uint(v) & 0x7f800000u) != 0x7f800000u; }
 
 template <typename T, bool kExact>
 __global__ void __launch_bounds__(kTrsmNb *kTrsmMaxMc) trsm_lookback(const T *__restrict__ M, int64_t ld, int64_t n,
@@ -227,6 +231,8 @@ __global__ void __launch_bounds__(kTrsmNb *kTrsmMaxMc) trsm_lookback(const T *__
     if (!kExact) __syncthreads();  // (the first block met no barrier after the scaling of td)
 
     if (!abort && col_ok) {
+        const T b0 = bv;
+        bool ok;
         if (scaled) {
             bv = Ar::fma_(bv, rinv, Ar::mul(bv, rlo));
 #pragma unroll 4
@@ -235,8 +241,10 @@ __global__ void __launch_bounds__(kTrsmNb *kTrsmMaxMc) trsm_lookback(const T *__
                 const T nb = Ar::fma_(-xy, td[y][tx], bv);
                 if (tx > y) bv = nb;
             }
+            // infinities and overflow on the way: products by a reciprocal are no longer what the
+            // division gives (inf * 0, inf - inf)
+            ok = trsm_finite(bv);
         } else {
-            const T b0 = bv;
             T num = bv;  // what this lane's row was divided from
 #pragma unroll 4
             for (int y = 0; y < bs; ++y) {
@@ -245,15 +253,20 @@ __global__ void __launch_bounds__(kTrsmNb *kTrsmMaxMc) trsm_lookback(const T *__
                 num = tx == y ? bv : num;
                 bv = tx == y ? xy : (tx > y ? nb : bv);
             }
-            const bool ok = tx >= bs || dq.ok(num, bv);
-            if (!__all_sync(0xffffffffu, ok)) {
-                bv = b0;
+            ok = dq.ok(num, bv);
+        }
+        if (!__all_sync(0xffffffffu, ok || tx >= bs)) {
+            bv = b0;
 #pragma unroll 1
-                for (int y = 0; y < bs; ++y) {
-                    const T xy = __shfl_sync(0xffffffffu, Ar::div(bv, dv), y);
-                    const T nb = kExact ? Ar::sub(bv, Ar::mul(xy, td[y][tx])) : Ar::fma_(-xy, td[y][tx], bv);
-                    bv = tx == y ? xy : (tx > y ? nb : bv);
+            for (int y = 0; y < bs; ++y) {
+                T t = td[y][tx];
+                if (scaled && tx > y && tx < bs) {  // as it was before the scaling
+                    const int64_t c = row_of(t0 + y);
+                    t = trans ? M[c + r_own * ld] : M[r_own + c * ld];
                 }
+                const T xy = __shfl_sync(0xffffffffu, Ar::div(bv, dv), y);
+                const T nb = kExact ? Ar::sub(bv, Ar::mul(xy, t)) : Ar::fma_(-xy, t, bv);
+                bv = tx == y ? xy : (tx > y ? nb : bv);
             }
         }
     }
