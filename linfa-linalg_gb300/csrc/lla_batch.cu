@@ -38,6 +38,7 @@
 #include "../../include/lla_gb300.h"
 #include "lla_autotune.h"
 #include "lla_common.cuh"
+#include "lla_device.h"
 #include "lla_int_math.h"
 #include "lla_kernels.h"
 #include "lla_oz_mma.cuh"
@@ -1061,13 +1062,7 @@ int serve_loop_launch(ServeRing *ring_dev, unsigned long long *d_next, double *s
                       double idle_us, cudaStream_t st) {
     const size_t smem = sizeof(BatchSmem<double>);
     static_assert(sizeof(BatchSmem<double>) >= sizeof(BatchSmem<float>), "one space for both types");
-    static bool attr = false;
-    if (!attr) {
-        if (cudaFuncSetAttribute(serve_loop_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-            cudaSuccess)
-            return -1;
-        attr = true;
-    }
+    if (allow_dynamic_smem(serve_loop_kernel, smem) != cudaSuccess) return -1;
     LaunchScope ls(K_BATCH, st);
     serve_loop_kernel<<<(unsigned)ctas, 256, smem, st>>>(ring_dev, d_next, scratch,
                                                          (unsigned long long)(idle_us * 1e3));
@@ -1106,17 +1101,6 @@ static size_t batch_smem(int dtype) { return dtype == 8 ? sizeof(BatchSmem<doubl
 static bool cache_lookup(const std::string &key, int &cps, int &thr) { return lla::autotune_lookup(key, cps, thr); }
 static void cache_store(const std::string &key, int cps, int thr) { lla::autotune_store(key, cps, thr); }
 
-static int sm_count() {
-    static int sms = 0;
-    if (!sms) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        if (sms <= 0) sms = 1;
-    }
-    return sms;
-}
-
 namespace lla {
 
 template <typename T>
@@ -1124,16 +1108,10 @@ int batch_launch_raw(const BatchItem *d_items, int64_t count, T *dA, T *dB, int3
                      int *d_counter, int ctas_per_sm, int threads, double flops, cudaStream_t st) {
     if (count <= 0) return 0;
     if (cudaMemsetAsync(d_counter, 0, sizeof(int), st) != cudaSuccess) return -1;
-    static bool attr[2] = {false, false};
     const size_t smem = batch_smem(sizeof(T));
-    if (!attr[sizeof(T) == 8]) {
-        if (cudaFuncSetAttribute(batch_posv_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)smem) != cudaSuccess)
-            return -1;
-        attr[sizeof(T) == 8] = true;
-    }
+    if (allow_dynamic_smem(batch_posv_kernel<T>, smem) != cudaSuccess) return -1;
     const unsigned grid =
-        (unsigned)std::max<int64_t>(1, std::min<int64_t>(count, (int64_t)ctas_per_sm * sm_count()));
+        (unsigned)std::max<int64_t>(1, std::min<int64_t>(count, (int64_t)ctas_per_sm * device_sms()));
     LaunchScope ls(K_BATCH, st, flops);
     batch_posv_kernel<T><<<grid, threads, smem, st>>>(d_items, count, dA, dB, d_info, d_counter);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
@@ -1154,7 +1132,7 @@ static cudaError_t batch_launch(lla_batch_plan *p, T *dA, T *dB, int32_t *d_info
     if (p->refined && sizeof(T) == 8) {
         if (cudaMemsetAsync(p->d_counter, 0, sizeof(int), st) != cudaSuccess) return cudaGetLastError();
         const int cps = refined_ctas_per_sm(p->ctas_per_sm);
-        const unsigned grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>(p->count, (int64_t)cps * sm_count()));
+        const unsigned grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>(p->count, (int64_t)cps * device_sms()));
         LaunchScope ls(K_BATCH, st, p->flops);
         batch_posv_refined_kernel<<<grid, p->threads, batch_refined_smem(), st>>>(
             p->d_items, p->count, (const double *)dA, (double *)dB, d_info, p->d_counter, p->d_scratch);
@@ -1229,10 +1207,8 @@ int lla_batch_plan_create(int64_t count, const int32_t *n, const int32_t *m, int
         e = cudaMemcpy(p->d_items, items.data(), sizeof(BatchItem) * count, cudaMemcpyHostToDevice);
     if (e == cudaSuccess) {
         const size_t smem = batch_smem(elem_bytes);
-        e = elem_bytes == 8 ? cudaFuncSetAttribute(batch_posv_kernel<double>,
-                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)
-                            : cudaFuncSetAttribute(batch_posv_kernel<float>,
-                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        e = elem_bytes == 8 ? allow_dynamic_smem(batch_posv_kernel<double>, smem)
+                            : allow_dynamic_smem(batch_posv_kernel<float>, smem);
     }
     if (e != cudaSuccess) {
         cudaFree(p->d_items);
@@ -1288,15 +1264,8 @@ int lla_batch_set_refined(lla_batch_plan *p, int refined, lla_error *err) {
     lla__set_status(err, LLA_OK);
     const bool want = refined != 0;
     if (want && !p->d_scratch) {
-        static bool attr = false;
-        if (!attr) {
-            const cudaError_t e = cudaFuncSetAttribute(batch_posv_refined_kernel,
-                                                       cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                       (int)batch_refined_smem());
-            if (e != cudaSuccess) return lla__set_cuda_error(err, e);
-            attr = true;
-        }
-        const cudaError_t e = cudaMalloc(&p->d_scratch, batch_refined_scratch_bytes(2 * sm_count()));
+        cudaError_t e = allow_dynamic_smem(batch_posv_refined_kernel, batch_refined_smem());
+        if (e == cudaSuccess) e = cudaMalloc(&p->d_scratch, batch_refined_scratch_bytes(2 * device_sms()));
         if (e != cudaSuccess) {
             p->d_scratch = nullptr;
             return lla__set_cuda_error(err, e);

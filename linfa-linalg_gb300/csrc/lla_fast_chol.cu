@@ -35,9 +35,9 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <atomic>
 
 #include "lla_common.cuh"
+#include "lla_device.h"
 #include "lla_int_math.h"
 #include "lla_kernels.h"
 #include "lla_oz_mma.cuh"
@@ -984,17 +984,6 @@ __global__ void fc_begin_kernel(const T *W, int64_t ld, int64_t n, T *out, int *
 
 // ---- host side --------------------------------------------------------------
 
-static int fc_sms() {
-    static int sms = 0;
-    if (!sms) {
-        int dev = 0, v = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
-        sms = v > 0 ? v : 1;
-    }
-    return sms;
-}
-
 static int fc_encode(PFN_cuTensorMapEncodeTiled_v12000 enc, CUtensorMap *m, void *planes, int64_t n, int digits,
                      int rows, int nplanes) {
     const cuuint32_t estr[3] = {1, 1, 1};
@@ -1012,13 +1001,8 @@ template <typename T>
 int potrf_fast_launch(T *W, int64_t n, int64_t ld, int64_t *d_info, T *diag0, double *min_ratio, int *err_word,
                       int *sticky, cudaStream_t st) {
     constexpr int ND = Fc<T>::kDigits;
-    static std::atomic<bool> attr{false};
-    if (!attr.load()) {
-        if (cudaFuncSetAttribute(fc_update_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFuSmem<T>) !=
-            cudaSuccess)
-            return -1;
-        attr.store(true);
-    }
+    if (allow_dynamic_smem(fc_update_kernel<T>, kFuSmem<T>) != cudaSuccess) return -1;
+    const int sms = device_sms();
     PFN_cuTensorMapEncodeTiled_v12000 enc = tma_encoder();
     if (!enc) return -1;
     // digit planes [ND][n][128], row exponents, reciprocal pivots, status word (own copy when
@@ -1054,7 +1038,7 @@ int potrf_fast_launch(T *W, int64_t n, int64_t ld, int64_t *d_info, T *diag0, do
         // algorithmic work: entries of the lower part x columns x 2
         LaunchScope ls(K_POTRF_FAST_UPDATE, st,
                        ((double)m * cols - (double)cols * (cols - 1) / 2) * 2.0 * kchunks * kFuK);
-        launch_maybe_pdl(true, fc_update_kernel<T>, dim3((unsigned)std::min<int64_t>(tiles, fc_sms())), dim3(kFuThreads),
+        launch_maybe_pdl(true, fc_update_kernel<T>, dim3((unsigned)std::min<int64_t>(tiles, sms)), dim3(kFuThreads),
                          (size_t)kFuSmem<T>, st, tmA, tmB, W, ld, q, n, p0, kchunks, (int)tiles, narrow,
                          (const int *)expo, (const T *)diag0, rinv, d_info, min_ratio, ew, sticky);
     };

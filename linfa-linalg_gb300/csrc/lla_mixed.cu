@@ -26,6 +26,7 @@
 #include "lla_api_internal.h"
 #include "lla_autotune.h"
 #include "lla_common.cuh"
+#include "lla_device.h"
 #include "lla_f32_bits.h"
 #include "lla_kernels.h"
 #include "lla_mixed.h"
@@ -557,13 +558,7 @@ static int res_rows(int64_t m) { return m <= 32 ? ResTile<4, 1>::kRows : ResTile
 static int res_cols(int64_t m) { return m <= 8 ? 8 : (m <= 16 ? 16 : (m <= 32 ? 32 : 64)); }
 
 int residual_splits(int64_t n, int64_t m) {
-    static int sms = 0;
-    if (!sms) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        if (sms <= 0) sms = 1;
-    }
+    const int sms = device_sms();
     const int64_t tiles = (int64_t)gx(n, res_rows(m)) * gx(m, res_cols(m));
     // smallest split giving at least four waves of CTAs (at most 8)
     int s = 1;

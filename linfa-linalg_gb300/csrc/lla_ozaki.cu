@@ -33,6 +33,7 @@
 #include <algorithm>
 
 #include "lla_common.cuh"
+#include "lla_device.h"
 #include "lla_mixed.h"
 #include "lla_oz_digits.h"
 #include "lla_prof.h"
@@ -441,13 +442,7 @@ struct OzState {
 };
 
 static int oz_splits(int64_t n) {
-    static int sms = 0;
-    if (!sms) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        if (sms <= 0) sms = 1;
-    }
+    const int sms = device_sms();
     // fewest splits whose CTAs fill the waves of one CTA per SM to within 5 %,
     // keeping at least 8 K-chunks per split
     const int64_t tiles = (n + kOzM - 1) / kOzM, chunks = oz_ldp(n) / kOzK;
@@ -505,13 +500,7 @@ int oz_prepare(const double *A, int64_t lda, int64_t n, int64_t m, void *ws, boo
 int oz_residual_launch(const double *X, int64_t ldx, const double *B, int64_t ldb, double *R, int64_t ldr,
                        int64_t n, int64_t m, const double *colmax_x, double *colmax_r, void *ws,
                        int *err_word, cudaStream_t st, const int *state) {
-    static bool attr = false;
-    if (!attr) {
-        if (cudaFuncSetAttribute(oz_residual_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kOzSmem) !=
-            cudaSuccess)
-            return -1;
-        attr = true;
-    }
+    if (allow_dynamic_smem(oz_residual_kernel, kOzSmem) != cudaSuccess) return -1;
     PFN_cuTensorMapEncodeTiled_v12000 enc = tma_encoder();
     if (!enc) return -1;
     OzState o;

@@ -1,11 +1,12 @@
 // lla_scratch.cpp -- see lla_scratch.h.
 #include "lla_scratch.h"
 
+#include "lla_device.h"
+
 #include <mutex>
 
 namespace lla {
 
-constexpr int kMaxDevices = 64;
 static std::mutex g_pool_mu;
 static cudaMemPool_t g_pool[kMaxDevices] = {};
 

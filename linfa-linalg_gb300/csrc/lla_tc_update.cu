@@ -30,6 +30,7 @@
 #include <cstring>
 
 #include "lla_common.cuh"
+#include "lla_device.h"
 #include "lla_tc.h"
 #include "lla_tcgen05.cuh"
 
@@ -514,14 +515,7 @@ int tc_update_launch(float *C, int64_t ld, int64_t q, int64_t n, void *planes, i
     const uint32_t ab = fp16 ? 0u : 1u;
     const uint32_t idesc = (1u << 4) | (ab << 7) | (ab << 10) | ((uint32_t)(kTcN >> 3) << 17) |
                            ((uint32_t)(kTcM >> 4) << 24);
-    static int sms = 0;
-    if (!sms) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        if (sms <= 0) sms = 1;
-    }
-    const unsigned grid = (unsigned)std::min<int64_t>(tiles, sms);
+    const unsigned grid = (unsigned)std::min<int64_t>(tiles, device_sms());
     // the pair lists are fixed per number of terms (small products first, (0, 0) last)
     if (pairs.n != (terms == 1 ? 1 : (terms == 2 ? 3 : 6)) || pairs.pa[pairs.n - 1] != 0 ||
         pairs.pb[pairs.n - 1] != 0)

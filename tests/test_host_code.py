@@ -1,0 +1,111 @@
+"""Host code of the library on a CUDA runtime without a GPU (tests/fake_cuda.cpp): what the
+entry points ask of the runtime, on two devices."""
+import ctypes
+import glob
+import os
+import shutil
+import subprocess
+import threading
+
+import numpy as np
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+PKG = os.path.join(ROOT, "linfa-linalg_gb300")
+CUDA = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+
+
+@pytest.fixture(scope="module")
+def fake(tmp_path_factory):
+    objs = sorted(glob.glob(os.path.join(PKG, "_build", "*.o")))
+    if not objs or not shutil.which("g++"):
+        pytest.skip("the library's objects are built by build()")
+    so = str(tmp_path_factory.mktemp("fake") / "liblla_fake.so")
+    subprocess.run(["g++", "-shared", "-fPIC", "-O1", "-I", os.path.join(CUDA, "include"), "-o", so,
+                    os.path.join(ROOT, "tests", "fake_cuda.cpp")] + objs +
+                   ["-Wl,-Bsymbolic", "-Wl,--no-undefined", "-lpthread", "-ldl", "-lm"], check=True)
+    lib = ctypes.CDLL(so)
+    lib.fake_log.restype = ctypes.c_char_p
+    return lib
+
+
+@pytest.fixture(autouse=True)
+def own_cache(tmp_path, monkeypatch):
+    """An autotune cache file of the test's own."""
+    monkeypatch.setenv("LLA_AUTOTUNE_CACHE", str(tmp_path / "autotune.txt"))
+    return tmp_path / "autotune.txt"
+
+
+def on_device(lib, dev, fn):
+    """fn() on a host thread of its own, bound to a device: its result."""
+    out = []
+
+    def body():
+        lib.fake_set_device(dev)
+        out.append(fn())
+
+    t = threading.Thread(target=body)
+    t.start()
+    t.join()
+    return out[0]
+
+
+I64, P = ctypes.c_int64, ctypes.c_void_p
+
+
+def _launches(lib, dev, kernel):
+    """Grid sizes of the launches of a kernel on a device since the last clear."""
+    rows = [r.split(" ", 2) for r in lib.fake_log().decode().splitlines()]
+    return [int(g) for d, g, name in rows if int(d) == dev and kernel in name]
+
+
+def _fast_factor(lib, fn, dtype):
+    a, info = np.eye(512, dtype=dtype), np.zeros(1, np.int64)
+    return fn(P(a.ctypes.data), I64(512), I64(512), 2, P(info.ctypes.data), None, None)
+
+
+def _batch(lib, elem, refined):
+    n, m = np.full(40, 16, np.int32), np.ones(40, np.int32)
+    plan = P()
+    assert lib.lla_batch_plan_create(I64(40), P(n.ctypes.data), P(m.ctypes.data), elem, ctypes.byref(plan), None) == 0
+    if refined:
+        st = lib.lla_batch_set_refined(plan, 1, None)
+        if st:
+            return st
+    a, b, info = np.zeros((40, 256)), np.zeros((40, 16)), np.zeros(40, np.int32)
+    fn = lib.lla_dbatch_posv_device if elem == 8 else lib.lla_sbatch_posv_device
+    st = fn(plan, P(a.ctypes.data), P(b.ctypes.data), P(info.ctypes.data), None, None)
+    lib.lla_batch_plan_destroy(plan)
+    return st
+
+
+def _residual(lib, method):
+    n, m = 300, 8
+    a, x, b, r = np.zeros((n, n)), np.zeros((m, n)), np.zeros((m, n)), np.zeros((m, n))
+    p = [P(v.ctypes.data) for v in (a, x, b, r)]
+    return lib.lla_dresidual_device(p[0], I64(n), I64(n), p[1], I64(n), p[2], I64(n), p[3], I64(n), I64(m), method,
+                                    None, None)
+
+
+# entry point, kernel with more than 48 KiB of dynamic shared memory (or a grid by the
+# multiprocessor count), and whether a multiprocessor holds several of its CTAs
+CALLS = {
+    "factor f64": (lambda lib: _fast_factor(lib, lib.lla_dpotrf_device, np.float64), "fc_update_kernel", 1),
+    "factor f32": (lambda lib: _fast_factor(lib, lib.lla_spotrf_device, np.float32), "fc_update_kernel", 1),
+    "batch f64": (lambda lib: _batch(lib, 8, False), "batch_posv_kernel", 4),
+    "batch f32": (lambda lib: _batch(lib, 4, False), "batch_posv_kernel", 4),
+    "batch refined": (lambda lib: _batch(lib, 8, True), "batch_posv_refined_kernel", 2),
+    "residual by slices": (lambda lib: _residual(lib, 1), "oz_residual_kernel", None),
+}
+
+
+@pytest.mark.parametrize("call", CALLS)
+def test_a_second_device_is_asked_for_itself(fake, call):
+    """Kernel attributes and multiprocessor counts belong to a device: the same call from threads
+    bound to two devices is launched on both, with each device's own grid."""
+    run, kernel, per_sm = CALLS[call]
+    for dev, sms in ((0, 5), (1, 7), (0, 5)):
+        fake.fake_clear()
+        assert on_device(fake, dev, lambda: run(fake)) == 0, f"refused on device {dev}"
+        grids = _launches(fake, dev, kernel)
+        assert grids and (per_sm is None or max(grids) == min(per_sm * sms, 40)), grids
