@@ -9,7 +9,6 @@
 #include <cstring>
 #include <map>
 #include <mutex>
-#include <set>
 #include <string>
 #include <utility>
 
@@ -20,8 +19,9 @@ struct State {
     std::map<const void *, std::string> names;
     std::map<std::pair<int, const void *>, int> smem;  // per device and function
     std::string log;
-    std::set<cudaStream_t> capturing;
-    int allocs_in_capture = 0;
+    std::map<cudaStream_t, cudaGraph_t> capturing;
+    std::map<cudaGraph_t, std::pair<cudaHostFn_t, void *>> kept;  // a graph's user object
+    int alloc_nodes = 0, pool_blocks = 0;                        // in graphs; from pools, not yet freed
 };
 State &state() {
     static State *s = new State();  // (kernels register before main, streams end after it)
@@ -57,6 +57,8 @@ void fake_set_device(int dev) { t_dev = dev; }
 void fake_set_hook(void (*hook)(const char *, void **)) { g_hook = hook; }
 const char *fake_log() { return state().log.c_str(); }
 void fake_clear() { state().log.clear(); }
+int fake_alloc_nodes() { return state().alloc_nodes; }
+int fake_pool_blocks() { return state().pool_blocks; }
 
 void **__cudaRegisterFatBinary(void *) { return (void **)calloc(1, 8); }
 void __cudaRegisterFatBinaryEnd(void **) {}
@@ -105,11 +107,12 @@ cudaError_t cudaDeviceSynchronize() { return cudaSuccess; }
 cudaError_t cudaMalloc(void **p, size_t n) { return memory(p, n); }
 cudaError_t cudaMallocAsync(void **p, size_t n, cudaStream_t) { return memory(p, n); }
 cudaError_t cudaMallocFromPoolAsync(void **p, size_t n, cudaMemPool_t, cudaStream_t st) {
-    state().allocs_in_capture += (int)state().capturing.count(st);
+    state().alloc_nodes += (int)state().capturing.count(st);
+    ++state().pool_blocks;
     return memory(p, n);
 }
 cudaError_t cudaFree(void *p) { return std::free(p), cudaSuccess; }
-cudaError_t cudaFreeAsync(void *p, cudaStream_t) { return std::free(p), cudaSuccess; }
+cudaError_t cudaFreeAsync(void *p, cudaStream_t) { return --state().pool_blocks, std::free(p), cudaSuccess; }
 cudaError_t cudaHostAlloc(void **p, size_t n, unsigned) { return memory(p, n); }
 cudaError_t cudaFreeHost(void *p) { return std::free(p), cudaSuccess; }
 cudaError_t cudaHostGetDevicePointer(void **d, void *h, unsigned) { return *d = h, cudaSuccess; }
@@ -144,13 +147,46 @@ cudaError_t cudaStreamDestroy(cudaStream_t s) { return std::free(s), cudaSuccess
 cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaStreamQuery(cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaStreamBeginCapture(cudaStream_t s, enum cudaStreamCaptureMode) {
-    return state().capturing.insert(s), cudaSuccess;
+    return memory((void **)&state().capturing[s], 8);
 }
+cudaError_t cudaStreamGetCaptureInfo(cudaStream_t s, enum cudaStreamCaptureStatus *st, unsigned long long *, cudaGraph_t *g,
+                                     const cudaGraphNode_t **, const cudaGraphEdgeData **, size_t *) {
+    const auto it = state().capturing.find(s);
+    *st = it == state().capturing.end() ? cudaStreamCaptureStatusNone : cudaStreamCaptureStatusActive;
+    if (g && it != state().capturing.end()) *g = it->second;
+    return cudaSuccess;
+}
+cudaError_t cudaThreadExchangeStreamCaptureMode(enum cudaStreamCaptureMode *) { return cudaSuccess; }
 cudaError_t cudaStreamEndCapture(cudaStream_t s, cudaGraph_t *g) {
+    *g = state().capturing[s];
     state().capturing.erase(s);
-    return memory((void **)g, 8);
+    return cudaSuccess;
 }
-cudaError_t cudaGraphDestroy(cudaGraph_t g) { return std::free(g), cudaSuccess; }
+cudaError_t cudaUserObjectCreate(cudaUserObject_t *o, void *arg, cudaHostFn_t fn, unsigned, unsigned) {
+    *o = (cudaUserObject_t) new std::pair<cudaHostFn_t, void *>(fn, arg);
+    return cudaSuccess;
+}
+cudaError_t cudaUserObjectRelease(cudaUserObject_t o, unsigned) {
+    auto *p = (std::pair<cudaHostFn_t, void *> *)o;
+    p->first(p->second);
+    delete p;
+    return cudaSuccess;
+}
+cudaError_t cudaGraphRetainUserObject(cudaGraph_t g, cudaUserObject_t o, unsigned, unsigned) {
+    auto *p = (std::pair<cudaHostFn_t, void *> *)o;
+    state().kept[g] = *p;
+    delete p;
+    return cudaSuccess;
+}
+cudaError_t cudaGraphDestroy(cudaGraph_t g) {
+    const auto it = state().kept.find(g);
+    if (it != state().kept.end()) {
+        const auto k = it->second;
+        state().kept.erase(it);
+        k.first(k.second);
+    }
+    return std::free(g), cudaSuccess;
+}
 cudaError_t cudaGraphInstantiate(cudaGraphExec_t *e, cudaGraph_t, unsigned long long) { return memory((void **)e, 8); }
 cudaError_t cudaGraphExecDestroy(cudaGraphExec_t e) { return std::free(e), cudaSuccess; }
 cudaError_t cudaGraphLaunch(cudaGraphExec_t, cudaStream_t) { return cudaSuccess; }

@@ -109,3 +109,30 @@ def test_a_second_device_is_asked_for_itself(fake, call):
         assert on_device(fake, dev, lambda: run(fake)) == 0, f"refused on device {dev}"
         grids = _launches(fake, dev, kernel)
         assert grids and (per_sm is None or max(grids) == min(per_sm * sms, 40)), grids
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+def test_a_captured_factor_allocates_beside_the_graph(fake, dtype):
+    """A captured FAST factor puts no allocation into the caller's graph, whose copies could not
+    run otherwise; the graph keeps the scratch, and once it is gone the next call frees it."""
+    fn = fake.lla_dpotrf_device if dtype == np.float64 else fake.lla_spotrf_device
+    a, info = np.eye(300, dtype=dtype), np.zeros(1, np.int64)
+
+    def factor(stream):
+        return fn(P(a.ctypes.data), I64(300), I64(300), 2, P(info.ctypes.data), stream, None)
+
+    def body():
+        stream, graph = P(), P()
+        fake.cudaStreamCreateWithFlags(ctypes.byref(stream), 1)
+        assert factor(stream) == 0  # creates the thread's workspace
+        blocks, nodes = fake.fake_pool_blocks(), fake.fake_alloc_nodes()
+        fake.cudaStreamBeginCapture(stream, 1)
+        assert factor(stream) == 0
+        fake.cudaStreamEndCapture(stream, ctypes.byref(graph))
+        assert fake.fake_alloc_nodes() == nodes
+        assert factor(stream) == 0 and fake.fake_pool_blocks() == blocks + 1  # the graph's
+        fake.cudaGraphDestroy(graph)
+        assert factor(stream) == 0 and fake.fake_pool_blocks() == blocks
+        return True
+
+    assert on_device(fake, 0, body)
