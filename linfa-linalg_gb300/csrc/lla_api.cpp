@@ -78,10 +78,6 @@ static int not_pd(lla_error *err, int64_t index) {
 
 static std::atomic<int> g_algo{LLA_ALGO_AUTO};
 static constexpr int64_t kAutoExactMaxN = 1024;
-// FAST factorisations whose smallest relative pivot falls below this are
-// re-run in EXACT order so that NotPositiveDefinite is decided by the
-// reference's own arithmetic.
-static constexpr double kPivotGuard = 1e-10;
 
 extern "C" int lla_set_algorithm(int algo) {
     if (algo < LLA_ALGO_AUTO || algo > LLA_ALGO_FAST) return -1;
@@ -305,18 +301,15 @@ cudaError_t download(Ctx &c, const View &v, DevBuf &raw, HostBuf &stage) {
 }
 
 // A download in two halves around one synchronisation of the stream, so that a
-// call with several results waits once: begin() copies a strided view, or a small
-// contiguous one, into its pinned staging buffer; finish(), after the caller has
-// synchronised and decided that the results stand, moves them into the view (a
-// large contiguous view is copied there directly and waited for: above 128 KiB
-// the driver's own staging beats a copy on this thread, invc of n = 300 948 us
-// against 1008).
+// call with several results waits once: begin() copies a small view into its pinned
+// staging buffer; finish(), after the caller has synchronised and decided that the
+// results stand, moves them into the view.  A larger view is copied then, and waited
+// for: a contiguous one goes through the driver's own staging, which beats a copy on
+// this thread (invc of n = 300, 720 KB: 948 us against 1008), and a call whose results
+// do not stand has not moved it for nothing.
 constexpr size_t kStageBytes = 1u << 17;
 
-bool staged_download(const View &v) {
-    const size_t bytes = (size_t)(v.rows * v.cols) * v.esz;
-    return !(colmajor_contig(v) || rowmajor_contig(v)) || bytes <= kStageBytes;
-}
+bool staged_download(const View &v) { return (size_t)(v.rows * v.cols) * v.esz <= kStageBytes; }
 cudaError_t begin_download(Ctx &c, const View &v, DevBuf &raw, HostBuf &stage) {
     const size_t bytes = (size_t)(v.rows * v.cols) * v.esz;
     if (bytes == 0 || !staged_download(v)) return cudaSuccess;
@@ -341,11 +334,10 @@ cudaError_t launch_status(int rc) {
     return e == cudaSuccess ? cudaErrorUnknown : e;
 }
 
-// Small device/host words: the factorisation's info, smallest relative pivot and
-// status (a bounded wait that gave up), the solves' status, the predicate's flag.
+// Small device/host words: the factorisation's verdict and status (a bounded wait
+// that gave up), the solves' status, the predicate's flag.
 struct Words {
-    int64_t info;
-    double min_ratio;
+    FactorVerdict factor;
     int32_t err_word;
     int32_t flag;
     int32_t factor_err;
@@ -353,8 +345,7 @@ struct Words {
 
 cudaError_t reset_words(Ctx &c) {
     Words *h = (Words *)c.small_host.p;
-    h->info = -1;
-    h->min_ratio = 1e300;
+    h->factor = {-1, 1e300};
     h->err_word = 0;
     h->flag = 1;
     h->factor_err = 0;
@@ -381,14 +372,16 @@ static cudaError_t factor_enqueue(Ctx &c, T *W, int64_t n, int64_t ld, bool exac
     cudaError_t e;
     if ((e = c.aux_d.ensure(sizeof(T) * n)) != cudaSuccess) return e;
     if (!exact)
-        return launch_status(potrf_fast_launch<T>(W, n, ld, &dev_words(c)->info, (T *)c.aux_d.p,
-                                                  &dev_words(c)->min_ratio, &dev_words(c)->factor_err, nullptr, c.stream));
+        return launch_status(potrf_fast_launch<T>(W, n, ld, &dev_words(c)->factor.info, (T *)c.aux_d.p,
+                                                  &dev_words(c)->factor.min_ratio, &dev_words(c)->factor_err, nullptr,
+                                                  c.stream));
     if ((e = c.aux_s.ensure(sizeof(T) * ld * n)) != cudaSuccess) return e;
-    return launch_status(potrf_exact_launch<T>(W, (T *)c.aux_s.p, (T *)c.aux_d.p, n, ld, &dev_words(c)->info, c.stream));
+    return launch_status(potrf_exact_launch<T>(W, (T *)c.aux_s.p, (T *)c.aux_d.p, n, ld, &dev_words(c)->factor.info,
+                                               c.stream));
 }
 
 // Whether a FAST factorisation's outcome has to be decided in EXACT order.
-static bool fast_undecided(const Words &w) { return w.info >= 0 || w.min_ratio < kPivotGuard; }
+static bool fast_undecided(const Words &w) { return w.factor.info >= 0 || w.factor.min_ratio < kPivotGuard; }
 
 // Factor the column-major n x n W in place.  On a FAST failure or a
 // near-singular FAST factorisation, W is re-imported from (R, drs, dcs) and
@@ -416,18 +409,19 @@ cudaError_t factor_on_device(Ctx &c, T *W, int64_t n, int64_t ld, bool exact, co
     }
     if ((e = factor_enqueue<T>(c, W, n, ld, true)) != cudaSuccess) return e;
     if ((e = read_words(c, w)) != cudaSuccess) return e;
-    *fail = w.info;
+    *fail = w.factor.info;
     return cudaSuccess;
 }
 
-// Enqueues a triangular solve (words reset before; err_word collects a timeout).
+// Enqueues a triangular solve (words reset before; err_word collects a timeout; without
+// a factorisation behind the words, their verdict is that one stands).
 template <typename T>
 static cudaError_t trsm_enqueue(Ctx &c, const T *M, int64_t ld, int64_t n, int lower, int trans, const T *diag, T *B,
                                 int64_t ldb, int64_t m, bool exact) {
     cudaError_t e = c.ws.ensure(sizeof(int) * trsm_ws_ints(n, m));
     if (e != cudaSuccess) return e;
     return launch_status(trsm_launch<T>(M, ld, n, lower, trans, diag, B, ldb, m, exact, (int *)c.ws.p,
-                                        &dev_words(c)->err_word, c.stream));
+                                        &dev_words(c)->err_word, c.stream, nullptr, &dev_words(c)->factor));
 }
 
 template <typename T>
@@ -474,7 +468,9 @@ bool bad_view(const void *p, int64_t rows, int64_t cols) {
 // with mode `good` and the downloads; the outcome is read together with the
 // results, and only if it is not a success are they dropped and the rest done
 // step by step: a FAST outcome that the reference's arithmetic has to decide, and
-// a failure, which exports only the rows the reference would have written.
+// a failure, which exports only the rows the reference would have written.  The work
+// behind the factor looks at the verdict itself: if it is not a success, it has cost
+// its launches and the raw copies still hold the caller's values.
 // `then` enqueues the work behind a factor in W (again after an EXACT re-run) and
 // its downloads' first half; `keep` moves its results to the caller once they stand.
 template <typename T, typename Then, typename Keep>
@@ -487,25 +483,24 @@ int factor_export(Ctx *c, const View &v, T *W, const T *R, int64_t drs, int64_t 
     LLA_TRY_CUDA(reset_words(*c));
     LLA_TRY_CUDA(factor_enqueue<T>(*c, W, n, n, exact));
     LLA_TRY_CUDA(then());
-    LLA_TRY_CUDA(launch_status(export_launch<T>(W, n, (T *)c->raw_a.p, drs, dcs, n, n, good, -1, c->stream)));
+    LLA_TRY_CUDA(launch_status(export_launch<T>(W, n, (T *)c->raw_a.p, drs, dcs, n, n, good, -1, c->stream,
+                                                &dev_words(*c)->factor)));
     LLA_TRY_CUDA(begin_download(*c, v, c->raw_a, c->stage_a));
     LLA_TRY_CUDA(read_words(*c, w));
     if (w.factor_err == LLA_ERR_TIMEOUT) return lla__set_status(err, LLA_ERR_TIMEOUT);
-    if (w.info >= 0 || (!exact && fast_undecided(w))) {
-        // the raw copy has been written to: the caller's view still holds the original
-        LLA_TRY_CUDA(upload(*c, v, c->raw_a, c->stage_a, drs, dcs));
+    if (fast_undecided(w)) {  // (an EXACT factorisation leaves the ratio as it was set)
         if (!exact) {
             LLA_TRY_CUDA(launch_status(import_launch<T>(R, drs, dcs, n, n, W, n, c->stream)));
             LLA_TRY_CUDA(reset_words(*c));
             LLA_TRY_CUDA(factor_enqueue<T>(*c, W, n, n, true));
             LLA_TRY_CUDA(read_words(*c, w));
         }
-        failed = w.info >= 0;
+        const int64_t row = w.factor.info;
+        failed = row >= 0;
         if (!failed) LLA_TRY_CUDA(then());
         LLA_TRY_CUDA(launch_status(export_launch<T>(W, n, (T *)c->raw_a.p, drs, dcs, n, n,
-                                                    failed ? EXPORT_FAIL : good, w.info, c->stream)));
+                                                    failed ? EXPORT_FAIL : good, row, c->stream)));
         LLA_TRY_CUDA(begin_download(*c, v, c->raw_a, c->stage_a));
-        const int64_t row = w.info;
         LLA_TRY_CUDA(read_words(*c, w));
         if (failed) {
             LLA_TRY_CUDA(finish_download(*c, v, c->raw_a, c->stage_a));
@@ -592,15 +587,12 @@ int solvec_impl(T *a, int64_t rows, int64_t cols, int64_t rs, int64_t cs, T *b, 
     LLA_TRY_CUDA(upload(*c, vb, c->raw_b, c->stage_b, drs, dcs));
     LLA_TRY_CUDA(c->work_b.ensure(sizeof(T) * n * bcols));
     T *WB = (T *)c->work_b.p, *RB = (T *)c->raw_b.p;
-    bool again = false;
     auto then = [&]() -> cudaError_t {  // solve, export, first half of the download
-        cudaError_t e = cudaSuccess;
-        if (again) e = upload(*c, vb, c->raw_b, c->stage_b, drs, dcs);  // raw_b has been written to
-        again = true;
-        if (e == cudaSuccess) e = launch_status(import_launch<T>(RB, drs, dcs, n, bcols, WB, n, c->stream));
+        cudaError_t e = launch_status(import_launch<T>(RB, drs, dcs, n, bcols, WB, n, c->stream));
         if (e == cudaSuccess) e = cholesky_solve_work<T>(c, n, WB, bcols);
         if (e == cudaSuccess)
-            e = launch_status(export_launch<T>(WB, n, RB, drs, dcs, n, bcols, EXPORT_FULL, -1, c->stream));
+            e = launch_status(export_launch<T>(WB, n, RB, drs, dcs, n, bcols, EXPORT_FULL, -1, c->stream,
+                                               &dev_words(*c)->factor));
         return e == cudaSuccess ? begin_download(*c, vb, c->raw_b, c->stage_b) : e;
     };
     return factor_export<T>(c, va, W, R, ars, acs, EXPORT_LOWER, then,
@@ -648,8 +640,8 @@ int invc_impl(T *a, int64_t rows, int64_t cols, int64_t rs, int64_t cs, T *out, 
             if (e == cudaSuccess) e = launch_status(symmetrize_launch<T>(WB, n, n, c->stream));
         }
         if (e == cudaSuccess)
-            e = launch_status(
-                export_launch<T>(WB, n, (T *)c->raw_b.p, drs, dcs, n, n, EXPORT_FULL, -1, c->stream));
+            e = launch_status(export_launch<T>(WB, n, (T *)c->raw_b.p, drs, dcs, n, n, EXPORT_FULL, -1, c->stream,
+                                               &dev_words(*c)->factor));
         return e == cudaSuccess ? begin_download(*c, vo, c->raw_b, c->stage_b) : e;
     };
     bool failed = false;

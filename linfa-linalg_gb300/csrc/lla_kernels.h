@@ -23,14 +23,32 @@ template <typename T>
 int potrf_fast_launch(T *W, int64_t n, int64_t ld, int64_t *d_info, T *diag0, double *min_ratio,
                       int *err_word, int *sticky, cudaStream_t st);
 
+// What a host call's factorisation leaves on the device.  Work that is enqueued behind
+// it, before the outcome is known, takes a pointer to it and returns at once unless the
+// factor stands: a pivot was not positive, or (FAST) the smallest one, relative to A's
+// diagonal, is so small that the reference's own arithmetic has to decide.
+struct FactorVerdict {
+    int64_t info;
+    double min_ratio;
+};
+constexpr double kPivotGuard = 1e-10;
+#ifdef __CUDACC__
+__device__ __forceinline__ bool factor_stands(const FactorVerdict *v) {
+    // (the ratio is not negative, so its bits compare like it)
+    return *(volatile const int64_t *)&v->info < 0 &&
+           *(volatile const long long *)&v->min_ratio >= __double_as_longlong(kPivotGuard);
+}
+#endif
+
 // Triangular solve op(T) X = B in place (see lla_trsm.cu).  ws: trsm_ws_ints
 // ints of scratch; err_word: device int, 0 on entry; sticky (optional): a
 // device status word that also receives LLA_ERR_TIMEOUT and is never cleared
-// by the launch (the record that lla_device_status reads).
+// by the launch (the record that lla_device_status reads); behind (optional): the
+// factorisation that M comes from.
 template <typename T>
 int trsm_launch(const T *M, int64_t ld, int64_t n, int lower, int trans, const T *diag, T *B,
                 int64_t ldb, int64_t m, bool exact, int *ws, int *err_word, cudaStream_t st,
-                int *sticky = nullptr);
+                int *sticky = nullptr, const FactorVerdict *behind = nullptr);
 size_t trsm_ws_ints(int64_t n, int64_t m);
 
 // One system of a batched solve: order n, m right-hand sides, caller index,
@@ -84,10 +102,11 @@ template <typename T>
 int import_launch(const T *R, int64_t rs, int64_t cs, int64_t rows, int64_t cols, T *W, int64_t ld,
                   cudaStream_t st);
 // R[i*rs + j*cs] = W[i + j*ld] for the entries selected by mode (fail_row
-// for EXPORT_FAIL: rows < f with j <= i, and row f with j < f).
+// for EXPORT_FAIL: rows < f with j <= i, and row f with j < f); behind (optional):
+// nothing, unless that factorisation stands.
 template <typename T>
 int export_launch(const T *W, int64_t ld, T *R, int64_t rs, int64_t cs, int64_t rows, int64_t cols,
-                  int mode, int64_t fail_row, cudaStream_t st);
+                  int mode, int64_t fail_row, cudaStream_t st, const FactorVerdict *behind = nullptr);
 // Zero the strict upper (uplo = LOWER) or strict lower (uplo = UPPER) part of R.
 template <typename T>
 int mask_launch(T *R, int64_t rs, int64_t cs, int64_t n, int uplo, cudaStream_t st);

@@ -47,7 +47,9 @@ __device__ __forceinline__ bool export_selected(int mode, int64_t i, int64_t j, 
 
 template <typename T>
 __global__ void export_kernel(const T *__restrict__ W, int64_t ld, T *__restrict__ R, int64_t rs,
-                              int64_t cs, int64_t rows, int64_t cols, int mode, int64_t f) {
+                              int64_t cs, int64_t rows, int64_t cols, int mode, int64_t f,
+                              const FactorVerdict *behind) {
+    if (behind != nullptr && !factor_stands(behind)) return;
     __shared__ T tile[32][33];
     const int64_t i0 = (int64_t)blockIdx.x * 32, j0 = (int64_t)blockIdx.y * 32;
     const bool row_major = (cs == 1);
@@ -117,11 +119,11 @@ int import_launch(const T *R, int64_t rs, int64_t cs, int64_t rows, int64_t cols
 
 template <typename T>
 int export_launch(const T *W, int64_t ld, T *R, int64_t rs, int64_t cs, int64_t rows, int64_t cols,
-                  int mode, int64_t fail_row, cudaStream_t st) {
+                  int mode, int64_t fail_row, cudaStream_t st, const FactorVerdict *behind) {
     if (rows == 0 || cols == 0) return 0;
     LaunchScope ls(K_LAYOUT, st);
     export_kernel<T><<<tiles2d(rows, cols), dim3(32, 8), 0, st>>>(W, ld, R, rs, cs, rows, cols,
-                                                                  mode, fail_row);
+                                                                  mode, fail_row, behind);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
@@ -183,7 +185,7 @@ int symmetrize_launch(T *W, int64_t ld, int64_t n, cudaStream_t st) {
     template int import_launch<T>(const T *, int64_t, int64_t, int64_t, int64_t, T *, int64_t,   \
                                   cudaStream_t);                                                 \
     template int export_launch<T>(const T *, int64_t, T *, int64_t, int64_t, int64_t, int64_t,   \
-                                  int, int64_t, cudaStream_t);                                   \
+                                  int, int64_t, cudaStream_t, const FactorVerdict *);            \
     template int mask_launch<T>(T *, int64_t, int64_t, int64_t, int, cudaStream_t);              \
     template int is_triangular_launch<T>(const T *, int64_t, int64_t, int64_t, int, int *,       \
                                          cudaStream_t);                                          \

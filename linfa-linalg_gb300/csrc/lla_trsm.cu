@@ -108,7 +108,8 @@ __global__ void __launch_bounds__(kTrsmNb *kTrsmMaxMc) trsm_lookback(const T *__
                                                                    int lower, int trans, const T *__restrict__ diag,
                                                                    T *B, int64_t ldb, int64_t m, int mc, int n_chunks,
                                                                    int *ws, int *err_word, int *sticky,
-                                                                   long long spin_limit, int lose_first) {
+                                                                   long long spin_limit, int lose_first,
+                                                                   const FactorVerdict *behind) {
     using Ar = Arith<T>;
     __shared__ T ts[2][kTrsmNb][kTrsmNb + 1];  // coupling tiles, [term][row]
     __shared__ T td[kTrsmNb][kTrsmNb + 1];     // diagonal block, [term][row]
@@ -117,8 +118,10 @@ __global__ void __launch_bounds__(kTrsmNb *kTrsmMaxMc) trsm_lookback(const T *__
     const int tx = threadIdx.x, ty = threadIdx.y;
     const int tid = ty * kTrsmNb + tx, nthr = kTrsmNb * blockDim.y;
     int *counter = ws, *flags = ws + 1;
+    const bool go = behind == nullptr || factor_stands(behind);  // (the same for every CTA)
     if (tid == 0) s_ticket = atomicAdd(counter, 1);
     __syncthreads();
+    if (!go) return;
     // failure injection (tests only): the first item is lost -- never solved,
     // never published -- so every wait on it runs out
     if (lose_first && s_ticket == 0) return;
@@ -294,7 +297,7 @@ static TrsmWaitCfg take_wait_cfg() {
 template <typename T>
 int trsm_launch(const T *M, int64_t ld, int64_t n, int lower, int trans, const T *diag, T *B,
                 int64_t ldb, int64_t m, bool exact, int *ws, int *err_word, cudaStream_t st,
-                int *sticky) {
+                int *sticky, const FactorVerdict *behind) {
     if (n == 0 || m == 0) return 0;
     const int mc = (int)std::min<int64_t>(kTrsmMc, m);
     const int64_t chunks = ceil_div(m, mc);
@@ -308,11 +311,11 @@ int trsm_launch(const T *M, int64_t ld, int64_t n, int lower, int trans, const T
     if (exact)
         trsm_lookback<T, true><<<grid, block, 0, st>>>(M, ld, n, lower, trans, diag, B, ldb, m, mc,
                                                        (int)chunks, ws, err_word, sticky,
-                                                       wc.spin_limit, wc.lose_first);
+                                                       wc.spin_limit, wc.lose_first, behind);
     else
         trsm_lookback<T, false><<<grid, block, 0, st>>>(M, ld, n, lower, trans, diag, B, ldb, m,
                                                         mc, (int)chunks, ws, err_word, sticky,
-                                                        wc.spin_limit, wc.lose_first);
+                                                        wc.spin_limit, wc.lose_first, behind);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
@@ -322,10 +325,10 @@ size_t trsm_ws_ints(int64_t n, int64_t m) {
     return (size_t)(1 + ceil_div(n, kTrsmNb) * ceil_div(m, mc));
 }
 
-template int trsm_launch<double>(const double *, int64_t, int64_t, int, int, const double *,
-                                 double *, int64_t, int64_t, bool, int *, int *, cudaStream_t, int *);
-template int trsm_launch<float>(const float *, int64_t, int64_t, int, int, const float *, float *,
-                                int64_t, int64_t, bool, int *, int *, cudaStream_t, int *);
+template int trsm_launch<double>(const double *, int64_t, int64_t, int, int, const double *, double *, int64_t,
+                                 int64_t, bool, int *, int *, cudaStream_t, int *, const FactorVerdict *);
+template int trsm_launch<float>(const float *, int64_t, int64_t, int, int, const float *, float *, int64_t,
+                                int64_t, bool, int *, int *, cudaStream_t, int *, const FactorVerdict *);
 
 }  // namespace lla
 
@@ -421,11 +424,11 @@ extern "C" int lla_dtrsm_device_noalloc(const double *dL, int64_t n, int64_t ld,
         if (algo == LLA_ALGO_EXACT)
             trsm_lookback<double, true><<<grid, block, 0, st>>>(
                 dL, ld, n, lower, trans ? 1 : 0, nullptr, dB, ldb, m, mc, (int)chunks, scratch, err_word,
-                scratch + kNoAllocStatus, wc.spin_limit, wc.lose_first);
+                scratch + kNoAllocStatus, wc.spin_limit, wc.lose_first, nullptr);
         else
             trsm_lookback<double, false><<<grid, block, 0, st>>>(
                 dL, ld, n, lower, trans ? 1 : 0, nullptr, dB, ldb, m, mc, (int)chunks, scratch, err_word,
-                scratch + kNoAllocStatus, wc.spin_limit, wc.lose_first);
+                scratch + kNoAllocStatus, wc.spin_limit, wc.lose_first, nullptr);
     }
     e = cudaGetLastError();
     if (e != cudaSuccess) return lla__set_cuda_error(err, e);
