@@ -1096,6 +1096,11 @@ struct lla_batch_plan {
     cudaStream_t g_stream = nullptr;
 };
 
+// Generation of the batched kernels, part of the cache's keys: a shape that was measured
+// with other kernels says nothing about these.  Raised with every change that moves
+// their best shape.
+constexpr int kBatchGeneration = 2;
+
 static size_t batch_smem(int dtype) { return dtype == 8 ? sizeof(BatchSmem<double>) : sizeof(BatchSmem<float>); }
 
 static bool cache_lookup(const std::string &key, int &cps, int &thr) { return lla::autotune_lookup(key, cps, thr); }
@@ -1189,10 +1194,11 @@ int lla_batch_plan_create(int64_t count, const int32_t *n, const int32_t *m, int
         const double ca = (double)a.n * a.n * (a.n + 6.0 * a.m), cb = (double)b.n * b.n * (b.n + 6.0 * b.m);
         return ca > cb;
     });
-    // autotune-cache key: element size, count, size-bucket histogram, widest RHS
+    // autotune-cache key: the kernels' generation, element size, count, size-bucket histogram,
+    // widest RHS
     char key[256];
-    std::snprintf(key, sizeof(key), "b%d:c%lld:h%d-%d-%d-%d-%d-%d-%d-%d-%d:m%d", elem_bytes,
-                  (long long)count, hist[0], hist[1], hist[2], hist[3], hist[4], hist[5], hist[6],
+    std::snprintf(key, sizeof(key), "k%d:b%d:c%lld:h%d-%d-%d-%d-%d-%d-%d-%d-%d:m%d",
+                  kBatchGeneration, elem_bytes, (long long)count, hist[0], hist[1], hist[2], hist[3], hist[4], hist[5], hist[6],
                   hist[7], hist[8], maxm);
     p->key = key;
     int cps, thr;

@@ -50,6 +50,26 @@ def on_device(lib, dev, fn):
     return out[0]
 
 
+def _plan(lib, refined=False):
+    n, m = np.full(40, 16, np.int32), np.ones(40, np.int32)
+    plan = P()
+    assert lib.lla_batch_plan_create(I64(40), P(n.ctypes.data), P(m.ctypes.data), 8, ctypes.byref(plan), None) == 0
+    if refined:
+        assert lib.lla_batch_set_refined(plan, 1, None) == 0
+    return plan
+
+
+def _shape(lib, plan):
+    c, t = ctypes.c_int(), ctypes.c_int()
+    assert lib.lla_batch_plan_info(plan, None, None, None, None, ctypes.byref(c), ctypes.byref(t), None) == 0
+    return c.value, t.value
+
+
+def _autotune(lib, plan):
+    a, b, info = np.zeros((40, 256)), np.zeros((40, 16)), np.zeros(40, np.int32)
+    assert lib.lla_batch_autotune(plan, P(a.ctypes.data), P(b.ctypes.data), P(info.ctypes.data), None, None, None) == 0
+
+
 I64, P = ctypes.c_int64, ctypes.c_void_p
 
 
@@ -136,3 +156,13 @@ def test_a_captured_factor_allocates_beside_the_graph(fake, dtype):
         return True
 
     assert on_device(fake, 0, body)
+
+
+def test_shapes_tuned_for_other_kernels_are_not_taken(fake, own_cache):
+    """Cache entries without this generation's mark leave the default shape; its own are taken up."""
+    key = "b8:c40:h40-0-0-0-0-0-0-0-0:m1"
+    own_cache.write_text(f"{key} 2 256\nk1:{key} 2 256\n{key}:r 1 128\n")
+    assert _shape(fake, _plan(fake)) == (4, 128) and _shape(fake, _plan(fake, True)) == (2, 256)
+    tuned = _plan(fake)
+    _autotune(fake, tuned)  # (every candidate takes the same time here: the first stays)
+    assert _shape(fake, tuned) == (1, 256) == _shape(fake, _plan(fake))
