@@ -1086,7 +1086,7 @@ struct lla_batch_plan {
     BatchItem *d_items = nullptr;
     int *d_counter = nullptr;
     int ctas_per_sm = 4, threads = 128;  // four latency chains a SM; measured best or equal at every order
-    bool tuned = false;     // the shape comes from the cache, the autotuner or the caller
+    bool by_caller = false;  // the caller set the shape (kept when the mode changes, as a tuned one is not)
     bool refined = false;   // f64 systems through an FP32 factor + FP64 refinement (A read only)
     char *d_scratch = nullptr;  // per-CTA scratch of the refined mode
     std::string key;
@@ -1205,7 +1205,6 @@ int lla_batch_plan_create(int64_t count, const int32_t *n, const int32_t *m, int
     if (cache_lookup(p->key, cps, thr)) {
         p->ctas_per_sm = cps;
         p->threads = thr;
-        p->tuned = true;
     }
     cudaError_t e = cudaMalloc(&p->d_items, sizeof(BatchItem) * std::max<int64_t>(1, count));
     if (e == cudaSuccess) e = cudaMalloc(&p->d_counter, sizeof(int));
@@ -1248,18 +1247,21 @@ int lla_batch_plan_info(const lla_batch_plan *p, int64_t *a_elems, int64_t *b_el
     return LLA_OK;
 }
 
+static void apply_shape(lla_batch_plan *p, int ctas_per_sm, int threads) {
+    if (p->ctas_per_sm == ctas_per_sm && p->threads == threads) return;
+    p->ctas_per_sm = ctas_per_sm;
+    p->threads = threads;
+    if (p->gexec) {
+        cudaGraphExecDestroy(p->gexec);
+        p->gexec = nullptr;
+    }
+}
+
 int lla_batch_set_shape(lla_batch_plan *p, int ctas_per_sm, int threads) {
     if (!p || ctas_per_sm < 1 || ctas_per_sm > 8 || (threads != 128 && threads != 256))
         return LLA_ERR_INVALID_ARG;
-    p->tuned = true;
-    if (p->ctas_per_sm != ctas_per_sm || p->threads != threads) {
-        p->ctas_per_sm = ctas_per_sm;
-        p->threads = threads;
-        if (p->gexec) {
-            cudaGraphExecDestroy(p->gexec);
-            p->gexec = nullptr;
-        }
-    }
+    p->by_caller = true;
+    apply_shape(p, ctas_per_sm, threads);
     return LLA_OK;
 }
 
@@ -1291,7 +1293,7 @@ int lla_batch_set_refined(lla_batch_plan *p, int refined, lla_error *err) {
         if (cache_lookup(p->key, cps, thr)) {
             p->ctas_per_sm = cps;
             p->threads = thr;
-        } else if (!p->tuned) {  // two CTAs of the refined kernel fit an SM
+        } else if (!p->by_caller) {  // two CTAs of the refined kernel fit an SM
             p->ctas_per_sm = want ? 2 : 4;
             p->threads = want ? 256 : 128;
         }
@@ -1424,9 +1426,8 @@ int lla_batch_autotune(lla_batch_plan *p, void *dA, void *dB, int32_t *d_info, v
     if (e1) cudaEventDestroy(e1);
     cudaFree(a0);
     cudaFree(b0);
-    lla_batch_set_shape(p, best_c, best_t);
+    apply_shape(p, best_c, best_t);
     if (e != cudaSuccess) return lla__set_cuda_error(err, e);
-    p->tuned = true;
     cache_store(p->key, best_c, best_t);
     if (best_ms) *best_ms = best;
     return LLA_OK;

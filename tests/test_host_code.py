@@ -166,3 +166,17 @@ def test_shapes_tuned_for_other_kernels_are_not_taken(fake, own_cache):
     tuned = _plan(fake)
     _autotune(fake, tuned)  # (every candidate takes the same time here: the first stays)
     assert _shape(fake, tuned) == (1, 256) == _shape(fake, _plan(fake))
+
+
+def test_a_shape_tuned_for_one_mode_stays_with_it(fake):
+    """Switching the mode takes that mode's tuned shape or its default, not the other mode's; a
+    shape that the caller set stays."""
+    plan = _plan(fake)
+    _autotune(fake, plan)
+    assert _shape(fake, plan) == (1, 256)
+    assert fake.lla_batch_set_refined(plan, 1, None) == 0 and _shape(fake, plan) == (2, 256)
+    assert fake.lla_batch_set_refined(plan, 0, None) == 0 and _shape(fake, plan) == (1, 256)
+    assert _shape(fake, _plan(fake, True)) == (2, 256)  # a plan that found the plain shape in the cache
+    own = _plan(fake)
+    assert fake.lla_batch_set_shape(own, 3, 128) == 0
+    assert fake.lla_batch_set_refined(own, 1, None) == 0 and _shape(fake, own) == (3, 128)
