@@ -739,6 +739,27 @@ __device__ __forceinline__ float fu_subtract(float w, long long T, int s) {
     return w - (fits ? t * __int_as_float((s + 127) << 23) : scalbnf(t, s));
 }
 
+// By the whole CTA, once a bounded wait has run out, instead of the rest of the kernel:
+// reports it, lets the copies and MMAs in flight end and frees the tensor memory.
+__device__ __forceinline__ void fu_give_up(uint32_t fullA0, uint32_t fullB0, const uint32_t *copied, const uint64_t *drain,
+                                        uint32_t tmem, int *err_word, int *sticky) {
+    const int tid = threadIdx.x;
+    if (tid == 0) {
+        atomicCAS(err_word, 0, (int)LLA_ERR_TIMEOUT);
+        if (sticky) atomicCAS(sticky, 0, (int)LLA_ERR_TIMEOUT);
+    } else if (tid == kFuEpi) {
+        ring_drain(fullA0, copied[0], kFuRing);
+        ring_drain(fullB0, copied[1], 2);
+    } else if (tid == kFuEpi + 32) {
+        tc_drain(smem_u32(drain));
+    }
+    __syncwarp();
+    __syncthreads();
+    tc_fence_after();
+    if (tid < 32)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kFuTmem) : "memory");
+}
+
 template <typename T>
 __global__ void __launch_bounds__(kFuThreads, 1) fc_update_kernel(
     const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, T *W, int64_t ld,
@@ -747,6 +768,8 @@ __global__ void __launch_bounds__(kFuThreads, 1) fc_update_kernel(
     constexpr int ND = Fc<T>::kDigits, SETS = kFuSets<T>, BSET = kFuBSet<T>;
     extern __shared__ uint8_t smem_raw[];
     __shared__ int s_abort, s_skip;
+    __shared__ __align__(8) uint64_t s_drain;
+    __shared__ uint32_t s_copied[2];  // planes of rows and of columns that the producer copied
     uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint8_t *sA = smem;
     uint8_t *sB = smem + kFuRing * kFuATile;
@@ -769,6 +792,7 @@ __global__ void __launch_bounds__(kFuThreads, 1) fc_update_kernel(
             mbar_init(tfull + 8 * s, 1);
             mbar_init(tempty + 8 * s, kFuEpi);
         }
+        mbar_init(smem_u32(&s_drain), 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         s_abort = 0;
     }
@@ -827,6 +851,8 @@ __global__ void __launch_bounds__(kFuThreads, 1) fc_update_kernel(
                     }
                 }
             }
+            s_copied[0] = ga;
+            s_copied[1] = gb;
         }
     } else if (warp == kFuEpi / 32 + 1) {
         if (lane == 0) {  // MMA issuer
@@ -955,9 +981,9 @@ __global__ void __launch_bounds__(kFuThreads, 1) fc_update_kernel(
     }
     __syncwarp();
     __syncthreads();
-    if (s_abort && tid == 0) {
-        atomicCAS(err_word, 0, (int)LLA_ERR_TIMEOUT);
-        if (sticky) atomicCAS(sticky, 0, (int)LLA_ERR_TIMEOUT);
+    if (s_abort) {
+        fu_give_up(fullA0, fullB0, s_copied, &s_drain, tmem, err_word, sticky);
+        return;
     }
     tc_fence_after();
     if (warp == 0)
@@ -969,7 +995,7 @@ __global__ void __launch_bounds__(kFuThreads, 1) fc_update_kernel(
     // has read its stages: the epilogue waited for the last one), while the other CTAs go on.  As a
     // kernel of its own between update and panel it left the other SMs idle (f64 n = 8192 15.0 ->
     // 13.6 ms, n = 2048 2.24 -> 2.22; f32 n = 6001 4.26 -> 3.73 ms).
-    if (blockIdx.x == 0 && tid < kFcDiagThreads && !s_abort)
+    if (blockIdx.x == 0 && tid < kFcDiagThreads)
         fc_diag_block(*reinterpret_cast<FcDiagSmem<T> *>(smem), W, ld, q, (int)min((int64_t)kFcNb, n - q), diag0, rinv,
                       info, min_ratio);
 }

@@ -220,6 +220,7 @@ __global__ void __launch_bounds__(kOzThreads, 1) oz_residual_kernel(
     if (refine_done(state)) return;
     extern __shared__ uint8_t smem_raw[];
     __shared__ int s_abort;
+    __shared__ __align__(8) uint64_t s_drain;
     uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint8_t *sA = smem;                              // kOzAStages x 16 KiB
     uint8_t *sX = smem + kOzAStages * kOzATile;      // 2 x 64 KiB
@@ -244,6 +245,7 @@ __global__ void __launch_bounds__(kOzThreads, 1) oz_residual_kernel(
         }
         mbar_init(tfull, 1);
         for (int h = 0; h < 2; ++h) mbar_init(tempty0 + 8 * h, 256);
+        mbar_init(smem_u32(&s_drain), 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         s_abort = 0;
     }
@@ -261,10 +263,11 @@ __global__ void __launch_bounds__(kOzThreads, 1) oz_residual_kernel(
     // instruction descriptor without N: D F32, A/B BF16, K-major, M = 128
     const uint32_t idesc0 = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kOzM >> 4) << 24);
 
+    int64_t ga = 0;  // A planes and chunks so far, copied or multiplied
+    int j = 0;
     if (warp == 8) {
         if (lane == 0) {  // TMA producer
-            int64_t ga = 0;
-            for (int kc = kc_beg, j = 0; kc < kc_end && !*(volatile int *)&s_abort; ++kc, ++j) {
+            for (int kc = kc_beg; kc < kc_end && !*(volatile int *)&s_abort; ++kc, ++j) {
                 const int xb = j & 1, use = j >> 1;
                 if (use > 0 && !mbar_wait(emptyX0 + 8 * xb, (uint32_t)((use - 1) & 1), err_word)) {
                     s_abort = 1;
@@ -286,9 +289,8 @@ __global__ void __launch_bounds__(kOzThreads, 1) oz_residual_kernel(
         }
     } else if (warp == 9) {
         if (lane == 0) {  // MMA issuer
-            int64_t ga = 0;
             int win = 0;
-            for (int kc = kc_beg, j = 0; kc < kc_end && !*(volatile int *)&s_abort; ++kc, ++j) {
+            for (int kc = kc_beg; kc < kc_end && !*(volatile int *)&s_abort; ++kc, ++j) {
                 const int xb = j & 1, use = j >> 1;
                 const bool wstart = (j % kOzWin) == 0;
                 if (!mbar_wait(fullX0 + 8 * xb, (uint32_t)(use & 1), err_word)) {
@@ -386,7 +388,17 @@ __global__ void __launch_bounds__(kOzThreads, 1) oz_residual_kernel(
     }
     __syncwarp();
     __syncthreads();
-    if (s_abort && tid == 0) atomicCAS(err_word, 0, (int)LLA_ERR_TIMEOUT);
+    if (s_abort) {
+        if (tid == 0) {
+            atomicCAS(err_word, 0, (int)LLA_ERR_TIMEOUT);
+        } else if (tid == 8 * 32) {
+            ring_drain(fullA0, (uint64_t)ga, kOzAStages);
+            ring_drain(fullX0, (uint64_t)j, 2);
+        } else if (tid == 9 * 32) {
+            tc_drain(smem_u32(&s_drain));
+        }
+        __syncthreads();
+    }
     tc_fence_after();
     if (warp == 0)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kOzCols)

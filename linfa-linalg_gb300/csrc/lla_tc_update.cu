@@ -135,6 +135,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_update_kernel(
     extern __shared__ uint8_t smem_raw[];
     __shared__ int s_abort, s_skip, s_epi_abort, s_epi_tile;
     __shared__ int s_tile[kTcTileRing];
+    __shared__ __align__(8) uint64_t s_drain;
     __shared__ __align__(8) uint64_t s_tbar[2 * kTcTileRing];  // tile ring: full[R], empty[R]
     uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     constexpr int kTile = tc_tile_bytes<KC>();
@@ -166,6 +167,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_update_kernel(
             mbar_init(rempty0 + 8 * r, EPI_TMA ? 2 : 9);
         }
         mbar_init(cfull, 1);
+        mbar_init(smem_u32(&s_drain), 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         s_abort = 0;
         s_epi_abort = 0;
@@ -195,9 +197,9 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_update_kernel(
         return;  // the launch is void (a failed or timed-out factorisation): its claims do not matter
     }
 
+    int64_t g = 0;  // K-chunks so far, copied or multiplied
     if (warp == 8) {
         if (lane == 0) {  // tile claims and TMA producer
-            int64_t g = 0;
             // one claim ahead: the next tile is claimed while this one's chunks load
             int64_t t_next = (int64_t)(atomicAdd(sched, 1u) - sched_base);
             for (int64_t lt = 0; !*(volatile int *)&s_abort; ++lt) {
@@ -230,7 +232,6 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_update_kernel(
         }
     } else if (warp == 9) {
         if (lane == 0) {  // MMA issuer
-            int64_t g = 0;
             for (int64_t lt = 0; !*(volatile int *)&s_abort; ++lt) {
                 const int slot = (int)(lt % kTcTileRing);
                 if (!mbar_wait(rfull0 + 8 * slot, (uint32_t)((lt / kTcTileRing) & 1), err_word)) {
@@ -431,7 +432,15 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_update_kernel(
     }
     __syncwarp();
     __syncthreads();
-    if (s_abort && tid == 0) atomicCAS(err_word, 0, (int)LLA_ERR_TIMEOUT);
+    if (s_abort) {
+        if (tid == 0)
+            atomicCAS(err_word, 0, (int)LLA_ERR_TIMEOUT);
+        else if (tid == 8 * 32)
+            ring_drain(full0, (uint64_t)g, (uint32_t)S);
+        else if (tid == 9 * 32)
+            tc_drain(smem_u32(&s_drain));
+        __syncthreads();
+    }
     tc_fence_after();
     if (warp == 0)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTcAlloc)

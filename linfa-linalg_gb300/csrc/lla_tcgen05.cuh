@@ -8,6 +8,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "lla_ring.h"
+
 namespace lla {
 
 constexpr long long kTcSpin = 1ll << 22;  // polls per bounded mbarrier wait
@@ -108,6 +110,27 @@ __device__ __forceinline__ void tc_mma(uint32_t dtmem, uint64_t adesc, uint64_t 
 __device__ __forceinline__ void tc_commit(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
                  : "memory");
+}
+
+// A kernel that gives up leaves nothing in flight behind: no copy that lands in shared
+// memory, and no MMA that writes tensor memory, after its CTA has gone.  Both waits
+// are bounded.
+//
+// By the thread that issued a ring's copies: those that have not landed yet.
+__device__ __forceinline__ void ring_drain(uint32_t full0, uint64_t issued, uint32_t stages) {
+#pragma unroll 1
+    for (uint32_t s = 0; s < stages; ++s) {
+        uint32_t parity;
+        if (!ring_last_phase(issued, stages, s, parity)) return;
+#pragma unroll 1
+        for (long long i = 0; i < kTcSpin && !mbar_try_wait(full0 + 8 * s, parity); ++i) {}
+    }
+}
+
+// By the thread that issued the MMAs; bar: a fresh barrier of count 1.
+__device__ __forceinline__ void tc_drain(uint32_t bar) {
+    tc_commit(bar);
+    for (long long i = 0; i < kTcSpin && !mbar_try_wait(bar, 0); ++i) {}
 }
 
 // 8 consecutive columns of one lane (32x32b shape, x8): no wait; pair with tc_wait_ld.
