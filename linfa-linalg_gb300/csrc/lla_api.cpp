@@ -793,7 +793,7 @@ int orthonormalize_impl(const T *v, int64_t rows, int64_t cols, int64_t rs, int6
     LLA_TRY_CUDA(launch_status(export_launch<T>(G, k, (T *)c->raw_c.p, lrs_d, lcs_d, k, k, EXPORT_LOWER_ZERO_UPPER,
                                                 -1, c->stream)));
     if (n > 0) {
-        if (k <= kSolveRowsMax) {  // U = V L^-T row by row, where V lies
+        if (solve_rows_pays<T>(n, k)) {  // U = V L^-T row by row, where V lies
             LLA_TRY_CUDA(launch_status(solve_rows_launch<T>(G, k, k, WV, n, n, use_exact(k), c->stream)));
         } else {  // V^T (k x n), L Z = V^T, U = Z^T
             LLA_TRY_CUDA(c->lob_t.ensure(sizeof(T) * k * n));

@@ -131,8 +131,19 @@ size_t atb_ws_elems(int64_t n, int64_t ka, int64_t kb);
 template <typename T>
 int atb_launch(const T *A, int64_t lda, const T *B, int64_t ldb, int64_t n, int64_t ka, int64_t kb, T *C,
                int64_t ldc, T *P, int symmetric, cudaStream_t st);
-// X (n x k) <- X L^-T, one row of X a thread (k <= kSolveRowsMax, n >= 2 k rows pay).
+// X (n x k) <- X L^-T, one row of X a thread; k <= kSolveRowsMax (the factor and 64 rows in
+// FP64 fill the 48 KiB of shared memory that a launch has without asking).
 constexpr int64_t kSolveRowsMax = 48;
+// Whether that beats the substitution kernel on X^T with its two transpositions.  A row is
+// a chain of k (k - 1) / 2 FP64 instructions of 64 cycles however few rows there are, so wide
+// short blocks are better off there.  Measured, a whole Cholesky-QR call, rows against
+// substitution: f64 k = 24, n = 200 155 us, 161; k = 32, n = 600 200, 185, n = 3000 208, 214;
+// k = 48, n = 600 342, 282, n = 3000 352, 343, n = 6000 359, 383; f32 k = 48, n = 600 172, 171,
+// and rows ahead everywhere else (k = 48, n = 200 157, 164).
+template <typename T>
+inline bool solve_rows_pays(int64_t n, int64_t k) {
+    return k <= kSolveRowsMax && (sizeof(T) == 4 || k <= 24 || n >= 80 * k);
+}
 template <typename T>
 int solve_rows_launch(const T *L, int64_t ldl, int64_t k, T *X, int64_t ldx, int64_t n, bool exact, cudaStream_t st);
 // V (n x k) -= Y (n x ky) U (ky x k).

@@ -180,3 +180,21 @@ def test_a_shape_tuned_for_one_mode_stays_with_it(fake):
     own = _plan(fake)
     assert fake.lla_batch_set_shape(own, 3, 128) == 0
     assert fake.lla_batch_set_refined(own, 1, None) == 0 and _shape(fake, own) == (3, 128)
+
+
+@pytest.mark.parametrize("dtype,n,k,rows", [
+    (np.float64, 100, 24, True), (np.float64, 600, 32, False), (np.float64, 2559, 32, False), (np.float64, 2560, 32, True),
+    (np.float64, 3839, 48, False), (np.float64, 3840, 48, True), (np.float64, 60000, 49, False),
+    (np.float32, 100, 48, True), (np.float32, 60000, 49, False)])
+def test_cholesky_qr_rows_or_substitution(fake, dtype, n, k, rows):
+    """Short blocks of many FP64 columns go through the substitution kernel."""
+    v, u, low = np.zeros((n, k), dtype), np.zeros((n, k), dtype), np.zeros((k, k), dtype)
+    fn = fake.lla_dorthonormalize if dtype == np.float64 else fake.lla_sorthonormalize
+
+    def body():
+        fake.fake_clear()
+        views = [x for m in (v, u, low) for x in (P(m.ctypes.data), I64(len(m)), I64(k), I64(k), I64(1))]
+        return fn(*views, None)
+
+    assert on_device(fake, 0, body) == 0
+    assert bool(_launches(fake, 0, "solve_rows_kernel")) == rows and bool(_launches(fake, 0, "trsm_lookback")) != rows
