@@ -1,5 +1,6 @@
-"""FP32 diagonal blocks on matrices that are hard on the pivots: nearly collinear
-neighbouring columns, values near the ends of the exponent range, against the bound of a column-by-column factor."""
+"""FAST, batched and mixed factors on matrices that are hard on them -- nearly collinear
+neighbouring columns, values near the ends of the exponent range, rows whose entries differ
+by orders of magnitude -- against the entrywise bound of a column-by-column factor."""
 import numpy as np
 import pytest
 
@@ -30,8 +31,8 @@ def _factor(gpu_lla, path, a):
     torch = _torch()
     n = len(a)
     if path == "batch":
-        plan = gpu_lla.BatchPlan(np.array([n], np.int32), np.array([1], np.int32), "f32")
-        ap, bp = plan.pack([a], [np.ones((n, 1), np.float32)])
+        plan = gpu_lla.BatchPlan(np.array([n], np.int32), np.array([1], np.int32), "f32" if a.dtype == np.float32 else "f64")
+        ap, bp = plan.pack([a], [np.ones((n, 1), a.dtype)])
         A, B = torch.from_numpy(ap.copy()).cuda(), torch.from_numpy(bp.copy()).cuda()
         info = torch.empty(1, dtype=torch.int32, device="cuda")
         plan.solve(A, B, info)
@@ -78,3 +79,27 @@ def test_pivots_near_the_ends_of_the_range(gpu_lla, path, n, scale):
     low = np.tril(fac).astype(np.float64)
     err = np.abs(low @ low.T - a) / scale
     assert err.max() <= (8 + n / 8) * np.finfo(np.float32).eps, err.max()
+
+
+@pytest.mark.parametrize("path,n", [("device", 65), ("device", 192), ("device", 500), ("batch", 33), ("batch", 200), ("batch", 256)])
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("groups", [2, 5])
+def test_weakly_coupled_interleaved_groups(gpu_lla, path, n, dtype, groups):
+    """Rows large in the columns of their own group and small in the others', which alternate, under a
+    diagonal scaling over six orders: the digits of a row hold its entries to a fraction of the
+    row's largest, so the bound is against sqrt(a_ii a_jj), as it is for FMAs, and no entry's own
+    relative accuracy is promised."""
+    rng = np.random.default_rng(n + groups)
+    g = rng.standard_normal((n, 2 * n))
+    own = (np.arange(n) % groups)[:, None] == (np.arange(2 * n) % groups)[None, :]
+    g = np.where(own, g, g * (1e-6 if dtype == np.float64 else 1e-3))
+    g /= np.sqrt((g * g).sum(1))[:, None]
+    d = 10.0 ** rng.uniform(-3, 3, n)
+    a = ((g @ g.T) * d[:, None] * d[None, :]).astype(dtype)
+    a = np.tril(a) + np.tril(a, -1).T
+    fac, info = _factor(gpu_lla, path, a)
+    assert info == -1
+    low = np.tril(fac).astype(np.longdouble)
+    scale = np.sqrt(np.diag(a).astype(np.float64))
+    err = np.abs((low @ low.T - a).astype(np.float64)) / scale[:, None] / scale[None, :]
+    assert err.max() <= (8 + n / 8) * np.finfo(dtype).eps, err.max()
