@@ -17,9 +17,9 @@
 //     block, one thread per remaining column after it.
 // A small system is a chain of latencies, so four CTAs of 128 threads share an SM
 // by default; a large FP64 one is bound by the FP64 pipe and the digits' integer
-// work.  10,000 systems of n 16-256 (before: one-warp diagonal blocks with library
-// divisions, FP64 updates on the FP64 pipe, two substitution passes): f64 20.1 ->
-// 5.8 ms, f32 5.4 -> 1.2 ms; 3,000 of n 16-64 1.60 -> 0.33 and 0.46 -> 0.13 ms.
+// work.  10,000 systems of n 16-256: f64 5.8 ms, f32 1.2 ms; 3,000 of n 16-64: 0.33
+// and 0.13 ms.  (One-warp diagonal blocks with library divisions, FP64 updates on the
+// FP64 pipe and two substitution passes: 20.1, 5.4, 1.60 and 0.46 ms.)
 // A non-positive pivot stops that system only: info[i] = first failing row
 // (-1 when the system solved).  The (CTAs per SM, threads) shape is chosen per
 // batch by lla_batch_autotune and cached on disk.
@@ -186,7 +186,7 @@ __device__ void batch_diag(BatchSmem<T> &sm, int kb) {
 // shared memory (the panel's space), every thread forms their pivots itself
 // (lla_pivot_pair.cuh), and the next pair is brought up to date and stored before the
 // columns right of it: one exchange and no shuffle on a pair's chain (10,000 systems
-// of n 16-256: 1.23 -> 1.12 ms against batch_diag).
+// of n 16-256: 1.12 ms in the kernel, 1.23 with batch_diag).
 __device__ bool batch_diag_quick(BatchSmem<float> &sm, int kb) {
     constexpr int DS = BatchSmem<float>::kBDs;
     const int tid = threadIdx.x;

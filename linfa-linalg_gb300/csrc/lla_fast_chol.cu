@@ -26,10 +26,11 @@
 // with the first panel alone (K = 64), then one update with both (K = 128) covers
 // the rest, so the trailing matrix is read and written once per 128 columns.
 //
-// Measured, FMA updates before -> now (error against 64 bits the same or lower):
-// f64 n = 8192 220 -> 12.3 ms, n = 2048 14.4 -> 2.0 ms; f32 n = 6001 14.6 ->
-// 2.8 ms.  There is no size at which the FMA form is faster: one 64 x 64 tile of
-// the FP64 one took 70 us on its SM.
+// Measured against updates by FMAs (error against 64 bits the same or lower over
+// matrices of that kind; not so for single small entries, include/lla_gb300.h):
+// f64 n = 8192 12.3 ms, 220 by FMAs, n = 2048 2.0 and 14.4; f32 n = 6001 2.8 and
+// 14.6.  There is no size at which FMAs are faster: one 64 x 64 tile in FP64 takes
+// them 70 us on its SM.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -113,7 +114,8 @@ __device__ __forceinline__ void atomic_min_pos_f64(double *addr, double v) {
 // the other three sub-partitions keep the rest in registers, in patches of 16
 // rows x 2 columns (one FP64 instruction per column applied), and hand pair
 // k + 2 to warp 0 through shared memory once pair k is in it.  One barrier per
-// pair.  160 -> 31 us a block (FP32, where fc_diag_quick cannot take it, 67 -> 13 us).
+// pair.  31 us a block (one warp for the chain and its columns alike: 160); FP32, where
+// fc_diag_quick cannot take it, 13.
 constexpr int kFcDiagThreads = 512;
 constexpr int kFcPatches = 80, kFcPatchWarps = 12, kFcSlots = 7;
 
@@ -230,7 +232,7 @@ __device__ __forceinline__ void fc_diag_sync() {
 // a warp), a pair of columns a step goes through shared memory, every thread forms
 // its pivots itself (lla_pivot_pair.cuh), and the next pair is brought up to date and
 // stored before the columns right of it.  No shuffle, one barrier a pair (of warps
-// 0 .. 7).  The factor of n = 6001: 3.12 -> 2.80 ms, of n = 1100 0.49 -> 0.40.
+// 0 .. 7).  The factor of n = 6001 takes 2.8 ms, 3.1 with the general form's shuffles.
 __device__ __forceinline__ void fc_diag_quick(FcDiagSmem<float> &sm) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, lr = 2 * lane, lc = 8 * warp;
     if (warp >= 8) return;
@@ -515,13 +517,12 @@ __device__ __forceinline__ void fc_half_product(double (*l11)[kFcNb], double (*x
 // 8 (w % 2) .., column quads w / 2 + 4 s).  Quads are finished in turn: their two
 // owners solve the four columns by shuffles and publish them, one barrier, every
 // warp applies them to its quads right of them; the next owners update and solve
-// their own quad before the others.  What bounds it is that chain: with pairs of
-// columns, twice the barriers and exchanges, n = 2048 took 21 us a panel in FP64
-// and 13 in FP32 (n = 6001), now 16 and 8; the loads, all in flight at once, take
-// 1.5 of them, 2 before.  In FP64 the pipe bounds a panel with more than one CTA an
-// SM, so the right half takes the left half's columns from the tensor cores instead
-// of by substitution, which halves the FP64 instructions.  n = 8192: 172 us a panel
-// on average at first, 32 with pairs by substitution alone, 27 in halves, now 24.
+// their own quad before the others.  What bounds it is that chain: 16 us a
+// panel of FP64 at n = 2048 and 8 of FP32 at n = 6001, against 21 and 13 by pairs of
+// columns, with twice the barriers and exchanges.  In FP64 the pipe bounds a panel
+// with more than one CTA an SM, so the right half takes the left half's columns from
+// the tensor cores instead of by substitution, which halves the FP64 instructions
+// (by pairs, n = 8192: 27 us a panel on average, 32 with substitution alone; by quads 24).
 // second: the pair of panels' second one -- the rows' first-panel entries are read
 // back and the digits of all 128 columns are formed with a common exponent.
 constexpr int kFcRows = 16;
@@ -686,9 +687,10 @@ __global__ void __launch_bounds__(kFcPanelThreads) fc_panel_kernel(T *W, int64_t
 // accumulators, one per level s + t (7 x 64 = 448 TMEM columns).  Sixteen warps
 // then read the levels, combine them in 64-bit integers, release the tensor
 // memory and subtract from W while the next tile's MMAs run.
-// Bound by the tensor pipe (28 products) and the digit planes' L2 traffic
-// (336 KB a tile); the FP64 pipe sees one add per entry.  n = 8192: 1403 -> 55 us
-// a panel on average.
+// Bound by the tensor pipe (28 products), which is 41% busy at n = 8192 because the
+// next tile's MMAs wait for the epilogue to have read all levels, and the digit
+// planes' L2 traffic (336 KB a tile); the FP64 pipe sees one add per entry.  n = 8192:
+// 55 us a panel on average, by FMAs 1403.
 constexpr int kFuM = 128, kFuN = 64, kFuK = 64;
 constexpr int kFuRing = 6;                         // stages of one row plane
 constexpr int kFuATile = kFuM * kFuK * 2;          // 16 KiB
@@ -993,8 +995,8 @@ __global__ void __launch_bounds__(kFuThreads, 1) fc_update_kernel(
     pdl_trigger();
     // The first tile holds the next diagonal block: factored here, in the ring's space (every MMA
     // has read its stages: the epilogue waited for the last one), while the other CTAs go on.  As a
-    // kernel of its own between update and panel it left the other SMs idle (f64 n = 8192 15.0 ->
-    // 13.6 ms, n = 2048 2.24 -> 2.22; f32 n = 6001 4.26 -> 3.73 ms).
+    // kernel of its own between update and panel it leaves the other SMs idle (measured when it went
+    // in: f64 n = 8192 13.6 ms, 15.0 as a kernel; n = 2048 2.22, 2.24; f32 n = 6001 3.73, 4.26).
     if (blockIdx.x == 0 && tid < kFcDiagThreads)
         fc_diag_block(*reinterpret_cast<FcDiagSmem<T> *>(smem), W, ld, q, (int)min((int64_t)kFcNb, n - q), diag0, rinv,
                       info, min_ratio);

@@ -33,10 +33,13 @@ struct FactorVerdict {
 };
 constexpr double kPivotGuard = 1e-10;
 #ifdef __CUDACC__
-__device__ __forceinline__ bool factor_stands(const FactorVerdict *v) {
+// (plain loads: an SM's L1 serves all but its first; the words change in no kernel that reads them)
+__device__ __forceinline__ FactorVerdict factor_verdict(const FactorVerdict *v) {
+    return v != nullptr ? *v : FactorVerdict{-1, 1.0};
+}
+__device__ __forceinline__ bool factor_stands(const FactorVerdict &v) {
     // (the ratio is not negative, so its bits compare like it)
-    return *(volatile const int64_t *)&v->info < 0 &&
-           *(volatile const long long *)&v->min_ratio >= __double_as_longlong(kPivotGuard);
+    return v.info < 0 && __double_as_longlong(v.min_ratio) >= __double_as_longlong(kPivotGuard);
 }
 #endif
 

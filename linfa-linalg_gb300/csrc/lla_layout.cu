@@ -49,8 +49,10 @@ template <typename T>
 __global__ void export_kernel(const T *__restrict__ W, int64_t ld, T *__restrict__ R, int64_t rs,
                               int64_t cs, int64_t rows, int64_t cols, int mode, int64_t f,
                               const FactorVerdict *behind) {
-    if (behind != nullptr && !factor_stands(behind)) return;
     __shared__ T tile[32][33];
+    // (the verdict's loads are in flight with the tile's: tested first, they cost an n = 1100
+    // export 5 us)
+    const FactorVerdict verdict = factor_verdict(behind);
     const int64_t i0 = (int64_t)blockIdx.x * 32, j0 = (int64_t)blockIdx.y * 32;
     const bool row_major = (cs == 1);
     for (int k = threadIdx.y; k < 32; k += blockDim.y) {
@@ -58,6 +60,7 @@ __global__ void export_kernel(const T *__restrict__ W, int64_t ld, T *__restrict
         if (i < rows && j < cols) tile[threadIdx.x][k] = W[i + j * ld];
     }
     __syncthreads();
+    if (!factor_stands(verdict)) return;
     for (int k = threadIdx.y; k < 32; k += blockDim.y) {
         const int64_t i = row_major ? i0 + k : i0 + threadIdx.x;
         const int64_t j = row_major ? j0 + threadIdx.x : j0 + k;

@@ -7,7 +7,7 @@
 //      defines.)
 //   2. Factor A^ ~= L L^T in low precision: FP32 diagonal blocks and panels,
 //      trailing updates on the tensor cores (BF16 or FP16 operand terms with
-//      FP32 accumulation, lla_tc_update.cu) or in FP32 SIMT.
+//      FP32 accumulation, lla_tc_update.cu), or the FAST FP32 factorisation.
 //   3. Refine in FP64: r = b - A x (FP64 tensor pipe), d = S L^-T L^-1 S r in
 //      FP32, x += d (FP64), until the normwise backward error
 //      max_j ||r_j||_inf / (||A||_inf ||x_j||_inf + ||b_j||_inf) <= tol.

@@ -25,9 +25,9 @@ namespace lla {
 // so: roots and quotients run in integer arithmetic (lla_int_math.h,
 // bit-identical to IEEE), the accumulators stay in registers as patches of 16
 // rows x 2 columns, and tiles are small, so that every SM's pipe has a share.
-// Per panel of a 512 x 512 factorisation, before -> now: diagonal block 53 ->
-// 18 us, panel 66 -> 15 us, update 82 -> 10 us (f64; the whole factor 3160 ->
-// 730 us).
+// Per panel of a 512 x 512 factorisation: diagonal block 18 us, panel 15, update 10
+// (f64; the whole factor 730 us).  With the library's roots and divisions, sums in
+// shared memory and 64 x 64 tiles: 53, 66, 82 (3160 us).
 constexpr int kNbExact = 32;
 
 // Asynchronous copy to shared memory: all of a thread's copies are in flight at once.
@@ -198,9 +198,9 @@ __global__ void __launch_bounds__(kExDiagThreads) potrf_exact_diag(T *W, const T
 // stay in registers as patches of 8 rows x 4 columns, two per warp (warp w: rows
 // 8 (w % 2) .., column quads w / 2 and w / 2 + 4); quads are finished in turn by
 // their two owners, one barrier each, the next owners bringing their own quad up to
-// date first.  The chain of divisions and sums bounds it; by pairs of columns, with
-// twice the barriers, a panel took 17 us (one copy of the division in a rolled loop:
-// 16, and the diagonal block so 20 instead of 18).  Warp 8 adds the rows' squares to D as their columns appear.
+// date first.  The chain of divisions and sums bounds it: 15 us a panel; 17 by pairs of
+// columns, with twice the barriers (one copy of the division in a rolled loop: 16, and
+// the diagonal block so 20 instead of 18).  Warp 8 adds the rows' squares to D as their columns appear.
 constexpr int kExRows = 16;
 constexpr int kExPanelThreads = 288;
 

@@ -29,11 +29,12 @@
 // first wait.  An FP64 instruction takes 64 cycles of its sub-partition, so the
 // solve of a block keeps few of them in its chain: in EXACT mode the division by
 // the diagonal is done in integers, for FP32 by FMAs (lla_int_math.h); in FAST mode
-// the rows are divided by their diagonal beforehand and a step is one FMA.  Four right-hand sides a CTA: one warp per sub-partition.
-// Per row block, before -> now: EXACT f64 25 -> 9.9 us (n = 512), EXACT f32 7.1 ->
-// 2.9 us (n = 1000, 8 right-hand sides), FAST f64 30 -> 7.3 us (n = 8192, 16
-// right-hand sides; 1.03 ms of the 1.9 ms solve is the FP64 pipe's share), FAST
-// f32 9.4 -> 2.0 us (n = 6001, 3 right-hand sides).
+// the rows are divided by their diagonal beforehand and a step is one FMA.  Four
+// right-hand sides a CTA: one warp per sub-partition.
+// Per row block: EXACT f64 9.9 us (n = 512; 25 with the library's division and the
+// hand-over by the whole CTA), EXACT f32 2.9 (n = 1000, 8 right-hand sides; 7.1), FAST
+// f64 7.3 (n = 8192, 16 right-hand sides; 30; 1.03 ms of the 1.9 ms solve is the FP64
+// pipe's share), FAST f32 2.0 (n = 6001, 3 right-hand sides; 9.4).
 //
 // T[r, c] (logical) = trans ? M[c, r] : M[r, c]; `diag` (optional) overrides
 // the diagonal as the reference's diag_fn does (src/triangular.rs:133-144).
@@ -74,8 +75,8 @@ static int trsm_warps(int mc) { return std::max(mc, kTrsmMc); }
 // without a test on its chain; ok says afterwards whether x is IEEE division's
 // num / d, and the solve repeats a block with IEEE division if one was not (so does
 // the FAST solve whose rows were divided beforehand, if a result is not finite).
-// (Tested in every step: EXACT f64 n = 512 190 us a solve, now 165; EXACT f32
-// n = 1000, with the general division 123 us, with the test 137, now 99.)
+// (EXACT f64 n = 512 165 us a solve, tested in every step 190; EXACT f32 n = 1000 99,
+// tested in every step 137, with the general division 123.)
 template <typename T>
 struct TrsmDivisor;
 template <>
@@ -104,13 +105,17 @@ __device__ __forceinline__ bool trsm_finite(double v) { return ((unsigned)__doub
 __device__ __forceinline__ bool trsm_finite(float v) { return (__float_as_uint(v) & 0x7f800000u) != 0x7f800000u; }
 
 // FAST, for a block that the products by reciprocals do not take: solved by division,
-// from M itself (mrow: this lane's row at the block's first term, mstep from one term
-// to the next).  Returns this lane's result.  Out of line, and apart from the other
-// form's repeat: sharing one repeat cost every block 2% (n = 2048, 16 right-hand sides).
+// from M itself.  Returns this lane's result.  Out of line with its addresses, and apart
+// from the other form's repeat: sharing one repeat cost every block 2% (n = 2048, 16
+// right-hand sides).
 template <typename T>
-__device__ __noinline__ T trsm_block_by_division(T bv, T dv, const T *mrow, int64_t mstep, int bs) {
+__device__ __noinline__ T trsm_block_by_division(T bv, T dv, const T *M, int64_t ld, int64_t n, int lower, int trans,
+                                                 int64_t t0, int bs) {
     using Ar = Arith<T>;
     const int tx = threadIdx.x;
+    const int64_t step = lower ? 1 : -1, c0 = lower ? t0 : n - 1 - t0, r = c0 + step * tx;  // (rows in processing order)
+    const T *const mrow = trans ? M + c0 + r * ld : M + r + c0 * ld;
+    const int64_t mstep = trans ? step : step * ld;
 #pragma unroll 1
     for (int y = 0; y < bs; ++y) {
         const T t = tx > y && tx < bs ? mrow[y * mstep] : T(0);
@@ -137,7 +142,7 @@ __global__ void __launch_bounds__(kTrsmNb *kTrsmMaxMc) trsm_lookback(const T *__
     const int tid = ty * kTrsmNb + tx, nthr = kTrsmNb * blockDim.y;
     int *counter = ws, *flags = ws + 1;
     // no ticket: the factorisation does not stand (the same for every CTA)
-    if (tid == 0) s_ticket = behind != nullptr && !factor_stands(behind) ? -1 : atomicAdd(counter, 1);
+    if (tid == 0) s_ticket = behind != nullptr && !factor_stands(factor_verdict(behind)) ? -1 : atomicAdd(counter, 1);
     __syncthreads();
     if (s_ticket < 0) return;
     // failure injection (tests only): the first item is lost -- never solved,
@@ -221,7 +226,7 @@ __global__ void __launch_bounds__(kTrsmNb *kTrsmMaxMc) trsm_lookback(const T *__
                 }
                 // only the block right before this one is worth polling without a pause: thousands of
                 // warps wait further back, on the same few lines (n = 8192, 16 right-hand sides:
-                // 1.98 -> 1.86 ms a solve)
+                // 1.98 ms a solve without the pause, 1.86 with it)
                 if (q + 1 < rb) {
                     if (spins > 2) __nanosleep(256);
                 } else if (spins > 64) {
@@ -264,9 +269,7 @@ __global__ void __launch_bounds__(kTrsmNb *kTrsmMaxMc) trsm_lookback(const T *__
             // infinities and overflow on the way: products by a reciprocal are no longer what the
             // division gives (inf * 0, inf - inf)
             if (!__all_sync(0xffffffffu, tx >= bs || trsm_finite(bv))) {
-                const int64_t c0 = row_of(t0);
-                bv = trsm_block_by_division<T>(b0, dv, trans ? M + c0 + r_own * ld : M + r_own + c0 * ld,
-                                               (lower ? 1 : -1) * (trans ? 1 : ld), bs);
+                bv = trsm_block_by_division<T>(b0, dv, M, ld, n, lower, trans, t0, bs);
             }
         } else {
             const T b0 = bv;
